@@ -238,3 +238,33 @@ def test_gated_activation(dtype, kind):
         x = torch.randn(rows, K, generator=g).to(dtype).cuda()
         w = (torch.randn(2 * F, K, generator=g) * K ** -0.5).to(dtype).cuda()
         assert torch.allclose(o.linear_glu(x, w, F, kind).float(), ref_ops.linear_glu(x, w, F, kind).float(), **tol(dtype)), (rows, K, F)
+
+
+@pytest.mark.parametrize("H,D,V", [(2, 64, 128), (3, 10, 14), (1, 128, 128), (2, 33, 31), (2, 16, 65), (5, 48, 64), (1, 1, 1)])
+def test_mlstm_in_chunks(H, D, V):
+    """The kernels that run a span in chunks of 64 rows, at every remainder that matters, behind a state of their own and
+    beside spans that are walked; gates that jump, close and stay open."""
+    o = ops()
+    g = torch.Generator().manual_seed(18)
+    at, cols = mlstm_columns(H, D, V)
+    bias_i, bias_f = (torch.randn(H, generator=g) - 1.0).cuda(), (torch.randn(H, generator=g) + 3.0).cuda()
+    norm_w = (1 + 0.1 * torch.randn(H * V, generator=g)).cuda()
+    state_a = torch.zeros(22, H, D + 1, V + 1).cuda()
+    state_b = state_a.clone()
+    for q_lens, impl in (([64, 1, 63, 65], "chunks"), ([129, 300, 2, 128], "chunks"), ([1, 64, 1, 200], None), ([63, 65, 5, 0], None), ([700], None)):
+        step = make_step(o, torch.bfloat16, [3] * len(q_lens), q_lens, 8, 256, 5)
+        N = sum(q_lens)
+        y = torch.randn(N, cols, generator=g)
+        y[:, at[4]:at[4] + H] *= 4.0                                   # input gates that jump by several units
+        y[N // 2:, at[5]:at[5] + H] -= 9.0                             # forget gates that close
+        y[N // 3:N // 3 + 70, at[4]:at[4] + H] -= 20.0                 # rows that hardly enter
+        y = y.to(torch.bfloat16).cuda()
+        ya = o.mlstm(y, at, bias_i, bias_f, 11.0, norm_w, 1e-5, state_a, step, H, D, V, True, impl=impl)
+        yb = ref_ops.mlstm(y, at, bias_i, bias_f, 11.0, norm_w, 1e-5, state_b, step, H, D, V, True, precision=torch.float64)
+        # the limits of test_mlstm: a bfloat16 result of a norm, and a state summed in 32-bit
+        assert torch.allclose(ya.float(), yb.float(), **tol(torch.bfloat16)), (q_lens, float((ya.float() - yb.float()).abs().max()))
+        assert torch.allclose(state_a, state_b, atol=1e-4, rtol=1e-4), q_lens
+    keep = state_a.clone()
+    o.mlstm(y, at, bias_i, bias_f, 11.0, norm_w, 1e-5, state_a, step, H, D, V, False, impl="chunks")
+    assert torch.equal(state_a, keep)
+    assert o.read_status() == 0

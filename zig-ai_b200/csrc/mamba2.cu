@@ -190,23 +190,6 @@ __device__ __forceinline__ void m2_load_rows(bf16* dst, int ld, const Mamba2Args
     }
 }
 
-// v as a sum of three bfloat16 numbers
-__device__ __forceinline__ void m2_split(float v, float& hi, float& mid, float& lo) {
-    hi = __bfloat162float(__float2bfloat16_rn(v));
-    const float r = v - hi;
-    mid = __bfloat162float(__float2bfloat16_rn(r));
-    lo = r - mid;
-}
-// two neighbouring values, each split: p[k] holds the k-th parts
-__device__ __forceinline__ void m2_split2(float v0, float v1, uint32_t (&p)[3]) {
-    float a0, a1, a2, b0, b1, b2;
-    m2_split(v0, a0, a1, a2);
-    m2_split(v1, b0, b1, b2);
-    p[0] = pack_bf16(a0, b0);
-    p[1] = pack_bf16(a1, b1);
-    p[2] = pack_bf16(a2, b2);
-}
-
 // pass 1: ends [chunk, H, N, V] and last [chunk, H] (the chunk's L_last).  VT columns of V a block; eight warps, each in turn
 // 16 states x 32 columns.
 template <int VT>
@@ -240,7 +223,7 @@ __global__ void __launch_bounds__(256) mamba2_chunk_state_kernel(const Mamba2Arg
         const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
         const float w = s_w[j];
         uint32_t q[3];
-        m2_split2(x.x * w, x.y * w, q);
+        split3_pair(x.x * w, x.y * w, q);
         p[0] = q[0];
         p[M2_Q * LDX / 2] = q[1];
         p[M2_Q * LDX] = q[2];
@@ -376,8 +359,8 @@ __global__ void __launch_bounds__(256) mamba2_chunk_out_kernel(const Mamba2Args 
                 const int i = i0 + 256 * k, n = i / PER, c = (i % PER) * 4;
                 if (n >= np) continue;
                 uint32_t p[3], q[3];
-                m2_split2(v[k].x, v[k].y, p);
-                m2_split2(v[k].z, v[k].w, q);
+                split3_pair(v[k].x, v[k].y, p);
+                split3_pair(v[k].z, v[k].w, q);
 #pragma unroll
                 for (int m = 0; m < 3; ++m) *reinterpret_cast<uint2*>(ss + (m * np + n) * LDX + c) = make_uint2(p[m], q[m]);
             }
@@ -386,7 +369,7 @@ __global__ void __launch_bounds__(256) mamba2_chunk_out_kernel(const Mamba2Args 
         for (int i = threadIdx.x; i < np * VT; i += 256) {
             const int n = i / VT, c = i % VT;
             float hi, mid, lo;
-            m2_split((n < a.N && c < nv) ? S[(size_t)n * a.V + c] : 0.f, hi, mid, lo);
+            split3((n < a.N && c < nv) ? S[(size_t)n * a.V + c] : 0.f, hi, mid, lo);
             ss[n * LDX + c] = __float2bfloat16_rn(hi);
             ss[(np + n) * LDX + c] = __float2bfloat16_rn(mid);
             ss[(2 * np + n) * LDX + c] = __float2bfloat16_rn(lo);
@@ -446,8 +429,8 @@ __global__ void __launch_bounds__(256) mamba2_chunk_out_kernel(const Mamba2Args 
             const float2 l0 = s_l[j], l1 = s_l[j + 1];
             const float* g4 = sco[2 * ks + half];
             uint32_t p[3], q[3];
-            m2_split2(j <= ra ? g4[0] * (fast_exp2(m2_between(la, l0)) * d0) : 0.f, j + 1 <= ra ? g4[1] * (fast_exp2(m2_between(la, l1)) * d1) : 0.f, p);
-            m2_split2(j <= rb ? g4[2] * (fast_exp2(m2_between(lb, l0)) * d0) : 0.f, j + 1 <= rb ? g4[3] * (fast_exp2(m2_between(lb, l1)) * d1) : 0.f, q);
+            split3_pair(j <= ra ? g4[0] * (fast_exp2(m2_between(la, l0)) * d0) : 0.f, j + 1 <= ra ? g4[1] * (fast_exp2(m2_between(la, l1)) * d1) : 0.f, p);
+            split3_pair(j <= rb ? g4[2] * (fast_exp2(m2_between(lb, l0)) * d0) : 0.f, j + 1 <= rb ? g4[3] * (fast_exp2(m2_between(lb, l1)) * d1) : 0.f, q);
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 f[k][2 * half] = p[k];

@@ -32,6 +32,22 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// v as a sum of three bfloat16 numbers, which hold its 24 bits: what is 32-bit goes into bfloat16 products as its three parts
+__device__ __forceinline__ void split3(float v, float& hi, float& mid, float& lo) {
+    hi = __bfloat162float(__float2bfloat16_rn(v));
+    const float r = v - hi;
+    mid = __bfloat162float(__float2bfloat16_rn(r));
+    lo = r - mid;
+}
+// two neighbouring values, each split: p[k] holds the k-th parts
+__device__ __forceinline__ void split3_pair(float v0, float v1, uint32_t (&p)[3]) {
+    float a0, a1, a2, b0, b1, b2;
+    split3(v0, a0, a1, a2);
+    split3(v1, b0, b1, b2);
+    p[0] = pack_bf16(a0, b0);
+    p[1] = pack_bf16(a1, b1);
+    p[2] = pack_bf16(a2, b2);
+}
 
 // 2^x by the special-function unit (2 ulp; x = -inf gives 0, which the masked scores rely on).  The
 // library's exp2f costs tens of cycles more per value, which showed as the largest part of a key

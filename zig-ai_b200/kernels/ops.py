@@ -96,7 +96,11 @@ _SIGNATURES = {
         "zai_paged_attention_scored": [_P, _P, _P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _P, _F, _P, _I, _P, _I, _P],
     },
     "mlstm": {"zai_mlstm": [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P, _F, _P, _F, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I,
-                            _P]},
+                            _P, _I, _P],
+              "zai_mlstm_chunk_rows": [],
+              "zai_mlstm_chunked_supports": [_I, _I],
+              "zai_mlstm_chunked": [_P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P, _F, _P, _F, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I,
+                                    _P, _P, _P, _I, _P]},
     "attention_mma": {
         "zai_attention_mma_supports": [_I, _I, _I],
         "zai_prefill_attention_mma": [_P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _P, _P],
@@ -1835,12 +1839,27 @@ def mamba2(y, at, conv_w, conv_b, dt_bias, a_log, d_skip, norm_w, eps, norm_part
     return out
 
 
+# Spans of this many rows or more run the matrix memory in chunks on the tensor cores (bfloat16): the walk takes about 12 us and
+# 0.25 us a row, the three kernels over chunks 25 to 30 us up to a thousand rows.  One request alone, heads of 64 x 128: 48 rows
+# 26 (walk) and 34 us (chunks), 64 rows 30 and 32, 128 rows 46 and 32; 16 requests of 32 rows 33 and 45, of 64 rows 50 and 43.
+MLSTM_CHUNKED_MIN = 64
+
+
+def _span_kinds(step, cut):
+    """Whether a step has spans of `cut` rows or more, and whether it has shorter ones.  A captured step shape is replayed with
+    other spans than it was captured with (it launches a bound of its attention tiles, `attn_tiles`): it may have both."""
+    if getattr(step, "attn_tiles", None) or not step.q_lens:
+        return step.n_tokens >= cut, True
+    return max(step.q_lens) >= cut, any(0 < n < cut for n in step.q_lens)
+
+
 @_timed("recurrence")
-def mlstm(y, at, bias_i, bias_f, cap, norm_w, eps, state, step, heads, dim, vdim, write_state=True):
+def mlstm(y, at, bias_i, bias_f, cap, norm_w, eps, state, step, heads, dim, vdim, write_state=True, impl=None):
     """The matrix memory with log gates.  y [N, cols]: the stacked projections, `at` the first columns of q (H D), k (H D), v (H
     Dv), the output gate (H Dv) and the inputs of the log input and forget gates (H each); bias_i, bias_f [H], norm_w [H Dv]
     32-bit; state [slots, H, D + 1, Dv + 1] 32-bit (the normaliser as the last column, every column's running maximum as
-    the last row).  Returns rms_per_head(o) * norm_w * sigmoid(gate), [N, H Dv]."""
+    the last row).  Returns rms_per_head(o) * norm_w * sigmoid(gate), [N, H Dv].  `impl` "walk" or "chunks" picks the kernels
+    whatever the spans' lengths."""
     _cuda(bias_i, bias_f, norm_w, state)
     yp, ys = _rows_view(y)
     N, H, D, Dv = y.shape[0], int(heads), int(dim), int(vdim)
@@ -1848,10 +1867,27 @@ def mlstm(y, at, bias_i, bias_f, cap, norm_w, eps, state, step, heads, dim, vdim
             or bias_f.dtype != torch.float32 or norm_w.dtype != torch.float32 or norm_w.numel() != H * Dv or N != step.n_tokens):
         raise KernelError("mlstm: operands do not fit together")
     out = torch.empty((N, H * Dv), dtype=y.dtype, device=y.device)
-    part = torch.empty((N, H, Dv + 2), dtype=torch.float32, device=y.device)
     q_at, k_at, v_at, g_at, i_at, f_at = (int(a) for a in at)
-    _check(_fn("mlstm", "zai_mlstm")(_ptr(out), _ptr(part), yp, ys, _dt(y), q_at, k_at, v_at, g_at, i_at, f_at, _ptr(bias_i),
-                                     _ptr(bias_f), float(cap), _ptr(norm_w), float(eps), _ptr(state), _ptr(step.cu_q),
-                                     _ptr(step.slot_ids), state.shape[0], _status_ptr(y.device), N, step.n_seqs, H, D, Dv,
-                                     int(bool(write_state)), _stream()), "mlstm", 2)
+    lib, status, wr = "mlstm", _status_ptr(y.device), int(bool(write_state))
+    # which kernels a span takes depends on its own length alone (a step may hold both kinds)
+    cut = 1 << 30
+    if impl != "walk" and not step.decode_only and y.dtype == torch.bfloat16 and _fn(lib, "zai_mlstm_chunked_supports")(D, Dv):
+        cut = 1 if impl == "chunks" else MLSTM_CHUNKED_MIN
+    long, short = _span_kinds(step, cut)
+    if long:
+        max_chunks = N // _fn(lib, "zai_mlstm_chunk_rows")() + step.n_seqs
+        ends = torch.empty((max_chunks, H, D, (Dv + 4) // 4 * 4), dtype=torch.float32, device=y.device)
+        gates = torch.empty((max_chunks, H, 2), dtype=torch.float64, device=y.device)
+        m_in = torch.empty((max_chunks, H), dtype=torch.float32, device=y.device)
+        _check(_fn(lib, "zai_mlstm_chunked")(_ptr(out), yp, ys, q_at, k_at, v_at, g_at, i_at, f_at, _ptr(bias_i), _ptr(bias_f), float(cap),
+                                             _ptr(norm_w), float(eps), _ptr(state), _ptr(step.cu_q), _ptr(step.slot_ids), state.shape[0],
+                                             status, step.n_seqs, H, D, Dv, wr, cut, _ptr(ends), _ptr(gates), _ptr(m_in), max_chunks,
+                                             _stream()), "mlstm_chunked", 3)
+        if not short or cut == 1:
+            return out
+    part = torch.empty((N, H, Dv + 2), dtype=torch.float32, device=y.device)
+    _check(_fn(lib, "zai_mlstm")(_ptr(out), _ptr(part), yp, ys, _dt(y), q_at, k_at, v_at, g_at, i_at, f_at, _ptr(bias_i),
+                                 _ptr(bias_f), float(cap), _ptr(norm_w), float(eps), _ptr(state), _ptr(step.cu_q),
+                                 _ptr(step.slot_ids), state.shape[0], status, N, step.n_seqs, H, D, Dv,
+                                 wr, _ptr(step.seq_idx) if long else None, cut - 1, _stream()), "mlstm", 2)
     return out
