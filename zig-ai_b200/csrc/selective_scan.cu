@@ -7,46 +7,23 @@
 //
 // Everything but the stored activations (x, p, z, y in the model's dtype) is 32-bit: the step size, the
 // decay, the state and the sums.  The products dt_in . Wdt^T of all rows are one matrix product made beforehand
-// (on the tensor cores where the model is bfloat16).  A lane holds K consecutive states of a channel in registers:
-// a whole channel where S <= 16, else G lanes of a warp share it.  Rows are taken two or four at a time: the loads,
-// step sizes and decays of the group do not depend on the state and are in flight together, only the state's own
-// multiply-adds wait for one another.
-//
-// Two ways through a step:
-//   * one pass (steps of single tokens and short portions): a block walks one request's rows in order;
-//   * three passes (long portions): the rows of every request are cut into chunks of `chunk` tokens.
-//     Pass 1 walks every chunk from a zero state and keeps its end state E and its summed step sizes
-//     (the chunk's decay is exp(A * sum dt)); pass 2 carries the state across the chunks of a request,
-//     h_in(j+1) = exp(A sum_j) h_in(j) + E_j, starting from the stored state, and stores the request's new
-//     state; pass 3 walks every chunk again from its h_in and writes y.  The recurrence is linear in h, so
-//     this is the same sum in another order (a difference of rounding only), and all chunks run at once.
-#include "common.cuh"
+// (on the tensor cores where the model is bfloat16).  Two kernels:
+//   * steps of single tokens: a lane holds K consecutive states of a channel (a whole channel where S <= 16, else G lanes
+//     of a warp share it), loads its row's values and sums its step size itself;
+//   * steps with portions: a block walks one request's rows in order, two states a lane, fed by warps of its own.
+#include "mma_helpers.cuh"
 
 // Exponentials and the softplus: exact library functions where the model is 32-bit; where activations are
 // bfloat16 the hardware approximations (relative error about 2^-21, far below the 2^-9 of a stored activation).
 template <typename T> __device__ __forceinline__ float exp_for(float v) { return expf(v); }
 template <> __device__ __forceinline__ float exp_for<bf16>(float v) { return __expf(v); }
 template <typename T> __device__ __forceinline__ float softplus_for(float v) { return v > 20.f ? v : log1pf(expf(v)); }
-template <> __device__ __forceinline__ float softplus_for<bf16>(float v) { return v > 20.f ? v : __logf(1.f + __expf(v)); }
+template <> __device__ __forceinline__ float softplus_for<bf16>(float v) {
+    const float s = __logf(1.f + __expf(v));           // (made for every value: a choice, not a branch)
+    return v > 20.f ? v : s;
+}
 template <typename T> __device__ __forceinline__ float silu_for(float v) { return v / (1.f + expf(-v)); }
 template <> __device__ __forceinline__ float silu_for<bf16>(float v) { return __fdividef(v, 1.f + __expf(-v)); }
-
-// The chunk with index b among all chunks of the step (requests in order, each cut into chunks of Lc rows).
-__device__ __forceinline__ bool zai_find_chunk(const int* __restrict__ cu_q, int n_seqs, int Lc, int b, int& seq, int& t0,
-                                               int& t1) {
-    for (int s = 0; s < n_seqs; ++s) {
-        const int a = cu_q[s], e = cu_q[s + 1];
-        const int nc = (e - a + Lc - 1) / Lc;
-        if (b < nc) {
-            seq = s;
-            t0 = a + b * Lc;
-            t1 = min(t0 + Lc, e);
-            return true;
-        }
-        b -= nc;
-    }
-    return false;
-}
 
 // K consecutive values as 32-bit; `vec`: the address is a multiple of 8 bytes and K of four (16-bit values, 8 bytes a load)
 template <int K>
@@ -70,13 +47,6 @@ __device__ __forceinline__ void load_run(const bf16* p, float (&d)[K], int n_val
     }
 }
 
-__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
-
-// Walks rows [t0, t1) of one request for channel c; this lane holds the states g*K .. g*K + K - 1 (with 16 states
-// or fewer one lane holds a channel's whole state: nothing is exchanged between lanes, and the rows' B and C are
-// the same addresses for every lane of a warp).  `dt_raw` [N, I] holds the step sizes' products dt_in . Wdt^T in
-// 32-bit (a matrix product made beforehand).  EMIT: writes y.  U rows are in flight together.  PREFETCH: the rows
-// are first asked into L1 (one trip to memory for a chunk, not one per group of rows).
 // dt_in . wrow over R terms, split over the G lanes of the channel (16 bytes a load where rows are aligned)
 template <typename T, int G>
 __device__ __forceinline__ float step_size_product(const T* __restrict__ wrow, const T* __restrict__ prow, int R, int g, bool vec) {
@@ -100,75 +70,6 @@ __device__ __forceinline__ float step_size_product(const T* __restrict__ wrow, c
     return s;
 }
 
-template <typename T, int K, int G, bool EMIT, int U, bool PREFETCH>
-__device__ __forceinline__ void scan_walk(float (&h)[K], const float (&a)[K], int t0, int t1, int c, int g, bool live,
-                                          T* __restrict__ y, const T* __restrict__ x, const T* __restrict__ proj, int proj_stride,
-                                          const T* __restrict__ z, int z_stride, const float* __restrict__ dt_raw,
-                                          const T* __restrict__ wrow, float bias, float dsk, int I, int S, int R, float* sum_dt) {
-    if (PREFETCH) {
-        const int c0 = blockIdx.y * (128 / G);
-        for (int tt = t0 + threadIdx.x; tt < t1; tt += 128) {
-            const T* p = proj + (size_t)tt * proj_stride + R;
-            for (int o = 0; o < (int)(2 * S * sizeof(T)); o += 128) prefetch_l1(reinterpret_cast<const char*>(p) + o);
-            for (int o = 0; o < 128 / G; o += 32) {
-                prefetch_l1(dt_raw + (size_t)tt * I + c0 + o);
-                if (o % 64 == 0) {
-                    prefetch_l1(x + (size_t)tt * I + c0 + o);
-                    if (EMIT) prefetch_l1(z + (size_t)tt * z_stride + c0 + o);
-                }
-            }
-        }
-    }
-    const int n_mine = max(min(S - g * K, K), 0);
-    const bool vec = sizeof(T) == 2 && ((proj_stride | R | S) & 3) == 0 && (reinterpret_cast<uintptr_t>(proj) & 7) == 0;
-    float total = 0.f;
-    for (int t = t0; t < t1; t += U) {
-        float dt[U], xv[U], zv[U], bv[U][K], cv[U][K];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const bool on = t + u < t1;
-            const int tt = on ? t + u : t;
-            const T* p = proj + (size_t)tt * proj_stride + R + g * K;
-            if (dt_raw) {
-                dt[u] = on ? dt_raw[(size_t)tt * I + c] : 0.f;
-            } else {                                   // (single-token steps: the product is summed here, no launch for it)
-                const bool vec8 = ((proj_stride | R) & 7) == 0 && ((reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(wrow)) & 15) == 0;
-                dt[u] = step_size_product<T, G>(wrow, proj + (size_t)tt * proj_stride, R, g, vec8);
-            }
-            xv[u] = on ? to_float(x[(size_t)tt * I + c]) : 0.f;
-            zv[u] = (EMIT && on) ? to_float(z[(size_t)tt * z_stride + c]) : 0.f;
-            load_run<K>(p, bv[u], on ? n_mine : 0, vec);
-            if (EMIT) load_run<K>(p + S, cv[u], on ? n_mine : 0, vec);
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) dt[u] = softplus_for<T>(dt[u] + bias);
-        float out[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            out[u] = 0.f;
-            if (t + u < t1) {
-                const float dx = dt[u] * xv[u];
-                total += dt[u];
-#pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    h[k] = exp_for<T>(dt[u] * a[k]) * h[k] + dx * bv[u][k];
-                    if (EMIT) out[u] += h[k] * cv[u][k];
-                }
-            }
-        }
-        if (EMIT) {
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                float s = out[u];
-#pragma unroll
-                for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-                if (g == 0 && live && t + u < t1) y[(size_t)(t + u) * I + c] = from_float<T>((s + dsk * xv[u]) * silu_for<T>(zv[u]));
-            }
-        }
-    }
-    if (sum_dt) *sum_dt = total;
-}
-
 // a lane's K states from / to memory (16 bytes a time where the run is aligned)
 template <int K>
 __device__ __forceinline__ void state_io(float* st, float (&h)[K], int n_valid, bool store) {
@@ -188,149 +89,434 @@ __device__ __forceinline__ void state_io(float* st, float (&h)[K], int n_valid, 
     }
 }
 
-// ---- one pass: a block walks one request's rows (U = 1: every request brings one token)
-template <typename T, int K, int G, int U>
-__global__ void __launch_bounds__(128) selective_scan_kernel(
+// ---- one row of a request, by 128 threads of a block: the step's only row of that request
+template <typename T, int K, int G>
+__device__ __forceinline__ void scan_one_row(T* __restrict__ y, const T* __restrict__ x, const T* __restrict__ proj, int proj_stride,
+                                             const T* __restrict__ z, int z_stride, const float* __restrict__ dt_raw, const T* __restrict__ w_dt,
+                                             const float* __restrict__ b_dt, const float* __restrict__ a_log, const float* __restrict__ d_skip,
+                                             float* __restrict__ state, int t, int slot, int I, int S, int R, int write_state) {
+    const int g = threadIdx.x % G;
+    int c = blockIdx.y * (128 / G) + threadIdx.x / G;
+    const bool live = c < I;
+    if (!live) c = I - 1;                              // (keeps the lane in the shuffles; it stores nothing)
+    const int n_mine = max(min(S - g * K, K), 0);
+    float* st = state + ((size_t)slot * I + c) * S + g * K;
+    float h[K], a[K], bv[K], cv[K];
+    state_io<K>(st, h, n_mine, false);
+#pragma unroll
+    for (int k = 0; k < K; ++k) a[k] = k < n_mine ? -expf(a_log[(size_t)c * S + g * K + k]) : 0.f;
+    const T* prow = proj + (size_t)t * proj_stride;
+    const bool vec = sizeof(T) == 2 && ((proj_stride | R | S) & 3) == 0 && (reinterpret_cast<uintptr_t>(proj) & 7) == 0;
+    load_run<K>(prow + R + g * K, bv, n_mine, vec);
+    load_run<K>(prow + R + S + g * K, cv, n_mine, vec);
+    const float xv = to_float(x[(size_t)t * I + c]), zv = to_float(z[(size_t)t * z_stride + c]);
+    float dt;
+    if (dt_raw) {
+        dt = dt_raw[(size_t)t * I + c];
+    } else {                                           // (the product is summed here, no launch for it)
+        const T* wrow = w_dt + (size_t)c * R;
+        const bool vec8 = ((proj_stride | R) & 7) == 0 && ((reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(wrow)) & 15) == 0;
+        dt = step_size_product<T, G>(wrow, prow, R, g, vec8);
+    }
+    dt = softplus_for<T>(dt + b_dt[c]);
+    const float dx = dt * xv;
+    float out = 0.f;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        h[k] = exp_for<T>(dt * a[k]) * h[k] + dx * bv[k];
+        out += h[k] * cv[k];
+    }
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) out += __shfl_xor_sync(0xffffffffu, out, o);
+    if (g == 0 && live) y[(size_t)t * I + c] = from_float<T>((out + d_skip[c] * xv) * silu_for<T>(zv));
+    if (write_state && live) state_io<K>(st, h, n_mine, true);
+}
+
+// ---- a step of single tokens, row i of request i
+template <typename T, int K, int G>
+__global__ void __launch_bounds__(128) selective_scan_single_kernel(
     T* __restrict__ y, const T* __restrict__ x, const T* __restrict__ proj, int proj_stride, const T* __restrict__ z,
     int z_stride, const float* __restrict__ dt_raw, const T* __restrict__ w_dt, const float* __restrict__ b_dt,
     const float* __restrict__ a_log, const float* __restrict__ d_skip, float* __restrict__ state, const int* __restrict__ cu_q,
     const int* __restrict__ slot_ids, int I, int S, int R, int write_state, int num_slots, int* __restrict__ status) {
     pdl_trigger();
     pdl_wait();
-    const int seq = blockIdx.x;
-    const int g = threadIdx.x % G;
-    int c = blockIdx.y * (128 / G) + threadIdx.x / G;
-    const bool live = c < I;
-    if (!live) c = I - 1;                              // (keeps the lane in the shuffles; it stores nothing)
+    const int t = cu_q[blockIdx.x];
+    if (cu_q[blockIdx.x + 1] <= t) return;
+    scan_one_row<T, K, G>(y, x, proj, proj_stride, z, z_stride, dt_raw, w_dt, b_dt, a_log, d_skip, state, t,
+                          zai_checked_slot(slot_ids[blockIdx.x], num_slots, status), I, S, R, write_state);
+}
+
+// ---- steps with portions.  A block walks one request's rows for 128 / G channels, in tiles of 64 rows (32 with more than
+// 64 states).  Four warps walk: a
+// lane holds K states of a channel, and what a row gives it comes out of shared memory as 32-bit numbers, four rows ahead of
+// their use.  Four more warps put the next tile there meanwhile (step sizes, their products with x, the gates; a tile's loads
+// are issued while the tile before it is walked) and take the read-outs of the tile before to y.  One barrier a tile.
+//
+// What bounds it: S exponentials a row and channel, which the special-function units make at 16 a cycle and SM.  Cutting the
+// rows into chunks that run at once (three passes: the chunks' end states, the carry, the rows again) makes them twice and moves
+// a state per chunk through memory; one walk makes them once, and with two states a lane 2048 channels give every scheduler of
+// the chip a warp.  A portion of 2048 rows with 16 states (us, its step sizes' product included): 134 for 4096 channels (three
+// passes: 309), 92 for 2048 (172), 91 for 1024 (129); 512 rows of 4096 channels 40 (104).  A row costs about 45 ns however few
+// the channels are (dependent instructions, one warp a scheduler): below 1024 channels and beyond 2048 rows chunks would be
+// faster again (8192 rows of 512 channels 331, in chunks 220).
+template <typename T> __device__ __forceinline__ float decay_scale(float a) { return a; }
+template <> __device__ __forceinline__ float decay_scale<bf16>(float a) { return a * 1.4426950408889634f; }
+template <typename T> __device__ __forceinline__ float decay_of(float v) { return expf(v); }
+template <> __device__ __forceinline__ float decay_of<bf16>(float v) { return fast_exp2(v); }
+
+// two 32-bit numbers in one register pair: one instruction multiplies (and adds) both, each rounded as by itself
+__device__ __forceinline__ uint64_t mul_pair(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t make_pair(float x, float y) {
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
+    return d;
+}
+__device__ __forceinline__ float2 pair_of(uint64_t v) {
+    float2 d;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(v));
+    return d;
+}
+
+// four neighbouring values as they lie in memory
+template <typename T> struct Four;
+template <> struct Four<float> {
+    float4 v;
+    __device__ __forceinline__ void load(const float* p) { v = *reinterpret_cast<const float4*>(p); }
+    __device__ __forceinline__ void zero() { v = make_float4(0.f, 0.f, 0.f, 0.f); }
+    __device__ __forceinline__ void load_some(const float* p, int n) {
+        v = make_float4(n > 0 ? p[0] : 0.f, n > 1 ? p[1] : 0.f, n > 2 ? p[2] : 0.f, n > 3 ? p[3] : 0.f);
+    }
+    __device__ __forceinline__ float4 get() const { return v; }
+    static __device__ __forceinline__ void store(float* p, const float (&o)[4]) { *reinterpret_cast<float4*>(p) = make_float4(o[0], o[1], o[2], o[3]); }
+};
+template <> struct Four<bf16> {
+    uint2 v;
+    __device__ __forceinline__ void load(const bf16* p) { v = *reinterpret_cast<const uint2*>(p); }
+    __device__ __forceinline__ void zero() { v = make_uint2(0u, 0u); }
+    __device__ __forceinline__ void load_some(const bf16* p, int n) {
+        v.x = pack_bf16(n > 0 ? to_float(p[0]) : 0.f, n > 1 ? to_float(p[1]) : 0.f);
+        v.y = pack_bf16(n > 2 ? to_float(p[2]) : 0.f, n > 3 ? to_float(p[3]) : 0.f);
+    }
+    __device__ __forceinline__ float4 get() const {
+        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x));
+        const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
+        return make_float4(a.x, a.y, b.x, b.y);
+    }
+    static __device__ __forceinline__ void store(bf16* p, const float (&o)[4]) {
+        *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]));
+    }
+};
+
+template <int K, int G>
+struct ScanTile {                                            // a tile in shared memory
+    static constexpr int CB = 128 / G, SP = K * G;           // channels and states (with padding) of a block
+    static constexpr int TT = SP > 64 ? 32 : 64;             // rows
+    static constexpr int LDS = CB + 8;                       // read-outs: four rows of a warp's channels lie in different banks
+    float4 step[TT][CB + 1];                                 // step size twice, its product with x twice (rows a bank group apart)
+    float2 last[TT][CB + 2];                                 // D x, silu(z)
+    float bc[TT][2 * SP];                                    // B | C
+    float sum[TT][LDS];                                      // the walk's read-outs
+};
+
+// the rows' way in and out, by 128 threads.  VEC: channels, states and every row of x, z, proj, dt_raw and y lie in fours on
+// boundaries of four
+template <typename T, int K, int G, bool VEC>
+__device__ __forceinline__ void scan_feed(ScanTile<K, G>* tiles, int tid, int c0, int start, int end, T* __restrict__ y,
+                                          const T* __restrict__ x, const T* __restrict__ proj, int proj_stride, const T* __restrict__ z,
+                                          int z_stride, const float* __restrict__ dt_raw, const float* __restrict__ b_dt,
+                                          const float* __restrict__ d_skip, int I, int S, int R) {
+    using Tile = ScanTile<K, G>;
+    constexpr int CB = Tile::CB, SP = Tile::SP, TT = Tile::TT, QC = CB / 4, ROWS = 128 / QC, PER = TT > ROWS ? TT / ROWS : 1;
+    constexpr int FOURS = TT * 2 * SP / 4, BC = FOURS / 128;          // fours of B and C: of a tile, of a thread
+    static_assert(BC >= 1 && FOURS % 128 == 0, "a tile is shared evenly");
+    const int cq = (tid % QC) * 4, r0 = tid / QC;            // this thread's four channels, and its rows r0 + i ROWS
+    const int n_c = min(I - c0 - cq, 4), n_tiles = (end - start + TT - 1) / TT;
+    float bias[4], skip[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        bias[k] = k < n_c ? b_dt[c0 + cq + k] : 0.f;
+        skip[k] = k < n_c ? d_skip[c0 + cq + k] : 0.f;
+    }
+    struct Raw { Four<float> dt[PER]; Four<T> xv[PER], zv[PER], bc[BC]; };
+    auto fetch = [&](int n, Raw& in) {
+        const int t0 = start + n * TT;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const int t = t0 + r0 + i * ROWS;
+            const int nc = (t < end && r0 + i * ROWS < TT) ? n_c : 0;
+            if (VEC) {
+                if (nc > 0) {
+                    in.dt[i].load(dt_raw + (size_t)t * I + c0 + cq);
+                    in.xv[i].load(x + (size_t)t * I + c0 + cq);
+                    in.zv[i].load(z + (size_t)t * z_stride + c0 + cq);
+                } else {
+                    in.dt[i].zero(); in.xv[i].zero(); in.zv[i].zero();
+                }
+            } else {
+                in.dt[i].load_some(dt_raw + (size_t)t * I + c0 + cq, nc);
+                in.xv[i].load_some(x + (size_t)t * I + c0 + cq, nc);
+                in.zv[i].load_some(z + (size_t)t * z_stride + c0 + cq, nc);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < BC; ++i) {
+            const int e = tid + i * 128, r = e / (2 * SP / 4), q = e % (2 * SP / 4) * 4, which = q >= SP, s = q - which * SP;
+            const int ns = t0 + r < end ? S - s : 0;
+            const T* p = proj + (size_t)(t0 + r) * proj_stride + R + which * S + s;
+            if (VEC) { if (ns > 0) in.bc[i].load(p); else in.bc[i].zero(); }
+            else in.bc[i].load_some(p, ns);
+        }
+    };
+    auto leave = [&](int n) {                                // the read-outs of tile n go to y
+        const Tile& tile = tiles[n & 1];
+        const int t0 = start + n * TT;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const int r = r0 + i * ROWS;
+            if (r >= TT || t0 + r >= end) continue;
+            float v[4];
+            const float4 m = *reinterpret_cast<const float4*>(&tile.sum[r][cq]);
+            const float4 l = *reinterpret_cast<const float4*>(&tile.last[r][cq]), k = *reinterpret_cast<const float4*>(&tile.last[r][cq + 2]);
+            v[0] = (m.x + l.x) * l.y;
+            v[1] = (m.y + l.z) * l.w;
+            v[2] = (m.z + k.x) * k.y;
+            v[3] = (m.w + k.z) * k.w;
+            T* p = y + (size_t)(t0 + r) * I + c0 + cq;
+            if (VEC) { if (n_c > 0) Four<T>::store(p, v); }
+            else {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (k < n_c) p[k] = from_float<T>(v[k]);
+            }
+        }
+    };
+    Raw in;
+    fetch(0, in);
+    for (int n = 0; n <= n_tiles; ++n) {
+        const int t0 = start + n * TT;
+        if (n >= 2) leave(n - 2);                            // (its buffer is the one that tile n is put into)
+        if (n < n_tiles) {
+            Tile& tile = tiles[n & 1];
+#pragma unroll
+            for (int i = 0; i < PER; ++i) {
+                const int r = r0 + i * ROWS;
+                if (r >= TT || t0 + r >= end + 3) continue;  // (rows in fours)
+                const bool on = t0 + r < end;
+                const float4 df = in.dt[i].get(), xf = in.xv[i].get(), zf = in.zv[i].get();
+                const float d4[4] = {df.x, df.y, df.z, df.w}, x4[4] = {xf.x, xf.y, xf.z, xf.w}, z4[4] = {zf.x, zf.y, zf.z, zf.w};
+                float2 l[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float d = on ? softplus_for<T>(d4[k] + bias[k]) : 0.f;          // (a row beyond the span changes no state)
+                    const float dx = d * x4[k];
+                    tile.step[r][cq + k] = make_float4(d, d, dx, dx);
+                    l[k] = make_float2(skip[k] * x4[k], silu_for<T>(z4[k]));
+                }
+#pragma unroll
+                for (int k = 0; k < 4; k += 2) *reinterpret_cast<float4*>(&tile.last[r][cq + k]) = make_float4(l[k].x, l[k].y, l[k + 1].x, l[k + 1].y);
+            }
+#pragma unroll
+            for (int i = 0; i < BC; ++i) *reinterpret_cast<float4*>(&tile.bc[0][0] + (tid + i * 128) * 4) = in.bc[i].get();
+            if (n + 1 < n_tiles) fetch(n + 1, in);
+        }
+        __syncthreads();                                     // tile n is there, tile n - 1 has been walked
+    }
+    leave(n_tiles - 1);
+}
+
+template <typename T, int K, int G>
+__global__ void __launch_bounds__(256) selective_scan_kernel(
+    T* __restrict__ y, const T* __restrict__ x, const T* __restrict__ proj, int proj_stride, const T* __restrict__ z,
+    int z_stride, const float* __restrict__ dt_raw, const float* __restrict__ b_dt,
+    const float* __restrict__ a_log, const float* __restrict__ d_skip, float* __restrict__ state, const int* __restrict__ cu_q,
+    const int* __restrict__ slot_ids, int I, int S, int R, int write_state, int num_slots, int* __restrict__ status, int vec) {
+    using Tile = ScanTile<K, G>;
+    constexpr int CB = Tile::CB, SP = Tile::SP, TT = Tile::TT;
+    extern __shared__ __align__(16) unsigned char scan_raw[];
+    Tile* tiles = reinterpret_cast<Tile*>(scan_raw);         // [2]
+    pdl_trigger();
+    pdl_wait();
+    const int seq = blockIdx.x, c0 = blockIdx.y * CB;
     const int start = cu_q[seq], end = cu_q[seq + 1];
     if (end <= start) return;
+    if (end - start == 1) {                                  // (a decoding request beside the portions: no tile for one row)
+        if (threadIdx.x < 128)
+            scan_one_row<T, K, G>(y, x, proj, proj_stride, z, z_stride, dt_raw, nullptr, b_dt, a_log, d_skip, state, start,
+                                  zai_checked_slot(slot_ids[seq], num_slots, status), I, S, R, write_state);
+        return;
+    }
+    const int n_tiles = (end - start + TT - 1) / TT;
+    if (threadIdx.x >= 128) {
+        if (vec) scan_feed<T, K, G, true>(tiles, threadIdx.x - 128, c0, start, end, y, x, proj, proj_stride, z, z_stride, dt_raw, b_dt, d_skip, I, S, R);
+        else scan_feed<T, K, G, false>(tiles, threadIdx.x - 128, c0, start, end, y, x, proj, proj_stride, z, z_stride, dt_raw, b_dt, d_skip, I, S, R);
+        return;
+    }
+
+    // ---- the walk
+    const int lane = threadIdx.x & 31, g = threadIdx.x % G, cl = threadIdx.x / G;
+    int c = c0 + cl;
+    const bool live = c < I;
+    if (!live) c = I - 1;
     const int slot = zai_checked_slot(slot_ids[seq], num_slots, status);
     const int n_mine = max(min(S - g * K, K), 0);
     float* st = state + ((size_t)slot * I + c) * S + g * K;
-    float h[K], a[K];
-    state_io<K>(st, h, n_mine, false);
+    float h1[K];
+    uint64_t h[K / 2], a[K / 2];                             // states in pairs
+    state_io<K>(st, h1, n_mine, false);
 #pragma unroll
-    for (int k = 0; k < K; ++k) a[k] = k < n_mine ? -expf(a_log[(size_t)c * S + g * K + k]) : 0.f;
-    scan_walk<T, K, G, true, U, false>(h, a, start, end, c, g, live, y, x, proj, proj_stride, z, z_stride, dt_raw,
-                                       w_dt + (size_t)c * R, b_dt[c], d_skip[c], I, S, R, nullptr);
-    if (write_state && live) state_io<K>(st, h, n_mine, true);
-}
-
-// ---- three passes.  ends [chunks, I, S]: a chunk's end state from zero, then (after pass 2) its start state;
-// sums [chunks, I]: its summed step sizes.
-template <typename T, int K, int G, bool EMIT>
-__global__ void __launch_bounds__(128) selective_scan_chunk_kernel(
-    T* __restrict__ y, const T* __restrict__ x, const T* __restrict__ proj, int proj_stride, const T* __restrict__ z,
-    int z_stride, const float* __restrict__ dt_raw, const float* __restrict__ b_dt, const float* __restrict__ a_log,
-    const float* __restrict__ d_skip, float* __restrict__ ends, float* __restrict__ sums, const int* __restrict__ cu_q,
-    int n_seqs, int Lc, int I, int S, int R) {
-    pdl_trigger();
-    pdl_wait();
-    int seq, t0, t1;
-    if (!zai_find_chunk(cu_q, n_seqs, Lc, blockIdx.x, seq, t0, t1)) return;
-    const int g = threadIdx.x % G;
-    int c = blockIdx.y * (128 / G) + threadIdx.x / G;
-    const bool live = c < I;
-    if (!live) c = I - 1;
-    const int n_mine = max(min(S - g * K, K), 0);
-    float* e = ends + ((size_t)blockIdx.x * I + c) * S + g * K;
-    float h[K], a[K];
-    if (EMIT) state_io<K>(e, h, n_mine, false);
+    for (int k = 0; k < K; k += 2) {
+        const float* al = a_log + (size_t)c * S + g * K + k;
+        h[k / 2] = make_pair(h1[k], h1[k + 1]);
+        a[k / 2] = make_pair(k < n_mine ? decay_scale<T>(-expf(al[0])) : 0.f, k + 1 < n_mine ? decay_scale<T>(-expf(al[1])) : 0.f);
+    }
+    struct Rows { ulonglong2 d[4]; uint64_t b[4][K / 2], c[4][K / 2]; };    // four rows' operands
+    auto take = [&](const Tile& tile, int r, Rows& o) {
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-        if (!EMIT) h[k] = 0.f;
-        a[k] = k < n_mine ? -expf(a_log[(size_t)c * S + g * K + k]) : 0.f;
-    }
-    float total = 0.f;
-    scan_walk<T, K, G, EMIT, (K > 8 ? 2 : 4), true>(h, a, t0, t1, c, g, live, y, x, proj, proj_stride, z, z_stride, dt_raw,
-                                                    (const T*)nullptr, b_dt[c], d_skip[c], I, S, R, &total);
-    if (!EMIT && live) {
-        state_io<K>(e, h, n_mine, true);
-        if (g == 0) sums[(size_t)blockIdx.x * I + c] = total;
-    }
-}
-
-// pass 2: one thread per (channel, state) carries the state across every request's chunks
-__global__ void selective_scan_carry_kernel(float* __restrict__ ends, const float* __restrict__ sums,
-                                            const float* __restrict__ a_log, float* __restrict__ state,
-                                            const int* __restrict__ cu_q, const int* __restrict__ slot_ids, int n_seqs, int Lc,
-                                            int I, int S, int write_state, int num_slots, int* __restrict__ status) {
-    pdl_trigger();
-    pdl_wait();
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= I * S) return;
-    const int c = idx / S;
-    const float a = -expf(a_log[idx]);
-    int chunk = 0;
-    for (int s = 0; s < n_seqs; ++s) {
-        const int len = cu_q[s + 1] - cu_q[s];
-        if (len <= 0) continue;
-        const int nc = (len + Lc - 1) / Lc;
-        const int slot = zai_checked_slot(slot_ids[s], num_slots, status);
-        float* st = state + (size_t)slot * I * S + idx;
-        float h = *st;
-        for (int j = 0; j < nc; ++j, ++chunk) {
-            float* e = ends + (size_t)chunk * I * S + idx;
-            const float h_in = h;
-            h = expf(a * sums[(size_t)chunk * I + c]) * h + *e;
-            *e = h_in;
+        for (int u = 0; u < 4; ++u) {
+            o.d[u] = *reinterpret_cast<const ulonglong2*>(&tile.step[r + u][cl]);
+            const uint64_t* p = reinterpret_cast<const uint64_t*>(&tile.bc[r + u][g * K]);
+#pragma unroll
+            for (int k = 0; k < K / 2; ++k) {
+                o.b[u][k] = p[k];
+                o.c[u][k] = p[SP / 2 + k];
+            }
         }
-        if (write_state) *st = h;
+    };
+    // the G lanes' sums of four rows at once, in steps that run beside the next rows' sums: each exchange halves the rows a lane
+    // goes on with
+    const bool b0 = lane & 1, b1 = lane & 2;
+    auto settle = [&](Tile& tile, int r, int at, float (&v)[4]) {
+        if (at == 0) {
+            v[0] = (b0 ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, b0 ? v[0] : v[1], 1);
+            v[2] = (b0 ? v[3] : v[2]) + __shfl_xor_sync(0xffffffffu, b0 ? v[2] : v[3], 1);
+        } else if (at == 1) {
+            v[0] = (b1 ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, b1 ? v[0] : v[2], 2);
+        } else if (at == 2) {
+#pragma unroll
+            for (int o = 4; o < G; o <<= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        } else if (G == 4 || g < 4) {
+            tile.sum[r + (lane & 3)][cl] = v[0];
+        }
+    };
+    __syncthreads();                                         // tile 0 is there
+    for (int n = 0; n < n_tiles; ++n) {
+        Tile& tile = tiles[n & 1];
+        const int rows = min(TT, end - start - n * TT);      // (up to three rows behind them change no state)
+        Rows now;
+        take(tile, 0, now);
+        float before[4] = {0.f, 0.f, 0.f, 0.f};
+        int r = 0;
+#pragma unroll 2
+        for (; r < rows; r += 4) {
+            Rows next;
+            take(tile, r + 4 < TT ? r + 4 : r, next);
+            float out[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                uint64_t sum = 0;
+#pragma unroll
+                for (int k = 0; k < K / 2; ++k) {
+                    const float2 v = pair_of(mul_pair(now.d[u].x, a[k]));
+                    h[k] = fma_pair(make_pair(decay_of<T>(v.x), decay_of<T>(v.y)), h[k], mul_pair(now.d[u].y, now.b[u][k]));
+                    sum = k ? fma_pair(h[k], now.c[u][k], sum) : mul_pair(h[k], now.c[u][k]);
+                }
+                const float2 both = pair_of(sum);
+                out[u] = both.x + both.y;
+                if (r > 0) settle(tile, r - 4, u, before);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) before[u] = out[u];
+            now = next;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) settle(tile, r - 4, u, before);
+        __syncthreads();                                     // this tile has been walked, the next one is there
+    }
+    if (write_state && live) {
+#pragma unroll
+        for (int k = 0; k < K; k += 2) {
+            const float2 v = pair_of(h[k / 2]);
+            h1[k] = v.x;
+            h1[k + 1] = v.y;
+        }
+        state_io<K>(st, h1, n_mine, true);
     }
 }
 
 template <typename T, int K, int G>
-static int launch_scan(void* y, const void* x, const void* proj, int proj_stride, const void* z, int z_stride, const float* dt_raw,
-                       const void* w_dt, const float* b_dt, const float* a_log, const float* d_skip, float* state, const int* cu_q,
-                       const int* slot_ids, int n_seqs, int I, int S, int R, int write_state, int num_slots, int* status,
-                       float* ends, float* sums, int chunk, int max_chunks, int single_tokens, cudaStream_t stream) {
-    const int per_block = 128 / G;
-    const unsigned cb = (unsigned)((I + per_block - 1) / per_block);
+static int launch_scan_single(void* y, const void* x, const void* proj, int proj_stride, const void* z, int z_stride, const float* dt_raw,
+                              const void* w_dt, const float* b_dt, const float* a_log, const float* d_skip, float* state, const int* cu_q,
+                              const int* slot_ids, int n_seqs, int I, int S, int R, int write_state, int num_slots, int* status,
+                              cudaStream_t stream) {
+    const unsigned cb = (unsigned)((I + 128 / G - 1) / (128 / G));
     if (cb > 65535) return ZAI_BAD_SIZE;
-    if (single_tokens)
-        return launch_pdl(selective_scan_kernel<T, K, G, 1>, dim3(n_seqs, cb), dim3(128), 0, stream, (T*)y, (const T*)x,
-                          (const T*)proj, proj_stride, (const T*)z, z_stride, dt_raw, (const T*)w_dt, b_dt, a_log, d_skip, state,
-                          cu_q, slot_ids, I, S, R, write_state, num_slots, status);
-    if (!dt_raw) return ZAI_BAD_SIZE;
-    if (!ends || chunk <= 0)
-        return launch_pdl(selective_scan_kernel<T, K, G, (K > 8 ? 2 : 4)>, dim3(n_seqs, cb), dim3(128), 0, stream, (T*)y,
-                          (const T*)x, (const T*)proj, proj_stride, (const T*)z, z_stride, dt_raw, (const T*)w_dt, b_dt, a_log, d_skip,
-                          state, cu_q, slot_ids, I, S, R, write_state, num_slots, status);
-    int rc = launch_pdl(selective_scan_chunk_kernel<T, K, G, false>, dim3(max_chunks, cb), dim3(128), 0, stream, (T*)y,
-                        (const T*)x, (const T*)proj, proj_stride, (const T*)z, z_stride, dt_raw, b_dt, a_log, d_skip, ends,
-                        sums, cu_q, n_seqs, chunk, I, S, R);
-    if (rc) return rc;
-    rc = launch_pdl(selective_scan_carry_kernel, dim3((I * S + 127) / 128), dim3(128), 0, stream, ends, (const float*)sums, a_log,
-                    state, cu_q, slot_ids, n_seqs, chunk, I, S, write_state, num_slots, status);
-    if (rc) return rc;
-    return launch_pdl(selective_scan_chunk_kernel<T, K, G, true>, dim3(max_chunks, cb), dim3(128), 0, stream, (T*)y, (const T*)x,
-                      (const T*)proj, proj_stride, (const T*)z, z_stride, dt_raw, b_dt, a_log, d_skip, ends, sums, cu_q,
-                      n_seqs, chunk, I, S, R);
+    return launch_pdl(selective_scan_single_kernel<T, K, G>, dim3(n_seqs, cb), dim3(128), 0, stream, (T*)y, (const T*)x,
+                      (const T*)proj, proj_stride, (const T*)z, z_stride, dt_raw, (const T*)w_dt, b_dt, a_log, d_skip, state,
+                      cu_q, slot_ids, I, S, R, write_state, num_slots, status);
+}
+
+template <typename T, int K, int G>
+static int launch_scan(void* y, const void* x, const void* proj, int proj_stride, const void* z, int z_stride, const float* dt_raw,
+                       const float* b_dt, const float* a_log, const float* d_skip, float* state, const int* cu_q,
+                       const int* slot_ids, int n_seqs, int I, int S, int R, int write_state, int num_slots, int* status,
+                       cudaStream_t stream) {
+    const unsigned cb = (unsigned)((I + 128 / G - 1) / (128 / G));
+    if (cb > 65535) return ZAI_BAD_SIZE;
+    constexpr size_t smem = 2 * sizeof(ScanTile<K, G>);
+    static_assert(smem <= 227 * 1024, "two tiles fit");
+    static unsigned long long done = 0;
+    if (zai_first_on_device(&done)) {
+        const cudaError_t e = cudaFuncSetAttribute(selective_scan_kernel<T, K, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+    }
+    const uintptr_t four = 4 * sizeof(T) - 1;
+    const int vec = ((I | S | R | proj_stride | z_stride) & 3) == 0 && (reinterpret_cast<uintptr_t>(dt_raw) & 15) == 0
+                    && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(proj)) & four) == 0;
+    return launch_pdl(selective_scan_kernel<T, K, G>, dim3(n_seqs, cb), dim3(256), smem, stream, (T*)y, (const T*)x, (const T*)proj,
+                      proj_stride, (const T*)z, z_stride, dt_raw, b_dt, a_log, d_skip, state, cu_q, slot_ids, I, S, R, write_state,
+                      num_slots, status, vec);
 }
 
 // y [N, I]; x [N, I]; proj [N, proj_stride] (dt_in | B | C, of which B and C are read here); z [N, z_stride];
 // dt_raw [N, I]: the products dt_in . w_dt^T in 32-bit (a matrix product made beforehand), or null in a step of single
 // tokens, which then sums them from w_dt [I, R] itself; state [slots, I, S].
-// With `ends` [max_chunks, I, S] and `sums` [max_chunks, I] (32-bit scratch) and chunk > 0 the step runs in three
-// passes over chunks of `chunk` rows; max_chunks >= the number of chunks of the step (N / chunk + n_seqs covers it).
 // single_tokens: every request brings one row (a leaner kernel).
 ZAI_API int zai_selective_scan(void* y, const void* x, const void* proj, int proj_stride, const void* z, int z_stride, int dtype,
                                const float* dt_raw, const void* w_dt, const float* b_dt, const float* a_log, const float* d_skip,
-                               float* state,
-                               const int* cu_q, const int* slot_ids, int N, int n_seqs, int I, int S, int R, int write_state,
-                               int num_slots, int* status, float* ends, float* sums, int chunk, int max_chunks,
-                               int single_tokens, cudaStream_t stream) {
+                               float* state, const int* cu_q, const int* slot_ids, int N, int n_seqs, int I, int S, int R, int write_state,
+                               int num_slots, int* status, int single_tokens, cudaStream_t stream) {
     if (N <= 0 || n_seqs <= 0) return ZAI_OK;
     if (I < 1 || S < 1 || S > 256 || R < 1 || (!dt_raw && !w_dt)) return ZAI_BAD_SIZE;
-#define ZAI_SCAN(KK, GG) ZAI_DISPATCH(dtype, return launch_scan<T, KK, GG>(y, x, proj, proj_stride, z, z_stride, dt_raw, w_dt, b_dt, a_log, \
-        d_skip, state, cu_q, slot_ids, n_seqs, I, S, R, write_state, num_slots, status, ends, sums, chunk, max_chunks, \
-        single_tokens && N == n_seqs, stream))
-    if (S <= 4) ZAI_SCAN(4, 1);
-    if (S <= 8) ZAI_SCAN(8, 1);
-    if (S <= 16) ZAI_SCAN(16, 1);
-    if (S <= 32) ZAI_SCAN(16, 2);
-    if (S <= 64) ZAI_SCAN(16, 4);
-    if (S <= 128) ZAI_SCAN(16, 8);
+    if (single_tokens && N == n_seqs) {
+#define ZAI_SCAN(KK, GG) ZAI_DISPATCH(dtype, return launch_scan_single<T, KK, GG>(y, x, proj, proj_stride, z, z_stride, dt_raw, w_dt, b_dt, \
+        a_log, d_skip, state, cu_q, slot_ids, n_seqs, I, S, R, write_state, num_slots, status, stream))
+        if (S <= 4) ZAI_SCAN(4, 1);
+        if (S <= 8) ZAI_SCAN(8, 1);
+        if (S <= 16) ZAI_SCAN(16, 1);
+        if (S <= 32) ZAI_SCAN(16, 2);
+        if (S <= 64) ZAI_SCAN(16, 4);
+        if (S <= 128) ZAI_SCAN(16, 8);
+        ZAI_SCAN(16, 16);
+#undef ZAI_SCAN
+    }
+    if (!dt_raw) return ZAI_BAD_SIZE;
+#define ZAI_SCAN(KK, GG) ZAI_DISPATCH(dtype, return launch_scan<T, KK, GG>(y, x, proj, proj_stride, z, z_stride, dt_raw, b_dt, a_log, \
+        d_skip, state, cu_q, slot_ids, n_seqs, I, S, R, write_state, num_slots, status, stream))
+    if (S <= 8) ZAI_SCAN(2, 4);
+    if (S <= 16) ZAI_SCAN(2, 8);
+    if (S <= 32) ZAI_SCAN(2, 16);
+    if (S <= 64) ZAI_SCAN(4, 16);
+    if (S <= 128) ZAI_SCAN(8, 16);
     ZAI_SCAN(16, 16);
 #undef ZAI_SCAN
 }

@@ -72,7 +72,7 @@ _SIGNATURES = {
                    "zai_weighted_sum": [_P, _P, _P, _I, _F, _F, ctypes.c_longlong, _P]},
     "causal_conv": {"zai_causal_conv": [_P, _I, _P, _I, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P]},
     "selective_scan": {"zai_selective_scan": [_P, _P, _P, _I, _P, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I,
-                                              _I, _P, _P, _P, _I, _I, _I, _P]},
+                                              _I, _P, _I, _P]},
     "min_gru": {"zai_min_gru": [_P, _P, _I, _I, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _I, _I, _P]},
     "gated_delta": {
         "zai_delta_prepare": [_P, _P, _P, _P, _I, _P, _I, _P, _I, _I, _P, _P, _I, _I, _I, _I, _F, _P],
@@ -1315,9 +1315,6 @@ def selective_scan(x, proj, z, w_dt, b_dt, a_log, d_skip, state, step, dt_rank, 
     if state.dtype != torch.float32 or tuple(state.shape[1:]) != (I, S):
         raise KernelError("the scan state is 32-bit [slots, inner, state]")
     y = torch.empty((N, I), dtype=x.dtype, device=x.device)
-    chunk, max_chunks = _scan_chunks(step, N, -(-I // (128 if S <= 16 else 64)))
-    ends = torch.empty((max_chunks, I, S), dtype=torch.float32, device=x.device) if chunk else None
-    sums = torch.empty((max_chunks, I), dtype=torch.float32, device=x.device) if chunk else None
     # the step sizes' products dt_in . w_dt^T for all rows as one matrix product with a 32-bit result; a step of
     # single tokens sums them inside its kernel (a launch less a layer, and the weights are read once either way)
     single = bool(step.decode_only and N == step.n_seqs)
@@ -1325,8 +1322,7 @@ def selective_scan(x, proj, z, w_dt, b_dt, a_log, d_skip, state, step, dt_rank, 
     _check(_fn("selective_scan", "zai_selective_scan")(
         _ptr(y), _ptr(x), pp, ps, zp, zs, _dt(x), _ptr(dt_raw), _ptr(w_dt), _ptr(b_dt), _ptr(a_log), _ptr(d_skip), _ptr(state),
         _ptr(step.cu_q), _ptr(step.slot_ids), N, step.n_seqs, I, S, R, int(bool(write_state)), state.shape[0],
-        _status_ptr(x.device), _ptr(ends), _ptr(sums), chunk, max_chunks, int(bool(step.decode_only)), _stream()),
-        "selective_scan", 3 if chunk else 1)
+        _status_ptr(x.device), int(bool(step.decode_only)), _stream()), "selective_scan")
     return y
 
 
