@@ -202,3 +202,39 @@ def test_value_norm_and_padding(dtype, H, G, D, Dv, normed):
     got = o.value_norm_pad(qkv, H, G, D, Dv, 1e-5, normed)
     assert got.shape == want.shape
     assert torch.allclose(got.float(), want.float(), **tol(dtype))
+
+
+@pytest.mark.parametrize("H,G,D,V", [(4, 2, 64, 128), (2, 2, 16, 24), (3, 1, 40, 33), (6, 2, 32, 40), (10, 5, 64, 256), (1, 1, 1, 1)])
+@pytest.mark.parametrize("channel", [False, True])
+def test_gated_delta_in_chunks(H, G, D, V, channel):
+    """The kernels that run a span in chunks of 64 rows, at every remainder that matters, behind a state and beside spans that
+    are walked; decays from next to none to ones that leave nothing of a state within a row, next to each other."""
+    o = ops()
+    g = torch.Generator().manual_seed(21)
+    cols_a = H * D if channel else H
+    a_log = torch.log(1 + 15 * torch.rand(H, generator=g)).cuda()
+    dt_bias = (torch.randn(cols_a, generator=g) * 2 - 3).cuda()
+    norm_w = (1 + 0.1 * torch.randn(V, generator=g)).cuda()
+    state_a = (torch.randn(22, H, D, V, generator=g) * 0.3).cuda()
+    state_b = state_a.clone()
+    for q_lens, impl in (([64, 1, 63, 65], "chunks"), ([129, 300, 2, 128], "chunks"), ([1, 160, 1, 400], None), ([159, 261, 5, 0], None), ([500], None)):
+        step = make_step(o, torch.bfloat16, [3] * len(q_lens), q_lens, 8, 256, 5)
+        N = sum(q_lens)
+        qkv = torch.randn(N, 2 * G * D + H * V, generator=g).bfloat16().cuda()
+        a = torch.randn(N, cols_a, generator=g)
+        a[N // 3:N // 3 + 20] += 30.0                                  # decays of hundreds of nats a row
+        a[N // 2:N // 2 + 40] -= 30.0                                  # and none at all
+        a = a.bfloat16().cuda()
+        rest = torch.randn(N, H * V + H, generator=g).bfloat16().cuda()
+        gate, b = rest[:, :H * V], rest[:, H * V:]
+        more = dict(channel_decay=channel, gate_act="sigmoid")
+        ya = o.gated_delta(qkv, b, a, gate, a_log, dt_bias, norm_w, 1e-5, state_a, step, H, G, D, V, True, impl=impl, **more)
+        yb = ref_ops.gated_delta(qkv, b, a, gate, a_log, dt_bias, norm_w, 1e-5, state_b, step, H, G, D, V, True, **more)
+        # the limits of test_gated_delta
+        assert torch.allclose(ya.float(), yb.float(), **tol(torch.bfloat16)), (q_lens, float((ya.float() - yb.float()).abs().max()))
+        assert torch.allclose(state_a, state_b, atol=1e-4, rtol=1e-4), q_lens
+    assert torch.equal(state_a[0], state_b[0])
+    keep = state_a.clone()
+    o.gated_delta(qkv, b, a, gate, a_log, dt_bias, norm_w, 1e-5, state_a, step, H, G, D, V, False, impl="chunks", **more)
+    assert torch.equal(state_a, keep)
+    assert o.read_status() == 0

@@ -6,15 +6,15 @@
 // beta = sigmoid(b), g = exp(-exp(A_log) softplus(a + dt_bias)): one decay per head, or (`channel`) one per head and
 // key channel, g [H, D], which then scales the rows of S one by one (a and dt_bias are [H D] wide, A_log stays per
 // head).  The output gate is silu or (`gate_act` 1) a sigmoid.  A step of single tokens is one kernel (a block per
-// request and head does all of it); steps with portions run three kernels:
-//   * prepare: unit norms, beta and g for every row of the step, all 32-bit;
-//   * the recurrence: the columns of S are independent, so a block owns some columns of one head of one
-//     request and walks the request's rows in order; P lanes of a warp share a column, each with DP of
-//     its D rows in registers; the operands of the next sixteen tokens come into shared memory by
-//     asynchronous copies while the current sixteen are computed;
-//   * the output norm: o / rms(o) * weight * silu(gate) per head, rounded to the model's dtype.
+// request and head does all of it); spans of rows go one of two ways, which differ by rounding only:
+//   * the walk (any sizes, both modes; shorter spans).  `prepare`: unit norms, beta and g for every row, all 32-bit.  The
+//     recurrence: the columns of S are independent, so a block owns some columns of one head of one request and walks the
+//     request's rows in order; P lanes of a warp share a column, each with DP of its D rows in registers; the operands of the
+//     next sixteen tokens come into shared memory by asynchronous copies while the current sixteen are computed.
+//   * chunks of 64 rows (bfloat16, longer spans, keys of up to 64): further below.
+// The output norm is a kernel of its own: o / rms(o) * weight * silu(gate) per head, rounded to the model's dtype.
 #include <cstdlib>
-#include "common.cuh"
+#include "mma_helpers.cuh"
 
 __device__ __forceinline__ float softplus_f(float v) { return v > 20.f ? v : log1pf(expf(v)); }
 
@@ -24,9 +24,14 @@ template <typename T>
 __global__ void delta_prepare_kernel(float* __restrict__ qk_out, float* __restrict__ bg_out, float* __restrict__ gch_out,
                                      const T* __restrict__ qkv, int qkv_stride, const T* __restrict__ b_in, int b_stride,
                                      const T* __restrict__ a_in, int a_stride, const float* __restrict__ a_log,
-                                     const float* __restrict__ dt_bias, int H, int G, int D, float unit_eps) {
+                                     const float* __restrict__ dt_bias, int H, int G, int D, float unit_eps,
+                                     const int* __restrict__ cu_q, const int* __restrict__ seq_idx, int max_rows) {
     pdl_trigger();
     pdl_wait();
+    if (seq_idx) {                                     // (rows of longer spans are another kernel's)
+        const int s = seq_idx[blockIdx.x];
+        if (cu_q[s + 1] - cu_q[s] > max_rows) return;
+    }
     const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
     const float q_scale = rsqrtf((float)D);
     for (int item = warp; item < 2 * G; item += nwarp) {
@@ -78,7 +83,7 @@ __global__ void __launch_bounds__(128) gated_delta_kernel(
     float* __restrict__ o_out, const float* __restrict__ qk, const float* __restrict__ bg, const float* __restrict__ gch,
     const T* __restrict__ v_in,
     int v_stride, float* __restrict__ state, const int* __restrict__ cu_q, const int* __restrict__ slot_ids, int H, int G,
-    int D, int V, int write_state, int num_slots, int* __restrict__ status) {
+    int D, int V, int write_state, int num_slots, int* __restrict__ status, int max_rows) {
     using St = DeltaStage<DP, P, CH>;
     constexpr int VB = St::VB, TB = St::TB, NG = St::NG;
     __shared__ __align__(16) float ring[2][TB][St::PER_TOKEN];
@@ -90,7 +95,7 @@ __global__ void __launch_bounds__(128) gated_delta_kernel(
     const bool live = j < V;
     if (!live) j = V - 1;                              // (stays for the shuffles, stores nothing)
     const int start = cu_q[seq], end = cu_q[seq + 1];
-    if (end <= start) return;
+    if (end <= start || end - start > max_rows) return;
     const int slot = zai_checked_slot(slot_ids[seq], num_slots, status);
     const int kvh = h / (H / G), d0 = p * DP;
     float* st = state + (((size_t)slot * H + h) * D) * V + j;
@@ -338,13 +343,16 @@ ZAI_API int zai_gated_delta_single(void* out, const void* qkv, int qkv_stride, c
 #undef ZAI_DELTA1
 }
 
-// gch_out null: one decay per head (into bg_out); else the decays per head and key channel [N, H, D]
+// gch_out null: one decay per head (into bg_out); else the decays per head and key channel [N, H, D].  With seq_idx [N] (the
+// rows' requests) only rows of spans of at most max_rows rows are made.
 ZAI_API int zai_delta_prepare(float* qk_out, float* bg_out, float* gch_out, const void* qkv, int qkv_stride, const void* b_in,
                               int b_stride, const void* a_in, int a_stride, int dtype, const float* a_log, const float* dt_bias,
-                              int N, int H, int G, int D, float unit_eps, cudaStream_t stream) {
+                              int N, int H, int G, int D, float unit_eps, const int* cu_q, const int* seq_idx, int max_rows,
+                              cudaStream_t stream) {
     if (N <= 0) return ZAI_OK;
     ZAI_DISPATCH(dtype, return launch_pdl(delta_prepare_kernel<T>, dim3(N), dim3(128), 0, stream, qk_out, bg_out, gch_out,
-        (const T*)qkv, qkv_stride, (const T*)b_in, b_stride, (const T*)a_in, a_stride, a_log, dt_bias, H, G, D, unit_eps));
+        (const T*)qkv, qkv_stride, (const T*)b_in, b_stride, (const T*)a_in, a_stride, a_log, dt_bias, H, G, D, unit_eps, cu_q,
+        seq_idx, max_rows));
 }
 
 // Dynamic shared memory that keeps more than `per_sm` blocks of `kernel` off one SM.  The recurrence is a chain of
@@ -379,28 +387,28 @@ static size_t delta_spread_smem(K kernel, long long blocks) {
 template <typename T, int DP, int P>
 static int launch_delta(float* o_out, const float* qk, const float* bg, const float* gch, const void* v_in, int v_stride,
                         float* state, const int* cu_q, const int* slot_ids, int n_seqs, int H, int G, int D, int V, int write_state,
-                        int num_slots, int* status, cudaStream_t stream) {
+                        int num_slots, int* status, int max_rows, cudaStream_t stream) {
     const int vb = 128 / P;
     const dim3 grid(n_seqs, H, (V + vb - 1) / vb);
     const long long blocks = (long long)grid.x * grid.y * grid.z;
     if (gch)
         return launch_pdl(gated_delta_kernel<T, DP, P, true>, grid, dim3(128), delta_spread_smem(gated_delta_kernel<T, DP, P, true>, blocks),
                           stream, o_out, qk, bg, gch, (const T*)v_in, v_stride, state, cu_q, slot_ids, H, G, D, V, write_state, num_slots,
-                          status);
+                          status, max_rows);
     return launch_pdl(gated_delta_kernel<T, DP, P, false>, grid, dim3(128), delta_spread_smem(gated_delta_kernel<T, DP, P, false>, blocks),
                       stream, o_out, qk, bg, gch, (const T*)v_in, v_stride, state, cu_q, slot_ids, H, G, D, V, write_state, num_slots,
-                      status);
+                      status, max_rows);
 }
 
 // o_out [N, H*V] 32-bit; qk, bg (and gch, or null) from zai_delta_prepare; v_in [N, v_stride] (heads of V values);
-// state [slots, H, D, V]
+// state [slots, H, D, V]; only spans of at most max_rows rows are run
 ZAI_API int zai_gated_delta(float* o_out, const float* qk, const float* bg, const float* gch, const void* v_in, int v_stride,
                             int dtype, float* state, const int* cu_q, const int* slot_ids, int N, int n_seqs, int H, int G, int D,
-                            int V, int write_state, int num_slots, int* status, cudaStream_t stream) {
+                            int V, int write_state, int num_slots, int* status, int max_rows, cudaStream_t stream) {
     if (N <= 0 || n_seqs <= 0) return ZAI_OK;
     if (D < 1 || D > 256 || V < 1 || G < 1 || H % G != 0 || H > 65535 || V > 65535 * 16) return ZAI_BAD_SIZE;
 #define ZAI_DELTA(DPV, PV) ZAI_DISPATCH(dtype, return launch_delta<T, DPV, PV>(o_out, qk, bg, gch, v_in, v_stride, state, cu_q, \
-        slot_ids, n_seqs, H, G, D, V, write_state, num_slots, status, stream))
+        slot_ids, n_seqs, H, G, D, V, write_state, num_slots, status, max_rows, stream))
     // four lanes a column (eight for the largest heads): measured against two and one (fewer exchanges, longer
     // chains of multiply-adds a lane), four was the fastest or level at 64-wide heads
     if (D <= 16) ZAI_DELTA(4, 4);
@@ -419,4 +427,703 @@ ZAI_API int zai_gated_rmsnorm(void* out, const float* o, const float* w, const v
     if (blocks > 0x7fffffffLL) return ZAI_BAD_SIZE;
     ZAI_DISPATCH(dtype, return launch_pdl(gated_rmsnorm_kernel<T>, dim3((unsigned)blocks), dim3(128), 0, stream, (T*)out, o, w,
         (const T*)gate, gate_stride, eps, (int)items, H, V, gate_act));
+}
+
+// ------------------------------------------------------------------------------------------------ chunks
+// The walk is a chain of one request's rows (0.28 us a row on a fraction of the SMs).  A portion of a prompt is cut into chunks
+// of DC rows instead.  With c_t the running sum of the log decays from the chunk's first row (one number a head, or one a key
+// channel) and S_0 the state before the chunk, the rule unrolls to
+//
+//   u_t = beta_t (v_t - S_0^T (e^(c_t) k_t) - sum_{s<t} A_ts u_s),    A_ts = sum_d k_t k_s e^(c_t - c_s)
+//   o_t = S_0^T (e^(c_t) q_t) + sum_{s<=t} P_ts u_s,                  P_ts = sum_d q_t k_s e^(c_t - c_s)
+//   S   = e^(c_last) S_0 + sum_s (e^(c_last - c_s) k_s) u_s^T
+//
+// The first line is a triangular system with the same matrix for every column: its solution for the right sides beta_t v_t (U0)
+// and beta_t e^(c_t) k_t (W) needs no state, and u = U0 - W S_0.  Two kernels:
+//   * `delta_chunk_kernel`, every chunk and head at once: unit norms, decays, A, P, and the system solved by substitution in
+//     32-bit, a thread a right side with its 64 unknowns in registers.  A and P are products of bfloat16 rows, or, with a decay per
+//     channel, of rows in three parts scaled by e^(c_t - c_first) and e^(c_first - c_s) around the first of 16 rows; inside 16 rows
+//     that decay by more than 2^-100 the pairs of rows are taken one by one instead.  Running sums are made in 64-bit and kept in
+//     two parts, so that a difference of two is good to the last bits.
+//   * `delta_carry_kernel`, a block a head and DN columns of S: carries S across a request's chunks on the tensor cores (four
+//     warps: u, then the new S) and makes the chunks' read-outs beside that (four more warps).  S, u, W, P and the scaled k and q
+//     are 32-bit and go into bfloat16 products as sums of three parts (24 bits; the six products that reach 2^-24 of the
+//     result), with 32-bit sums by size.  What comes from the first kernel is laid out as a lane's operands of one m16n8k16
+//     product lie, three parts beforehand: 16 bytes a load, nothing to convert.
+// 2048 rows of 16 heads of 64 x 128 (norms, recurrence and output norm): 136 us where the walk takes 480, with a decay per channel
+// 172 (601); of 32 heads 233 (581) and 292 (660).  The first kernel (53 and 88 us of 16 heads) is bound by its phases' latencies
+// with two blocks an SM, the second (58) by a chunk's two dependent products, 1.8 us a chunk at 43 % of the tensor pipe.
+#define DC 64                       // rows of a chunk
+#define DCD 64                      // key size the chunk kernels are made for (smaller heads are filled up with zeros)
+#define DC_LD 68                    // 32-bit row stride in shared memory
+
+// A 64 x 64 operand of the carry in three parts: [part][tile of 16 rows][tile of 16 columns][lane], a lane's four registers
+struct DeltaOperand { uint4 v[3][4][4][32]; };
+struct DeltaChunk {                 // what the first kernel leaves for a chunk and head (U0 lies behind all of them)
+    DeltaOperand w, k, q, p;        // W [t, d]; e^(c_last - c_s) k_s [d, s]; e^(c_t) q_t [t, d]; P [t, s]
+    float keep[DCD];                // e^(c_last)
+};
+
+struct DeltaArgs {
+    const bf16* qkv;                // [N, qkv_stride]: q heads, k heads, v heads
+    const bf16 *b, *a;              // [N, b_stride] (H a row), [N, a_stride] (H, or H D with a decay per channel)
+    int qkv_stride, b_stride, a_stride;
+    const float *a_log, *dt_bias;
+    float unit_eps;
+    float* state;                   // [num_slots, H, D, V]
+    const int *cu_q, *slot_ids;
+    int* status;
+    int num_slots, n_seqs, H, G, D, V, write_state, min_rows;
+    DeltaChunk* chunks;             // [chunks, H]
+    float* u0;                      // [chunks, H, DC, VP]
+    int VP;                         // V rounded up to 32
+    float* o;                       // [N, H V]
+};
+
+// Chunk b among all chunks of the step: the spans of min_rows rows or more in order, each cut into chunks of DC rows.
+__device__ __forceinline__ bool delta_find_chunk(const DeltaArgs& a, int b, int& t0, int& t1) {
+    for (int s = 0; s < a.n_seqs; ++s) {
+        const int lo = a.cu_q[s], hi = a.cu_q[s + 1];
+        if (hi - lo < a.min_rows) continue;
+        const int n = (hi - lo + DC - 1) / DC;
+        if (b < n) {
+            t0 = lo + b * DC;
+            t1 = min(t0 + DC, hi);
+            return true;
+        }
+        b -= n;
+    }
+    return false;
+}
+
+__device__ __forceinline__ float delta_minus(float2 a, float2 b) { return (a.x - b.x) + (a.y - b.y); }
+// log decay in units of ln 2.  Below 2^-1000 a decay is zero in 32-bit however it is split up: the sums stay finite.
+__device__ __forceinline__ double delta_log_decay(float rate, float a) {
+    const double l = -1.4426950408889634 * (double)(rate * softplus_f(a));
+    return l < -1000.0 ? -1000.0 : l;
+}
+// 2^(x + y) for a small y
+__device__ __forceinline__ float delta_exp2(float x, float y) {
+    const float e = fast_exp2(x);
+    return fmaf(e, 0.69314718f * y, e);
+}
+
+// 16 sums over 16 neighbouring lanes at once: lane i of the 16 ends with the sum of v[i] in v[0]
+__device__ __forceinline__ void sum16(float (&v)[16], int lane) {
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+            const float send = up ? v[i] : v[i + o], keep = up ? v[i + o] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+}
+
+// Writes an operand: get(row, column) gives two neighbouring columns (the first even); all 256 threads
+template <typename F>
+__device__ __forceinline__ void delta_put(DeltaOperand* out, F get) {
+    for (int i = threadIdx.x; i < 4 * 4 * 32; i += 256) {
+        const int lane = i & 31, kt = (i >> 5) & 3, mt = i >> 7, g = lane >> 2, tq = lane & 3;
+        uint32_t part[4][3];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int row = mt * 16 + g + 8 * (r & 1), col = kt * 16 + 2 * tq + 8 * (r >> 1);
+            const float2 x = get(row, col);
+            split3_pair(x.x, x.y, part[r]);
+        }
+#pragma unroll
+        for (int p = 0; p < 3; ++p) out->v[p][mt][kt][lane] = make_uint4(part[0][p], part[1][p], part[2][p], part[3][p]);
+    }
+}
+
+#define DR_LD (DCD + 8)             // bfloat16 row stride of rows in shared memory
+#define DELTA_V_MAX 256             // value sizes up to which a chunk's rows of v are put into shared memory
+#define DELTA_FAST 100.f            // log2 decays over 16 rows up to which e^(-c) is kept as a number of its own
+
+struct DeltaShared {
+    bf16 qk[2][DC][DR_LD];                                   // the rows of q and k as they came
+    float inv[2][DC];                                        // what makes them unit rows (q: times D^-1/2)
+    union {
+        struct {
+            bf16 left[2][3][16][DR_LD];                      // 16 rows of q and k times e^(c_t - c at their first), in three parts
+            bf16 right[3][DC][DR_LD];                        // the rows of k up to them times e^(c at their first - c_s), likewise
+        };
+        bf16 v[DC * (DELTA_V_MAX + 8)];                      // then: the rows of v, V + 8 values apart
+    };
+    float m[DC][DC_LD];                                      // beta_t A_ts below the diagonal, P_ts at [s][t] on and above it
+    union {
+        struct {
+            float hi[DC][DCD];                               // running log decays inside the 16 rows (one column: the chunk's), in
+            bf16 lo[DC][DCD];                                // two parts (32 bits of their sums)
+        } c;
+        float w[DC][DC_LD];                                  // W, when the decays are no longer needed
+    };
+    float sum[4][DCD], sum_lo[4][DCD];                       // log decay of every 16 rows, in two parts
+    float before[5][DCD], after[4][DCD];                     // ... of all 16s before (4: of the chunk), and after
+    float beta[DC];
+    double carry;
+    // (which: 0 q, 1 k) a unit row's value; two neighbouring ones (d even)
+    __device__ __forceinline__ float unit(int which, int t, int d) const { return to_float(qk[which][t][d]) * inv[which][t]; }
+    __device__ __forceinline__ float2 unit_two(int which, int t, int d) const {
+        const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&qk[which][t][d]));
+        const float i = inv[which][t];
+        return make_float2(x.x * i, x.y * i);
+    }
+    __device__ __forceinline__ float2 at(int t, int d) const { return make_float2(c.hi[t][d], to_float(c.lo[t][d])); }
+    // two neighbouring sums: their leading parts and what is left
+    __device__ __forceinline__ void at_two(int t, int d, float2& x, float2& y) const {
+        x = *reinterpret_cast<const float2*>(&c.hi[t][d]);
+        y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&c.lo[t][d]));
+    }
+    __device__ __forceinline__ void keep(int t, int d, double v) {
+        c.hi[t][d] = (float)v;
+        c.lo[t][d] = __float2bfloat16_rn((float)(v - (double)(float)v));
+    }
+};
+
+// CH: a decay per key channel
+template <bool CH>
+__global__ void __launch_bounds__(256, 2) delta_chunk_kernel(const DeltaArgs a) {
+    extern __shared__ __align__(16) unsigned char delta_raw[];
+    DeltaShared& sm = *reinterpret_cast<DeltaShared*>(delta_raw);
+    pdl_trigger();
+    pdl_wait();
+    int t0, t1;
+    if (!delta_find_chunk(a, blockIdx.x, t0, t1)) return;
+    const int h = blockIdx.y, kvh = h / (a.H / a.G), n = t1 - t0;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int D = a.D, V = a.V;
+
+    // the rows of q and k (zeros beyond the chunk and beyond D)
+    if (((D | a.qkv_stride) & 7) == 0 && (reinterpret_cast<uintptr_t>(a.qkv) & 15) == 0) {
+        for (int i = tid; i < 2 * DC * 8; i += 256) {
+            const int which = i >> 9, t = (i >> 3) & 63, d = (i & 7) * 8;
+            const bool ok = t < n && d < D;
+            cp_async16(&sm.qk[which][t][d], a.qkv + (ok ? (size_t)(t0 + t) * a.qkv_stride + (size_t)(which * a.G + kvh) * D + d : 0), ok);
+        }
+    } else {
+        for (int i = tid; i < 2 * DC * DCD; i += 256) {
+            const int which = i >> 12, t = (i >> 6) & 63, d = i & 63;
+            sm.qk[which][t][d] = (t < n && d < D) ? a.qkv[(size_t)(t0 + t) * a.qkv_stride + (size_t)(which * a.G + kvh) * D + d] : __float2bfloat16_rn(0.f);
+        }
+    }
+    cp_async_commit();
+    // decays and beta
+    if (tid < DC) sm.beta[tid] = tid < n ? 1.f / (1.f + expf(-to_float(a.b[(size_t)(t0 + tid) * a.b_stride + h]))) : 0.f;
+    const float rate = expf(a.a_log[h]);
+    if constexpr (CH) {
+        const int d = tid & 63, seg = tid >> 6;              // 16 rows of a channel a thread
+        double acc = 0.0;
+        float x[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const int t = seg * 16 + i;
+            x[i] = (t < n && d < D) ? to_float(a.a[(size_t)(t0 + t) * a.a_stride + h * D + d]) : 0.f;
+        }
+        const float bias = d < D ? a.dt_bias[h * D + d] : 0.f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const int t = seg * 16 + i;
+            if (t < n && d < D) acc += delta_log_decay(rate, x[i] + bias);
+            sm.keep(t, d, acc);
+        }
+        sm.sum[seg][d] = (float)acc;
+        sm.sum_lo[seg][d] = (float)(acc - (double)(float)acc);
+    } else {
+        double l = 0.0;
+        if (tid < DC) {
+            if (tid < n) l = delta_log_decay(rate, to_float(a.a[(size_t)(t0 + tid) * a.a_stride + h]) + a.dt_bias[h]);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const double up = __shfl_up_sync(0xffffffffu, l, o);
+                if (lane >= o) l += up;
+            }
+            if (tid == 31) sm.carry = l;
+        }
+        __syncthreads();
+        if (tid < DC) sm.keep(tid, 0, tid >= 32 ? l + sm.carry : l);
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    // what makes the rows unit rows: two threads a row
+    {
+        const int which = tid >> 7, t = (tid >> 1) & 63, part = tid & 1;
+        float ss = 0.f;
+#pragma unroll
+        for (int i = 0; i < DCD / 2; i += 2) {
+            const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&sm.qk[which][t][part * (DCD / 2) + i]));
+            ss = fmaf(x.x, x.x, fmaf(x.y, x.y, ss));
+        }
+        ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+        if (part == 0) sm.inv[which][t] = rsqrtf(ss + a.unit_eps) * (which ? 1.f : rsqrtf((float)D));
+    }
+    if constexpr (CH) {
+        if (tid < DCD) {                                     // (sums of numbers of one sign: their rounding is as small as their terms')
+            float acc = 0.f;
+            sm.before[0][tid] = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                acc += sm.sum[j][tid];
+                sm.before[j + 1][tid] = acc;
+            }
+            acc = 0.f;
+#pragma unroll
+            for (int j = 3; j >= 0; --j) {
+                sm.after[j][tid] = acc;
+                acc += sm.sum[j][tid];
+            }
+        }
+    }
+    __syncthreads();
+
+    // A and P on the tensor cores, 16 rows (I) at a time; a warp takes eight columns of one of the two
+    const int mi = lane >> 3, r8 = lane & 7, g = lane >> 2, tq = lane & 3;
+    for (int I = 0; I < 4; ++I) {
+        bool fast = true;
+        if constexpr (CH) {
+            // the largest decay of these 16 rows says whether e^(-c) inside them can be a factor by itself
+            fast = !__syncthreads_or(tid < DCD && !(sm.sum[I][tid & 63] > -DELTA_FAST));
+            const int rows = 16 * I + (fast ? 16 : 0);
+            for (int i = tid; i < (rows + 32) * (DCD / 2); i += 256) {
+                const int row = i / (DCD / 2), d = (i % (DCD / 2)) * 2;
+                float2 e, x, hi, lo;
+                if (row < rows) {                            // right: k_s e^(c at the first of the 16 - c_s)
+                    const int s = row, J = s >> 4;
+                    sm.at_two(s, d, hi, lo);
+                    if (J == I) {
+                        e = make_float2(delta_exp2(-hi.x, -lo.x), delta_exp2(-hi.y, -lo.y));
+                    } else {
+                        const float2 a0 = *reinterpret_cast<const float2*>(&sm.sum[J][d]), a1 = *reinterpret_cast<const float2*>(&sm.sum_lo[J][d]);
+                        float2 f = make_float2((a0.x - hi.x) + (a1.x - lo.x), (a0.y - hi.y) + (a1.y - lo.y));
+                        for (int K = J + 1; K < I; ++K) {
+                            const float2 more = *reinterpret_cast<const float2*>(&sm.sum[K][d]);
+                            f.x += more.x;
+                            f.y += more.y;
+                        }
+                        e = make_float2(fast_exp2(f.x), fast_exp2(f.y));
+                    }
+                    x = sm.unit_two(1, s, d);
+                } else {                                     // left: q_t, k_t times e^(c_t - c at the first)
+                    const int which = (row - rows) >> 4, t = 16 * I + ((row - rows) & 15);
+                    sm.at_two(t, d, hi, lo);
+                    e = make_float2(delta_exp2(hi.x, lo.x), delta_exp2(hi.y, lo.y));
+                    x = sm.unit_two(which, t, d);
+                }
+                uint32_t p[3];
+                split3_pair(x.x * e.x, x.y * e.y, p);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    bf16* dst = row < rows ? &sm.right[k][row][d] : &sm.left[(row - rows) >> 4][k][(row - rows) & 15][d];
+                    *reinterpret_cast<uint32_t*>(dst) = p[k];
+                }
+            }
+            __syncthreads();
+        }
+        for (int unit = warp; unit < (I + (fast ? 1 : 0)) * 4; unit += 8) {
+            const int which = unit & 1, nt = unit >> 1;      // which: 0 P (rows of q), 1 A (rows of k); columns 8 nt ..
+            float acc[3][4] = {};
+#pragma unroll
+            for (int kt = 0; kt < 4; ++kt) {
+                if constexpr (CH) {
+                    uint32_t fa[3][4], fb[3][2];
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) {
+                        ldmatrix_x4(fa[k], &sm.left[which][k][(mi & 1) * 8 + r8][kt * 16 + (mi >> 1) * 8]);
+                        fb[k][0] = *reinterpret_cast<const uint32_t*>(&sm.right[k][nt * 8 + g][kt * 16 + 2 * tq]);
+                        fb[k][1] = *reinterpret_cast<const uint32_t*>(&sm.right[k][nt * 8 + g][kt * 16 + 2 * tq + 8]);
+                    }
+#pragma unroll
+                    for (int pa = 0; pa < 3; ++pa)
+#pragma unroll
+                        for (int pb = 0; pa + pb < 3; ++pb) mma_bf16(acc[pa + pb], fa[pa], fb[pb][0], fb[pb][1]);
+                } else {                                     // (rows as they came are bfloat16: one product)
+                    uint32_t fa[4];
+                    ldmatrix_x4(fa, &sm.qk[which][16 * I + (mi & 1) * 8 + r8][kt * 16 + (mi >> 1) * 8]);
+                    mma_bf16(acc[0], fa, *reinterpret_cast<const uint32_t*>(&sm.qk[1][nt * 8 + g][kt * 16 + 2 * tq]),
+                             *reinterpret_cast<const uint32_t*>(&sm.qk[1][nt * 8 + g][kt * 16 + 2 * tq + 8]));
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int t = 16 * I + g + 8 * (e >> 1), s = nt * 8 + 2 * tq + (e & 1);
+                if (s > t) continue;                         // (what lies there is no part of the sums)
+                float v = acc[0][e] + (acc[1][e] + acc[2][e]);
+                if constexpr (!CH) v = acc[0][e] * sm.inv[which][t] * sm.inv[1][s] * fast_exp2(delta_minus(sm.at(t, 0), sm.at(s, 0)));
+                if (which == 0) sm.m[s][t] = v;
+                else if (s < t) sm.m[t][s] = sm.beta[t] * v;
+            }
+        }
+        if (CH && !fast) {
+            // strong decays inside the 16 rows: every pair of rows by itself.  Thread (row r, four channels); the 16 threads of a
+            // row add up its columns
+            const int r = tid >> 4, dq = tid & 15, d0 = dq * 4, t = 16 * I + r;
+            float2 ct[4];
+            float kk[4], qq[4], va[16], vp[16];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                ct[j] = sm.at(t, d0 + j);
+                kk[j] = sm.unit(1, t, d0 + j);
+                qq[j] = sm.unit(0, t, d0 + j);
+            }
+#pragma unroll
+            for (int s = 0; s < 16; ++s) {
+                float x = 0.f, y = 0.f;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float w = sm.unit(1, 16 * I + s, d0 + j) * fast_exp2(delta_minus(ct[j], sm.at(16 * I + s, d0 + j)));
+                    x = fmaf(kk[j], w, x);
+                    y = fmaf(qq[j], w, y);
+                }
+                va[s] = s <= r ? x : 0.f;                    // (later rows have exponents above zero)
+                vp[s] = s <= r ? y : 0.f;
+            }
+            sum16(va, lane);
+            sum16(vp, lane);
+            if (dq < r) sm.m[t][16 * I + dq] = sm.beta[t] * va[0];
+            if (dq <= r) sm.m[16 * I + dq][t] = vp[0];
+        }
+        if (CH) __syncthreads();                             // (the next 16 rows' operands take the place of these)
+    }
+    __syncthreads();
+
+    DeltaChunk* out = a.chunks + (size_t)blockIdx.x * a.H + h;
+    // the rows of v come while the operands are put down
+    const bool v_here = V <= DELTA_V_MAX;
+    const bf16* v = a.qkv + (size_t)t0 * a.qkv_stride + (size_t)2 * a.G * D + (size_t)h * V;
+    const bool v_vec = v_here && ((V | a.qkv_stride | (2 * a.G * D)) & 7) == 0 && (reinterpret_cast<uintptr_t>(a.qkv) & 15) == 0;
+    if (v_vec) {
+        const int per = V >> 3;
+        for (int i = tid; i < DC * per; i += 256) {
+            const int t = i / per, c = (i - t * per) * 8;
+            cp_async16(&sm.v[t * (V + 8) + c], v + (size_t)(t < n ? t : 0) * a.qkv_stride + c, t < n);
+        }
+    } else if (v_here) {
+        for (int i = tid; i < DC * V; i += 256) {
+            const int t = i / V, c = i - t * V;
+            sm.v[t * (V + 8) + c] = t < n ? v[(size_t)t * a.qkv_stride + c] : __float2bfloat16_rn(0.f);
+        }
+    }
+    cp_async_commit();
+    auto from_start = [&](int t, int d) { return CH ? sm.before[t >> 4][d] + sm.c.hi[t][d] : sm.c.hi[t][0]; };
+    delta_put(&out->q, [&](int t, int d) {
+        const float2 x = sm.unit_two(0, t, d);
+        if (!CH) {
+            const float e = fast_exp2(sm.c.hi[t][0]);
+            return make_float2(x.x * e, x.y * e);
+        }
+        const float2 hi = *reinterpret_cast<const float2*>(&sm.c.hi[t][d]), b = *reinterpret_cast<const float2*>(&sm.before[t >> 4][d]);
+        return make_float2(x.x * fast_exp2(b.x + hi.x), x.y * fast_exp2(b.y + hi.y));
+    });
+    delta_put(&out->p, [&](int t, int s) { return make_float2(s <= t ? sm.m[s][t] : 0.f, s < t ? sm.m[s + 1][t] : 0.f); });
+    delta_put(&out->k, [&](int d, int s) {
+        float e[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            if (CH) e[i] = sm.after[s >> 4][d] + delta_minus(make_float2(sm.sum[s >> 4][d], sm.sum_lo[s >> 4][d]), sm.at(s + i, d));
+            else e[i] = delta_minus(sm.at(DC - 1, 0), sm.at(s + i, 0));
+        }
+        return make_float2(sm.unit(1, s, d) * fast_exp2(e[0]), sm.unit(1, s + 1, d) * fast_exp2(e[1]));
+    });
+    if (tid < DCD) out->keep[tid] = fast_exp2(CH ? sm.before[4][tid] : sm.c.hi[DC - 1][0]);
+
+    cp_async_wait<0>();
+    __syncthreads();
+    // the triangular system, a right side a thread: the columns of e^(c_t) k_t, then those of v
+    float* u0 = a.u0 + ((size_t)blockIdx.x * a.H + h) * DC * a.VP;
+    const int total = V + DCD;
+    for (int c0 = 0; c0 < total; c0 += 256) {
+        const int d = c0 + tid, col = d - DCD;
+        float u[DC];
+        if (col >= 0) {
+            if (v_here) {
+#pragma unroll
+                for (int t = 0; t < DC; ++t) u[t] = col < V ? to_float(sm.v[t * (V + 8) + col]) : 0.f;
+            } else {
+#pragma unroll
+                for (int t = 0; t < DC; ++t) u[t] = (t < n && col < V) ? to_float(v[(size_t)t * a.qkv_stride + col]) : 0.f;
+            }
+        } else {
+#pragma unroll
+            for (int t = 0; t < DC; ++t) u[t] = sm.unit(1, t, d) * fast_exp2(from_start(t, d));
+        }
+        __syncthreads();                                     // (W takes the decays' place)
+        if (c0 + warp * 32 >= total) continue;
+#pragma unroll
+        for (int t = 0; t < DC; ++t) {
+            float p0 = sm.beta[t] * u[t], p1 = 0.f, p2 = 0.f, p3 = 0.f;
+#pragma unroll
+            for (int s = 0; s + 4 <= t; s += 4) {
+                const float4 m4 = *reinterpret_cast<const float4*>(&sm.m[t][s]);
+                p0 = fmaf(-m4.x, u[s], p0);
+                p1 = fmaf(-m4.y, u[s + 1], p1);
+                p2 = fmaf(-m4.z, u[s + 2], p2);
+                p3 = fmaf(-m4.w, u[s + 3], p3);
+            }
+#pragma unroll
+            for (int s = t & ~3; s < t; ++s) p1 = fmaf(-sm.m[t][s], u[s], p1);
+            u[t] = (p0 + p1) + (p2 + p3);
+        }
+        if (col < 0) {
+#pragma unroll
+            for (int t = 0; t < DC; ++t) sm.w[t][d] = u[t];
+        } else if (col < V) {
+#pragma unroll
+            for (int t = 0; t < DC; ++t) u0[(size_t)t * a.VP + col] = u[t];
+        }
+    }
+    __syncthreads();
+    delta_put(&out->w, [&](int t, int d) { return *reinterpret_cast<const float2*>(&sm.w[t][d]); });
+}
+
+__device__ __forceinline__ void stmatrix_x4_trans(void* p, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};\n" ::"r"(smem_u32(p)), "r"(r0), "r"(r1),
+                 "r"(r2), "r"(r3) : "memory");
+}
+
+#define DB_LD (DC + 8)              // bfloat16 row stride of the columns in shared memory
+
+// Columns of a 64-row matrix in three parts as the second operand: [part][column][row]
+template <int DN> struct DeltaColumns { bf16 v[3][DN][DB_LD]; };
+
+// 16 rows (tile mt) x DN columns of a product's layout (rows g, g + 8; columns 2 tq, + 1 of every 8) into the columns' parts
+template <int DN>
+__device__ __forceinline__ void delta_put_columns(DeltaColumns<DN>& c, const float (&x)[DN / 8][4], int mt, int lane) {
+#pragma unroll
+    for (int nt = 0; nt < DN / 8; nt += 2) {
+        uint32_t lo[2][3], hi[2][3];                         // rows g and g + 8 of the two tiles of eight columns
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            split3_pair(x[nt + j][0], x[nt + j][1], lo[j]);
+            split3_pair(x[nt + j][2], x[nt + j][3], hi[j]);
+        }
+        const int mi = lane >> 3, r8 = lane & 7;
+#pragma unroll
+        for (int p = 0; p < 3; ++p)
+            stmatrix_x4_trans(&c.v[p][(nt + (mi >> 1)) * 8 + r8][mt * 16 + (mi & 1) * 8], lo[0][p], hi[0][p], lo[1][p], hi[1][p]);
+    }
+}
+
+// acc[s] += (operand tile row: fa[part][kt]) x columns, sorted by size: s = 0 the leading parts, 2 the smallest products
+template <int DN>
+__device__ __forceinline__ void delta_product(float (&acc)[3][DN / 8][4], const uint4 (&fa)[3][4], const DeltaColumns<DN>& c, int kts, int lane) {
+    const int mi = lane >> 3, r8 = lane & 7;
+#pragma unroll
+    for (int kt = 0; kt < 4; ++kt) {
+        if (kt >= kts) continue;
+#pragma unroll
+        for (int nt = 0; nt < DN / 8; nt += 2) {
+            uint32_t fb[3][4];
+#pragma unroll
+            for (int p = 0; p < 3; ++p) ldmatrix_x4(fb[p], &c.v[p][(nt + (mi >> 1)) * 8 + r8][kt * 16 + (mi & 1) * 8]);
+#pragma unroll
+            for (int pa = 0; pa < 3; ++pa) {
+                const uint32_t f[4] = {fa[pa][kt].x, fa[pa][kt].y, fa[pa][kt].z, fa[pa][kt].w};
+#pragma unroll
+                for (int pb = 0; pa + pb < 3; ++pb) {
+                    mma_bf16(acc[pa + pb][nt], f, fb[pb][0], fb[pb][1]);
+                    mma_bf16(acc[pa + pb][nt + 1], f, fb[pb][2], fb[pb][3]);
+                }
+            }
+        }
+    }
+}
+__device__ __forceinline__ void delta_fetch(uint4 (&f)[3][4], const DeltaOperand& x, int mt, int lane, int kts) {
+#pragma unroll
+    for (int p = 0; p < 3; ++p)
+#pragma unroll
+        for (int kt = 0; kt < 4; ++kt)
+            if (kt < kts) f[p][kt] = x.v[p][mt][kt][lane];
+}
+
+// named barriers: of the carry's four warps (128 threads), and between them and the read-outs' four (256: one side arrives and
+// goes on, the other waits)
+__device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+#define DB_CARRY 1
+#define DB_STATE 2                  // + turn: S before a chunk is there
+#define DB_U 4                      // + turn: u of a chunk is there
+#define DB_FREE 6                   // + turn: a chunk's read-outs are made, its buffers may be filled again
+
+template <int DN>
+__global__ void __launch_bounds__(256) delta_carry_kernel(const DeltaArgs a) {
+    constexpr int NT = DN / 8;
+    extern __shared__ __align__(16) unsigned char delta_raw[];
+    DeltaColumns<DN>* ss = reinterpret_cast<DeltaColumns<DN>*>(delta_raw);    // [2] S before the chunk, by turns
+    DeltaColumns<DN>* su = ss + 2;                                            // [2] u
+    pdl_trigger();
+    pdl_wait();
+    const int seq = blockIdx.z, h = blockIdx.y, v0 = blockIdx.x * DN;
+    const int r0 = a.cu_q[seq], rows = a.cu_q[seq + 1] - r0;
+    if (rows < a.min_rows) return;
+    int first = 0;
+    for (int s = 0; s < seq; ++s) {
+        const int n = a.cu_q[s + 1] - a.cu_q[s];
+        if (n >= a.min_rows) first += (n + DC - 1) / DC;
+    }
+    const int nc = (rows + DC - 1) / DC;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, mt = warp & 3, g = lane >> 2, tq = lane & 3;
+    const DeltaChunk* ch = a.chunks + (size_t)first * a.H + h;
+    const int D = a.D, V = a.V;
+
+    if (warp >= 4) {                                         // ---- the read-outs
+        uint4 fq[3][4], fp[3][4];
+        delta_fetch(fq, ch->q, mt, lane, 4);
+        delta_fetch(fp, ch->p, mt, lane, mt + 1);
+        for (int c = 0; c < nc; ++c) {
+            float acc[3][NT][4] = {};
+            bar_sync(DB_STATE + (c & 1), 256);
+            delta_product<DN>(acc, fq, ss[c & 1], 4, lane);
+            ch += a.H;
+            if (c + 1 < nc) delta_fetch(fq, ch->q, mt, lane, 4);
+            bar_sync(DB_U + (c & 1), 256);
+            delta_product<DN>(acc, fp, su[c & 1], mt + 1, lane);
+            if (c + 2 < nc) bar_arrive(DB_FREE + (c & 1), 256);
+            if (c + 1 < nc) delta_fetch(fp, ch->p, mt, lane, mt + 1);
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int t = c * DC + mt * 16 + g + 8 * half;
+                if (t >= rows) continue;
+                float* o = a.o + ((size_t)(r0 + t) * a.H + h) * V;
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) {
+                    const int col = v0 + nt * 8 + 2 * tq;
+                    const float y0 = acc[0][nt][2 * half] + (acc[1][nt][2 * half] + acc[2][nt][2 * half]);
+                    const float y1 = acc[0][nt][2 * half + 1] + (acc[1][nt][2 * half + 1] + acc[2][nt][2 * half + 1]);
+                    if ((V & 1) == 0 && col < V) *reinterpret_cast<float2*>(o + col) = make_float2(y0, y1);
+                    else {
+                        if (col < V) o[col] = y0;
+                        if (col + 1 < V) o[col + 1] = y1;
+                    }
+                }
+            }
+        }
+        return;
+    }
+
+    // ---- u and the state: warp mt has rows 16 mt .. of both
+    const int slot = zai_checked_slot(a.slot_ids[seq], a.num_slots, a.status);
+    float* st = a.state + ((size_t)slot * a.H + h) * D * V;
+    float S[NT][4];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int d = mt * 16 + g + 8 * (e >> 1), col = v0 + nt * 8 + 2 * tq + (e & 1);
+            S[nt][e] = (d < D && col < V) ? st[(size_t)d * V + col] : 0.f;
+        }
+    const size_t u_step = (size_t)a.H * DC * a.VP;
+    const float* u0 = a.u0 + ((size_t)first * a.H + h) * DC * a.VP + (size_t)(mt * 16 + g) * a.VP + v0 + 2 * tq;
+    uint4 fw[3][4], fk[3][4];
+    float2 ua[NT], ub[NT];
+    float keep_a, keep_b;
+    auto fetch_u = [&]() {
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+            ua[nt] = *reinterpret_cast<const float2*>(u0 + nt * 8);
+            ub[nt] = *reinterpret_cast<const float2*>(u0 + (size_t)8 * a.VP + nt * 8);
+        }
+    };
+    delta_fetch(fw, ch->w, mt, lane, 4);
+    delta_fetch(fk, ch->k, mt, lane, 4);
+    fetch_u();
+    keep_a = ch->keep[mt * 16 + g];
+    keep_b = ch->keep[mt * 16 + g + 8];
+    delta_put_columns<DN>(ss[0], S, mt, lane);
+    bar_arrive(DB_STATE, 256);
+    for (int c = 0; c < nc; ++c) {
+        const bool more = c + 1 < nc;
+        bar_sync(DB_CARRY, 128);                             // S before chunk c is there
+        float x[NT][4];
+        {
+            float acc[3][NT][4] = {};
+            delta_product<DN>(acc, fw, ss[c & 1], 4, lane);
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+                x[nt][0] = ua[nt].x - (acc[0][nt][0] + (acc[1][nt][0] + acc[2][nt][0]));
+                x[nt][1] = ua[nt].y - (acc[0][nt][1] + (acc[1][nt][1] + acc[2][nt][1]));
+                x[nt][2] = ub[nt].x - (acc[0][nt][2] + (acc[1][nt][2] + acc[2][nt][2]));
+                x[nt][3] = ub[nt].y - (acc[0][nt][3] + (acc[1][nt][3] + acc[2][nt][3]));
+            }
+        }
+        delta_put_columns<DN>(su[c & 1], x, mt, lane);
+        bar_arrive(DB_U + (c & 1), 256);
+        ch += a.H;
+        u0 += u_step;
+        if (more) {
+            delta_fetch(fw, ch->w, mt, lane, 4);
+            fetch_u();
+        }
+        bar_sync(DB_CARRY, 128);                             // u of chunk c is there
+        {
+            float acc[3][NT][4] = {};
+            delta_product<DN>(acc, fk, su[c & 1], 4, lane);
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    S[nt][e] = fmaf(e < 2 ? keep_a : keep_b, S[nt][e], acc[0][nt][e] + (acc[1][nt][e] + acc[2][nt][e]));
+        }
+        if (more) {
+            if (c > 0) bar_sync(DB_FREE + ((c + 1) & 1), 256);       // (chunk c - 1's, whose turn chunk c + 1 has)
+            delta_put_columns<DN>(ss[(c + 1) & 1], S, mt, lane);
+            bar_arrive(DB_STATE + ((c + 1) & 1), 256);
+            delta_fetch(fk, ch->k, mt, lane, 4);
+            keep_a = ch->keep[mt * 16 + g];
+            keep_b = ch->keep[mt * 16 + g + 8];
+        }
+    }
+    if (a.write_state) {
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int d = mt * 16 + g + 8 * (e >> 1), col = v0 + nt * 8 + 2 * tq + (e & 1);
+                if (d < D && col < V) st[(size_t)d * V + col] = S[nt][e];
+            }
+    }
+}
+
+template <int DN>
+static int delta_carry(const DeltaArgs& a, cudaStream_t stream) {
+    constexpr size_t smem = 4 * sizeof(DeltaColumns<DN>);
+    static unsigned long long done = 0;
+    if (zai_first_on_device(&done)) {
+        const cudaError_t e = cudaFuncSetAttribute(delta_carry_kernel<DN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+    }
+    return launch_pdl(delta_carry_kernel<DN>, dim3((a.V + DN - 1) / DN, a.H, a.n_seqs), dim3(256), smem, stream, a);
+}
+
+ZAI_API int zai_gated_delta_chunk_rows() { return DC; }
+ZAI_API int zai_gated_delta_chunked_supports(int D, int V) { return D >= 1 && D <= DCD && V >= 1 && V <= 65535 * 16; }
+// bytes of scratch a chunk and head takes
+ZAI_API int zai_gated_delta_chunk_bytes(int V) { return (int)(sizeof(DeltaChunk) + (size_t)DC * ((V + 31) & ~31) * sizeof(float)); }
+
+// o_out [N, H V] 32-bit and the state of every span of min_rows rows or more, bfloat16, in chunks.  scratch: max_chunks x H x
+// zai_gated_delta_chunk_bytes(V) bytes, on a boundary of 16; rows / DC + n_seqs chunks are always enough.  `channel`: a decay per
+// head and key channel (a and dt_bias H D wide).
+ZAI_API int zai_gated_delta_chunked(float* o_out, const void* qkv, int qkv_stride, const void* b_in, int b_stride, const void* a_in,
+                                    int a_stride, const float* a_log, const float* dt_bias, float unit_eps, float* state, const int* cu_q,
+                                    const int* slot_ids, int num_slots, int* status, int n_seqs, int H, int G, int D, int V, int channel,
+                                    int write_state, int min_rows, void* scratch, int max_chunks, cudaStream_t stream) {
+    if (n_seqs <= 0 || max_chunks <= 0) return ZAI_OK;
+    if (H < 1 || H > 65535 || n_seqs > 65535 || G < 1 || H % G || !zai_gated_delta_chunked_supports(D, V)) return ZAI_BAD_SIZE;
+    DeltaChunk* chunks = (DeltaChunk*)scratch;
+    const DeltaArgs a = {(const bf16*)qkv, (const bf16*)b_in, (const bf16*)a_in, qkv_stride, b_stride, a_stride, a_log, dt_bias, unit_eps,
+                         state, cu_q, slot_ids, status, num_slots, n_seqs, H, G, D, V, write_state, min_rows < 1 ? 1 : min_rows,
+                         chunks, (float*)(chunks + (size_t)max_chunks * H), (V + 31) & ~31, o_out};
+    static unsigned long long done = 0;
+    if (zai_first_on_device(&done)) {
+        cudaError_t e = cudaFuncSetAttribute(delta_chunk_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DeltaShared));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DeltaShared));
+        if (e != cudaSuccess) return (int)e;
+    }
+    const int rc = channel ? launch_pdl(delta_chunk_kernel<true>, dim3(max_chunks, H), dim3(256), sizeof(DeltaShared), stream, a)
+                           : launch_pdl(delta_chunk_kernel<false>, dim3(max_chunks, H), dim3(256), sizeof(DeltaShared), stream, a);
+    if (rc) return rc;
+    // 16 columns a block while that leaves no SM with two, else 32 (half the operand loads a column)
+    if ((V + 15) / 16 * H <= 148) return delta_carry<16>(a, stream);
+    return delta_carry<32>(a, stream);
 }

@@ -75,8 +75,12 @@ _SIGNATURES = {
                                               _I, _P, _I, _P]},
     "min_gru": {"zai_min_gru": [_P, _P, _I, _I, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _I, _I, _P]},
     "gated_delta": {
-        "zai_delta_prepare": [_P, _P, _P, _P, _I, _P, _I, _P, _I, _I, _P, _P, _I, _I, _I, _I, _F, _P],
-        "zai_gated_delta": [_P, _P, _P, _P, _P, _I, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P],
+        "zai_delta_prepare": [_P, _P, _P, _P, _I, _P, _I, _P, _I, _I, _P, _P, _I, _I, _I, _I, _F, _P, _P, _I, _P],
+        "zai_gated_delta": [_P, _P, _P, _P, _P, _I, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _I, _P],
+        "zai_gated_delta_chunk_rows": [],
+        "zai_gated_delta_chunked_supports": [_I, _I],
+        "zai_gated_delta_chunk_bytes": [_I],
+        "zai_gated_delta_chunked": [_P, _P, _I, _P, _I, _P, _I, _P, _P, _F, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _I, _P],
         "zai_gated_rmsnorm": [_P, _P, _P, _P, _I, _I, _F, _I, _I, _I, _I, _P],
         "zai_gated_delta_single_supports": [_I, _I],
         "zai_gated_delta_single": [_P, _P, _I, _P, _I, _P, _I, _P, _I, _I, _P, _P, _P, _F, _F, _P, _P, _I, _I, _I, _I, _I, _I, _I,
@@ -1274,6 +1278,14 @@ def _scan_chunks(step, n_rows, channel_blocks=16):
     return chunk, n_rows // chunk + step.n_seqs
 
 
+def _span_kinds(step, cut):
+    """Whether a step has spans of `cut` rows or more, and whether it has shorter ones.  A captured step shape is replayed with
+    other spans than it was captured with (it launches a bound of its attention tiles, `attn_tiles`): it may have both."""
+    if getattr(step, "attn_tiles", None) or not step.q_lens:
+        return step.n_tokens >= cut, True
+    return max(step.q_lens) >= cut, any(0 < n < cut for n in step.q_lens)
+
+
 def _rows_view(x):
     """(pointer, row stride) of a 2-D tensor whose rows are contiguous (a column slice of a wider matrix)."""
     if x.dim() != 2 or x.stride(1) != 1 or not x.is_cuda:
@@ -1345,13 +1357,46 @@ def min_gru(zxg, b_z, b_x, state, step, write_state=True):
     return out
 
 
+# Microseconds that the delta rule's kernels take (measured at 16 and 32 heads of 64 x 128): the walk 12 and 0.25 for every row of
+# its longest span, or 0.0040 for every row and head together where many requests fill the chip; the chunks' kernels 20 and 0.0040
+# a row and head.  2048 rows of 16 heads: one span 480 (walk) and 136 (chunks), eight spans 129 and 136; of 32 heads 580 and
+# 233, 260 and 244.
+DELTA_WALK, DELTA_CHUNKS = (12.0, 0.25, 0.0040), (20.0, 0.0040)
+DELTA_CHUNKED_LEAST = 64
+
+
+def _delta_cut(step, n_rows, load):
+    """The rows from which on a step's spans run in chunks: the choice that the figures above make the quickest.  `load`: heads,
+    in units of 128 values.  A captured step shape is replayed with other spans than it has now: there a span goes in chunks if
+    walking it takes longer than the whole step in chunks, which is no slower whatever the other spans are."""
+    fixed, by_row, by_load = DELTA_WALK
+    if getattr(step, "attn_tiles", None) or not step.q_lens:
+        return max(DELTA_CHUNKED_LEAST, int((DELTA_CHUNKS[0] + DELTA_CHUNKS[1] * n_rows * load) / by_row))
+    lens = sorted(step.q_lens, reverse=True)
+    best, cut, rows = None, 1 << 30, 0
+    for i in range(len(lens) + 1):
+        # the first i spans in chunks, the others walked
+        left = lens[i] if i < len(lens) else 0
+        if i == 0 or lens[i - 1] != left:
+            us = (DELTA_CHUNKS[0] + DELTA_CHUNKS[1] * rows * load) if i else 0.0
+            if left:
+                us += fixed + max(by_row * left, by_load * (n_rows - rows) * load)
+            if best is None or us < best:
+                best, cut = us, (lens[i - 1] if i else 1 << 30)
+        if left < DELTA_CHUNKED_LEAST:
+            break
+        rows += left
+    return cut
+
+
 @_timed("recurrence")
 def gated_delta(qkv, b, a, gate, a_log, dt_bias, norm_w, eps, state, step, heads, kv_heads, dim, vdim, write_state=True,
-                unit_eps=1e-6, channel_decay=False, gate_act="silu"):
+                unit_eps=1e-6, channel_decay=False, gate_act="silu", impl=None):
     """The gated delta rule over the rows of a step.  qkv [N, 2 G D + H V] (q heads, k heads, v heads, after their
     convolutions), b [N, H], a [N, H] (with `channel_decay` [N, H D]: a decay per head and key channel, `dt_bias` as wide),
     gate [N, H V] (column slices are fine), state [slots, H, D, V] 32-bit.
-    Returns rms(o) * norm_w * act(gate) per head (`gate_act`: silu or sigmoid), [N, H V] in qkv's dtype."""
+    Returns rms(o) * norm_w * act(gate) per head (`gate_act`: silu or sigmoid), [N, H V] in qkv's dtype.
+    `impl` "walk" or "chunks" picks the kernels for spans whatever their length."""
     _cuda(a_log, dt_bias, norm_w, state)
     N = qkv.shape[0]
     H, G, D, V = int(heads), int(kv_heads), int(dim), int(vdim)
@@ -1375,17 +1420,30 @@ def gated_delta(qkv, b, a, gate, a_log, dt_bias, norm_w, eps, state, step, heads
             float(unit_eps), _ptr(state), _ptr(step.slot_ids), N, H, G, D, V, int(bool(write_state)), state.shape[0],
             _status_ptr(dev), ch, act, _stream()), "gated_delta_single")
         return out
-    qk = torch.empty((N, 2, G, D), dtype=torch.float32, device=dev)
-    bg = torch.empty((N, 2, H), dtype=torch.float32, device=dev)
-    gch = torch.empty((N, H, D), dtype=torch.float32, device=dev) if ch else None
     o = torch.empty((N, H * V), dtype=torch.float32, device=dev)
     out = torch.empty((N, H * V), dtype=qkv.dtype, device=dev)
-    _check(_fn(lib, "zai_delta_prepare")(_ptr(qk), _ptr(bg), _ptr(gch), qp, qs, bp, bs, ap, as_, _dt(qkv), _ptr(a_log), _ptr(dt_bias),
-                                         N, H, G, D, float(unit_eps), _stream()), "delta_prepare")
-    vp = qp + 2 * G * D * qkv.element_size()
-    _check(_fn(lib, "zai_gated_delta")(_ptr(o), _ptr(qk), _ptr(bg), _ptr(gch), vp, qs, _dt(qkv), _ptr(state), _ptr(step.cu_q),
-                                       _ptr(step.slot_ids), N, step.n_seqs, H, G, D, V, int(bool(write_state)), state.shape[0],
-                                       _status_ptr(dev), _stream()), "gated_delta")
+    cut = 1 << 30                                              # (spans of that many rows or more run in chunks, the others are walked)
+    if impl != "walk" and not step.decode_only and qkv.dtype == torch.bfloat16 and _fn(lib, "zai_gated_delta_chunked_supports")(D, V):
+        cut = 1 if impl == "chunks" else _delta_cut(step, N, H * V / 128)
+    long, short = _span_kinds(step, cut)
+    if long:
+        max_chunks = N // _fn(lib, "zai_gated_delta_chunk_rows")() + step.n_seqs
+        scratch = torch.empty(max_chunks * H * _fn(lib, "zai_gated_delta_chunk_bytes")(V), dtype=torch.uint8, device=dev)
+        _check(_fn(lib, "zai_gated_delta_chunked")(
+            _ptr(o), qp, qs, bp, bs, ap, as_, _ptr(a_log), _ptr(dt_bias), float(unit_eps), _ptr(state), _ptr(step.cu_q), _ptr(step.slot_ids),
+            state.shape[0], _status_ptr(dev), step.n_seqs, H, G, D, V, ch, int(bool(write_state)), cut, _ptr(scratch), max_chunks,
+            _stream()), "gated_delta_chunked", 2)
+    if short and cut > 1:
+        qk = torch.empty((N, 2, G, D), dtype=torch.float32, device=dev)
+        bg = torch.empty((N, 2, H), dtype=torch.float32, device=dev)
+        gch = torch.empty((N, H, D), dtype=torch.float32, device=dev) if ch else None
+        _check(_fn(lib, "zai_delta_prepare")(_ptr(qk), _ptr(bg), _ptr(gch), qp, qs, bp, bs, ap, as_, _dt(qkv), _ptr(a_log), _ptr(dt_bias),
+                                             N, H, G, D, float(unit_eps), _ptr(step.cu_q), _ptr(step.seq_idx) if long else None, cut - 1,
+                                             _stream()), "delta_prepare")
+        vp = qp + 2 * G * D * qkv.element_size()
+        _check(_fn(lib, "zai_gated_delta")(_ptr(o), _ptr(qk), _ptr(bg), _ptr(gch), vp, qs, _dt(qkv), _ptr(state), _ptr(step.cu_q),
+                                           _ptr(step.slot_ids), N, step.n_seqs, H, G, D, V, int(bool(write_state)), state.shape[0],
+                                           _status_ptr(dev), cut - 1, _stream()), "gated_delta")
     _check(_fn(lib, "zai_gated_rmsnorm")(_ptr(out), _ptr(o), _ptr(norm_w), gp, gs, _dt(qkv), float(eps), N, H, V, act, _stream()),
            "gated_rmsnorm")
     return out
@@ -1839,14 +1897,6 @@ def mamba2(y, at, conv_w, conv_b, dt_bias, a_log, d_skip, norm_w, eps, norm_part
 # 0.25 us a row, the three kernels over chunks 25 to 30 us up to a thousand rows.  One request alone, heads of 64 x 128: 48 rows
 # 26 (walk) and 34 us (chunks), 64 rows 30 and 32, 128 rows 46 and 32; 16 requests of 32 rows 33 and 45, of 64 rows 50 and 43.
 MLSTM_CHUNKED_MIN = 64
-
-
-def _span_kinds(step, cut):
-    """Whether a step has spans of `cut` rows or more, and whether it has shorter ones.  A captured step shape is replayed with
-    other spans than it was captured with (it launches a bound of its attention tiles, `attn_tiles`): it may have both."""
-    if getattr(step, "attn_tiles", None) or not step.q_lens:
-        return step.n_tokens >= cut, True
-    return max(step.q_lens) >= cut, any(0 < n < cut for n in step.q_lens)
 
 
 @_timed("recurrence")
