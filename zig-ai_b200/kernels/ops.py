@@ -1357,11 +1357,11 @@ def min_gru(zxg, b_z, b_x, state, step, write_state=True):
     return out
 
 
-# Microseconds that the delta rule's kernels take (measured at 16 and 32 heads of 64 x 128): the walk 12 and 0.25 for every row of
-# its longest span, or 0.0040 for every row and head together where many requests fill the chip; the chunks' kernels 20 and 0.0040
-# a row and head.  2048 rows of 16 heads: one span 480 (walk) and 136 (chunks), eight spans 129 and 136; of 32 heads 580 and
-# 233, 260 and 244.
-DELTA_WALK, DELTA_CHUNKS = (12.0, 0.25, 0.0040), (20.0, 0.0040)
+# Microseconds that the delta rule's kernels take (16 and 32 heads of 64 x 128): the walk 12 and 0.28 for every row of its longest
+# span, or 0.0040 for every row and head together where many requests fill the chip; the chunks' kernels 25 and 0.0036 a row and
+# head, rows in 64s.  2048 rows of 16 heads: one span 480 (walk) and 136 (chunks), four spans 168 and 138, eight spans 129
+# and 137; of 32 heads 580 and 233, 261 and 239, 261 and 245; eight spans of 160 rows of 16 heads 90 and 106.
+DELTA_WALK, DELTA_CHUNKS = (12.0, 0.28, 0.0040), (25.0, 0.0036)
 DELTA_CHUNKED_LEAST = 64
 
 
@@ -1373,12 +1373,12 @@ def _delta_cut(step, n_rows, load):
     if getattr(step, "attn_tiles", None) or not step.q_lens:
         return max(DELTA_CHUNKED_LEAST, int((DELTA_CHUNKS[0] + DELTA_CHUNKS[1] * n_rows * load) / by_row))
     lens = sorted(step.q_lens, reverse=True)
-    best, cut, rows = None, 1 << 30, 0
+    best, cut, rows, padded = None, 1 << 30, 0, 0
     for i in range(len(lens) + 1):
         # the first i spans in chunks, the others walked
         left = lens[i] if i < len(lens) else 0
         if i == 0 or lens[i - 1] != left:
-            us = (DELTA_CHUNKS[0] + DELTA_CHUNKS[1] * rows * load) if i else 0.0
+            us = (DELTA_CHUNKS[0] + DELTA_CHUNKS[1] * padded * load) if i else 0.0
             if left:
                 us += fixed + max(by_row * left, by_load * (n_rows - rows) * load)
             if best is None or us < best:
@@ -1386,6 +1386,7 @@ def _delta_cut(step, n_rows, load):
         if left < DELTA_CHUNKED_LEAST:
             break
         rows += left
+        padded += -(-left // 64) * 64
     return cut
 
 
