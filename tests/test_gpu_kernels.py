@@ -929,3 +929,24 @@ def test_qk_norm_rope_many_rows(Hq, Hkv, D, ps, qk_norm):
     assert torch.allclose(ka.float(), kb.float(), **tol(dtype))
     assert torch.allclose(pages_a.float(), pages_b.float(), **tol(dtype))
     assert pages_a[0].abs().sum() == 0 and o.read_status() == 0
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("Hq,Hkv,D", [(4, 2, 64), (3, 3, 24), (6, 2, 100), (32, 1, 12), (33, 1, 20), (5, 1, 128), (2, 1, 1)])
+def test_attention_in_tiles_of_rows(dtype, Hq, Hkv, D):
+    """Spans around the tiles' edges (32 pairs of row and head, 64 keys) in the general path, against its kernel of one warp a row."""
+    o = ops()
+    g = torch.Generator().manual_seed(31)
+    ps = 16
+    bias, sink = torch.randn(19, Hq, generator=g).cuda(), torch.randn(Hq, generator=g).cuda()
+    for ctx, q_lens in (([0, 63, 64, 65, 200], [16, 17, 1, 33, 130]), ([0, 0, 5, 300], [1, 2, 64, 1]), ([127, 1000], [65, 3])):
+        num_pages = sum(-(-(c + n) // ps) for c, n in zip(ctx, q_lens)) + 8
+        step = make_step(o, dtype, ctx, q_lens, ps, num_pages, 9)
+        pages = torch.randn(num_pages, 2, Hkv, ps, D, generator=g).to(dtype).cuda()
+        q = torch.randn(sum(q_lens), Hq * D, generator=g).to(dtype).cuda()
+        view = CacheView(0, pages, step.block_tables[0], ps)
+        for opts in (dict(), dict(window=50), dict(chunk=48), dict(softcap=2.0, bias=bias, sink=sink), dict(window=70, keep_first=5), dict(window=9, keep_first=130)):
+            a = o.paged_attention(q, step, view, Hq, Hkv, D, D ** -0.5, impl=None, **opts)
+            b = o.paged_attention(q, step, view, Hq, Hkv, D, D ** -0.5, impl="general", **opts)
+            assert torch.allclose(a.float(), b.float(), **tol(dtype)), (ctx, sorted(opts), float((a.float() - b.float()).abs().max()))
+    assert o.read_status() == 0

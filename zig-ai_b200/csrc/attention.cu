@@ -1,5 +1,5 @@
-// Causal grouped-query attention over the paged cache, general kernel (any element type, head size,
-// page size, window): one warp per (row, query head).
+// Causal grouped-query attention over the paged cache, general kernels (any element type, head size, page size, window): one
+// warp per (row, query head), and for steps with spans of rows tiles of 32 (row, query head) pairs (further below).
 //
 //   s_j = q . k_j * scale  for cached positions j <= pos (and j > pos - window, or j in the chunk of pos), same request
 //   o   = sum_j softmax(s)_j v_j
@@ -98,6 +98,262 @@ __global__ void paged_attention_warp_kernel(T* __restrict__ out, const T* __rest
         const int d = lane + 32 * r;
         if (d < D) orow[d] = from_float<T>(acc[r] * inv);
     }
+}
+
+// ---- spans of rows: a block owns AT_M (row, query head) pairs of one key/value head and one request (neighbouring rows, the heads
+// that share the keys) and walks the keys in tiles of AT_N, 32-bit multiply-adds throughout.  A thread makes 4 pairs x 4 keys of the
+// scores (rows ty 4 .., keys tx + 16 j) and 4 pairs x DM / 16 columns of the output; the 16 threads of a row are neighbouring lanes,
+// so its maximum, sum and weights need no block barrier.  Key tiles start at multiples of AT_N whatever the span, so a row's result
+// does not depend on how the request was cut into steps or on its batch.
+//
+// What bounds it: 32-bit multiply-adds; eight 16-byte loads from shared memory feed 64 of them, and four blocks an SM (two at 128)
+// cover each other's loads and barriers.  A warp a row read every key and value from L2 once per row and head, keys by 32 lanes on
+// 32 rows at a time.  32-bit, 16 heads
+// of 64 over 8: 384 rows behind 128 positions 585 -> 64 us, 2048 rows 8585 -> 394 us (22 TFLOP/s of the about 70 of the units),
+// 2 rows behind 2000 positions 403 -> 150; 32 rows alone 18 -> 22 (the call's host time).
+#define AT_M 32
+#define AT_N 64
+
+template <int DM>
+struct AtTile {
+    static constexpr int LD = DM + 4;                        // (rows four banks apart)
+    float q[AT_M][LD], k[AT_N][LD], v[AT_N][LD], p[AT_M][AT_N + 4];
+    long long row[2][AT_N];                                  // where a tile's keys lie in the pages
+};
+
+// four neighbouring values of a row of D as 32-bit numbers, zeros beyond D; `vec`: D and the address are multiples of four
+__device__ __forceinline__ float4 at_four(const float* p, int d, int D, bool vec) {
+    if (vec && d < D) return *reinterpret_cast<const float4*>(p + d);
+    return make_float4(d < D ? p[d] : 0.f, d + 1 < D ? p[d + 1] : 0.f, d + 2 < D ? p[d + 2] : 0.f, d + 3 < D ? p[d + 3] : 0.f);
+}
+__device__ __forceinline__ float4 at_four(const bf16* p, int d, int D, bool vec) {
+    if (vec && d < D) {
+        const uint2 v = *reinterpret_cast<const uint2*>(p + d);
+        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x));
+        const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
+        return make_float4(a.x, a.y, b.x, b.y);
+    }
+    return make_float4(d < D ? to_float(p[d]) : 0.f, d + 1 < D ? to_float(p[d + 1]) : 0.f, d + 2 < D ? to_float(p[d + 2]) : 0.f,
+                       d + 3 < D ? to_float(p[d + 3]) : 0.f);
+}
+
+template <typename T, int DM, bool EXT>
+__global__ void __launch_bounds__(128) paged_attention_tile_kernel(
+    T* __restrict__ out, const T* __restrict__ q, const T* __restrict__ pages, const int* __restrict__ block_table, int table_width,
+    const int* __restrict__ positions, const int* __restrict__ cu_q, int n_seqs, int page_size, int Hq, int Hkv, int D, float scale,
+    int window, int num_pages, int* __restrict__ status, const ZaiScoreOptions opt) {
+    using Tile = AtTile<DM>;
+    constexpr int NC = DM / 16;                              // output columns of a thread: fours (twos) 64 (32) apart
+    extern __shared__ __align__(16) unsigned char at_raw[];
+    Tile& sm = *reinterpret_cast<Tile*>(at_raw);
+    pdl_trigger();
+    pdl_wait();
+    const int kvh = blockIdx.y, group = Hq / Hkv, rows_of = AT_M / group;
+    int seq = 0, r0 = 0, n_rows = 0, b = blockIdx.x;
+    for (; seq < n_seqs; ++seq) {
+        const int lo = cu_q[seq], len = cu_q[seq + 1] - lo, nt = (len + rows_of - 1) / rows_of;
+        if (b < nt) {
+            r0 = lo + b * rows_of;
+            n_rows = min(rows_of, lo + len - r0);
+            break;
+        }
+        b -= nt;
+    }
+    if (n_rows <= 0) return;
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, n_pairs = n_rows * group;
+    const ZaiTableRow table{block_table + (size_t)seq * table_width, table_width, num_pages, status};
+    const size_t page_stride = (size_t)2 * Hkv * page_size * D, v_off = (size_t)Hkv * page_size * D;
+    const bool vec = (D & 3) == 0 && ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(pages)) & (4 * sizeof(T) - 1)) == 0;
+    const int first_pos = positions[r0], last_pos = positions[r0 + n_rows - 1];
+    // a pair's query (scaled); pairs that do not exist are zeros
+    for (int i = tid; i < AT_M * (DM / 4); i += 128) {
+        const int p = i / (DM / 4), d = (i % (DM / 4)) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (p < n_pairs) v = at_four(q + ((size_t)(r0 + p / group) * Hq + kvh * group + p % group) * D, d, D, vec);
+        *reinterpret_cast<float4*>(&sm.q[p][d]) = make_float4(v.x * scale, v.y * scale, v.z * scale, v.w * scale);
+    }
+    int pos[4], from[4], kept[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int p = ty * 4 + i;
+        pos[i] = p < n_pairs ? first_pos + p / group : -1;   // (-1: sees no key)
+        from[i] = zai_first_visible(pos[i], window);
+        kept[i] = EXT && window > 0 ? min(opt.keep_first, from[i]) : 0;
+    }
+    // the tiles: those of the kept first positions, then from the first row's first visible one on
+    const int seen_from = zai_first_visible(first_pos, window), start = seen_from / AT_N * AT_N;
+    const int keep_end = EXT && window > 0 ? min(opt.keep_first, zai_first_visible(last_pos, window)) : 0;
+    const int n_kept = min((keep_end + AT_N - 1) / AT_N, start / AT_N), n_tiles = n_kept + (last_pos - start) / AT_N + 1;
+    auto base_of = [&](int n) { return n < n_kept ? n * AT_N : start + (n - n_kept) * AT_N; };
+    auto find_rows = [&](int n) {
+        if (tid < AT_N && n < n_tiles) {
+            const int j = base_of(n) + tid;
+            long long at = -1;                               // (no row sees it: zeros)
+            if (j <= last_pos && (j >= seen_from || j < keep_end)) at = (long long)((size_t)table.page(j / page_size) * page_stride + ((size_t)kvh * page_size + j % page_size) * D);
+            sm.row[n & 1][tid] = at;
+        }
+    };
+    float m[4], l[4], o[4][NC];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        m[i] = -INFINITY;
+        l[i] = 0.f;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) o[i][c] = 0.f;
+    }
+    find_rows(0);
+    for (int n = 0; n < n_tiles; ++n) {
+        __syncthreads();                                     // the tile before has been used; this one's rows are known
+#pragma unroll 4
+        for (int i = tid; i < AT_N * (DM / 4); i += 128) {
+            const int j = i / (DM / 4), d = (i % (DM / 4)) * 4;
+            const long long at = sm.row[n & 1][j];
+            float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), vv = kv;
+            if (at >= 0) {
+                kv = at_four(pages + at, d, D, vec);
+                vv = at_four(pages + at + v_off, d, D, vec);
+            }
+            *reinterpret_cast<float4*>(&sm.k[j][d]) = kv;
+            *reinterpret_cast<float4*>(&sm.v[j][d]) = vv;
+        }
+        find_rows(n + 1);
+        __syncthreads();
+        float s[4][4] = {};
+#pragma unroll 4
+        for (int d = 0; d < DM; d += 4) {
+            float4 a[4], k4[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(&sm.q[ty * 4 + i][d]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) k4[j] = *reinterpret_cast<const float4*>(&sm.k[tx + 16 * j][d]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) s[i][j] = fmaf(a[i].w, k4[j].w, fmaf(a[i].z, k4[j].z, fmaf(a[i].y, k4[j].y, fmaf(a[i].x, k4[j].x, s[i][j]))));
+        }
+        const int base = base_of(n);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float top = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int key = base + tx + 16 * j;
+                const bool seen = key <= pos[i] && (key >= from[i] || key < kept[i]);
+                if (EXT && seen) {
+                    if (opt.softcap > 0.f) s[i][j] = opt.softcap * tanhf(s[i][j] / opt.softcap);
+                    if (opt.bias) s[i][j] += opt.bias[(size_t)min(pos[i] - key, opt.bias_rows - 1) * Hq + kvh * group + (ty * 4 + i) % group];
+                }
+                if (!seen) s[i][j] = -INFINITY;
+                top = fmaxf(top, s[i][j]);
+            }
+#pragma unroll
+            for (int w = 8; w > 0; w >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, w));
+            const float m_new = fmaxf(m[i], top);
+            const float ref = m_new == -INFINITY ? 0.f : m_new;               // (no key of the row so far: weights of zero)
+            float sum = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float w = expf(s[i][j] - ref);
+                sm.p[ty * 4 + i][tx + 16 * j] = w;
+                sum += w;
+            }
+#pragma unroll
+            for (int w = 8; w > 0; w >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, w);
+            const float corr = expf(m[i] - ref);                              // m = -inf at first: 0
+            l[i] = l[i] * corr + sum;
+            m[i] = m_new;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) o[i][c] *= corr;
+        }
+        __syncwarp();                                        // (a row's weights come from its own 16 lanes)
+#pragma unroll 2
+        for (int j = 0; j < AT_N; j += 4) {
+            float4 w[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const float4*>(&sm.p[ty * 4 + i][j]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                float v[NC];
+                if constexpr (NC == 2) {
+                    const float2 x = *reinterpret_cast<const float2*>(&sm.v[j + e][tx * 2]);
+                    v[0] = x.x; v[1] = x.y;
+                } else {
+#pragma unroll
+                    for (int c = 0; c < NC; c += 4) {
+                        const float4 x = *reinterpret_cast<const float4*>(&sm.v[j + e][c * 16 + tx * 4]);
+                        v[c] = x.x; v[c + 1] = x.y; v[c + 2] = x.z; v[c + 3] = x.w;
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float p = e == 0 ? w[i].x : e == 1 ? w[i].y : e == 2 ? w[i].z : w[i].w;
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) o[i][c] = fmaf(p, v[c], o[i][c]);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int p = ty * 4 + i;
+        if (p >= n_pairs) continue;
+        const int h = kvh * group + p % group;
+        if (EXT && opt.sink) {                               // the sink: a term of the denominator alone
+            const float sk = opt.sink[h], m_new = fmaxf(m[i], sk), corr = expf(m[i] - m_new);
+            l[i] = l[i] * corr + expf(sk - m_new);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) o[i][c] *= corr;
+        }
+        const float inv = 1.f / l[i];
+        T* orow = out + ((size_t)(r0 + p / group) * Hq + h) * D;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const int d = NC == 2 ? tx * 2 + c : (c / 4) * 64 + tx * 4 + c % 4;
+            if (d < D) orow[d] = from_float<T>(o[i][c] * inv);
+        }
+    }
+}
+
+ZAI_API int zai_paged_attention_tiles_supports(int D, int Hq, int Hkv) { return D >= 1 && D <= 128 && Hkv >= 1 && Hq % Hkv == 0 && Hq / Hkv <= AT_M && Hkv <= 65535; }
+// rows of a tile: n_tiles of the launcher is the sum over the spans of their rows divided by this, rounded up (or more)
+ZAI_API int zai_paged_attention_tile_rows(int Hq, int Hkv) { return AT_M / (Hq / Hkv); }
+
+template <typename T, int DM, bool EXT>
+static int launch_tiles(void* out, const void* q, const void* pages, const int* block_table, int table_width, const int* positions,
+                        const int* cu_q, int n_seqs, int n_tiles, int page_size, int Hq, int Hkv, int D, float scale, int window,
+                        int num_pages, int* status, const ZaiScoreOptions& opt, cudaStream_t stream) {
+    static unsigned long long done = 0;
+    if (zai_first_on_device(&done)) {
+        const cudaError_t e = cudaFuncSetAttribute(paged_attention_tile_kernel<T, DM, EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AtTile<DM>));
+        if (e != cudaSuccess) return (int)e;
+    }
+    return launch_pdl(paged_attention_tile_kernel<T, DM, EXT>, dim3(n_tiles, Hkv), dim3(128), sizeof(AtTile<DM>), stream, (T*)out,
+                      (const T*)q, (const T*)pages, block_table, table_width, positions, cu_q, n_seqs, page_size, Hq, Hkv, D, scale,
+                      window, num_pages, status, opt);
+}
+
+// A step's spans in tiles of rows (positions of a span's rows follow one another); the score options as below, all off by zeros
+// and null pointers.
+ZAI_API int zai_paged_attention_tiles(void* out, const void* q, const void* pages, int dtype, const int* block_table, int table_width,
+                                      const int* positions, const int* cu_q, int n_seqs, int n_tiles, int page_size, int Hq, int Hkv,
+                                      int D, float scale, int window, int num_pages, int* status, float softcap, const float* bias,
+                                      int bias_rows, const float* sink, int keep_first, cudaStream_t stream) {
+    if (softcap < 0.f || (bias && bias_rows < 1) || keep_first < 0 || (keep_first && window <= 0)) return ZAI_BAD_SIZE;
+    if (n_tiles <= 0 || n_seqs <= 0) return ZAI_OK;
+    if (!zai_paged_attention_tiles_supports(D, Hq, Hkv)) return ZAI_BAD_SIZE;
+    const ZaiScoreOptions opt = {softcap, bias, bias_rows, sink, keep_first, scale};
+    const bool ext = softcap > 0.f || bias || sink || keep_first;
+#define ZAI_TILES(DM, EXT) ZAI_DISPATCH(dtype, return launch_tiles<T, DM, EXT>(out, q, pages, block_table, table_width, positions, cu_q, n_seqs, \
+        n_tiles, page_size, Hq, Hkv, D, scale, window, num_pages, status, opt, stream))
+    if (ext) {
+        if (D <= 32) ZAI_TILES(32, true);
+        if (D <= 64) ZAI_TILES(64, true);
+        ZAI_TILES(128, true);
+    }
+    if (D <= 32) ZAI_TILES(32, false);
+    if (D <= 64) ZAI_TILES(64, false);
+    ZAI_TILES(128, false);
+#undef ZAI_TILES
 }
 
 ZAI_API int zai_paged_attention_general(void* out, const void* q, const void* pages, int dtype, const int* block_table,

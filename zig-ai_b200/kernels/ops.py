@@ -97,6 +97,9 @@ _SIGNATURES = {
     },
     "attention": {
         "zai_paged_attention_general": [_P, _P, _P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _P, _P],
+        "zai_paged_attention_tiles_supports": [_I, _I, _I],
+        "zai_paged_attention_tile_rows": [_I, _I],
+        "zai_paged_attention_tiles": [_P, _P, _P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _F, _I, _I, _P, _F, _P, _I, _P, _I, _P],
         "zai_paged_attention_scored": [_P, _P, _P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _P, _F, _P, _I, _P, _I, _P],
     },
     "mlstm": {"zai_mlstm": [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P, _F, _P, _F, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I,
@@ -988,13 +991,29 @@ def _attention_tickets(device, n):
         _span_tickets[device] = t
     return t
 
+def _attention_tiles(out, q, step, cache, heads, kv_heads, head_dim, scale, window, shaped):
+    """Attention of a step with spans of rows in tiles of rows, 32-bit arithmetic; False if the sizes are not the kernel's, or in
+    steps of single tokens (a tile would hold one row's heads alone)."""
+    if step.decode_only or not _fn("attention", "zai_paged_attention_tiles_supports")(head_dim, heads, kv_heads):
+        return False
+    rows, n = _fn("attention", "zai_paged_attention_tile_rows")(heads, kv_heads), step.n_tokens
+    tiles = n // rows + step.n_seqs if getattr(step, "attn_tiles", None) or not step.q_lens else sum(-(-x // rows) for x in step.q_lens)
+    bt = cache.block_table
+    _check(_fn("attention", "zai_paged_attention_tiles")(
+        _ptr(out), _ptr(q), _ptr(cache.pages), _dt(q), _ptr(bt), bt.shape[1], _ptr(step.positions), _ptr(step.cu_q), step.n_seqs, tiles,
+        cache.page_size, heads, kv_heads, head_dim, float(scale), int(window or 0), cache.pages.shape[0], _status_ptr(q.device), *shaped,
+        _stream()), "paged_attention (tiles)")
+    return True
+
+
 @_timed("attention")
 def paged_attention(q, step, cache, heads, kv_heads, head_dim, scale, window=None, impl=None, chunk=None, softcap=None, bias=None,
                     sink=None, keep_first=0):
     """Causal attention of the step's rows over their requests' pages.  bfloat16 runs on the
     tensor cores (a split-key kernel when every span is one token, else the flash-style kernel)
-    for the head sizes those kernels have; everything else, and `impl="general"`, runs the
-    general kernel.  `impl="mma"` / `impl="tcgen05"` pick between the two span kernels.
+    for the head sizes those kernels have; everything else runs
+    the general kernels in 32-bit arithmetic: spans of rows in tiles of rows (head sizes up to 128), single tokens and
+    `impl="general"` with one warp a row and head.  `impl="mma"` / `impl="tcgen05"` pick between the two span kernels.
     `window`: a query sees the last `window` positions; `chunk`: it sees back to the start of its chunk of that
     many positions (the kernels take the chunk as a negative window).
     Shaped scores (the general kernel): `softcap` (s <- cap tanh(s / cap)), `bias` [distances, heads] 32-bit (added after the
@@ -1038,6 +1057,8 @@ def paged_attention(q, step, cache, heads, kv_heads, head_dim, scale, window=Non
                 _ptr(out), _ptr(q), _ptr(cache.pages), _ptr(bt[ns:]), bt.shape[1], _ptr(step.cu_q[ns:]), _ptr(step.ctx_lens[ns:]),
                 step.n_seqs - ns, n_tiles, cache.page_size, heads, kv_heads, head_dim, float(scale), int(window or 0),
                 cache.pages.shape[0], _status_ptr(q.device), *shaped, _stream()), "prefill attention (scored)")
+            return out
+        if impl != "general" and _attention_tiles(out, q, step, cache, heads, kv_heads, head_dim, scale, window, shaped):
             return out
         _check(_fn("attention", "zai_paged_attention_scored")(
             _ptr(out), _ptr(q), _ptr(cache.pages), _dt(q), _ptr(bt), bt.shape[1], _ptr(step.positions), _ptr(step.seq_idx),
@@ -1101,6 +1122,8 @@ def paged_attention(q, step, cache, heads, kv_heads, head_dim, scale, window=Non
                 _ptr(out), _ptr(q), _ptr(cache.pages), _ptr(bt), bt.shape[1], _ptr(cu_q), _ptr(ctx_lens),
                 S, n_tiles, cache.page_size, heads, kv_heads, head_dim, float(scale), int(window or 0),
                 cache.pages.shape[0], _status_ptr(q.device), _stream()), "prefill attention")
+        return out
+    if impl != "general" and _attention_tiles(out, q, step, cache, heads, kv_heads, head_dim, scale, window, (0.0, None, 0, None, 0)):
         return out
     _check(_fn("attention", "zai_paged_attention_general")(
         _ptr(out), _ptr(q), _ptr(cache.pages), _dt(q), _ptr(bt), bt.shape[1],
