@@ -335,3 +335,26 @@ def test_layer_norm_inside_the_few_rows_product(M, K, O):
         got = o.linear_clamped_glu(LazyNorm(res, delta, gamma, 1e-5, dt, beta=beta), w, O // 2, 0.8, 1.702)
         want = ref_ops.linear_clamped_glu(x_ref, w, O // 2, 0.8, 1.702)
         assert got.shape == (M, O // 2) and torch.allclose(got.float(), want.float(), atol=3e-2, rtol=3e-2)
+
+
+@pytest.mark.parametrize("H,R,Dr,ps", [(16, 256, 32, 64), (8, 256, 32, 16), (24, 128, 64, 8), (3, 64, 0, 128), (130, 192, 16, 32), (1, 256, 48, 64)])
+def test_latent_attention_in_tiles_of_pairs(H, R, Dr, ps):
+    """The tcgen05 kernel: tiles of 128 (row, head) pairs that end inside a row, spans of one row beside portions, cached rows
+    up to and just beyond a tile of 64, a sink that counts and one that takes nearly everything."""
+    o = ops()
+    g = torch.Generator().manual_seed(41)
+    dtype = torch.bfloat16
+    for ctx, q_lens in (([0, 63, 64, 65], [70, 1, 9, 130]), ([0, 300, 5], [1, 17, 64]), ([1000], [33]), ([0, 3], [16, 0])):
+        num_pages = sum(-(-(c + n) // ps) for c, n in zip(ctx, q_lens)) + 8
+        step = make_step(o, dtype, ctx, q_lens, ps, num_pages, 22)
+        pages = latent_pages(step, ctx, q_lens, ps, R + Dr, dtype, num_pages, g)
+        N = sum(q_lens)
+        q_lat = torch.randn(N, H, R, generator=g).to(dtype).cuda()
+        q_rot = torch.randn(N, H, Dr, generator=g).to(dtype).cuda()
+        view = CacheView(0, pages, step.block_tables[0], ps)
+        scale = (R + Dr) ** -0.5
+        for sink in (None, torch.randn(H, generator=g).cuda(), torch.full((H,), 30.0).cuda()):
+            a = o.latent_attention(q_lat, q_rot, step, view, H, R, Dr, scale, impl="tcgen05", sink=sink)
+            b = ref_ops.latent_attention(q_lat, q_rot, step, view, H, R, Dr, scale, sink=sink)
+            assert torch.allclose(a.float(), b.float(), **tol(dtype)), (ctx, sink is not None, float((a.float() - b.float()).abs().max()))
+    assert o.read_status() == 0

@@ -63,6 +63,11 @@ _SIGNATURES = {
         "zai_latent_attention_mma_supports": [_I, _I],
         "zai_latent_attention_mma": [_P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P, _P],
     },
+    "latent_attention_tc": {
+        "zai_latent_attention_tc_supports": [_I, _I, _I, _I],
+        "zai_latent_attention_tc_pairs": [],
+        "zai_latent_attention_tc": [_P, _P, _P, _P, _I, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _P, _P],
+    },
     "activation": {"zai_silu_mul": [_P, _P, _I, _I, _I, _P],
                    "zai_clamped_glu": [_P, _P, _I, _I, _I, _F, _F, _P],
                    "zai_act_mul": [_P, _P, _I, _I, _I, _I, _P],
@@ -203,7 +208,7 @@ def _check(code: int, what: str, n: int = 1) -> None:
 CORE_LIBS = ("embed", "norm", "activation", "rope_kv")
 BF16_LIBS = ("decode_gemm",)
 # libraries that a part may name and only a bfloat16 model uses
-BF16_ONLY = ("gemm_tc", "gemm_tc_pair", "stream_gemm", "attention_mma", "attention_tma", "attention_tc")
+BF16_ONLY = ("gemm_tc", "gemm_tc_pair", "stream_gemm", "attention_mma", "attention_tma", "attention_tc", "latent_attention_tc")
 ATTENTION_LIBS = ("attention", "attention_mma", "attention_tma", "attention_tc")
 
 
@@ -1590,6 +1595,11 @@ def latent_prepare(q, dkv, norm_w, eps, table, step, cache, heads, dim, rot_dim,
     return q_rot
 
 
+# From this many rows x groups of 16 heads on, steps with portions run latent attention in tiles of 128 (row, head) pairs on tcgen05:
+# a tile walks its keys at 29 us a thousand whatever the step's size, and the mma.sync kernels take 0.3 us a row, group and thousand
+# keys.  16 heads: 32 rows behind 8000 positions 90 (mma.sync) and 234 us, 128 behind 4000 160 and 124, 512 behind 6000 902
+# and 191, 2048 alone 282 and 66; 16 single tokens and 20 rows behind 6000 87 and 178.
+LATENT_TC_ROWS = 112
 LATENT_SPLIT_KEYS = 256          # keys per range where a step's rows are too few to fill the device
 LATENT_WARPS_WANTED = 1024       # from this many warps (rows x groups of 16 heads x blocks of output columns) on, no ranges
 USE_LATENT_MMA = os.environ.get("ZAI_LATENT_MMA", "1") == "1"
@@ -1598,8 +1608,9 @@ USE_LATENT_MMA = os.environ.get("ZAI_LATENT_MMA", "1") == "1"
 @_timed("attention")
 def latent_attention(q_lat, q_rot, step, cache, heads, rank, rot_dim, scale, impl=None, sink=None):
     """Causal attention of every head against the cached rows [latent | rotated key part]: scores
-    (q_lat . latent + q_rot . key part) * scale, output sum_j p_j latent_j, [N, H, rank].  bfloat16 with a rank
-    that is a multiple of 32 and rank + rot_dim a multiple of 16 runs on the tensor cores (steps of many rows: the four
+    (q_lat . latent + q_rot . key part) * scale, output sum_j p_j latent_j, [N, H, rank].  bfloat16 steps with
+    many rows run on tcgen05 where the rank is a multiple of 64 up to 256 and rot_dim one of 16 up to 64 (`impl="tcgen05"` whatever
+    their size); else bfloat16 with a rank that is a multiple of 32 and rank + rot_dim a multiple of 16 runs on the tensor cores (steps of many rows: the four
     warps of a block share the tiles of cached rows; steps of few rows: a warp a row and range of keys, the ranges added
     up by a second kernel); everything else, and `impl="general"`, runs the general kernel.  `sink` [H] 32-bit: one more
     term exp(sink_h) in every row's denominator (no key, no value, not scaled)."""
@@ -1612,6 +1623,17 @@ def latent_attention(q_lat, q_rot, step, cache, heads, rank, rot_dim, scale, imp
     if N != step.n_tokens or pages.dtype != q_lat.dtype or tuple(pages.shape[1:]) != (cache.page_size, R + Dr):
         raise KernelError("latent_attention: operands do not fit together")
     out = torch.empty((N, H, R), dtype=q_lat.dtype, device=q_lat.device)
+    if (impl in (None, "tcgen05") and q_lat.dtype == torch.bfloat16 and not step.decode_only
+            and _fn("latent_attention_tc", "zai_latent_attention_tc_supports")(H, R, Dr, cache.page_size)):
+        if impl == "tcgen05" or N * -(-H // 16) >= LATENT_TC_ROWS:
+            pairs = _fn("latent_attention_tc", "zai_latent_attention_tc_pairs")()
+            captured = getattr(step, "attn_tiles", None) or not step.q_lens
+            tiles = N * H // pairs + step.n_seqs if captured else sum(-(-n * H // pairs) for n in step.q_lens)
+            _check(_fn("latent_attention_tc", "zai_latent_attention_tc")(
+                _ptr(out), _ptr(q_lat), _ptr(q_rot), _ptr(pages), pages.shape[0], _status_ptr(q_lat.device), _ptr(bt), bt.shape[1],
+                _ptr(step.cu_q), _ptr(step.ctx_lens), N, step.n_seqs, tiles, cache.page_size, H, R, Dr, float(scale), _ptr(sink),
+                _stream()), "latent_attention_tc")
+            return out
     if (impl != "general" and (USE_LATENT_MMA or impl in ("mma", "mma_rows", "mma_ranges")) and q_lat.dtype == torch.bfloat16
             and _fn("latent_attention", "zai_latent_attention_mma_supports")(R, Dr)):
         warps = N * (-(-H // 16)) * (-(-R // (128 if R <= 128 else 256)))

@@ -44,7 +44,7 @@ DEFAULT_NAMES = {"q": "attn_q.weight", "dkv": "attn_kv_down.weight", "dkv_norm":
 class LatentAttention(Mixer):
     accepts_lazy_input = True     # x goes straight into a product
     graph_safe = True             # forward launches kernels only; nothing is read back to the host
-    kernel_libs = ("latent_attention", "qkv_prepare")
+    kernel_libs = ("latent_attention", "latent_attention_tc", "qkv_prepare")      # (the second: bfloat16 only)
 
     def __init__(self, hidden: int, heads: int, dim: int, rot_dim: int, vdim: int, rank: int, scale: float, eps: float,
                  position: PartSpec, kv_proj: bool = True, gate="element", names=None, q_rank=None, sink: bool = False):
