@@ -129,6 +129,36 @@ def test_span_attention_few_rows_over_long_contexts(ps, window, padded):
     assert o.read_status() == 0
 
 
+@pytest.mark.parametrize("ps,opts", [(64, dict(softcap=2.0, bias=600, sink=True)), (16, dict(window=5000, keep_first=130, sink=True)),
+                                     (128, dict(softcap=30.0)), (32, dict(window=700, keep_first=65, bias=7168))])
+def test_shaped_span_attention_few_rows_over_long_contexts(ps, opts):
+    """Shared tiles with shaped scores: the kept first positions are tiles of the first shares, the sink counts once, a bias table
+    shorter than some contexts and longer than others; twice in a row.  A result is a weighted mean of values below 5.2: weights and
+    both results rounded to bfloat16, 3 * 2^-9 * 5.2."""
+    o = ops()
+    from zig_ai_b200.kernels import ops as ops_module
+    g = torch.Generator().manual_seed(75)
+    ctx, q_lens = [16000, 5, 700, 9000], [40, 3, 130, 2]
+    num_pages = sum(-(-(c + n) // ps) for c, n in zip(ctx, q_lens)) + 8
+    step = make_step(o, BF16, ctx, q_lens, ps, num_pages, 76)
+    pages = fill_pages(step, ctx, q_lens, ps, Hkv, D, BF16, num_pages, g).clamp(-5.2, 5.2)
+    q = torch.randn(sum(q_lens), Hq * D, generator=g).to(BF16).cuda()
+    opts = dict(opts)
+    if "bias" in opts:
+        opts["bias"] = (torch.randn(opts["bias"], Hq, generator=g) * 1.5).cuda()
+    if "sink" in opts:
+        opts["sink"] = (torch.randn(Hq, generator=g) * 2 + 4).cuda()
+    view = CacheView(0, pages, step.block_tables[0], ps)
+    n_tiles = sum(-(-n // 128) for n in q_lens)
+    assert ops_module._fn("attention_tc", "zai_prefill_attention_tc_shaped_splits")(n_tiles, Hq, step.block_tables[0].shape[1], ps) > 1
+    want = ref_ops.paged_attention(q, step, view, Hq, Hkv, D, D ** -0.5, **opts)
+    for _ in range(2):
+        got = o.paged_attention(q, step, view, Hq, Hkv, D, D ** -0.5, **opts)
+        assert torch.allclose(got.float(), want.float(), atol=3e-2, rtol=0), (got.float() - want.float()).abs().max()
+        assert int(ops_module._span_tickets[q.device].abs().sum()) == 0
+    assert o.read_status() == 0
+
+
 @pytest.mark.parametrize("tma", [True, False])
 @pytest.mark.parametrize("ps,window", [(64, None), (16, None), (64, 1500)])
 def test_decode_attention_batch_64_at_contexts_2048_to_4095(tma, ps, window):

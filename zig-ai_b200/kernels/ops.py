@@ -160,8 +160,10 @@ _SIGNATURES = {
     },
     "attention_tc": {
         "zai_prefill_attention_tc_supports": [_I, _I, _I, _I],
-        "zai_prefill_attention_tc": [_P, _P, _P, _I, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _P, _P, _P, _P],
+        "zai_prefill_attention_tc": [_P, _P, _P, _I, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _P, _P, _P, _F, _P, _I, _P, _I, _P],
         "zai_prefill_attention_tc_splits": [_I, _I, _I, _I],
+        "zai_prefill_attention_tc_shaped_splits": [_I, _I, _I, _I],
+        "zai_prefill_attention_tc_max_bias": [],
     },
     "sampling": {
         "zai_argmax": [_P, _P, _I, _I, _P, _P],
@@ -996,6 +998,18 @@ def _attention_tickets(device, n):
         _span_tickets[device] = t
     return t
 
+
+def _attention_splits(device, n_tiles, heads, bt, page_size, shaped=False):
+    """How many blocks share a tile of query rows' keys, and the scratch for it.  Few tiles over long contexts: several blocks share
+    a tile's keys and leave their parts in scratch, the last to finish combines them (tickets: zero before and after)."""
+    splits = _fn("attention_tc", f"zai_prefill_attention_tc{'_shaped' if shaped else ''}_splits")(n_tiles, heads, bt.shape[1], page_size)
+    tickets = _attention_tickets(device, n_tiles * heads if splits > 1 else 0)   # (made at the first call, which no graph captures)
+    if splits <= 1:
+        return splits, None, None, tickets
+    parts = torch.empty((n_tiles * heads * splits * (64 + 2), 128), dtype=torch.float32, device=device)      # one allocation: O's parts, then references and sums
+    return splits, parts, parts[n_tiles * heads * splits * 64:], tickets
+
+
 def _attention_tiles(out, q, step, cache, heads, kv_heads, head_dim, scale, window, shaped):
     """Attention of a step with spans of rows in tiles of rows, 32-bit arithmetic; False if the sizes are not the kernel's, or in
     steps of single tokens (a tile would hold one row's heads alone)."""
@@ -1058,6 +1072,17 @@ def paged_attention(q, step, cache, heads, kv_heads, head_dim, scale, window=Non
                 single_tokens(ns)
             block_rows = _fn("attention_mma", "zai_prefill_block_rows")()
             n_tiles = (step.attn_tiles - ns) if getattr(step, "attn_tiles", None) else sum(-(-n // block_rows) for n in step.q_lens[ns:])
+            # head size 64 on tcgen05 at every size: 8 x 100 rows behind 500 positions with 16 heads of 64 are the one form found where the
+            # walk by mma.sync is level (41 us to 43), long contexts gain most (684 to 100, 32 rows behind 16 384).  TMA wants 16 bytes.
+            if (impl != "mma" and (USE_TC_ATTENTION or impl == "tcgen05") and not (q.data_ptr() | out.data_ptr() | cache.pages.data_ptr()) & 15
+                    and _fn("attention_tc", "zai_prefill_attention_tc_supports")(head_dim, heads, kv_heads, cache.page_size)
+                    and (bias is None or bias.shape[0] <= _fn("attention_tc", "zai_prefill_attention_tc_max_bias")())):
+                splits, part_o, part_ml, tickets = _attention_splits(q.device, n_tiles, heads, bt[ns:], cache.page_size, shaped=True)
+                _check(_fn("attention_tc", "zai_prefill_attention_tc")(
+                    _ptr(out), _ptr(q), _ptr(cache.pages), cache.pages.shape[0], _status_ptr(q.device), _ptr(bt[ns:]), bt.shape[1],
+                    _ptr(step.cu_q[ns:]), _ptr(step.ctx_lens[ns:]), N, step.n_seqs - ns, n_tiles, cache.page_size, heads, kv_heads, head_dim,
+                    float(scale), int(window or 0), splits, _ptr(part_o), _ptr(part_ml), _ptr(tickets), *shaped, _stream()), "prefill attention (tcgen05, scored)")
+                return out
             _check(_fn("attention_mma", "zai_prefill_attention_mma_scored")(
                 _ptr(out), _ptr(q), _ptr(cache.pages), _ptr(bt[ns:]), bt.shape[1], _ptr(step.cu_q[ns:]), _ptr(step.ctx_lens[ns:]),
                 step.n_seqs - ns, n_tiles, cache.page_size, heads, kv_heads, head_dim, float(scale), int(window or 0),
@@ -1109,19 +1134,12 @@ def paged_attention(q, step, cache, heads, kv_heads, head_dim, scale, window=Non
             n_tiles = (step.attn_tiles - ns) if getattr(step, "attn_tiles", None) else sum(-(-n // block_rows) for n in step.q_lens[ns:])
             if (impl != "mma" and (USE_TC_ATTENTION or impl == "tcgen05") and q.is_contiguous()
                     and _fn("attention_tc", "zai_prefill_attention_tc_supports")(head_dim, heads, kv_heads, cache.page_size)):
-                # few tiles of query rows over long contexts: several blocks share a tile's keys and leave their
-                # parts in scratch, the last to finish combines them (tickets: zero before and after)
-                splits = _fn("attention_tc", "zai_prefill_attention_tc_splits")(n_tiles, heads, bt.shape[1], cache.page_size)
-                part_o = part_ml = None
-                tickets = _attention_tickets(q.device, n_tiles * heads if splits > 1 else 0)   # (made at the first call, which no graph captures)
-                if splits > 1:
-                    part_o = torch.empty((n_tiles * heads * splits, 64 * 128), dtype=torch.float32, device=q.device)
-                    part_ml = torch.empty((n_tiles * heads * splits, 2 * 128), dtype=torch.float32, device=q.device)
+                splits, part_o, part_ml, tickets = _attention_splits(q.device, n_tiles, heads, bt, cache.page_size)
                 _check(_fn("attention_tc", "zai_prefill_attention_tc")(
                     _ptr(out), _ptr(q), _ptr(cache.pages), cache.pages.shape[0], _status_ptr(q.device), _ptr(bt), bt.shape[1],
                     _ptr(cu_q), _ptr(ctx_lens), N, S, n_tiles, cache.page_size, heads, kv_heads,
                     head_dim, float(scale), int(window or 0), splits, _ptr(part_o), _ptr(part_ml), _ptr(tickets),
-                    _stream()), "prefill attention (tcgen05)")
+                    0.0, None, 0, None, 0, _stream()), "prefill attention (tcgen05)")
                 return out
             _check(_fn("attention_mma", "zai_prefill_attention_mma")(
                 _ptr(out), _ptr(q), _ptr(cache.pages), _ptr(bt), bt.shape[1], _ptr(cu_q), _ptr(ctx_lens),
