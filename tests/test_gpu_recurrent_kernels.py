@@ -238,3 +238,28 @@ def test_gated_delta_in_chunks(H, G, D, V, channel):
     o.gated_delta(qkv, b, a, gate, a_log, dt_bias, norm_w, 1e-5, state_a, step, H, G, D, V, False, impl="chunks", **more)
     assert torch.equal(state_a, keep)
     assert o.read_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("V,H,stride,off", [(32, 3, 4, 0), (64, 5, 8, 0), (128, 1, 0, 0), (256, 3, 4, 0), (128, 3, 2, 0), (64, 3, 4, 1), (48, 3, 0, 0)])
+def test_gated_rmsnorm_in_fours_and_one_by_one(dtype, V, H, stride, off):
+    """Head sizes that are read four columns a load, with rows on and off such a load's boundary, and one that is not; item counts that
+    fill no block.  32-bit sums of V terms: 1e-5; bfloat16 results round at 2^-9."""
+    from zig_ai_b200.kernels import ops as o
+    o.require(extra=("gated_delta",))
+    g = torch.Generator().manual_seed(V + H)
+    for N, with_w, act in ((1, True, 0), (37, False, 1), (130, True, 0)):
+        x = torch.randn(N, H, V, generator=g).cuda()
+        w = (1 + 0.1 * torch.randn(V, generator=g)).cuda() if with_w else None
+        gs = H * V + stride
+        gate = torch.randn(N * gs + off, generator=g).to(dtype).cuda()[off:]
+        out = torch.empty(N, H, V, dtype=dtype, device="cuda")
+        code = o._fn("gated_delta", "zai_gated_rmsnorm")(out.data_ptr(), x.data_ptr(), o._ptr(w), gate.data_ptr(), gs, o._dt(out), 1e-5, N, H, V, act,
+                                                          o._stream())
+        assert code == 0
+        gv = gate.view(N, gs)[:, :H * V].reshape(N, H, V).double()
+        s = torch.sigmoid(gv)
+        want = x.double() * torch.rsqrt((x.double() ** 2).mean(-1, keepdim=True) + 1e-5) * (w.double() if with_w else 1) * (s if act else gv * s)
+        bound = 1e-5 if dtype is torch.float32 else 2.0 ** -8
+        assert ((out.double() - want).abs() <= bound * (want.abs() + 1e-3)).all()
+    assert o.read_status() == 0
