@@ -229,7 +229,7 @@ __global__ void gated_rmsnorm_kernel(T* __restrict__ out, const float* __restric
 
 // The same for head sizes 4 L R: L lanes an item, four neighbouring columns a lane and load (R times), all of them asked for before the
 // sum.  What bounds it is memory (8 bytes a column in bfloat16); with one column a lane and load the warps waited for loads one after
-// another: a whole delta layer, 2048 rows 226 -> 224 us, a mixed step of 1280 rows 271 -> 267.
+// another: 2048 rows of 32 heads of 128 25.5 -> 19.3 us, of 64 22.2 -> 10.8; of a delta layer of 2048 rows 226 -> 224.
 template <typename T>
 __device__ __forceinline__ void delta_four(const T* p, float (&v)[4]) {
     if (sizeof(T) == 4) {
