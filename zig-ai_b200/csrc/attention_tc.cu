@@ -77,8 +77,8 @@ struct AtArgs {
     ZaiScoreOptions opt;        // (shaped scores)
 };
 
-// tanh without a branch: the Taylor series up to x^9 below 0.3 (the next term is under 6e-8 of it there), 1 - 2 / (1 + e^2x) beyond
-// (a relative error of 4e-7 at most).  The library's tanhf branches at 0.55, which a warp of mixed scores takes both ways.
+// tanh without a branch, so that a warp of mixed scores takes one way: the Taylor series up to x^9 below 0.3 (the next term is under
+// 6e-8 of it there), the identity 1 - 2 / (1 + e^2x) beyond (a relative error of 4e-7 at most).
 __device__ __forceinline__ float at_tanh(float x) {
     const float q = x * x;
     const float small = fmaf(x * q, fmaf(q, fmaf(q, fmaf(q, 62.f / 2835.f, -17.f / 315.f), 2.f / 15.f), -1.f / 3.f), x);
