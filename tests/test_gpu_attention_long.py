@@ -238,3 +238,54 @@ def test_planted_keys_at_every_edge_other_head_sizes(dtype, heads, kv_heads, hea
         tol = dict(atol=2e-4, rtol=2e-4) if dtype == torch.float32 else dict(atol=3e-2, rtol=3e-2)
         assert want.float().abs().max() > 5.0
         assert torch.allclose(got.float(), want.float(), **tol), (q_lens, (got.float() - want.float()).abs().max())
+
+
+FORMS = [dict(), dict(window=100), dict(chunk=96), dict(softcap=20.0, bias=300, sink=True), dict(window=90, keep_first=70, sink=True)]
+
+
+@pytest.mark.parametrize("ps", [16, 64, 128])
+@pytest.mark.parametrize("form", range(len(FORMS)))
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_span_attention_and_values_that_are_not_finite(ps, form, bad):
+    """A page's last owner may have left anything behind: what no row sees (unused ends of pages, the null page, positions before
+    every row's window) does not change a result, and a value that some rows see does not reach the rows that don't."""
+    o = ops()
+    g = torch.Generator().manual_seed(77)
+    opts = dict(FORMS[form])
+    if "bias" in opts:
+        opts["bias"] = torch.randn(opts["bias"], Hq, generator=g).cuda()
+    if "sink" in opts:
+        opts["sink"] = torch.randn(Hq, generator=g).cuda()
+    impl = "tcgen05"
+    for ctx, q_lens in (([0, 300, 5], [200, 130, 3]), ([6000], [40]), ([61, 0], [64, 128])):
+        num_pages = sum(-(-(c + n) // ps) for c, n in zip(ctx, q_lens)) + 8
+        step = make_step(o, BF16, ctx, q_lens, ps, num_pages, 78)
+        clean = fill_pages(step, ctx, q_lens, ps, Hkv, D, BF16, num_pages, torch.Generator().manual_seed(79), junk=0.0)
+        dirty = fill_pages(step, ctx, q_lens, ps, Hkv, D, BF16, num_pages, torch.Generator().manual_seed(79), junk=bad)
+        q = torch.randn(sum(q_lens), Hq * D, generator=g).to(BF16).cuda()
+
+        def run(pages):
+            return o.paged_attention(q, step, CacheView(0, pages, step.block_tables[0], ps), Hq, Hkv, D, D ** -0.5, impl=impl, **opts)
+        want = run(clean)
+        assert torch.isfinite(want).all()
+        assert torch.equal(run(dirty), want), (ctx, q_lens)
+        # one value of one key/value head of request 0, at positions that rows behind them see and rows before them don't
+        kv, col, n, c = 3, 17, q_lens[0], ctx[0]
+        for p in sorted({c, c + 1, c + n // 2, c + n - 1, c + 63 if n > 63 else c, max(c - 90, 0), max(c - 130, 0)}):
+            pages = dirty.clone()
+            pages[int(step.block_tables[0][0, p // ps]), 1, kv, p % ps, col] = bad
+            pos = torch.arange(c, c + n)
+            if "window" in opts:
+                lo = (pos - opts["window"] + 1).clamp(min=0)
+            elif "chunk" in opts:
+                lo = pos // opts["chunk"] * opts["chunk"]
+            else:
+                lo = torch.zeros_like(pos)
+            sees = (p <= pos) & ((p >= lo) | (p < opts.get("keep_first", 0)))
+            hit = torch.zeros(sum(q_lens), Hq, D, dtype=torch.bool)
+            hit[:n, kv * G:(kv + 1) * G, col] = sees[:, None]
+            hit = hit.view(-1, Hq * D).cuda()
+            got = run(pages)
+            assert not torch.isfinite(got[hit]).any(), (ctx, p)
+            assert torch.equal(got[~hit], want[~hit]), (ctx, p)
+    assert o.read_status() == 0

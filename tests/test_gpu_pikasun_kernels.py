@@ -358,3 +358,37 @@ def test_latent_attention_in_tiles_of_pairs(H, R, Dr, ps):
             b = ref_ops.latent_attention(q_lat, q_rot, step, view, H, R, Dr, scale, sink=sink)
             assert torch.allclose(a.float(), b.float(), **tol(dtype)), (ctx, sink is not None, float((a.float() - b.float()).abs().max()))
     assert o.read_status() == 0
+
+
+@pytest.mark.parametrize("H,R,Dr,ps", [(16, 256, 32, 64), (8, 128, 32, 16), (1, 64, 0, 128), (40, 192, 64, 32)])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_latent_attention_and_rows_that_are_not_finite(H, R, Dr, ps, bad):
+    """What a page's last owner left behind a request's last position (or in the null page) does not change a result, and a cached
+    row that some rows of the step see does not reach the rows before it."""
+    o = ops()
+    g = torch.Generator().manual_seed(43)
+    dtype = torch.bfloat16
+    for ctx, q_lens in (([0, 63, 64], [70, 1, 130]), ([300], [17]), ([61], [67])):
+        num_pages = sum(-(-(c + n) // ps) for c, n in zip(ctx, q_lens)) + 8
+        step = make_step(o, dtype, ctx, q_lens, ps, num_pages, 22)
+        clean = latent_pages(step, ctx, q_lens, ps, R + Dr, dtype, num_pages, g)
+        dirty = torch.where(clean == 60.0, torch.full_like(clean, bad), clean)
+        N = sum(q_lens)
+        q_lat = torch.randn(N, H, R, generator=g).to(dtype).cuda()
+        q_rot = torch.randn(N, H, Dr, generator=g).to(dtype).cuda()
+        sink = torch.randn(H, generator=g).cuda()
+
+        def run(pages):
+            return o.latent_attention(q_lat, q_rot, step, CacheView(0, pages, step.block_tables[0], ps), H, R, Dr, (R + Dr) ** -0.5,
+                                      impl="tcgen05", sink=sink)
+        want = run(clean)
+        assert torch.isfinite(want).all()
+        assert torch.equal(run(dirty), want), (ctx, q_lens)
+        c, n = ctx[0], q_lens[0]
+        for r in (0, 1, n // 2, n - 1):
+            pages = dirty.clone()
+            pages[int(step.block_tables[0][0, (c + r) // ps]), (c + r) % ps] = bad
+            got = run(pages)
+            assert not torch.isfinite(got[r:n]).any(), (ctx, r)
+            assert torch.equal(got[:r], want[:r]) and torch.equal(got[n:], want[n:]), (ctx, r)
+    assert o.read_status() == 0

@@ -57,6 +57,7 @@
 #define AT_TMEM_COLS 256                              // two score buffers in columns 0..127, O in 128..191, two P buffers in 192..255
 #define AT_COL_O (2 * AT_BN)
 #define AT_COL_P (2 * AT_BN + AT_D)
+#define AT_HIDDEN_BYTES 1600                          // AtHidden<AT_D>
 
 struct AtArgs {
     bf16* out;                  // [rows of the step, Hq, 64]
@@ -109,10 +110,13 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
     int& s_seq = words[1];
     int& s_i0 = words[2];
     float* exch = reinterpret_cast<float*>(words + 4);          // [2][2][128]: a tile's maxima by half, by turns; then the sums
-    float* bias = exch + 4 * AT_BM;                             // [bias_rows] the head's bias by distance
+    AtHidden<AT_D>& hid = *reinterpret_cast<AtHidden<AT_D>*>(exch + 4 * AT_BM);
+    float* bias = exch + 4 * AT_BM + AT_HIDDEN_BYTES / 4;       // [bias_rows] the head's bias by distance
     volatile int* failed = &failed_flag;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
+    if (tid < AT_D)
+        for (int t = 0; t < 3; ++t) hid.clear(t, tid, AT_D);
     if (tid == 0) {
         failed_flag = (at_smem(base) & 1023u) ? 1 : 0;          // the swizzled tiles need 1024-byte alignment
         at_mbar_init(&q_full, 1);
@@ -162,6 +166,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
     }
     // the softmax threads' state, kept past the roles for a shared tile's combination
     float m = -INFINITY, l = 0.f;                               // m: the row's reference, in units of the scores
+    uint32_t nans = 0;                                          // which of the thread's 32 columns have met a value that is not finite
     bool have_o = false;                                        // the row's O in TMEM is complete
     int row0 = 0, rows = 0;
     if (s < a.S && !failed_flag) {
@@ -284,12 +289,36 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
             const uint32_t tS = tmem_base + ((uint32_t)(qd * 32) << 16) + half * 32, tO = tS + AT_COL_O, tP = tmem_base + ((uint32_t)(qd * 32) << 16) + AT_COL_P + half * 16;
             const float c = SHAPED ? 1.f : a.scale_log2;        // (shaped scores are made in the exponent's units)
             const float unit = SHAPED && a.opt.softcap > 0.f ? a.opt.scale / a.opt.softcap : 0.f, cap = a.opt.softcap * 1.4426950408889634f;
+            // (a key is hidden from some row of the block if it lies behind the first row, or before the last row's first one and is not kept)
+            const int keep = SHAPED && a.window > 0 ? a.opt.keep_first : 0, klast = zai_first_visible(kend - 1, a.window);
+            int turn3 = 0;
             bool alive = true;
             for (int i = 0; i < n_tiles; ++i) {
                 const int key0 = key_of(i) + half * 32;
                 if (alive && !at_mbar_wait_warp(&s_ready[i & 1], (i >> 1) & 1, failed)) alive = false;      // (the warp together)
                 const uint32_t tSi = tS + (i & 1) * AT_BN, tPi = tP + (i & 1) * (AT_BN / 2);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const int tile_key = key_of(i);
+                if (tile_key + AT_BN - 1 > ctx + i0 || (tile_key < klast && tile_key + AT_BN > keep)) {
+                    const int st = i % STAGES;
+                    hid.clear(turn3 == 2 ? 0 : turn3 + 1, tid - 64, 256);            // (all have left the tile that used it)
+                    if (alive && !at_mbar_wait_warp(&kv_full[st], (i / STAGES) & 1, failed)) alive = false;    // (long since there)
+                    if (alive) {
+                        unsigned char* values = sKV + (size_t)st * AT_KV_BYTES + AT_KV_BYTES / 2;
+                        for (int e = tid - 64; e < AT_BN * 8; e += 256) {
+                            const int key = tile_key + (e >> 3);
+                            hid.clean(values, e, 0, key >= kend || (key < kbeg && key >= keep), turn3);
+                        }
+                        at_proxy_fence();
+                    }
+                    asm volatile("bar.sync 6, 256;" ::: "memory");
+                    if (hid.any[turn3]) {
+                        const unsigned long long sees = (at_below(qpos + 1 - tile_key) & ~at_below(klo - tile_key)) | at_below(kept - tile_key);
+                        for (int j = 0; j < 32; ++j)
+                            if (hid.keys[turn3][half * 32 + j] & sees) nans |= 1u << j;
+                    }
+                    turn3 = turn3 == 2 ? 0 : turn3 + 1;
+                }
                 // keys of this half that the row sees: [lo, hi), and those below `first`
                 const int lo = valid ? max(klo - key0, 0) : 32, hi = valid ? min(qpos + 1 - key0, 32) : 0;
                 const int first = valid ? kept - key0 : 0;
@@ -406,6 +435,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
                 if (!SHARED) {
                     uint32_t r[32];
                     at_tmem_ld32(tO, r);
+                    if (nans) at_put_nans(r, nans);
                     if (valid) {
 #pragma unroll
                         for (int d = 0; d < 32; d += 8) {
@@ -438,6 +468,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
         if (ok) {
             uint32_t r[32];
             at_tmem_ld32(tO, r);
+            if (nans) at_put_nans(r, nans);
 #pragma unroll
             for (int j = 0; j < 32; ++j) po[j * AT_BM + row] = __uint_as_float(r[j]);
         }
@@ -562,7 +593,8 @@ ZAI_API int zai_prefill_attention_tc(void* out, const void* q, const void* pages
     while ((1 << a.page_shift) < page_size) ++a.page_shift;
     const bool shaped = softcap > 0.f || bias || sink || keep_first > 0;
     a.opt = {softcap, bias, bias_rows, sink, keep_first, scale};
-    constexpr size_t words = 256 + 4 * AT_BM * sizeof(float);
+    constexpr size_t words = 256 + 4 * AT_BM * sizeof(float) + AT_HIDDEN_BYTES;
+    static_assert(sizeof(AtHidden<AT_D>) <= AT_HIDDEN_BYTES && AT_HIDDEN_BYTES % 16 == 0, "the notes fit");
     constexpr size_t smem = AT_Q_BYTES + (size_t)AT_STAGES * AT_KV_BYTES + words;
     constexpr size_t smem_shaped = AT_Q_BYTES + (size_t)AT_SHAPED_STAGES * AT_KV_BYTES + words;
     static_assert(2 * (smem + 1024) <= 233472 && 2 * (smem_shaped + AT_MAX_BIAS * sizeof(float) + 1024) <= 233472, "two blocks an SM");

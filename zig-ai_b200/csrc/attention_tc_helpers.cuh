@@ -111,6 +111,53 @@ __device__ __forceinline__ void at_tmem_wait_ld(uint32_t (&r)[32]) {
                  :: "memory");
 }
 
+// ---- values that some rows of a block do not see.  A tile's hidden keys have weights of exactly zero, but zero times NaN or
+// infinity is NaN in the product: a recycled page's last owner, or a later row of the span, would reach every row of the block.  So
+// in tiles that some row sees a part of, before their product, the softmax threads put zeros over the values that no row sees, and take
+// what is not finite out of the others: AtHidden notes it by column and key, and a row that sees such a key ends as NaN in that
+// column.  Zeros and notes are generic writes: at_proxy_fence() orders them before the product's reads (asynchronous proxy).
+__device__ __forceinline__ void at_proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+// eight bfloat16 values: is one of them infinite or NaN (an exponent of ones)?
+__device__ __forceinline__ bool at_not_finite(const uint4& v) {
+    auto two = [](uint32_t x) { return ((x & 0x7f807f80u) + 0x00800080u) & 0x80008000u; };
+    return (two(v.x) | two(v.y) | two(v.z) | two(v.w)) != 0;
+}
+// the lowest n of 64 bits
+__device__ __forceinline__ unsigned long long at_below(int n) { return n <= 0 ? 0ull : n >= 64 ? ~0ull : (1ull << n) - 1; }
+template <int COLS>
+struct AtHidden {                                               // three tiles' notes, by turns
+    unsigned long long keys[3][COLS];                           // a column's keys of the tile whose value is not finite
+    int any[3];
+    __device__ __forceinline__ void clear(int turn, int tid, int threads) {
+        for (int c = tid; c < COLS; c += threads) keys[turn][c] = 0;
+        if (tid == 0) any[turn] = 0;
+    }
+    // 16 bytes of a tile's values (swizzled rows of 128 bytes; `chunk` counts 16 bytes from the tile's first row; columns from
+    // `col0`): zeros if no row sees the key, else without what is not finite
+    __device__ __forceinline__ void clean(unsigned char* tile, int chunk, int col0, bool hidden, int turn) {
+        uint4* p = reinterpret_cast<uint4*>(tile) + chunk;
+        if (hidden) {
+            *p = make_uint4(0u, 0u, 0u, 0u);
+            return;
+        }
+        if (!at_not_finite(*p)) return;
+        const int key = chunk >> 3, c0 = col0 + ((chunk & 7) ^ (key & 7)) * 8;
+        unsigned short* v = reinterpret_cast<unsigned short*>(p);
+        for (int e = 0; e < 8; ++e)
+            if ((v[e] & 0x7f80) == 0x7f80) {
+                v[e] = 0;
+                atomicOr(&keys[turn][c0 + e], 1ull << key);
+            }
+        any[turn] = 1;
+    }
+};
+
+__device__ __forceinline__ void at_put_nans(uint32_t (&r)[32], uint32_t which) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+        if (which >> j & 1) r[j] = 0x7fc00000u;
+}
+
 // ------------------------------------------------------------------------------------------ host side
 typedef CUresult (*AtEncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                     const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,

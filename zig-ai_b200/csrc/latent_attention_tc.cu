@@ -75,9 +75,13 @@ __global__ void __launch_bounds__(LT_THREADS) latent_attention_tc_kernel(const _
     int& failed_flag = words[0];
     int& s_seq = words[1];
     int& s_i0 = words[2];
+    AtHidden<LT_MAX_R>& hid = *reinterpret_cast<AtHidden<LT_MAX_R>*>(words + 4);
+    uint32_t* nans = reinterpret_cast<uint32_t*>(&hid + 1);     // [8][LT_BM] the columns of a pair that have met a value that is not finite
     volatile int* failed = &failed_flag;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
+    for (int t = 0; t < 3; ++t) hid.clear(t, tid, LT_THREADS);
+    for (int i = tid; i < LT_MAX_R / 32 * LT_BM; i += LT_THREADS) nans[i] = 0;
     if (tid == 0) {
         failed_flag = (at_smem(smem_raw) & 1023u) ? 1 : 0;      // the swizzled tiles need 1024-byte alignment
         at_mbar_init(&q_full, 1);
@@ -204,11 +208,34 @@ __global__ void __launch_bounds__(LT_THREADS) latent_attention_tc_kernel(const _
             const uint32_t tS = tmem_base + ((uint32_t)(qd * 32) << 16), tO = tS + LT_COL_O, tP = tS + LT_COL_P;
             const float c = a.scale_log2;
             float m = -INFINITY, l = 0.f;                       // m: the pair's reference, in units of the scores
-            bool alive = true;
-            for (int i = 0; i < n_tiles && alive; ++i) {
-                if (!at_mbar_wait_warp(&s_ready[i & 1], (i >> 1) & 1, failed)) { alive = false; break; }    // (the warp leaves together)
+            int turn3 = 0;
+            bool alive = true, bad = false;
+            for (int i = 0; i < n_tiles; ++i) {
+                if (alive && !at_mbar_wait_warp(&s_ready[i & 1], (i >> 1) & 1, failed)) alive = false;      // (the warp together)
                 const uint32_t tSi = tS + (i & 1) * LT_BN, tPi = tP + (i & 1) * (LT_BN / 2);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (i * LT_BN + LT_BN - 1 > ctx + i0 / a.H) {   // some pair sees a part of this tile (a warp that has given up takes part)
+                    const int st = i % LT_STAGES;
+                    hid.clear(turn3 == 2 ? 0 : turn3 + 1, tid - 64, LT_BM);           // (all have left the tile that used it)
+                    if (alive && !at_mbar_wait_warp(&kv_full[st], (i / LT_STAGES) & 1, failed)) alive = false;    // (long since there)
+                    if (alive) {
+                        unsigned char* rows = sKV + (size_t)st * kv_bytes;           // (as keys they have been used: the scores are there)
+                        for (int e = tid - 64; e < n_lat * LT_BN * 8; e += LT_BM) {
+                            const int b = e / (LT_BN * 8), chunk = e % (LT_BN * 8);
+                            hid.clean(rows + (size_t)b * LT_K_BLOCK, chunk, b * 64, i * LT_BN + (chunk >> 3) >= kend, turn3);
+                        }
+                        at_proxy_fence();
+                    }
+                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                    if (hid.any[turn3]) {
+                        bad = true;
+                        const unsigned long long sees = at_below(qpos + 1 - i * LT_BN);
+                        for (int c = 0; c < a.R; ++c)
+                            if (hid.keys[turn3][c] & sees) nans[(c >> 5) * LT_BM + row] |= 1u << (c & 31);
+                    }
+                    turn3 = turn3 == 2 ? 0 : turn3 + 1;
+                }
+                if (!alive) continue;                           // (the other warps' barriers still count on this one)
                 const int hi = valid ? min(qpos + 1 - i * LT_BN, LT_BN) : 0;      // keys of this tile that the pair sees: below hi
                 const bool full = hi >= LT_BN;
                 // the pair's 64 scores: their maximum, their weights against the reference into P, the weights' sum
@@ -236,7 +263,7 @@ __global__ void __launch_bounds__(LT_THREADS) latent_attention_tc_kernel(const _
                     m = mx;
                 }
                 if (i > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
-                    if (!at_mbar_wait_warp(&o_ready[(i - 1) & 1], ((i - 1) >> 1) & 1, failed)) { alive = false; break; }   // the product before has added to O
+                    if (!at_mbar_wait_warp(&o_ready[(i - 1) & 1], ((i - 1) >> 1) & 1, failed)) { alive = false; continue; }   // the product before has added to O
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     for (int c0 = 0; c0 < a.R; c0 += 32) {
                         uint32_t o[32];
@@ -282,6 +309,7 @@ __global__ void __launch_bounds__(LT_THREADS) latent_attention_tc_kernel(const _
                 for (int c0 = 0; c0 < a.R; c0 += 32) {
                     uint32_t o[32];
                     at_tmem_ld32(tO + c0, o);
+                    if (bad) at_put_nans(o, nans[(c0 >> 5) * LT_BM + row]);
                     if (valid) {
 #pragma unroll
                         for (int d = 0; d < 32; d += 8) {
@@ -339,11 +367,13 @@ ZAI_API int zai_latent_attention_tc(void* out, const void* q_lat, const void* q_
     a.page_shift = 0;
     while ((1 << a.page_shift) < page_size) ++a.page_shift;
     const int n_blocks = R / 64 + (Dr > 0 ? 1 : 0);
-    const size_t smem = (size_t)n_blocks * (LT_Q_BLOCK + LT_STAGES * LT_K_BLOCK) + 256;
+    constexpr size_t words = 256 + sizeof(AtHidden<LT_MAX_R>) + LT_MAX_R / 32 * LT_BM * sizeof(uint32_t);
+    static_assert(LT_MAX_BLOCKS * (LT_Q_BLOCK + LT_STAGES * LT_K_BLOCK) + words <= 227 * 1024, "one block an SM");
+    const size_t smem = (size_t)n_blocks * (LT_Q_BLOCK + LT_STAGES * LT_K_BLOCK) + words;
     static unsigned long long configured = 0;
     if (zai_first_on_device(&configured)) {
         const cudaError_t err = cudaFuncSetAttribute(latent_attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     LT_MAX_BLOCKS * (LT_Q_BLOCK + LT_STAGES * LT_K_BLOCK) + 256);
+                                                     (int)(LT_MAX_BLOCKS * (LT_Q_BLOCK + LT_STAGES * LT_K_BLOCK) + words));
         if (err != cudaSuccess) return (int)err;
     }
     return launch_pdl(latent_attention_tc_kernel, dim3(n_tiles), dim3(LT_THREADS), smem, stream, ml, mr, mkv, a);
