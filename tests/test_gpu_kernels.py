@@ -950,3 +950,31 @@ def test_attention_in_tiles_of_rows(dtype, Hq, Hkv, D):
             b = o.paged_attention(q, step, view, Hq, Hkv, D, D ** -0.5, impl="general", **opts)
             assert torch.allclose(a.float(), b.float(), **tol(dtype)), (ctx, sorted(opts), float((a.float() - b.float()).abs().max()))
     assert o.read_status() == 0
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("Hq,Hkv,D", [(6, 2, 100), (4, 2, 64), (3, 3, 24)])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_attention_in_tiles_and_values_that_are_not_finite(dtype, Hq, Hkv, D, bad):
+    """A value that some rows of a tile see does not reach the rows that don't: not finite where the kernel of one warp a row is not, the
+    same elsewhere as with a clean value."""
+    if dtype == torch.bfloat16 and D == 64:
+        pytest.skip("a head size of the tensor-core kernels")
+    o = ops()
+    g = torch.Generator().manual_seed(33)
+    ps, ctx, q_lens = 16, [0, 63, 200], [70, 33, 130]
+    num_pages = sum(-(-(c + n) // ps) for c, n in zip(ctx, q_lens)) + 8
+    step = make_step(o, dtype, ctx, q_lens, ps, num_pages, 9)
+    clean = torch.randn(num_pages, 2, Hkv, ps, D, generator=g).to(dtype).cuda()
+    q = torch.randn(sum(q_lens), Hq * D, generator=g).to(dtype).cuda()
+    for at in (0, 37, 69):
+        pages = clean.clone()
+        pages[int(step.block_tables[0][0, at // ps]), 1, 1, at % ps, 5] = bad
+        view, was = CacheView(0, pages, step.block_tables[0], ps), CacheView(0, clean, step.block_tables[0], ps)
+        for opts in (dict(), dict(window=20), dict(chunk=32), dict(window=9, keep_first=40)):
+            a = o.paged_attention(q, step, view, Hq, Hkv, D, D ** -0.5, **opts)
+            b = o.paged_attention(q, step, view, Hq, Hkv, D, D ** -0.5, impl="general", **opts)
+            assert torch.equal(torch.isfinite(a), torch.isfinite(b)), (at, sorted(opts))
+            keep = torch.isfinite(a)
+            assert not keep.all() and torch.equal(a[keep], o.paged_attention(q, step, was, Hq, Hkv, D, D ** -0.5, **opts)[keep])
+    assert o.read_status() == 0

@@ -203,6 +203,7 @@ __global__ void __launch_bounds__(128) paged_attention_tile_kernel(
     }
     find_rows(0);
     for (int n = 0; n < n_tiles; ++n) {
+        bool odd = false;                                    // one of the thread's values is infinite or NaN
         __syncthreads();                                     // the tile before has been used; this one's rows are known
 #pragma unroll 4
         for (int i = tid; i < AT_N * (DM / 4); i += 128) {
@@ -215,9 +216,10 @@ __global__ void __launch_bounds__(128) paged_attention_tile_kernel(
             }
             *reinterpret_cast<float4*>(&sm.k[j][d]) = kv;
             *reinterpret_cast<float4*>(&sm.v[j][d]) = vv;
+            odd |= !(fmaf(vv.x, 0.f, fmaf(vv.y, 0.f, fmaf(vv.z, 0.f, vv.w * 0.f))) == 0.f);       // (NaN for either)
         }
         find_rows(n + 1);
-        __syncthreads();
+        odd = __syncthreads_or(odd);
         float s[4][4] = {};
 #pragma unroll 4
         for (int d = 0; d < DM; d += 4) {
@@ -266,6 +268,20 @@ __global__ void __launch_bounds__(128) paged_attention_tile_kernel(
             for (int c = 0; c < NC; ++c) o[i][c] *= corr;
         }
         __syncwarp();                                        // (a row's weights come from its own 16 lanes)
+        if (odd) {
+            // a hidden key's weight is zero, and zero times such a value is NaN: each pair takes the keys that it sees, one by one
+            for (int j = 0; j < AT_N; ++j) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int key = base + j;
+                    if (!(key <= pos[i] && (key >= from[i] || key < kept[i]))) continue;
+#pragma unroll
+                    for (int c = 0; c < NC; ++c)
+                        o[i][c] = fmaf(sm.p[ty * 4 + i][j], sm.v[j][NC == 2 ? tx * 2 + c : (c / 4) * 64 + tx * 4 + c % 4], o[i][c]);
+                }
+            }
+            continue;
+        }
 #pragma unroll 2
         for (int j = 0; j < AT_N; j += 4) {
             float4 w[4];
