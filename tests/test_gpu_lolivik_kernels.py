@@ -268,3 +268,28 @@ def test_mlstm_in_chunks(H, D, V):
     o.mlstm(y, at, bias_i, bias_f, 11.0, norm_w, 1e-5, state_a, step, H, D, V, False, impl="chunks")
     assert torch.equal(state_a, keep)
     assert o.read_status() == 0
+
+
+@pytest.mark.parametrize("H,D,V", [(2, 64, 128), (3, 10, 14), (1, 128, 65)])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_mlstm_in_chunks_and_values_that_are_not_finite(H, D, V, bad):
+    """A value that is not finite reaches its own head from its own row on, and nothing else."""
+    o = ops()
+    g = torch.Generator().manual_seed(19)
+    at, cols = mlstm_columns(H, D, V)
+    bias_i, bias_f, norm_w = (torch.randn(H, generator=g) - 1.0).cuda(), (torch.randn(H, generator=g) + 3.0).cuda(), torch.ones(H * V).cuda()
+    q_lens = [200, 70]
+    step = make_step(o, torch.bfloat16, [3, 3], q_lens, 8, 256, 5)
+    y = torch.randn(270, cols, generator=g).to(torch.bfloat16).cuda()
+    run = lambda rows: o.mlstm(rows, at, bias_i, bias_f, 11.0, norm_w, 1e-5, torch.zeros(5, H, D + 1, V + 1).cuda(), step, H, D, V, True, impl="chunks").view(270, H, V)
+    want = run(y)
+    assert torch.isfinite(want).all()
+    for r in (0, 1, 15, 16, 63, 64, 100, 199):
+        dirty = y.clone()
+        dirty[r, at[2] + V // 2] = bad                                 # one value of head 0
+        got = run(dirty)
+        hit = torch.zeros(270, H, dtype=torch.bool)
+        hit[r:200, 0] = True
+        assert torch.equal(got[~hit], want[~hit]), r
+        assert not torch.isfinite(got[hit]).all(1).any(), r
+    assert o.read_status() == 0

@@ -444,6 +444,7 @@ __global__ void __launch_bounds__(256) mlstm_chunk_out_kernel(const MlstmArgs a,
     __shared__ float2 s_u[MLSTM_Q];
     __shared__ double s_top[MLSTM_Q], s_f[MLSTM_Q], s_carry[2];
     __shared__ float s_nq[MLSTM_Q], s_ss[2][MLSTM_Q];
+    __shared__ int s_odd, s_from[VT];                        // a value of v that is infinite or NaN: whether, and a column's first row with one
     constexpr int LDX = VT + MLSTM_PAD, VW = VT / 2;
     const int dp = (a.D + 15) & ~15, ldk = dp + MLSTM_PAD;
     bf16* sq = reinterpret_cast<bf16*>(ml_raw);              // [Q][ldk]
@@ -456,6 +457,8 @@ __global__ void __launch_bounds__(256) mlstm_chunk_out_kernel(const MlstmArgs a,
     pdl_wait();
     int t0, t1, first;
     if (!mlstm_find_chunk(a, blockIdx.x, t0, t1, first)) return;
+    if (threadIdx.x < VT) s_from[threadIdx.x] = MLSTM_Q;
+    if (threadIdx.x == 0) s_odd = 0;
     const int h = blockIdx.y;
     mlstm_load_rows(sq, ldk, a, a.q_at + h * a.D, a.D, dp, t0, t1);
     mlstm_load_rows(sk, ldk, a, a.k_at + h * a.D, a.D, dp, t0, t1);
@@ -503,6 +506,19 @@ __global__ void __launch_bounds__(256) mlstm_chunk_out_kernel(const MlstmArgs a,
         n += __shfl_xor_sync(0xffffffffu, n, 2);
         if (part == 0) s_nq[r] = n;
     }
+    // (a later row's weight is zero, and zero times such a value is NaN: it leaves the product, and its column ends as NaN from its row on)
+    for (int i = threadIdx.x; i < MLSTM_Q * (VT / 8); i += 256) {
+        const int r = i / (VT / 8), c = (i % (VT / 8)) * 8;
+        uint32_t* p = reinterpret_cast<uint32_t*>(sv + r * LDX + c);
+        const uint4 x = *reinterpret_cast<const uint4*>(p);
+        if ((not_finite_pair(x.x) | not_finite_pair(x.y) | not_finite_pair(x.z) | not_finite_pair(x.w)) == 0) continue;
+        for (int k = 0; k < 8; ++k)
+            if (not_finite_pair(p[k >> 1]) >> (k & 1 ? 31 : 15) & 1) {
+                sv[r * LDX + c + k] = __float2bfloat16_rn(0.f);
+                atomicMin(&s_from[c + k], r);
+            }
+        s_odd = 1;
+    }
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, mi = lane >> 3, r8 = lane & 7, tq = lane & 3;
     const int wr = warp & 3, side = warp >> 2, vb = side * VW;
@@ -544,6 +560,13 @@ __global__ void __launch_bounds__(256) mlstm_chunk_out_kernel(const MlstmArgs a,
 #pragma unroll
     for (int i = 0; i < VW / 8; ++i) {
         acc[i][0] *= ea; acc[i][1] *= ea; acc[i][2] *= eb; acc[i][3] *= eb;
+    }
+    if (s_odd) {
+#pragma unroll
+        for (int i = 0; i < VW / 8; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if ((e < 2 ? ra : rb) >= s_from[vb + i * 8 + 2 * tq + (e & 1)]) acc[i][e] = __int_as_float(0x7fc00000);
     }
     // the chunk's own rows
     float na = 0.f, nb = 0.f;

@@ -32,6 +32,9 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// two bfloat16 values: the sign bit of each that is infinite or NaN (an exponent of ones)
+__device__ __forceinline__ uint32_t not_finite_pair(uint32_t v) { return ((v & 0x7f807f80u) + 0x00800080u) & 0x80008000u; }
+
 // v as a sum of three bfloat16 numbers, which hold its 24 bits: what is 32-bit goes into bfloat16 products as its three parts
 __device__ __forceinline__ void split3(float v, float& hi, float& mid, float& lo) {
     hi = __bfloat162float(__float2bfloat16_rn(v));
