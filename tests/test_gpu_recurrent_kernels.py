@@ -263,3 +263,35 @@ def test_gated_rmsnorm_in_fours_and_one_by_one(dtype, V, H, stride, off):
         bound = 1e-5 if dtype is torch.float32 else 2.0 ** -8
         assert ((out.double() - want).abs() <= bound * (want.abs() + 1e-3)).all()
     assert o.read_status() == 0
+
+
+def delta_inputs(H, G, D, V, N, channel, g):
+    cols_a = H * D if channel else H
+    a_log, dt_bias = torch.log(1 + 15 * torch.rand(H, generator=g)).cuda(), (torch.randn(cols_a, generator=g) - 3).cuda()
+    qkv, a = torch.randn(N, 2 * G * D + H * V, generator=g).bfloat16().cuda(), torch.randn(N, cols_a, generator=g).bfloat16().cuda()
+    gate, b = torch.randn(N, H * V, generator=g).bfloat16().cuda(), torch.randn(N, H, generator=g).bfloat16().cuda()
+    return qkv, b, a, gate, a_log, dt_bias, torch.ones(V).cuda()
+
+
+@pytest.mark.parametrize("H,G,D,V", [(4, 2, 64, 128), (2, 2, 24, 40)])
+@pytest.mark.parametrize("channel", [False, True])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_gated_delta_in_chunks_and_values_that_are_not_finite(H, G, D, V, channel, bad):
+    """A value (or a key) that is not finite reaches its own heads from its own row on, and nothing else."""
+    o = ops()
+    g = torch.Generator().manual_seed(23)
+    step = make_step(o, torch.bfloat16, [3, 3], [200, 70], 8, 256, 5)
+    qkv, *rest = delta_inputs(H, G, D, V, 270, channel, g)
+    run = lambda rows: o.gated_delta(rows, *rest, 1e-5, torch.zeros(5, H, D, V).cuda(), step, H, G, D, V, True, channel_decay=channel, impl="chunks").view(270, H, V)
+    want = run(qkv)
+    assert torch.isfinite(want).all()
+    for r in (0, 1, 7, 8, 15, 16, 30, 63, 64, 100, 199):
+        for col, heads in ((2 * G * D + V // 2, [0]), (G * D, list(range(H // G)))):       # a value of head 0; a key of the first key head
+            dirty = qkv.clone()
+            dirty[r, col] = bad
+            got = run(dirty)
+            hit = torch.zeros(270, H, dtype=torch.bool)
+            hit[r:200, heads] = True
+            assert torch.equal(got[~hit], want[~hit]), (r, col)
+            assert not torch.isfinite(got[hit]).all(1).any(), (r, col)
+    assert o.read_status() == 0

@@ -971,8 +971,37 @@ __device__ __forceinline__ void delta_put_columns(DeltaColumns<DN>& c, const flo
     }
 }
 
-// acc[s] += (operand tile row: fa[part][kt]) x columns, sorted by size: s = 0 the leading parts, 2 the smallest products
-template <int DN>
+// The part of a product's second operand that CAUSAL rows see only some of (16 rows, two tiles of eight columns; a lane has rows
+// 2 tq, + 1, + 8, + 9 of columns g): a row's weight for what lies behind it is zero, and zero times infinity or NaN is NaN.  Such
+// values leave the operand; rows from a column's first one on become NaN there.
+template <int NT>
+__device__ __forceinline__ void delta_take_odd(float (&acc)[NT][4], uint32_t (&fb)[3][4], int nt, int lane) {
+    const int tq = lane & 3;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        int from = 16;
+#pragma unroll
+        for (int r = 1; r >= 0; --r) {
+            const uint32_t odd = not_finite_pair(fb[0][2 * j + r]);
+            if (odd >> 31) from = 2 * tq + 8 * r + 1;
+            if (odd >> 15 & 1) from = 2 * tq + 8 * r;
+            const uint32_t keep = (odd >> 31 ? 0u : 0xffff0000u) | (odd >> 15 & 1 ? 0u : 0x0000ffffu);
+#pragma unroll
+            for (int p = 0; p < 3; ++p) fb[p][2 * j + r] &= keep;
+        }
+        from = min(from, __shfl_xor_sync(0xffffffffu, from, 1));
+        from = min(from, __shfl_xor_sync(0xffffffffu, from, 2));
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int first = __shfl_sync(0xffffffffu, from, (2 * tq + (e & 1)) * 4);
+            if ((lane >> 2) + 8 * (e >> 1) >= first) acc[nt + j][e] = __int_as_float(0x7fc00000);
+        }
+    }
+}
+
+// acc[s] += (operand tile row: fa[part][kt]) x columns, sorted by size: s = 0 the leading parts, 2 the smallest products.  CAUSAL:
+// in the last of the kts tiles of 16 rows a row sees those up to its own
+template <int DN, bool CAUSAL = false>
 __device__ __forceinline__ void delta_product(float (&acc)[3][DN / 8][4], const uint4 (&fa)[3][4], const DeltaColumns<DN>& c, int kts, int lane) {
     const int mi = lane >> 3, r8 = lane & 7;
 #pragma unroll
@@ -983,6 +1012,9 @@ __device__ __forceinline__ void delta_product(float (&acc)[3][DN / 8][4], const 
             uint32_t fb[3][4];
 #pragma unroll
             for (int p = 0; p < 3; ++p) ldmatrix_x4(fb[p], &c.v[p][(nt + (mi >> 1)) * 8 + r8][kt * 16 + (mi & 1) * 8]);
+            if (CAUSAL && kt == kts - 1
+                && __any_sync(0xffffffffu, (not_finite_pair(fb[0][0]) | not_finite_pair(fb[0][1]) | not_finite_pair(fb[0][2]) | not_finite_pair(fb[0][3])) != 0))
+                delta_take_odd(acc[0], fb, nt, lane);
 #pragma unroll
             for (int pa = 0; pa < 3; ++pa) {
                 const uint32_t f[4] = {fa[pa][kt].x, fa[pa][kt].y, fa[pa][kt].z, fa[pa][kt].w};
@@ -1044,7 +1076,7 @@ __global__ void __launch_bounds__(256) delta_carry_kernel(const DeltaArgs a) {
             ch += a.H;
             if (c + 1 < nc) delta_fetch(fq, ch->q, mt, lane, 4);
             bar_sync(DB_U + (c & 1), 256);
-            delta_product<DN>(acc, fp, su[c & 1], mt + 1, lane);
+            delta_product<DN, true>(acc, fp, su[c & 1], mt + 1, lane);
             if (c + 2 < nc) bar_arrive(DB_FREE + (c & 1), 256);
             if (c + 1 < nc) delta_fetch(fp, ch->p, mt, lane, mt + 1);
 #pragma unroll
