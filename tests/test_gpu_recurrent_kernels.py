@@ -295,3 +295,19 @@ def test_gated_delta_in_chunks_and_values_that_are_not_finite(H, G, D, V, channe
             assert torch.equal(got[~hit], want[~hit]), (r, col)
             assert not torch.isfinite(got[hit]).all(1).any(), (r, col)
     assert o.read_status() == 0
+
+
+@pytest.mark.parametrize("channel", [False, True])
+def test_gated_delta_in_chunks_with_a_unit_norm_without_epsilon(channel):
+    """A span whose last chunk is not full: its spare rows are zeros, which a norm without an epsilon would divide by zero."""
+    o = ops()
+    g = torch.Generator().manual_seed(24)
+    H, G, D, V = 4, 2, 64, 128
+    step = make_step(o, torch.bfloat16, [3, 3], [100, 65], 8, 256, 5)
+    inputs = delta_inputs(H, G, D, V, 165, channel, g)
+    state_a = (torch.randn(5, H, D, V, generator=g) * 0.3).cuda()
+    state_b = state_a.clone()
+    ya = o.gated_delta(*inputs, 1e-5, state_a, step, H, G, D, V, True, unit_eps=0.0, channel_decay=channel, impl="chunks")
+    yb = ref_ops.gated_delta(*inputs, 1e-5, state_b, step, H, G, D, V, True, unit_eps=0.0, channel_decay=channel)
+    assert torch.allclose(ya.float(), yb.float(), **tol(torch.bfloat16))
+    assert torch.allclose(state_a, state_b, atol=1e-4, rtol=1e-4)

@@ -723,7 +723,8 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_kernel(const DeltaArgs a) 
             ss = fmaf(x.x, x.x, fmaf(x.y, x.y, ss));
         }
         ss += __shfl_xor_sync(0xffffffffu, ss, 1);
-        if (part == 0) sm.inv[which][t] = rsqrtf(ss + a.unit_eps) * (which ? 1.f : rsqrtf((float)D));
+        // (rows beyond the chunk stay zeros, whatever the norm's epsilon)
+        if (part == 0) sm.inv[which][t] = t < n ? rsqrtf(ss + a.unit_eps) * (which ? 1.f : rsqrtf((float)D)) : 0.f;
     }
     if constexpr (CH) {
         if (tid < DCD) {                                     // (sums of numbers of one sign: their rounding is as small as their terms')
