@@ -311,3 +311,23 @@ def test_gated_delta_in_chunks_with_a_unit_norm_without_epsilon(channel):
     yb = ref_ops.gated_delta(*inputs, 1e-5, state_b, step, H, G, D, V, True, unit_eps=0.0, channel_decay=channel)
     assert torch.allclose(ya.float(), yb.float(), **tol(torch.bfloat16))
     assert torch.allclose(state_a, state_b, atol=1e-4, rtol=1e-4)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_selective_scan_with_rates_that_overflow(dtype):
+    """exp(A_log) beyond the largest number: the state is gone after each row (as by any rate that large), and rows that fill up a tile
+    change nothing."""
+    o = ops()
+    g = torch.Generator().manual_seed(25)
+    I, S, R = 32, 16, 4
+    step = make_step(o, dtype, [3, 3], [5, 66], 8, 256, 5)
+    w_dt, b_dt, d = (torch.randn(I, R, generator=g) * 0.5).to(dtype).cuda(), (torch.randn(I, generator=g) * 0.5).cuda(), torch.randn(I, generator=g).cuda()
+    x, proj, z = (torch.randn(71, n, generator=g).to(dtype).cuda() for n in (I, R + 2 * S, I))
+    out = []
+    for rate in (100.0, 30.0):                                 # e^100 is infinite in 32 bits, e^30 is not; both leave nothing
+        a_log = (torch.randn(I, S, generator=torch.Generator().manual_seed(1)) * 0.5).cuda()
+        a_log[::3] = rate
+        state = torch.randn(5, I, S, generator=torch.Generator().manual_seed(2)).cuda()
+        out.append((o.selective_scan(x, proj, z, w_dt, b_dt, a_log, d, state, step, R, True), state))
+    assert torch.isfinite(out[0][0]).all() and torch.isfinite(out[0][1]).all()
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])

@@ -11,6 +11,7 @@
 //   * steps of single tokens: a lane holds K consecutive states of a channel (a whole channel where S <= 16, else G lanes
 //     of a warp share it), loads its row's values and sums its step size itself;
 //   * steps with portions: a block walks one request's rows in order, two states a lane, fed by warps of its own.
+#include <cfloat>
 #include "mma_helpers.cuh"
 
 // Exponentials and the softplus: exact library functions where the model is 32-bit; where activations are
@@ -160,8 +161,10 @@ __global__ void __launch_bounds__(128) selective_scan_single_kernel(
 // passes: 309), 92 for 2048 (172), 91 for 1024 (129); 512 rows of 4096 channels 40 (104).  A row costs about 45 ns however few
 // the channels are (dependent instructions, one warp a scheduler): below 1024 channels and beyond 2048 rows chunks would be
 // faster again (8192 rows of 512 channels 331, in chunks 220).
-template <typename T> __device__ __forceinline__ float decay_scale(float a) { return a; }
-template <> __device__ __forceinline__ float decay_scale<bf16>(float a) { return a * 1.4426950408889634f; }
+// (a rate beyond the largest number counts as that: a row with a step of zero leaves the state alone, zero times infinity would not)
+__device__ __forceinline__ float decay_bound(float a) { return a < -FLT_MAX ? -FLT_MAX : a; }
+template <typename T> __device__ __forceinline__ float decay_scale(float a) { return decay_bound(a); }
+template <> __device__ __forceinline__ float decay_scale<bf16>(float a) { return decay_bound(a * 1.4426950408889634f); }
 template <typename T> __device__ __forceinline__ float decay_of(float v) { return expf(v); }
 template <> __device__ __forceinline__ float decay_of<bf16>(float v) { return fast_exp2(v); }
 
