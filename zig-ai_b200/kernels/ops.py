@@ -1332,6 +1332,14 @@ def _span_kinds(step, cut):
     return max(step.q_lens) >= cut, any(0 < n < cut for n in step.q_lens)
 
 
+def _chunk_bound(step, cut, rows):
+    """How many chunks of `rows` rows a step's spans of `cut` rows or more make; of a captured step shape, the most that its rows and
+    spans allow (at most n_tokens // cut spans are that long, and each may end with a part of a chunk)."""
+    if getattr(step, "attn_tiles", None) or not step.q_lens:
+        return step.n_tokens // rows + min(step.n_seqs, step.n_tokens // cut)
+    return sum(-(-n // rows) for n in step.q_lens if n >= cut)
+
+
 def _rows_view(x):
     """(pointer, row stride) of a 2-D tensor whose rows are contiguous (a column slice of a wider matrix)."""
     if x.dim() != 2 or x.stride(1) != 1 or not x.is_cuda:
@@ -1474,7 +1482,7 @@ def gated_delta(qkv, b, a, gate, a_log, dt_bias, norm_w, eps, state, step, heads
         cut = 1 if impl == "chunks" else _delta_cut(step, N, H * V / 128)
     long, short = _span_kinds(step, cut)
     if long:
-        max_chunks = N // _fn(lib, "zai_gated_delta_chunk_rows")() + step.n_seqs
+        max_chunks = _chunk_bound(step, cut, _fn(lib, "zai_gated_delta_chunk_rows")())
         scratch = torch.empty(max_chunks * H * _fn(lib, "zai_gated_delta_chunk_bytes")(V), dtype=torch.uint8, device=dev)
         _check(_fn(lib, "zai_gated_delta_chunked")(
             _ptr(o), qp, qs, bp, bs, ap, as_, _ptr(a_log), _ptr(dt_bias), float(unit_eps), _ptr(state), _ptr(step.cu_q), _ptr(step.slot_ids),
@@ -1985,7 +1993,7 @@ def mlstm(y, at, bias_i, bias_f, cap, norm_w, eps, state, step, heads, dim, vdim
         cut = 1 if impl == "chunks" else MLSTM_CHUNKED_MIN
     long, short = _span_kinds(step, cut)
     if long:
-        max_chunks = N // _fn(lib, "zai_mlstm_chunk_rows")() + step.n_seqs
+        max_chunks = _chunk_bound(step, cut, _fn(lib, "zai_mlstm_chunk_rows")())
         ends = torch.empty((max_chunks, H, D, (Dv + 4) // 4 * 4), dtype=torch.float32, device=y.device)
         gates = torch.empty((max_chunks, H, 2), dtype=torch.float64, device=y.device)
         m_in = torch.empty((max_chunks, H), dtype=torch.float32, device=y.device)
