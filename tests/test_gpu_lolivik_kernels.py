@@ -293,3 +293,25 @@ def test_mlstm_in_chunks_and_values_that_are_not_finite(H, D, V, bad):
         assert torch.equal(got[~hit], want[~hit]), r
         assert not torch.isfinite(got[hit]).all(1).any(), r
     assert o.read_status() == 0
+
+
+@pytest.mark.parametrize("H,D,V", [(4, 64, 128), (8, 16, 32)])
+def test_mlstm_does_not_depend_on_neighbours_or_capture(H, D, V):
+    from test_gpu_recurrent_kernels import same_alone_and_beside
+    o = ops()
+    g = torch.Generator().manual_seed(20)
+    at, cols = mlstm_columns(H, D, V)
+    most = 1100
+    y = torch.randn(most, cols, generator=g).to(torch.bfloat16).cuda()
+    bias_i, bias_f, norm_w = (torch.randn(H, generator=g) - 1.0).cuda(), (torch.randn(H, generator=g) + 3.0).cuda(), torch.ones(H * V).cuda()
+    first = torch.randn(H, D + 1, V + 1, generator=g).cuda()
+    first[:, D] = first[:, D, :1].clone()
+
+    def run(q_lens, shift, captured):
+        step = make_step(o, torch.bfloat16, [3] * len(q_lens), q_lens, 8, 2 * sum(q_lens) // 8 + 8 * len(q_lens) + 8, 5)
+        if captured:
+            step.attn_tiles = sum(q_lens) // 128 + len(q_lens)
+        rows = torch.cat([(torch.arange(n) + k) % most for n, k in zip(q_lens, shift)]).cuda()
+        state = first.repeat(len(q_lens) + 2, 1, 1, 1)
+        return o.mlstm(y[rows], at, bias_i, bias_f, 11.0, norm_w, 1e-5, state, step, H, D, V, True), state[1:]
+    same_alone_and_beside(run, (1, 5, 63, 64, 65, 191, 192, 300), ([2, 70], [1, 0, 600], [64, 192, 64]))

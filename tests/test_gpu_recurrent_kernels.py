@@ -331,3 +331,39 @@ def test_selective_scan_with_rates_that_overflow(dtype):
         out.append((o.selective_scan(x, proj, z, w_dt, b_dt, a_log, d, state, step, R, True), state))
     assert torch.isfinite(out[0][0]).all() and torch.isfinite(out[0][1]).all()
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
+def same_alone_and_beside(run, lens, others):
+    """run(q_lens, rows) -> (output rows, states by request) of a step whose requests hold the given rows of the inputs.  A request's rows
+    alone, in front of, between and behind others, and in a step that is laid out like a captured one (spans without rows among them)
+    must give the same bits."""
+    for n in lens:
+        want, state = run([n], [0], None)
+        for q_lens in others:
+            for at in range(len(q_lens) + 1):
+                spans = q_lens[:at] + [n] + q_lens[at:]
+                first = sum(spans[:at])
+                for captured in (None, 1):
+                    got, states = run(spans, [200 + i if i != at else 0 for i in range(len(spans))], captured)
+                    assert torch.equal(got[first:first + n], want), (n, spans, at, captured)
+                    assert torch.equal(states[at], state[0]), (n, spans, at, captured)
+
+
+@pytest.mark.parametrize("H,G,D,V", [(16, 8, 64, 128), (4, 2, 16, 32), (32, 16, 64, 64)])
+@pytest.mark.parametrize("channel", [False, True])
+def test_gated_delta_does_not_depend_on_neighbours_or_capture(H, G, D, V, channel):
+    o = ops()
+    g = torch.Generator().manual_seed(26)
+    most = 1100
+    qkv, b, a, gate, a_log, dt_bias, norm_w = delta_inputs(H, G, D, V, most, channel, g)
+    first = (torch.randn(H, D, V, generator=g) * 0.3).cuda()
+
+    def run(q_lens, shift, captured):
+        step = make_step(o, torch.bfloat16, [3] * len(q_lens), q_lens, 8, 2 * sum(q_lens) // 8 + 8 * len(q_lens) + 8, 5)
+        if captured:
+            step.attn_tiles = sum(q_lens) // 128 + len(q_lens)
+        rows = torch.cat([(torch.arange(n) + k) % most for n, k in zip(q_lens, shift)]).cuda()
+        state = first.repeat(len(q_lens) + 2, 1, 1, 1)
+        y = o.gated_delta(qkv[rows], b[rows], a[rows], gate[rows], a_log, dt_bias, norm_w, 1e-5, state, step, H, G, D, V, True, channel_decay=channel)
+        return y, state[1:]
+    same_alone_and_beside(run, (2, 5, 64, 127, 128, 130, 256, 700), ([2, 130], [1, 0, 600], [128, 128, 128]))

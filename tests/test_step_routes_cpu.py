@@ -2,6 +2,8 @@
 import random
 from types import SimpleNamespace
 
+import pytest
+
 from zig_ai_b200.kernels import ops
 
 
@@ -21,3 +23,11 @@ def test_chunk_scratch_holds_every_chunk_and_little_more():
     # one portion beside decoding requests, as a captured shape sees it (its spans rounded up): no chunk a request
     assert ops._chunk_bound(step_of([1] * 64 + [2048] + [0] * 63, True), 128, 64) == 33 + 16
     assert ops._chunk_bound(step_of([1] * 256 + [2048]), 128, 64) == 32
+
+
+@pytest.mark.parametrize("cut", [lambda h, d, v: ops._delta_cut(h, d, v), lambda h, d, v: ops._mlstm_cut(d, v)])
+def test_spans_take_their_kernels_by_the_layers_sizes_alone(cut):
+    for h in (1, 4, 16, 64):
+        for d in (1, 8, 16, 32, 64):
+            for v in (1, 8, 33, 64, 128, 256):
+                assert 64 <= cut(h, d, v) <= max(256, 32 * h)

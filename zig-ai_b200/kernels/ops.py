@@ -1411,37 +1411,19 @@ def min_gru(zxg, b_z, b_x, state, step, write_state=True):
     return out
 
 
-# Microseconds that the delta rule's kernels take (16 and 32 heads of 64 x 128): the walk 12 and 0.28 for every row of its longest
-# span, or 0.0040 for every row and head together where many requests fill the chip; the chunks' kernels 25 and 0.0036 a row and
-# head, rows in 64s.  2048 rows of 16 heads: one span 480 (walk) and 136 (chunks), four spans 168 and 138, eight spans 129
-# and 137; of 32 heads 580 and 233, 261 and 239, 261 and 245; eight spans of 160 rows of 16 heads 90 and 106.
-DELTA_WALK, DELTA_CHUNKS = (12.0, 0.28, 0.0040), (25.0, 0.0036)
-DELTA_CHUNKED_LEAST = 64
-
-
-def _delta_cut(step, n_rows, load):
-    """The rows from which on a step's spans run in chunks: the choice that the figures above make the quickest.  `load`: heads,
-    in units of 128 values.  A captured step shape is replayed with other spans than it has now: there a span goes in chunks if
-    walking it takes longer than the whole step in chunks, which is no slower whatever the other spans are."""
-    fixed, by_row, by_load = DELTA_WALK
-    if getattr(step, "attn_tiles", None) or not step.q_lens:
-        return max(DELTA_CHUNKED_LEAST, int((DELTA_CHUNKS[0] + DELTA_CHUNKS[1] * n_rows * load) / by_row))
-    lens = sorted(step.q_lens, reverse=True)
-    best, cut, rows, padded = None, 1 << 30, 0, 0
-    for i in range(len(lens) + 1):
-        # the first i spans in chunks, the others walked
-        left = lens[i] if i < len(lens) else 0
-        if i == 0 or lens[i - 1] != left:
-            us = (DELTA_CHUNKS[0] + DELTA_CHUNKS[1] * padded * load) if i else 0.0
-            if left:
-                us += fixed + max(by_row * left, by_load * (n_rows - rows) * load)
-            if best is None or us < best:
-                best, cut = us, (lens[i - 1] if i else 1 << 30)
-        if left < DELTA_CHUNKED_LEAST:
-            break
-        rows += left
-        padded += -(-left // 64) * 64
-    return cut
+def _delta_cut(heads, dim, vdim):
+    """Spans of this many rows or more run the delta rule in chunks (bfloat16).  It depends on the layer's sizes alone, so that a
+    request's results depend neither on its neighbours nor on capture.  us walked and in chunks, spans x rows: a span alone gains from
+    about 64 rows on (16 heads of 64 x 128: 1x128 39 and 27, 1x2048 474 and 132; 32 heads of 32 x 64: 1x256 60 and 35), and beside longer
+    spans a shorter one had better not be a chain of its own (32 heads of 64 x 128, 777 and 301 rows with 130 and 64: 307 with the 64
+    walked, 266 with all in chunks).  Where spans fill the chip the walk costs by D x V and the chunks by the head: 16 heads of 64 x
+    128, 8x256 125 and 133, 32x64 125 and 185; 32 of 64 x 64, 4x512 177 and 177, 8x128 70 and 91; of 32 x 64, 4x512 133 and 177; of 16 x
+    32, 8x256 68 and 135, 1x2048 367 and 170.  The lines lie where a full chip loses about a third at most."""
+    if dim * vdim >= 64 * 128:
+        return 64
+    if dim * vdim >= 64 * 64:
+        return 128
+    return max(256, heads * (8 if dim * vdim >= 1024 else 32))
 
 
 @_timed("recurrence")
@@ -1479,7 +1461,7 @@ def gated_delta(qkv, b, a, gate, a_log, dt_bias, norm_w, eps, state, step, heads
     out = torch.empty((N, H * V), dtype=qkv.dtype, device=dev)
     cut = 1 << 30                                              # (spans of that many rows or more run in chunks, the others are walked)
     if impl != "walk" and not step.decode_only and qkv.dtype == torch.bfloat16 and _fn(lib, "zai_gated_delta_chunked_supports")(D, V):
-        cut = 1 if impl == "chunks" else _delta_cut(step, N, H * V / 128)
+        cut = 1 if impl == "chunks" else _delta_cut(H, D, V)
     long, short = _span_kinds(step, cut)
     if long:
         max_chunks = _chunk_bound(step, cut, _fn(lib, "zai_gated_delta_chunk_rows")())
@@ -1965,10 +1947,12 @@ def mamba2(y, at, conv_w, conv_b, dt_bias, a_log, d_skip, norm_w, eps, norm_part
     return out
 
 
-# Spans of this many rows or more run the matrix memory in chunks on the tensor cores (bfloat16): the walk takes about 12 us and
-# 0.25 us a row, the three kernels over chunks 25 to 30 us up to a thousand rows.  One request alone, heads of 64 x 128: 48 rows
-# 26 (walk) and 34 us (chunks), 64 rows 30 and 32, 128 rows 46 and 32; 16 requests of 32 rows 33 and 45, of 64 rows 50 and 43.
-MLSTM_CHUNKED_MIN = 64
+def _mlstm_cut(dim, vdim):
+    """Spans of this many rows or more run the matrix memory in chunks on the tensor cores (bfloat16).  The walk costs by D x Dv and a
+    row, the chunks some 20 to 30 us up to a thousand rows.  us walked and in chunks, spans x rows: 8 heads of 64 x 128, 1x64 31 and
+    28, 16x64 51 and 43; of 64 x 64, 1x64 29 and 21, 16x64 37 and 29; of 32 x 64, 16x64 27 and 27; of 16 x 32, 16x64 18 and 26, 8x160
+    31 and 25, 1x192 34 and 21."""
+    return 64 if dim * vdim >= 64 * 64 else 192
 
 
 @_timed("recurrence")
@@ -1990,7 +1974,7 @@ def mlstm(y, at, bias_i, bias_f, cap, norm_w, eps, state, step, heads, dim, vdim
     # which kernels a span takes depends on its own length alone (a step may hold both kinds)
     cut = 1 << 30
     if impl != "walk" and not step.decode_only and y.dtype == torch.bfloat16 and _fn(lib, "zai_mlstm_chunked_supports")(D, Dv):
-        cut = 1 if impl == "chunks" else MLSTM_CHUNKED_MIN
+        cut = 1 if impl == "chunks" else _mlstm_cut(D, Dv)
     long, short = _span_kinds(step, cut)
     if long:
         max_chunks = _chunk_bound(step, cut, _fn(lib, "zai_mlstm_chunk_rows")())
