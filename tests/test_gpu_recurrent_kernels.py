@@ -367,3 +367,25 @@ def test_gated_delta_does_not_depend_on_neighbours_or_capture(H, G, D, V, channe
         y = o.gated_delta(qkv[rows], b[rows], a[rows], gate[rows], a_log, dt_bias, norm_w, 1e-5, state, step, H, G, D, V, True, channel_decay=channel)
         return y, state[1:]
     same_alone_and_beside(run, (2, 5, 64, 127, 128, 130, 256, 700), ([2, 130], [1, 0, 600], [128, 128, 128]))
+
+
+def test_recurrences_in_chunks_beside_very_many_requests():
+    """More requests than a grid's second and third dimension hold."""
+    o = ops()
+    o.require(extra=("mlstm",))
+    g = torch.Generator().manual_seed(27)
+    q_lens = [1] * 65600 + [300]
+    N = sum(q_lens)
+    step = make_step(o, torch.bfloat16, [0] * len(q_lens), q_lens, 8, len(q_lens) + 100, 5)
+    y = torch.randn(N, 6 * 8 + 2, generator=g).bfloat16().cuda()
+    one = torch.ones(1).cuda()
+    outs = []
+    for impl in ("walk", None):
+        state = torch.zeros(len(q_lens) + 1, 1, 9, 17).cuda()
+        outs.append((o.mlstm(y, [0, 8, 16, 32, 48, 49], one, 3 * one, 11.0, torch.ones(16).cuda(), 1e-5, state, step, 1, 8, 16, True, impl=impl), state))
+        state = torch.zeros(len(q_lens) + 1, 1, 8, 16).cuda()
+        outs.append((o.gated_delta(y[:, :32], y[:, 48:49], y[:, 49:], y[:, 32:48], one, one, torch.ones(16).cuda(), 1e-5, state, step, 1, 1, 8, 16, True, impl=impl), state))
+    for (a, sa), (b, sb) in zip(outs[:2], outs[2:]):
+        assert torch.equal(a[:65600], b[:65600]) and torch.equal(sa[1:65601], sb[1:65601])
+        assert torch.allclose(a.float(), b.float(), **tol(torch.bfloat16)) and torch.allclose(sa, sb, atol=1e-4, rtol=1e-4)
+    assert o.read_status() == 0

@@ -1053,7 +1053,7 @@ __global__ void __launch_bounds__(256) delta_carry_kernel(const DeltaArgs a) {
     DeltaColumns<DN>* su = ss + 2;                                            // [2] u
     pdl_trigger();
     pdl_wait();
-    const int seq = blockIdx.z, h = blockIdx.y, v0 = blockIdx.x * DN;
+    const int seq = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * DN;
     const int r0 = a.cu_q[seq], rows = a.cu_q[seq + 1] - r0;
     if (rows < a.min_rows) return;
     int first = 0;
@@ -1192,7 +1192,7 @@ static int delta_carry(const DeltaArgs& a, cudaStream_t stream) {
         const cudaError_t e = cudaFuncSetAttribute(delta_carry_kernel<DN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
     }
-    return launch_pdl(delta_carry_kernel<DN>, dim3((a.V + DN - 1) / DN, a.H, a.n_seqs), dim3(256), smem, stream, a);
+    return launch_pdl(delta_carry_kernel<DN>, dim3(a.n_seqs, a.H, (a.V + DN - 1) / DN), dim3(256), smem, stream, a);
 }
 
 ZAI_API int zai_gated_delta_chunk_rows() { return DC; }
@@ -1208,7 +1208,7 @@ ZAI_API int zai_gated_delta_chunked(float* o_out, const void* qkv, int qkv_strid
                                     const int* slot_ids, int num_slots, int* status, int n_seqs, int H, int G, int D, int V, int channel,
                                     int write_state, int min_rows, void* scratch, int max_chunks, cudaStream_t stream) {
     if (n_seqs <= 0 || max_chunks <= 0) return ZAI_OK;
-    if (H < 1 || H > 65535 || n_seqs > 65535 || G < 1 || H % G || !zai_gated_delta_chunked_supports(D, V)) return ZAI_BAD_SIZE;
+    if (H < 1 || H > 65535 || G < 1 || H % G || !zai_gated_delta_chunked_supports(D, V)) return ZAI_BAD_SIZE;
     DeltaChunk* chunks = (DeltaChunk*)scratch;
     const DeltaArgs a = {(const bf16*)qkv, (const bf16*)b_in, (const bf16*)a_in, qkv_stride, b_stride, a_stride, a_log, dt_bias, unit_eps,
                          state, cu_q, slot_ids, status, num_slots, n_seqs, H, G, D, V, write_state, min_rows < 1 ? 1 : min_rows,

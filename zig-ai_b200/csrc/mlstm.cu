@@ -375,13 +375,13 @@ __global__ void __launch_bounds__(256) mlstm_chunk_state_kernel(const MlstmArgs 
     }
 }
 
-// pass 2: a thread carries four neighbouring columns of one row of S across every chunk of a request (blockIdx.z); the maximum's
+// pass 2: a thread carries four neighbouring columns of one row of S across every chunk of a request (blockIdx.x); the maximum's
 // way is the same sum in every thread.
 __global__ void __launch_bounds__(128) mlstm_state_pass_kernel(const MlstmArgs a) {
     constexpr int AHEAD = 8;                                 // chunks whose loads are in flight
     pdl_trigger();
     pdl_wait();
-    const int s = blockIdx.z, h = blockIdx.y;
+    const int s = blockIdx.x, h = blockIdx.y;
     const int rows = a.cu_q[s + 1] - a.cu_q[s];
     if (rows < a.min_rows) return;
     int c0 = 0;
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(128) mlstm_state_pass_kernel(const MlstmArgs a
         if (n >= a.min_rows) c0 += (n + MLSTM_Q - 1) / MLSTM_Q;
     }
     const int nc = (rows + MLSTM_Q - 1) / MLSTM_Q, per = a.VP / 4;
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    const int idx = blockIdx.z * blockDim.x + threadIdx.x;
     if (idx >= a.D * per) return;
     const int d = idx / per, col = (idx % per) * 4, cols = a.Dv + 1;
     const int slot = zai_checked_slot(a.slot_ids[s], a.num_slots, a.status);
@@ -682,7 +682,7 @@ ZAI_API int zai_mlstm_chunked(void* out, const void* y, int y_stride, int q_at, 
                               const int* cu_q, const int* slot_ids, int num_slots, int* status, int n_seqs, int H, int D, int Dv,
                               int write_state, int min_rows, float* ends, double* gates, float* m_in, int max_chunks, cudaStream_t stream) {
     if (n_seqs <= 0 || max_chunks <= 0) return ZAI_OK;
-    if (H < 1 || H > 65535 || n_seqs > 65535 || cap <= 0.f || !zai_mlstm_chunked_supports(D, Dv)) return ZAI_BAD_SIZE;
+    if (H < 1 || H > 65535 || cap <= 0.f || !zai_mlstm_chunked_supports(D, Dv)) return ZAI_BAD_SIZE;
     const MlstmArgs a = {(const bf16*)y, y_stride, q_at, k_at, v_at, g_at, i_at, f_at, bias_i, bias_f, cap, state, cu_q, slot_ids, status,
                          num_slots, n_seqs, H, D, Dv, write_state, min_rows < 1 ? 1 : min_rows, ends, gates, m_in, (Dv + 4) & ~3};
     static unsigned long long done = 0;
@@ -692,7 +692,7 @@ ZAI_API int zai_mlstm_chunked(void* out, const void* y, int y_stride, int q_at, 
     }
     int rc = launch_pdl(mlstm_chunk_state_kernel, dim3(max_chunks, H, (Dv + 63) / 64), dim3(256), mlstm_state_smem(D), stream, a);
     if (rc) return rc;
-    rc = launch_pdl(mlstm_state_pass_kernel, dim3((D * (a.VP / 4) + 127) / 128, H, n_seqs), dim3(128), 0, stream, a);
+    rc = launch_pdl(mlstm_state_pass_kernel, dim3(n_seqs, H, (D * (a.VP / 4) + 127) / 128), dim3(128), 0, stream, a);
     if (rc) return rc;
     return Dv <= 64 ? mlstm_chunk_out<64>(a, (bf16*)out, weight, eps, max_chunks, stream)
                     : mlstm_chunk_out<128>(a, (bf16*)out, weight, eps, max_chunks, stream);
