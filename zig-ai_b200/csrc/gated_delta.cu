@@ -1202,11 +1202,11 @@ ZAI_API int zai_gated_delta_chunk_bytes(int V) { return (int)(sizeof(DeltaChunk)
 
 // o_out [N, H V] 32-bit and the state of every span of min_rows rows or more, bfloat16, in chunks.  scratch: max_chunks x H x
 // zai_gated_delta_chunk_bytes(V) bytes, on a boundary of 16; rows / DC + n_seqs chunks are always enough.  `channel`: a decay per
-// head and key channel (a and dt_bias H D wide).
+// head and key channel (a and dt_bias H D wide).  n_spans: how many such spans there are (or the most there may be).
 ZAI_API int zai_gated_delta_chunked(float* o_out, const void* qkv, int qkv_stride, const void* b_in, int b_stride, const void* a_in,
                                     int a_stride, const float* a_log, const float* dt_bias, float unit_eps, float* state, const int* cu_q,
                                     const int* slot_ids, int num_slots, int* status, int n_seqs, int H, int G, int D, int V, int channel,
-                                    int write_state, int min_rows, void* scratch, int max_chunks, cudaStream_t stream) {
+                                    int write_state, int min_rows, int n_spans, void* scratch, int max_chunks, cudaStream_t stream) {
     if (n_seqs <= 0 || max_chunks <= 0) return ZAI_OK;
     if (H < 1 || H > 65535 || G < 1 || H % G || !zai_gated_delta_chunked_supports(D, V)) return ZAI_BAD_SIZE;
     DeltaChunk* chunks = (DeltaChunk*)scratch;
@@ -1222,7 +1222,12 @@ ZAI_API int zai_gated_delta_chunked(float* o_out, const void* qkv, int qkv_strid
     const int rc = channel ? launch_pdl(delta_chunk_kernel<true>, dim3(max_chunks, H), dim3(256), sizeof(DeltaShared), stream, a)
                            : launch_pdl(delta_chunk_kernel<false>, dim3(max_chunks, H), dim3(256), sizeof(DeltaShared), stream, a);
     if (rc) return rc;
-    // 16 columns a block while that leaves no SM with two, else 32 (half the operand loads a column)
-    if ((V + 15) / 16 * H <= 148) return delta_carry<16>(a, stream);
+    // 16 columns a block while that leaves no SM with two, else 32 (half the operand loads a column; the same sums a column)
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 148;
+    }
+    if ((long long)((V + 15) / 16) * H * n_spans <= sms) return delta_carry<16>(a, stream);
     return delta_carry<32>(a, stream);
 }

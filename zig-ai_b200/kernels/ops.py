@@ -85,7 +85,7 @@ _SIGNATURES = {
         "zai_gated_delta_chunk_rows": [],
         "zai_gated_delta_chunked_supports": [_I, _I],
         "zai_gated_delta_chunk_bytes": [_I],
-        "zai_gated_delta_chunked": [_P, _P, _I, _P, _I, _P, _I, _P, _P, _F, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _I, _P],
+        "zai_gated_delta_chunked": [_P, _P, _I, _P, _I, _P, _I, _P, _P, _F, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _I, _P],
         "zai_gated_rmsnorm": [_P, _P, _P, _P, _I, _I, _F, _I, _I, _I, _I, _P],
         "zai_gated_delta_single_supports": [_I, _I],
         "zai_gated_delta_single": [_P, _P, _I, _P, _I, _P, _I, _P, _I, _I, _P, _P, _P, _F, _F, _P, _P, _I, _I, _I, _I, _I, _I, _I,
@@ -1332,11 +1332,17 @@ def _span_kinds(step, cut):
     return max(step.q_lens) >= cut, any(0 < n < cut for n in step.q_lens)
 
 
-def _chunk_bound(step, cut, rows):
-    """How many chunks of `rows` rows a step's spans of `cut` rows or more make; of a captured step shape, the most that its rows and
-    spans allow (at most n_tokens // cut spans are that long, and each may end with a part of a chunk)."""
+def _chunked_spans(step, cut):
+    """How many spans of `cut` rows or more a step has; of a captured step shape, the most that its rows and spans allow."""
     if getattr(step, "attn_tiles", None) or not step.q_lens:
-        return step.n_tokens // rows + min(step.n_seqs, step.n_tokens // cut)
+        return min(step.n_seqs, step.n_tokens // cut)
+    return sum(n >= cut for n in step.q_lens)
+
+
+def _chunk_bound(step, cut, rows):
+    """How many chunks of `rows` rows those spans make (each may end with a part of a chunk), or the most they may make."""
+    if getattr(step, "attn_tiles", None) or not step.q_lens:
+        return step.n_tokens // rows + _chunked_spans(step, cut)
     return sum(-(-n // rows) for n in step.q_lens if n >= cut)
 
 
@@ -1468,8 +1474,8 @@ def gated_delta(qkv, b, a, gate, a_log, dt_bias, norm_w, eps, state, step, heads
         scratch = torch.empty(max_chunks * H * _fn(lib, "zai_gated_delta_chunk_bytes")(V), dtype=torch.uint8, device=dev)
         _check(_fn(lib, "zai_gated_delta_chunked")(
             _ptr(o), qp, qs, bp, bs, ap, as_, _ptr(a_log), _ptr(dt_bias), float(unit_eps), _ptr(state), _ptr(step.cu_q), _ptr(step.slot_ids),
-            state.shape[0], _status_ptr(dev), step.n_seqs, H, G, D, V, ch, int(bool(write_state)), cut, _ptr(scratch), max_chunks,
-            _stream()), "gated_delta_chunked", 2)
+            state.shape[0], _status_ptr(dev), step.n_seqs, H, G, D, V, ch, int(bool(write_state)), cut, _chunked_spans(step, cut),
+            _ptr(scratch), max_chunks, _stream()), "gated_delta_chunked", 2)
     if short and cut > 1:
         qk = torch.empty((N, 2, G, D), dtype=torch.float32, device=dev)
         bg = torch.empty((N, 2, H), dtype=torch.float32, device=dev)
