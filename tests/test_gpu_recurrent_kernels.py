@@ -389,3 +389,49 @@ def test_recurrences_in_chunks_beside_very_many_requests():
         assert torch.equal(a[:65600], b[:65600]) and torch.equal(sa[1:65601], sb[1:65601])
         assert torch.allclose(a.float(), b.float(), **tol(torch.bfloat16)) and torch.allclose(sa, sb, atol=1e-4, rtol=1e-4)
     assert o.read_status() == 0
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("I,S,R", [(96, 16, 8), (36, 12, 4), (68, 4, 4), (20, 28, 8), (24, 64, 8), (20, 100, 8), (12, 200, 4), (256, 16, 16)])
+@pytest.mark.parametrize("impl", [None, "chunks"])
+def test_selective_scan_of_spans_in_fours(dtype, I, S, R, impl):
+    """Rows that are read four values a load (channels, states and strides in fours), at the remainders of tiles of 32 and 64 rows, of
+    the channels of a block and of chunks of 512 rows, beside single tokens and a span without rows."""
+    o = ops()
+    g = torch.Generator().manual_seed(28)
+    w_dt, b_dt, d = (torch.randn(I, R, generator=g) * 0.5).to(dtype).cuda(), (torch.randn(I, generator=g) * 0.5 - 1).cuda(), torch.randn(I, generator=g).cuda()
+    a_log = (torch.randn(I, S, generator=g) * 0.5 - 1).cuda()
+    state_a = torch.randn(9, I, S, generator=g).cuda()
+    state_b = state_a.clone()
+    for q_lens in ([2, 1, 61, 64, 3], [1, 129, 0, 300], [63, 65, 1, 1], [32, 33], [511, 1, 512], [513, 2, 1025]):
+        step = make_step(o, dtype, [3] * len(q_lens), q_lens, 8, 600, 5)
+        N = sum(q_lens)
+        x, proj, z = (torch.randn(N, n, generator=g).to(dtype).cuda() for n in (I, R + 2 * S, I))
+        ya = o.selective_scan(x, proj, z, w_dt, b_dt, a_log, d, state_a, step, R, True, impl=impl)
+        yb = ref_ops.selective_scan(x, proj, z, w_dt, b_dt, a_log, d, state_b, step, R, True)
+        # the limits of test_selective_scan
+        assert torch.allclose(ya.float(), yb.float(), **tol(dtype)), (q_lens, float((ya.float() - yb.float()).abs().max()))
+        assert torch.allclose(state_a, state_b, atol=1e-4, rtol=1e-4), (q_lens, float((state_a - state_b).abs().max()))
+        state_a.copy_(state_b)
+    keep = state_a.clone()
+    o.selective_scan(x, proj, z, w_dt, b_dt, a_log, d, state_a, step, R, False, impl=impl)
+    assert torch.equal(state_a, keep)
+    assert o.read_status() == 0
+
+
+def test_selective_scan_does_not_depend_on_neighbours_or_capture():
+    o = ops()
+    g = torch.Generator().manual_seed(29)
+    I, S, R, most, dtype = 48, 16, 4, 3000, torch.bfloat16
+    w_dt, b_dt, d = (torch.randn(I, R, generator=g) * 0.5).to(dtype).cuda(), (torch.randn(I, generator=g) * 0.5 - 1).cuda(), torch.randn(I, generator=g).cuda()
+    a_log, first = (torch.randn(I, S, generator=g) * 0.5 - 1).cuda(), torch.randn(I, S, generator=g).cuda()
+    x, proj, z = (torch.randn(most, n, generator=g).to(dtype).cuda() for n in (I, R + 2 * S, I))
+
+    def run(q_lens, shift, captured):
+        step = make_step(o, dtype, [3] * len(q_lens), q_lens, 8, 2 * sum(q_lens) // 8 + 8 * len(q_lens) + 8, 5)
+        if captured:
+            step.attn_tiles = sum(q_lens) // 128 + len(q_lens)
+        rows = torch.cat([(torch.arange(n) + k) % most for n, k in zip(q_lens, shift)]).cuda()
+        state = first.repeat(len(q_lens) + 2, 1, 1)
+        return o.selective_scan(x[rows], proj[rows], z[rows], w_dt, b_dt, a_log, d, state, step, R, True), state[1:]
+    same_alone_and_beside(run, (2, 300, 2047, 2048, 2600), ([2, 130], [1, 0, 2100]))

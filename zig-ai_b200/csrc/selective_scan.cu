@@ -10,7 +10,8 @@
 // (on the tensor cores where the model is bfloat16).  Two kernels:
 //   * steps of single tokens: a lane holds K consecutive states of a channel (a whole channel where S <= 16, else G lanes
 //     of a warp share it), loads its row's values and sums its step size itself;
-//   * steps with portions: a block walks one request's rows in order, two states a lane, fed by warps of its own.
+//   * steps with portions: a block walks one request's rows in order, two states a lane (four and eight beyond 64 and 128), fed by warps
+//     of its own; long spans of few channels are cut into chunks that are walked at once (below).
 #include <cfloat>
 #include "mma_helpers.cuh"
 
@@ -149,18 +150,18 @@ __global__ void __launch_bounds__(128) selective_scan_single_kernel(
 }
 
 // ---- steps with portions.  A block walks one request's rows for 128 / G channels, in tiles of 64 rows (32 with more than
-// 64 states).  Four warps walk: a
-// lane holds K states of a channel, and what a row gives it comes out of shared memory as 32-bit numbers, four rows ahead of
-// their use.  Four more warps put the next tile there meanwhile (step sizes, their products with x, the gates; a tile's loads
-// are issued while the tile before it is walked) and take the read-outs of the tile before to y.  One barrier a tile.
+// 64 states).  Four warps walk: a lane holds K states of a channel, and what a row gives it comes out of shared memory as 32-bit
+// numbers, four rows ahead of their use.  Four more warps put the next tile there meanwhile (step sizes, their products with x, the
+// gates; a tile's loads are issued while the tile before it is walked) and take the read-outs of the tile before to y.  One barrier
+// a tile.
 //
-// What bounds it: S exponentials a row and channel, which the special-function units make at 16 a cycle and SM.  Cutting the
-// rows into chunks that run at once (three passes: the chunks' end states, the carry, the rows again) makes them twice and moves
-// a state per chunk through memory; one walk makes them once, and with two states a lane 2048 channels give every scheduler of
-// the chip a warp.  A portion of 2048 rows with 16 states (us, its step sizes' product included): 134 for 4096 channels (three
-// passes: 309), 92 for 2048 (172), 91 for 1024 (129); 512 rows of 4096 channels 40 (104).  A row costs about 45 ns however few
-// the channels are (dependent instructions, one warp a scheduler): below 1024 channels and beyond 2048 rows chunks would be
-// faster again (8192 rows of 512 channels 331, in chunks 220).
+// What bounds it: S exponentials a row and channel, which the special-function units make at 16 a cycle and SM, and, where the
+// channels are few, a row's chain of dependent instructions (38 ns with two states a lane, 53 with four).  A walk makes the exponentials
+// once; with two states a lane 2048 channels of 16 states give every scheduler of the chip a warp.  One span of 2048 rows, 16 states
+// (us, without the step sizes' product): 119 for 4096 channels (three passes over chunks of 16 to 64 rows: 296), 82 for 2048 (160);
+// 512 rows of 4096 channels 31 (94).  States a lane, by S: up to 16 states 2 on 8 lanes (8 states, 4096 channels: 118, 2 on 4 lanes
+// 150, whose feeding warps are too slow), 64 states 4 on 16 lanes (1024 channels: 109; 2 on 32 lanes 130), 128 states 4 on 32 lanes
+// (512 channels: 212; 8 on 16 lanes 281), 256 states 8 on 32 lanes (200 states, 512 channels: 447; 16 on 16 lanes, which spills, 1018).
 // (a rate beyond the largest number counts as that: a row with a step of zero leaves the state alone, zero times infinity would not)
 __device__ __forceinline__ float decay_bound(float a) { return a < -FLT_MAX ? -FLT_MAX : a; }
 template <typename T> __device__ __forceinline__ float decay_scale(float a) { return decay_bound(a); }
@@ -232,8 +233,8 @@ struct ScanTile {                                            // a tile in shared
 };
 
 // the rows' way in and out, by 128 threads.  VEC: channels, states and every row of x, z, proj, dt_raw and y lie in fours on
-// boundaries of four
-template <typename T, int K, int G, bool VEC>
+// boundaries of four.  ENDS: nothing goes out
+template <typename T, int K, int G, bool VEC, bool ENDS>
 __device__ __forceinline__ void scan_feed(ScanTile<K, G>* tiles, int tid, int c0, int start, int end, T* __restrict__ y,
                                           const T* __restrict__ x, const T* __restrict__ proj, int proj_stride, const T* __restrict__ z,
                                           int z_stride, const float* __restrict__ dt_raw, const float* __restrict__ b_dt,
@@ -261,14 +262,14 @@ __device__ __forceinline__ void scan_feed(ScanTile<K, G>* tiles, int tid, int c0
                 if (nc > 0) {
                     in.dt[i].load(dt_raw + (size_t)t * I + c0 + cq);
                     in.xv[i].load(x + (size_t)t * I + c0 + cq);
-                    in.zv[i].load(z + (size_t)t * z_stride + c0 + cq);
+                    if (!ENDS) in.zv[i].load(z + (size_t)t * z_stride + c0 + cq);
                 } else {
                     in.dt[i].zero(); in.xv[i].zero(); in.zv[i].zero();
                 }
             } else {
                 in.dt[i].load_some(dt_raw + (size_t)t * I + c0 + cq, nc);
                 in.xv[i].load_some(x + (size_t)t * I + c0 + cq, nc);
-                in.zv[i].load_some(z + (size_t)t * z_stride + c0 + cq, nc);
+                if (!ENDS) in.zv[i].load_some(z + (size_t)t * z_stride + c0 + cq, nc);
             }
         }
 #pragma unroll
@@ -307,7 +308,7 @@ __device__ __forceinline__ void scan_feed(ScanTile<K, G>* tiles, int tid, int c0
     fetch(0, in);
     for (int n = 0; n <= n_tiles; ++n) {
         const int t0 = start + n * TT;
-        if (n >= 2) leave(n - 2);                            // (its buffer is the one that tile n is put into)
+        if (!ENDS && n >= 2) leave(n - 2);                   // (its buffer is the one that tile n is put into)
         if (n < n_tiles) {
             Tile& tile = tiles[n & 1];
 #pragma unroll
@@ -315,7 +316,7 @@ __device__ __forceinline__ void scan_feed(ScanTile<K, G>* tiles, int tid, int c0
                 const int r = r0 + i * ROWS;
                 if (r >= TT || t0 + r >= end + 3) continue;  // (rows in fours)
                 const bool on = t0 + r < end;
-                const float4 df = in.dt[i].get(), xf = in.xv[i].get(), zf = in.zv[i].get();
+                const float4 df = in.dt[i].get(), xf = in.xv[i].get(), zf = ENDS ? make_float4(0.f, 0.f, 0.f, 0.f) : in.zv[i].get();
                 const float d4[4] = {df.x, df.y, df.z, df.w}, x4[4] = {xf.x, xf.y, xf.z, xf.w}, z4[4] = {zf.x, zf.y, zf.z, zf.w};
                 float2 l[4];
 #pragma unroll
@@ -323,10 +324,12 @@ __device__ __forceinline__ void scan_feed(ScanTile<K, G>* tiles, int tid, int c0
                     const float d = on ? softplus_for<T>(d4[k] + bias[k]) : 0.f;          // (a row beyond the span changes no state)
                     const float dx = d * x4[k];
                     tile.step[r][cq + k] = make_float4(d, d, dx, dx);
-                    l[k] = make_float2(skip[k] * x4[k], silu_for<T>(z4[k]));
+                    if (!ENDS) l[k] = make_float2(skip[k] * x4[k], silu_for<T>(z4[k]));
                 }
+                if (!ENDS) {
 #pragma unroll
-                for (int k = 0; k < 4; k += 2) *reinterpret_cast<float4*>(&tile.last[r][cq + k]) = make_float4(l[k].x, l[k].y, l[k + 1].x, l[k + 1].y);
+                    for (int k = 0; k < 4; k += 2) *reinterpret_cast<float4*>(&tile.last[r][cq + k]) = make_float4(l[k].x, l[k].y, l[k + 1].x, l[k + 1].y);
+                }
             }
 #pragma unroll
             for (int i = 0; i < BC; ++i) *reinterpret_cast<float4*>(&tile.bc[0][0] + (tid + i * 128) * 4) = in.bc[i].get();
@@ -334,15 +337,43 @@ __device__ __forceinline__ void scan_feed(ScanTile<K, G>* tiles, int tid, int c0
         }
         __syncthreads();                                     // tile n is there, tile n - 1 has been walked
     }
-    leave(n_tiles - 1);
+    if (!ENDS) leave(n_tiles - 1);
 }
 
-template <typename T, int K, int G>
+// A walk is one chain of rows: where a layer's channels are few blocks and a span is long, most of the chip waits for it.  Spans of
+// min_rows rows or more are cut into chunks of SCAN_CHUNK rows there, which run as
+//   ENDS      every chunk walked from a state of zero: its end state E and, state by state, the product P of its decays
+//   carry     across a request's chunks, in order: E <- the state before the chunk, which becomes P state + E
+//   the walk  of every chunk from its own first state
+// The recurrence is linear in its state: the same sums in another order.  One span of 16 states, walked and in chunks (us): 2048 rows
+// of 256 channels 82 and 37, of 1024 80 and 51, of 2048 (128 blocks) 82 and 84; 8192 rows of 512 channels 313 and 100.
+#define SCAN_CHUNK 512
+struct ScanChunks {
+    float *ends, *decays;                                    // [chunks, I, S]; null: spans are walked whole
+    int n_seqs, min_rows, max_rows;                          // (whole: spans of up to max_rows)
+};
+// the rows of chunk b among all chunks of the step: those of the spans of min_rows rows or more, in order
+__device__ __forceinline__ bool scan_find_chunk(const int* __restrict__ cu_q, const ScanChunks& ch, int b, int& start, int& end) {
+    for (int s = 0; s < ch.n_seqs; ++s) {
+        const int lo = cu_q[s], hi = cu_q[s + 1];
+        if (hi - lo < ch.min_rows) continue;
+        const int n = (hi - lo + SCAN_CHUNK - 1) / SCAN_CHUNK;
+        if (b < n) {
+            start = lo + b * SCAN_CHUNK;
+            end = min(start + SCAN_CHUNK, hi);
+            return true;
+        }
+        b -= n;
+    }
+    return false;
+}
+
+template <typename T, int K, int G, bool ENDS>
 __global__ void __launch_bounds__(256) selective_scan_kernel(
     T* __restrict__ y, const T* __restrict__ x, const T* __restrict__ proj, int proj_stride, const T* __restrict__ z,
     int z_stride, const float* __restrict__ dt_raw, const float* __restrict__ b_dt,
     const float* __restrict__ a_log, const float* __restrict__ d_skip, float* __restrict__ state, const int* __restrict__ cu_q,
-    const int* __restrict__ slot_ids, int I, int S, int R, int write_state, int num_slots, int* __restrict__ status, int vec) {
+    const int* __restrict__ slot_ids, int I, int S, int R, int write_state, int num_slots, int* __restrict__ status, int vec, const ScanChunks ch) {
     using Tile = ScanTile<K, G>;
     constexpr int CB = Tile::CB, SP = Tile::SP, TT = Tile::TT;
     extern __shared__ __align__(16) unsigned char scan_raw[];
@@ -350,9 +381,14 @@ __global__ void __launch_bounds__(256) selective_scan_kernel(
     pdl_trigger();
     pdl_wait();
     const int seq = blockIdx.x, c0 = blockIdx.y * CB;
-    const int start = cu_q[seq], end = cu_q[seq + 1];
-    if (end <= start) return;
-    if (end - start == 1) {                                  // (a decoding request beside the portions: no tile for one row)
+    int start, end;
+    if (ch.ends) {
+        if (!scan_find_chunk(cu_q, ch, blockIdx.x, start, end)) return;
+    } else {
+        start = cu_q[seq], end = cu_q[seq + 1];
+        if (end <= start || end - start > ch.max_rows) return;
+    }
+    if (!ENDS && !ch.ends && end - start == 1) {             // (a decoding request beside the portions: no tile for one row)
         if (threadIdx.x < 128)
             scan_one_row<T, K, G>(y, x, proj, proj_stride, z, z_stride, dt_raw, nullptr, b_dt, a_log, d_skip, state, start,
                                   zai_checked_slot(slot_ids[seq], num_slots, status), I, S, R, write_state);
@@ -360,8 +396,8 @@ __global__ void __launch_bounds__(256) selective_scan_kernel(
     }
     const int n_tiles = (end - start + TT - 1) / TT;
     if (threadIdx.x >= 128) {
-        if (vec) scan_feed<T, K, G, true>(tiles, threadIdx.x - 128, c0, start, end, y, x, proj, proj_stride, z, z_stride, dt_raw, b_dt, d_skip, I, S, R);
-        else scan_feed<T, K, G, false>(tiles, threadIdx.x - 128, c0, start, end, y, x, proj, proj_stride, z, z_stride, dt_raw, b_dt, d_skip, I, S, R);
+        if (vec) scan_feed<T, K, G, true, ENDS>(tiles, threadIdx.x - 128, c0, start, end, y, x, proj, proj_stride, z, z_stride, dt_raw, b_dt, d_skip, I, S, R);
+        else scan_feed<T, K, G, false, ENDS>(tiles, threadIdx.x - 128, c0, start, end, y, x, proj, proj_stride, z, z_stride, dt_raw, b_dt, d_skip, I, S, R);
         return;
     }
 
@@ -370,16 +406,17 @@ __global__ void __launch_bounds__(256) selective_scan_kernel(
     int c = c0 + cl;
     const bool live = c < I;
     if (!live) c = I - 1;
-    const int slot = zai_checked_slot(slot_ids[seq], num_slots, status);
     const int n_mine = max(min(S - g * K, K), 0);
-    float* st = state + ((size_t)slot * I + c) * S + g * K;
-    float h1[K];
-    uint64_t h[K / 2], a[K / 2];                             // states in pairs
-    state_io<K>(st, h1, n_mine, false);
+    float* st = ch.ends ? ch.ends + ((size_t)blockIdx.x * I + c) * S + g * K
+                        : state + ((size_t)zai_checked_slot(slot_ids[seq], num_slots, status) * I + c) * S + g * K;
+    float h1[K] = {};
+    uint64_t h[K / 2], a[K / 2], product[K / 2];             // states in pairs
+    if (!ENDS) state_io<K>(st, h1, n_mine, false);
 #pragma unroll
     for (int k = 0; k < K; k += 2) {
         const float* al = a_log + (size_t)c * S + g * K + k;
         h[k / 2] = make_pair(h1[k], h1[k + 1]);
+        product[k / 2] = make_pair(1.f, 1.f);
         a[k / 2] = make_pair(k < n_mine ? decay_scale<T>(-expf(al[0])) : 0.f, k + 1 < n_mine ? decay_scale<T>(-expf(al[1])) : 0.f);
     }
     struct Rows { ulonglong2 d[4]; uint64_t b[4][K / 2], c[4][K / 2]; };    // four rows' operands
@@ -391,7 +428,7 @@ __global__ void __launch_bounds__(256) selective_scan_kernel(
 #pragma unroll
             for (int k = 0; k < K / 2; ++k) {
                 o.b[u][k] = p[k];
-                o.c[u][k] = p[SP / 2 + k];
+                if (!ENDS) o.c[u][k] = p[SP / 2 + k];
             }
         }
     };
@@ -430,22 +467,26 @@ __global__ void __launch_bounds__(256) selective_scan_kernel(
 #pragma unroll
                 for (int k = 0; k < K / 2; ++k) {
                     const float2 v = pair_of(mul_pair(now.d[u].x, a[k]));
-                    h[k] = fma_pair(make_pair(decay_of<T>(v.x), decay_of<T>(v.y)), h[k], mul_pair(now.d[u].y, now.b[u][k]));
-                    sum = k ? fma_pair(h[k], now.c[u][k], sum) : mul_pair(h[k], now.c[u][k]);
+                    const uint64_t decay = make_pair(decay_of<T>(v.x), decay_of<T>(v.y));
+                    h[k] = fma_pair(decay, h[k], mul_pair(now.d[u].y, now.b[u][k]));
+                    if (ENDS) product[k] = mul_pair(product[k], decay);
+                    else sum = k ? fma_pair(h[k], now.c[u][k], sum) : mul_pair(h[k], now.c[u][k]);
                 }
                 const float2 both = pair_of(sum);
                 out[u] = both.x + both.y;
-                if (r > 0) settle(tile, r - 4, u, before);
+                if (!ENDS && r > 0) settle(tile, r - 4, u, before);
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) before[u] = out[u];
             now = next;
         }
+        if (!ENDS) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) settle(tile, r - 4, u, before);
+            for (int u = 0; u < 4; ++u) settle(tile, r - 4, u, before);
+        }
         __syncthreads();                                     // this tile has been walked, the next one is there
     }
-    if (write_state && live) {
+    if (live && (ENDS || (write_state && !ch.ends))) {
 #pragma unroll
         for (int k = 0; k < K; k += 2) {
             const float2 v = pair_of(h[k / 2]);
@@ -453,7 +494,40 @@ __global__ void __launch_bounds__(256) selective_scan_kernel(
             h1[k + 1] = v.y;
         }
         state_io<K>(st, h1, n_mine, true);
+        if (ENDS) {
+#pragma unroll
+            for (int k = 0; k < K; k += 2) {
+                const float2 v = pair_of(product[k / 2]);
+                h1[k] = v.x;
+                h1[k + 1] = v.y;
+            }
+            state_io<K>(ch.decays + ((size_t)blockIdx.x * I + c) * S + g * K, h1, n_mine, true);
+        }
     }
+}
+
+// a thread carries one state of a request (blockIdx.x) across its chunks
+__global__ void __launch_bounds__(128) selective_scan_carry_kernel(float* __restrict__ state, const int* __restrict__ cu_q, const int* __restrict__ slot_ids,
+                                                                   int IS, int write_state, int num_slots, int* __restrict__ status, const ScanChunks ch) {
+    pdl_trigger();
+    pdl_wait();
+    const int seq = blockIdx.x, rows = cu_q[seq + 1] - cu_q[seq], idx = blockIdx.y * blockDim.x + threadIdx.x;
+    if (rows < ch.min_rows || idx >= IS) return;
+    int first = 0;
+    for (int s = 0; s < seq; ++s) {
+        const int n = cu_q[s + 1] - cu_q[s];
+        if (n >= ch.min_rows) first += (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
+    }
+    const int nc = (rows + SCAN_CHUNK - 1) / SCAN_CHUNK;
+    float* st = state + (size_t)zai_checked_slot(slot_ids[seq], num_slots, status) * IS + idx;
+    float h = *st;
+    for (int c = 0; c < nc; ++c) {
+        float* e = ch.ends + (size_t)(first + c) * IS + idx;
+        const float end = *e, decay = ch.decays[(size_t)(first + c) * IS + idx];
+        *e = h;
+        h = fmaf(decay, h, end);
+    }
+    if (write_state) *st = h;
 }
 
 template <typename T, int K, int G>
@@ -472,32 +546,53 @@ template <typename T, int K, int G>
 static int launch_scan(void* y, const void* x, const void* proj, int proj_stride, const void* z, int z_stride, const float* dt_raw,
                        const float* b_dt, const float* a_log, const float* d_skip, float* state, const int* cu_q,
                        const int* slot_ids, int n_seqs, int I, int S, int R, int write_state, int num_slots, int* status,
-                       cudaStream_t stream) {
+                       const ScanChunks& chunks, int max_chunks, cudaStream_t stream) {
     const unsigned cb = (unsigned)((I + 128 / G - 1) / (128 / G));
     if (cb > 65535) return ZAI_BAD_SIZE;
     constexpr size_t smem = 2 * sizeof(ScanTile<K, G>);
     static_assert(smem <= 227 * 1024, "two tiles fit");
     static unsigned long long done = 0;
     if (zai_first_on_device(&done)) {
-        const cudaError_t e = cudaFuncSetAttribute(selective_scan_kernel<T, K, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(selective_scan_kernel<T, K, G, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(selective_scan_kernel<T, K, G, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
     }
     const uintptr_t four = 4 * sizeof(T) - 1;
     const int vec = ((I | S | R | proj_stride | z_stride) & 3) == 0 && (reinterpret_cast<uintptr_t>(dt_raw) & 15) == 0
                     && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(proj)) & four) == 0;
-    return launch_pdl(selective_scan_kernel<T, K, G>, dim3(n_seqs, cb), dim3(256), smem, stream, (T*)y, (const T*)x, (const T*)proj,
-                      proj_stride, (const T*)z, z_stride, dt_raw, b_dt, a_log, d_skip, state, cu_q, slot_ids, I, S, R, write_state,
-                      num_slots, status, vec);
+    auto walk = [&](void (*kernel)(T*, const T*, const T*, int, const T*, int, const float*, const float*, const float*, const float*, float*,
+                                   const int*, const int*, int, int, int, int, int, int*, int, const ScanChunks), int blocks, const ScanChunks& ch) {
+        return launch_pdl(kernel, dim3(blocks, cb), dim3(256), smem, stream, (T*)y, (const T*)x, (const T*)proj, proj_stride, (const T*)z,
+                          z_stride, dt_raw, b_dt, a_log, d_skip, state, cu_q, slot_ids, I, S, R, write_state, num_slots, status, vec, ch);
+    };
+    if (max_chunks > 0) {
+        if ((long long)I * S > 65535LL * 128) return ZAI_BAD_SIZE;
+        int rc = walk(selective_scan_kernel<T, K, G, true>, max_chunks, chunks);
+        if (rc) return rc;
+        rc = launch_pdl(selective_scan_carry_kernel, dim3(n_seqs, (I * S + 127) / 128), dim3(128), 0, stream, state, cu_q, slot_ids, I * S, write_state,
+                        num_slots, status, chunks);
+        if (rc) return rc;
+        rc = walk(selective_scan_kernel<T, K, G, false>, max_chunks, chunks);
+        if (rc || chunks.max_rows < 1) return rc;
+    }
+    return walk(selective_scan_kernel<T, K, G, false>, n_seqs, ScanChunks{nullptr, nullptr, n_seqs, 0, chunks.max_rows});
 }
+
+// channels of a block of the kernel that walks portions, by the number of states
+ZAI_API int zai_selective_scan_channels(int S) { return S <= 16 ? 16 : S <= 64 ? 8 : 4; }
+ZAI_API int zai_selective_scan_chunk_rows() { return SCAN_CHUNK; }
 
 // y [N, I]; x [N, I]; proj [N, proj_stride] (dt_in | B | C, of which B and C are read here); z [N, z_stride];
 // dt_raw [N, I]: the products dt_in . w_dt^T in 32-bit (a matrix product made beforehand), or null in a step of single
 // tokens, which then sums them from w_dt [I, R] itself; state [slots, I, S].
 // single_tokens: every request brings one row (a leaner kernel).
+// With max_chunks > 0 spans of min_rows rows or more run in chunks of SCAN_CHUNK rows: ends and decays [max_chunks, I, S] 32-bit scratch,
+// max_chunks at least the number of their chunks; `others`: there may be shorter spans too.
 ZAI_API int zai_selective_scan(void* y, const void* x, const void* proj, int proj_stride, const void* z, int z_stride, int dtype,
                                const float* dt_raw, const void* w_dt, const float* b_dt, const float* a_log, const float* d_skip,
                                float* state, const int* cu_q, const int* slot_ids, int N, int n_seqs, int I, int S, int R, int write_state,
-                               int num_slots, int* status, int single_tokens, cudaStream_t stream) {
+                               int num_slots, int* status, int single_tokens, float* ends, float* decays, int max_chunks, int min_rows, int others,
+                               cudaStream_t stream) {
     if (N <= 0 || n_seqs <= 0) return ZAI_OK;
     if (I < 1 || S < 1 || S > 256 || R < 1 || (!dt_raw && !w_dt)) return ZAI_BAD_SIZE;
     if (single_tokens && N == n_seqs) {
@@ -512,14 +607,14 @@ ZAI_API int zai_selective_scan(void* y, const void* x, const void* proj, int pro
         ZAI_SCAN(16, 16);
 #undef ZAI_SCAN
     }
-    if (!dt_raw) return ZAI_BAD_SIZE;
+    if (!dt_raw || (max_chunks > 0 && (!ends || !decays || min_rows < 1))) return ZAI_BAD_SIZE;
+    const ScanChunks chunks = {ends, decays, n_seqs, min_rows, max_chunks <= 0 ? 0x7fffffff : others ? min_rows - 1 : 0};
 #define ZAI_SCAN(KK, GG) ZAI_DISPATCH(dtype, return launch_scan<T, KK, GG>(y, x, proj, proj_stride, z, z_stride, dt_raw, b_dt, a_log, \
-        d_skip, state, cu_q, slot_ids, n_seqs, I, S, R, write_state, num_slots, status, stream))
-    if (S <= 8) ZAI_SCAN(2, 4);
+        d_skip, state, cu_q, slot_ids, n_seqs, I, S, R, write_state, num_slots, status, chunks, max_chunks, stream))
     if (S <= 16) ZAI_SCAN(2, 8);
     if (S <= 32) ZAI_SCAN(2, 16);
     if (S <= 64) ZAI_SCAN(4, 16);
-    if (S <= 128) ZAI_SCAN(8, 16);
-    ZAI_SCAN(16, 16);
+    if (S <= 128) ZAI_SCAN(4, 32);
+    ZAI_SCAN(8, 32);
 #undef ZAI_SCAN
 }

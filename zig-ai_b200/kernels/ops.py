@@ -77,7 +77,9 @@ _SIGNATURES = {
                    "zai_weighted_sum": [_P, _P, _P, _I, _F, _F, ctypes.c_longlong, _P]},
     "causal_conv": {"zai_causal_conv": [_P, _I, _P, _I, _I, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P]},
     "selective_scan": {"zai_selective_scan": [_P, _P, _P, _I, _P, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I,
-                                              _I, _P, _I, _P]},
+                                              _I, _P, _I, _P, _P, _I, _I, _I, _P],
+                       "zai_selective_scan_channels": [_I],
+                       "zai_selective_scan_chunk_rows": []},
     "min_gru": {"zai_min_gru": [_P, _P, _I, _I, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P, _I, _I, _P]},
     "gated_delta": {
         "zai_delta_prepare": [_P, _P, _P, _P, _I, _P, _I, _P, _I, _I, _P, _P, _I, _I, _I, _I, _F, _P, _P, _I, _P],
@@ -1372,11 +1374,18 @@ def causal_conv(x, taps, bias, state, step, act=True, write_state=True):
     return out
 
 
+def _scan_cut(channel_blocks):
+    """Spans of this many rows or more run the selective scan in chunks: by the layer's sizes alone.  A walk is one chain of rows, 38 ns
+    each (53 with 64 states, 110 with 128), on `channel_blocks` SMs; chunks walk the rows twice, all chunks at once.  One span of 2048
+    rows, walked and in chunks: 32 blocks 82 and 37 us, 64 blocks 80 and 51, 128 blocks 82 and 84."""
+    return 2048 if channel_blocks <= 64 else 1 << 30
+
+
 @_timed("recurrence")
-def selective_scan(x, proj, z, w_dt, b_dt, a_log, d_skip, state, step, dt_rank, write_state=True):
+def selective_scan(x, proj, z, w_dt, b_dt, a_log, d_skip, state, step, dt_rank, write_state=True, impl=None):
     """The selective-scan recurrence: x [N, I] (after its convolution), proj [N, R + 2S] = (dt_in | B | C), z [N, I]
     (a column slice is fine), w_dt [I, R], b_dt [I], a_log [I, S], d_skip [I], state [slots, I, S] 32-bit.
-    Returns (scan + d_skip * x) * silu(z) in x's dtype."""
+    Returns (scan + d_skip * x) * silu(z) in x's dtype.  `impl` "walk" or "chunks" picks the way of spans whatever their length."""
     _cuda(x, w_dt, b_dt, a_log, d_skip, state)
     N, I = x.shape
     S, R = a_log.shape[1], int(dt_rank)
@@ -1390,11 +1399,19 @@ def selective_scan(x, proj, z, w_dt, b_dt, a_log, d_skip, state, step, dt_rank, 
     # the step sizes' products dt_in . w_dt^T for all rows as one matrix product with a 32-bit result; a step of
     # single tokens sums them inside its kernel (a launch less a layer, and the weights are read once either way)
     single = bool(step.decode_only and N == step.n_seqs)
+    cut, max_chunks, ends, decays, short = 1 << 30, 0, None, None, True
+    if not step.decode_only and impl != "walk":
+        cut = 1 if impl == "chunks" else _scan_cut(-(-I // _fn("selective_scan", "zai_selective_scan_channels")(S)))
+    long, short = _span_kinds(step, cut)
+    if long:
+        max_chunks = _chunk_bound(step, cut, _fn("selective_scan", "zai_selective_scan_chunk_rows")())
+        ends, decays = torch.empty((2, max_chunks, I, S), dtype=torch.float32, device=x.device)
     dt_raw = None if single else linear(proj[:, :R], w_dt, out_dtype=torch.float32)
     _check(_fn("selective_scan", "zai_selective_scan")(
         _ptr(y), _ptr(x), pp, ps, zp, zs, _dt(x), _ptr(dt_raw), _ptr(w_dt), _ptr(b_dt), _ptr(a_log), _ptr(d_skip), _ptr(state),
         _ptr(step.cu_q), _ptr(step.slot_ids), N, step.n_seqs, I, S, R, int(bool(write_state)), state.shape[0],
-        _status_ptr(x.device), int(bool(step.decode_only)), _stream()), "selective_scan")
+        _status_ptr(x.device), int(bool(step.decode_only)), _ptr(ends), _ptr(decays), max_chunks, cut, int(short and cut > 1), _stream()),
+        "selective_scan", 1 if not long else 4 if short and cut > 1 else 3)
     return y
 
 
