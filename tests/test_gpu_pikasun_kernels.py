@@ -392,3 +392,28 @@ def test_latent_attention_and_rows_that_are_not_finite(H, R, Dr, ps, bad):
             assert not torch.isfinite(got[r:n]).any(), (ctx, r)
             assert torch.equal(got[:r], want[:r]) and torch.equal(got[n:], want[n:]), (ctx, r)
     assert o.read_status() == 0
+
+
+def latent_case(H, R, Dr, ps, ctx, q_lens, seed, shift=0):
+    """(operands of a step, its cached rows); `shift`: the queries start that many values behind a 16-byte boundary."""
+    o = ops()
+    g = torch.Generator().manual_seed(seed)
+    num_pages = sum(-(-(c + n) // ps) for c, n in zip(ctx, q_lens)) + 8
+    step = make_step(o, torch.bfloat16, ctx, q_lens, ps, num_pages, 22)
+    pages = latent_pages(step, ctx, q_lens, ps, R + Dr, torch.bfloat16, num_pages, g)
+    N = sum(q_lens)
+    q = [torch.randn(N * H * n + shift, generator=g).to(torch.bfloat16).cuda()[shift:].view(N, H, n) for n in (R, Dr)]
+    return o, (q[0], q[1], step, CacheView(0, pages, step.block_tables[0], ps), H, R, Dr, (R + Dr) ** -0.5)
+
+
+@pytest.mark.parametrize("q_lens", [[200], [1, 1, 1]])
+def test_latent_attention_leaves_calls_to_the_general_kernel(q_lens, monkeypatch):
+    """With the tensor-core kernels switched off, and for operands off their copies' boundaries."""
+    o, case = latent_case(16, 256, 32, 64, [5] * len(q_lens), q_lens, 44)
+    assert not torch.equal(o.latent_attention(*case), o.latent_attention(*case, impl="general"))       # (the switch makes a difference)
+    monkeypatch.setattr(o, "USE_LATENT_MMA", False)
+    assert torch.equal(o.latent_attention(*case), o.latent_attention(*case, impl="general"))
+    monkeypatch.undo()
+    o, case = latent_case(16, 256, 32, 64, [5] * len(q_lens), q_lens, 44, shift=1)
+    assert torch.equal(o.latent_attention(*case), o.latent_attention(*case, impl="general"))
+    assert o.read_status() == 0

@@ -1654,7 +1654,9 @@ def latent_attention(q_lat, q_rot, step, cache, heads, rank, rot_dim, scale, imp
     if N != step.n_tokens or pages.dtype != q_lat.dtype or tuple(pages.shape[1:]) != (cache.page_size, R + Dr):
         raise KernelError("latent_attention: operands do not fit together")
     out = torch.empty((N, H, R), dtype=q_lat.dtype, device=q_lat.device)
-    if (impl in (None, "tcgen05") and q_lat.dtype == torch.bfloat16 and not step.decode_only
+    # (the tensor-core kernels' copies start on 16 bytes; ZAI_LATENT_MMA=0 leaves every call to the general kernel)
+    tensor_cores = q_lat.dtype == torch.bfloat16 and not (q_lat.data_ptr() | (q_rot.data_ptr() if Dr else 0) | pages.data_ptr()) & 15
+    if (tensor_cores and (impl == "tcgen05" or (impl is None and USE_LATENT_MMA)) and not step.decode_only
             and _fn("latent_attention_tc", "zai_latent_attention_tc_supports")(H, R, Dr, cache.page_size)):
         if impl == "tcgen05" or N * -(-H // 16) >= LATENT_TC_ROWS:
             pairs = _fn("latent_attention_tc", "zai_latent_attention_tc_pairs")()
@@ -1665,7 +1667,7 @@ def latent_attention(q_lat, q_rot, step, cache, heads, rank, rot_dim, scale, imp
                 _ptr(step.cu_q), _ptr(step.ctx_lens), N, step.n_seqs, tiles, cache.page_size, H, R, Dr, float(scale), _ptr(sink),
                 _stream()), "latent_attention_tc")
             return out
-    if (impl != "general" and (USE_LATENT_MMA or impl in ("mma", "mma_rows", "mma_ranges")) and q_lat.dtype == torch.bfloat16
+    if (impl != "general" and (USE_LATENT_MMA or impl in ("mma", "mma_rows", "mma_ranges")) and tensor_cores
             and _fn("latent_attention", "zai_latent_attention_mma_supports")(R, Dr)):
         warps = N * (-(-H // 16)) * (-(-R // (128 if R <= 128 else 256)))
         n_splits = 1 if warps >= LATENT_WARPS_WANTED else max(-(-int(step.max_kv_len) // LATENT_SPLIT_KEYS), 1)
