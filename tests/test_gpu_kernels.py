@@ -978,3 +978,19 @@ def test_attention_in_tiles_and_values_that_are_not_finite(dtype, Hq, Hkv, D, ba
             keep = torch.isfinite(a)
             assert not keep.all() and torch.equal(a[keep], o.paged_attention(q, step, was, Hq, Hkv, D, D ** -0.5, **opts)[keep])
     assert o.read_status() == 0
+
+
+@pytest.mark.parametrize("q_lens", [[200, 3], [1, 1, 1]])
+def test_attention_of_queries_off_the_tensor_cores_boundaries(q_lens):
+    """bfloat16 queries that start between 16-byte boundaries go to the general kernels."""
+    o = ops()
+    g = torch.Generator().manual_seed(34)
+    Hq, Hkv, D, ps, ctx = 8, 2, 64, 16, [70] * len(q_lens)
+    num_pages = sum(-(-(c + n) // ps) for c, n in zip(ctx, q_lens)) + 8
+    step = make_step(o, torch.bfloat16, ctx, q_lens, ps, num_pages, 9)
+    view = CacheView(0, fill_pages(step, ctx, q_lens, ps, Hkv, D, torch.bfloat16, num_pages, g), step.block_tables[0], ps)
+    q = torch.randn(sum(q_lens) * Hq * D + 1, generator=g).bfloat16().cuda()[1:].view(sum(q_lens), Hq * D)
+    for opts in (dict(), dict(window=20), dict(softcap=5.0, sink=torch.randn(Hq, generator=g).cuda())):
+        want = ref_ops.paged_attention(q, step, view, Hq, Hkv, D, D ** -0.5, **opts)
+        assert torch.allclose(o.paged_attention(q, step, view, Hq, Hkv, D, D ** -0.5, **opts).float(), want.float(), **tol(torch.bfloat16))
+    assert o.read_status() == 0

@@ -1041,6 +1041,7 @@ def paged_attention(q, step, cache, heads, kv_heads, head_dim, scale, window=Non
     cap by min(distance, last row)), `sink` [heads] 32-bit (a term of the denominator alone), `keep_first` (with a window:
     the request's first positions stay visible)."""
     _cuda(q, bias, sink)
+    aligned = not (q.data_ptr() | cache.pages.data_ptr()) & 15               # (the tensor-core kernels' copies start on 16 bytes)
     if softcap or bias is not None or sink is not None or keep_first:
         if chunk is not None or (keep_first and not window):
             raise KernelError("shaped scores go with a window or none; kept first positions need a window")
@@ -1051,7 +1052,7 @@ def paged_attention(q, step, cache, heads, kv_heads, head_dim, scale, window=Non
                 or (sink is not None and (sink.dtype != torch.float32 or sink.numel() != heads))):
             raise KernelError("paged_attention: operands do not fit together")
         shaped = (float(softcap or 0.0), _ptr(bias), 0 if bias is None else bias.shape[0], _ptr(sink), int(keep_first or 0))
-        if (impl != "general" and q.dtype == torch.bfloat16 and q.is_contiguous()
+        if (impl != "general" and q.dtype == torch.bfloat16 and aligned and q.is_contiguous()
                 and _fn("attention_mma", "zai_attention_mma_supports")(head_dim, heads, kv_heads)):
             # the tensor-core kernels with the scores shaped inside them
             def single_tokens(n):
@@ -1075,8 +1076,8 @@ def paged_attention(q, step, cache, heads, kv_heads, head_dim, scale, window=Non
             block_rows = _fn("attention_mma", "zai_prefill_block_rows")()
             n_tiles = (step.attn_tiles - ns) if getattr(step, "attn_tiles", None) else sum(-(-n // block_rows) for n in step.q_lens[ns:])
             # head size 64 on tcgen05 at every size: 8 x 100 rows behind 500 positions with 16 heads of 64 are the one form found where the
-            # walk by mma.sync is level (41 us to 43), long contexts gain most (684 to 100, 32 rows behind 16 384).  TMA wants 16 bytes.
-            if (impl != "mma" and (USE_TC_ATTENTION or impl == "tcgen05") and not (q.data_ptr() | out.data_ptr() | cache.pages.data_ptr()) & 15
+            # walk by mma.sync is level (41 us to 43), long contexts gain most (684 to 100, 32 rows behind 16 384).
+            if (impl != "mma" and (USE_TC_ATTENTION or impl == "tcgen05")
                     and _fn("attention_tc", "zai_prefill_attention_tc_supports")(head_dim, heads, kv_heads, cache.page_size)
                     and (bias is None or bias.shape[0] <= _fn("attention_tc", "zai_prefill_attention_tc_max_bias")())):
                 splits, part_o, part_ml, tickets = _attention_splits(q.device, n_tiles, heads, bt[ns:], cache.page_size, shaped=True)
@@ -1109,7 +1110,7 @@ def paged_attention(q, step, cache, heads, kv_heads, head_dim, scale, window=Non
     if cache.pages.dtype != q.dtype:
         raise KernelError("the pages and the queries should have one dtype")
     bt = cache.block_table
-    if (impl != "general" and q.dtype == torch.bfloat16
+    if (impl != "general" and q.dtype == torch.bfloat16 and aligned
             and _fn("attention_mma", "zai_attention_mma_supports")(head_dim, heads, kv_heads)):
         def single_tokens(n):
             # rows 0..n-1 are one token each, row i of span i: keys split over blocks, then combined
