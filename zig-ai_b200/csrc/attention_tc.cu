@@ -36,8 +36,8 @@
 // Their error against 64 bits is 0.93 to 1.00 of that walk's (relative 1.71e-3 to 2.10e-3, what bfloat16 P and results make it).
 //
 // Q, K and V reach shared memory by TMA (cp.async.bulk.tensor, no multicast), K and V page by page
-// through the block table into five stages of 16 KB.  Roles: warp 0 one lane issues the loads, warp 1
-// one lane the products, warps 2-9 are the softmax.
+// through the block table into five stages of 16 KB.  Roles: warp 0 one lane issues the loads (and the warp cleans the values of
+// tiles that not every row sees whole), warp 1 one lane the products, warps 2-9 are the softmax.
 //
 // Blocks are handed out heads first, tiles of query rows from the last rows backwards: under the causal
 // mask the last rows of a long span walk many more key tiles than the first, a block's tiles are a chain
@@ -57,7 +57,8 @@
 #define AT_TMEM_COLS 256                              // two score buffers in columns 0..127, O in 128..191, two P buffers in 192..255
 #define AT_COL_O (2 * AT_BN)
 #define AT_COL_P (2 * AT_BN + AT_D)
-#define AT_HIDDEN_BYTES 1600                          // AtHidden<AT_D>
+#define AT_LAG 2                                      // tiles that the cleaning is behind the loads (below the number of stages)
+typedef AtNotes<1, 128> AtTileNotes;
 
 struct AtArgs {
     bf16* out;                  // [rows of the step, Hq, 64]
@@ -104,23 +105,24 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
     uint64_t* s_ready = bars + 1 + 2 * STAGES;               // [2] scores of tile i in buffer i & 1
     uint64_t* p_ready = bars + 3 + 2 * STAGES;               // [2] P of tile i in buffer i & 1
     uint64_t* o_ready = bars + 5 + 2 * STAGES;               // [2] the product of tile i has read P buffer i & 1 and added to O
-    uint32_t& tmem_base_holder = *reinterpret_cast<uint32_t*>(bars + 7 + 2 * STAGES);
-    int* words = reinterpret_cast<int*>(bars + 8 + 2 * STAGES);
+    uint64_t* v_ready = bars + 7 + 2 * STAGES;               // [STAGES] the values of a stage are there and clean
+    uint32_t& tmem_base_holder = *reinterpret_cast<uint32_t*>(bars + 7 + 3 * STAGES);
+    int* words = reinterpret_cast<int*>(bars + 8 + 3 * STAGES);
     int& failed_flag = words[0];
     int& s_seq = words[1];
     int& s_i0 = words[2];
     float* exch = reinterpret_cast<float*>(words + 4);          // [2][2][128]: a tile's maxima by half, by turns; then the sums
-    AtHidden<AT_D>& hid = *reinterpret_cast<AtHidden<AT_D>*>(exch + 4 * AT_BM);
-    float* bias = exch + 4 * AT_BM + AT_HIDDEN_BYTES / 4;       // [bias_rows] the head's bias by distance
+    AtTileNotes& notes = *reinterpret_cast<AtTileNotes*>(exch + 4 * AT_BM);
+    float* bias = reinterpret_cast<float*>(&notes + 1);         // [bias_rows] the head's bias by distance
     volatile int* failed = &failed_flag;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-    if (tid < AT_D)
-        for (int t = 0; t < 3; ++t) hid.clear(t, tid, AT_D);
     if (tid == 0) {
         failed_flag = (at_smem(base) & 1023u) ? 1 : 0;          // the swizzled tiles need 1024-byte alignment
+        notes.clear();
         at_mbar_init(&q_full, 1);
         for (int s = 0; s < STAGES; ++s) {
+            at_mbar_init(&v_ready[s], 1);
             at_mbar_init(&kv_full[s], 1);
             at_mbar_init(&kv_empty[s], 1);
         }
@@ -186,36 +188,66 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
             n_tiles = min(per, n_tiles - from);
         }
         auto key_of = [&](int i) { return (SHAPED && from + i < n_kept ? from + i : tile0 + from + i - n_kept) * AT_BN; };   // the first key of tile i
+        // the tiles that some row does not see whole: those that end behind the first row (from tile p0 on; the last one counts as such:
+        // when its values are ready, so are all), and those before the last row's first key that are not kept (p1 to p2)
+        const int keep = SHAPED && a.window > 0 ? a.opt.keep_first : 0;
+        auto index_of = [&](int t) { return min(max((t < n_kept ? t : max(t, tile0) - tile0 + n_kept) - from, 0), n_tiles); };
+        const int p0 = min(index_of((ctx + i0 + 1) / AT_BN), n_tiles - 1), p1 = index_of(keep / AT_BN);
+        const int whole = index_of((zai_first_visible(kend - 1, a.window) + AT_BN - 1) / AT_BN), p2 = p1 < whole ? whole : 0;
+        auto part = [&](int i) { return i >= p0 || (i >= p1 && i < p2); };
 
         if (warp == 0) {
-            if (lane == 0 && n_tiles > 0) {
+            if (n_tiles > 0) {
                 // ---- loads: the block's queries, then a stage of keys and values per tile, page by page
                 const int* table = a.block_table + (size_t)s * a.table_width;
                 const int ps = a.page_size, box_rows = ps < AT_BN ? ps : AT_BN, per_tile = AT_BN / box_rows;
-                at_mbar_expect_tx(&q_full, AT_Q_BYTES);
-                at_tma_load_2d(sQ, &map_q, h * AT_D, row0 + i0, &q_full);
-                int issued = 0;
-                for (int i = 0; i < n_tiles; ++i) {
-                    const int st = i % STAGES;
-                    if (!at_mbar_wait(&kv_empty[st], ((i / STAGES) & 1) ^ 1, failed)) break;
-                    at_mbar_expect_tx(&kv_full[st], AT_KV_BYTES);
-                    unsigned char* dst = sKV + (size_t)st * AT_KV_BYTES;
-                    for (int p = 0; p < per_tile; ++p) {
-                        const int key0 = key_of(i) + p * box_rows;
-                        const int idx = key0 >> a.page_shift, off = key0 & (ps - 1);
-                        int page = idx < a.table_width ? table[idx] : 0;              // beyond the table: the null page
-                        if ((unsigned)page >= (unsigned)a.num_pages) {                // outside the pool: page 0, and the step is void
-                            zai_raise(a.status, ZAI_ST_PAGE);
-                            page = 0;
-                        }
-                        const int krow = ((page * 2 + 0) * a.Hkv + hk) * ps + off;
-                        const int vrow = ((page * 2 + 1) * a.Hkv + hk) * ps + off;
-                        at_tma_load_2d(dst + (size_t)p * box_rows * 128, &map_kv, 0, krow, &kv_full[st]);
-                        at_tma_load_2d(dst + AT_BN * 128 + (size_t)p * box_rows * 128, &map_kv, 0, vrow, &kv_full[st]);
-                    }
-                    issued = i + 1;
+                if (lane == 0) {
+                    at_mbar_expect_tx(&q_full, AT_Q_BYTES);
+                    at_tma_load_2d(sQ, &map_q, h * AT_D, row0 + i0, &q_full);
                 }
-                if (*failed) {                                  // loads already issued still land here: wait for them
+                int issued = 0;
+                for (int i = 0; i < n_tiles; ++i) {             // (i: the next tile whose values may need cleaning)
+                    i = min(i < p2 ? max(i, p1) : n_tiles, max(i, p0));
+                    bool ok = true;
+                    if (lane == 0)                              // one lane issues all loads up to AT_LAG tiles behind it
+                        for (const int end = min(i + AT_LAG + 1, n_tiles); issued < end && ok; ++issued) {
+                            const int st = issued % STAGES;
+                            ok = at_mbar_wait(&kv_empty[st], ((issued / STAGES) & 1) ^ 1, failed);
+                            if (!ok) break;
+                            at_mbar_expect_tx(&kv_full[st], AT_KV_BYTES);
+                            unsigned char* dst = sKV + (size_t)st * AT_KV_BYTES;
+                            for (int p = 0; p < per_tile; ++p) {
+                                const int key0 = key_of(issued) + p * box_rows;
+                                const int idx = key0 >> a.page_shift, off = key0 & (ps - 1);
+                                int page = idx < a.table_width ? table[idx] : 0;      // beyond the table: the null page
+                                if ((unsigned)page >= (unsigned)a.num_pages) {        // outside the pool: page 0, and the step is void
+                                    zai_raise(a.status, ZAI_ST_PAGE);
+                                    page = 0;
+                                }
+                                const int krow = ((page * 2 + 0) * a.Hkv + hk) * ps + off;
+                                const int vrow = ((page * 2 + 1) * a.Hkv + hk) * ps + off;
+                                at_tma_load_2d(dst + (size_t)p * box_rows * 128, &map_kv, 0, krow, &kv_full[st]);
+                                at_tma_load_2d(dst + AT_BN * 128 + (size_t)p * box_rows * 128, &map_kv, 0, vrow, &kv_full[st]);
+                            }
+                            if (!part(issued)) at_mbar_arrive(&v_ready[st]);
+                        }
+                    const int st = i % STAGES, tile_key = key_of(i);
+                    if (!__shfl_sync(0xffffffffu, ok, 0) || !at_mbar_wait_warp(&kv_full[st], (i / STAGES) & 1, failed)) break;
+                    unsigned char* values = sKV + (size_t)st * AT_KV_BYTES + AT_KV_BYTES / 2;
+                    const unsigned long long shown = at_below(kend - tile_key) & (~at_below(kbeg - tile_key) | at_below(keep - tile_key));
+                    if (__any_sync(0xffffffffu, at_clean<4>(values, lane >> 3, shown)))
+                        for (int k0 = 0; k0 < AT_BN; k0 += 4) {
+                            const unsigned long long odd = at_take_odd(values, k0 + (lane >> 3), true);
+                            if ((lane & 7) == 0 && odd) {
+                                const int e = notes.add(tile_key + k0 + (lane >> 3));
+                                if (e >= 0) notes.cols[e][0] = odd;
+                            }
+                        }
+                    at_proxy_fence();                           // (generic writes, which the product reads)
+                    __syncwarp();
+                    if (lane == 0) at_mbar_arrive(&v_ready[st]);
+                }
+                if (lane == 0 && *failed) {                     // loads already issued still land here: wait for them
                     for (int i = max(issued - STAGES, 0); i < issued; ++i) {
                         const uint32_t addr = at_smem(&kv_full[i % STAGES]);
                         const uint32_t ph = (i / STAGES) & 1;
@@ -263,7 +295,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
                 if (ok && n_tiles > 1) ok = scores(1);
                 for (int i = 0; i < n_tiles && ok; ++i) {
                     const int st = i % STAGES;
-                    ok = at_mbar_wait(&p_ready[i & 1], (i >> 1) & 1, failed);
+                    ok = at_mbar_wait(&p_ready[i & 1], (i >> 1) & 1, failed) && (!part(i) || at_mbar_wait(&v_ready[st], (i / STAGES) & 1, failed));
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t aV = at_smem(sKV + (size_t)st * AT_KV_BYTES + AT_BN * 128);
@@ -289,36 +321,12 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
             const uint32_t tS = tmem_base + ((uint32_t)(qd * 32) << 16) + half * 32, tO = tS + AT_COL_O, tP = tmem_base + ((uint32_t)(qd * 32) << 16) + AT_COL_P + half * 16;
             const float c = SHAPED ? 1.f : a.scale_log2;        // (shaped scores are made in the exponent's units)
             const float unit = SHAPED && a.opt.softcap > 0.f ? a.opt.scale / a.opt.softcap : 0.f, cap = a.opt.softcap * 1.4426950408889634f;
-            // (a key is hidden from some row of the block if it lies behind the first row, or before the last row's first one and is not kept)
-            const int keep = SHAPED && a.window > 0 ? a.opt.keep_first : 0, klast = zai_first_visible(kend - 1, a.window);
-            int turn3 = 0;
             bool alive = true;
             for (int i = 0; i < n_tiles; ++i) {
                 const int key0 = key_of(i) + half * 32;
                 if (alive && !at_mbar_wait_warp(&s_ready[i & 1], (i >> 1) & 1, failed)) alive = false;      // (the warp together)
                 const uint32_t tSi = tS + (i & 1) * AT_BN, tPi = tP + (i & 1) * (AT_BN / 2);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const int tile_key = key_of(i);
-                if (tile_key + AT_BN - 1 > ctx + i0 || (tile_key < klast && tile_key + AT_BN > keep)) {
-                    const int st = i % STAGES;
-                    hid.clear(turn3 == 2 ? 0 : turn3 + 1, tid - 64, 256);            // (all have left the tile that used it)
-                    if (alive && !at_mbar_wait_warp(&kv_full[st], (i / STAGES) & 1, failed)) alive = false;    // (long since there)
-                    if (alive) {
-                        unsigned char* values = sKV + (size_t)st * AT_KV_BYTES + AT_KV_BYTES / 2;
-                        for (int e = tid - 64; e < AT_BN * 8; e += 256) {
-                            const int key = tile_key + (e >> 3);
-                            hid.clean(values, e, 0, key >= kend || (key < kbeg && key >= keep), turn3);
-                        }
-                        at_proxy_fence();
-                    }
-                    asm volatile("bar.sync 6, 256;" ::: "memory");
-                    if (hid.any[turn3]) {
-                        const unsigned long long sees = (at_below(qpos + 1 - tile_key) & ~at_below(klo - tile_key)) | at_below(kept - tile_key);
-                        for (int j = 0; j < 32; ++j)
-                            if (hid.keys[turn3][half * 32 + j] & sees) nans |= 1u << j;
-                    }
-                    turn3 = turn3 == 2 ? 0 : turn3 + 1;
-                }
                 // keys of this half that the row sees: [lo, hi), and those below `first`
                 const int lo = valid ? max(klo - key0, 0) : 32, hi = valid ? min(qpos + 1 - key0, 32) : 0;
                 const int first = valid ? kept - key0 : 0;
@@ -424,7 +432,8 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
             l += turn[(half ^ 1) * AT_BM + row];
             if (alive && at_mbar_wait_warp(&o_ready[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1, failed)) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                have_o = true;
+                have_o = at_mbar_wait_warp(&v_ready[(n_tiles - 1) % STAGES], ((n_tiles - 1) / STAGES) & 1, failed);    // (long since; the notes are seen)
+                if (notes.count) nans = notes.met(half, qpos, klo, kept);
                 float inv = l > 0.f ? 1.f / l : 0.f;
                 if (SHAPED && a.opt.sink) {                     // one more term of the denominator
                     const float M = m * c, sk = a.opt.sink[h] * 1.4426950408889634f, top = fmaxf(M, sk);
@@ -593,8 +602,7 @@ ZAI_API int zai_prefill_attention_tc(void* out, const void* q, const void* pages
     while ((1 << a.page_shift) < page_size) ++a.page_shift;
     const bool shaped = softcap > 0.f || bias || sink || keep_first > 0;
     a.opt = {softcap, bias, bias_rows, sink, keep_first, scale};
-    constexpr size_t words = 256 + 4 * AT_BM * sizeof(float) + AT_HIDDEN_BYTES;
-    static_assert(sizeof(AtHidden<AT_D>) <= AT_HIDDEN_BYTES && AT_HIDDEN_BYTES % 16 == 0, "the notes fit");
+    constexpr size_t words = 256 + 4 * AT_BM * sizeof(float) + sizeof(AtTileNotes);
     constexpr size_t smem = AT_Q_BYTES + (size_t)AT_STAGES * AT_KV_BYTES + words;
     constexpr size_t smem_shaped = AT_Q_BYTES + (size_t)AT_SHAPED_STAGES * AT_KV_BYTES + words;
     static_assert(2 * (smem + 1024) <= 233472 && 2 * (smem_shaped + AT_MAX_BIAS * sizeof(float) + 1024) <= 233472, "two blocks an SM");

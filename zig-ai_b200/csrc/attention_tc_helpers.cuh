@@ -113,45 +113,77 @@ __device__ __forceinline__ void at_tmem_wait_ld(uint32_t (&r)[32]) {
 
 // ---- values that some rows of a block do not see.  A tile's hidden keys have weights of exactly zero, but zero times NaN or
 // infinity is NaN in the product: a recycled page's last owner, or a later row of the span, would reach every row of the block.  So
-// in tiles that some row sees a part of, before their product, the softmax threads put zeros over the values that no row sees, and take
-// what is not finite out of the others: AtHidden notes it by column and key, and a row that sees such a key ends as NaN in that
-// column.  Zeros and notes are generic writes: at_proxy_fence() orders them before the product's reads (asynchronous proxy).
+// before the product of a tile that not every row sees whole, the warp that loads tiles puts zeros over the values that no row
+// sees and takes what is not finite out of the others; AtNotes holds those keys and their columns, and a row that sees such a key
+// ends as NaN there.  The softmax warps, whose chain bounds these kernels, have no part in it (there it cost 4 to 13 %).
 __device__ __forceinline__ void at_proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 // eight bfloat16 values: is one of them infinite or NaN (an exponent of ones)?
 __device__ __forceinline__ bool at_not_finite(const uint4& v) {
     auto two = [](uint32_t x) { return ((x & 0x7f807f80u) + 0x00800080u) & 0x80008000u; };
     return (two(v.x) | two(v.y) | two(v.z) | two(v.w)) != 0;
 }
-// the lowest n of 64 bits
-__device__ __forceinline__ unsigned long long at_below(int n) { return n <= 0 ? 0ull : n >= 64 ? ~0ull : (1ull << n) - 1; }
-template <int COLS>
-struct AtHidden {                                               // three tiles' notes, by turns
-    unsigned long long keys[3][COLS];                           // a column's keys of the tile whose value is not finite
-    int any[3];
-    __device__ __forceinline__ void clear(int turn, int tid, int threads) {
-        for (int c = tid; c < COLS; c += threads) keys[turn][c] = 0;
-        if (tid == 0) any[turn] = 0;
+// A lane's part of a tile's values, 16 bytes of every STEP-th key from `key` on (a key's 64 columns are one swizzled row of 128 bytes,
+// eight lanes): zeros where the tile's key is not among `shown`.  Returns whether another value is not finite.
+template <int STEP>
+__device__ __forceinline__ bool at_clean(unsigned char* tile, int key, unsigned long long shown) {
+    uint4* p = reinterpret_cast<uint4*>(tile) + (threadIdx.x & 7);
+    bool odd = false;
+#pragma unroll 8
+    for (int t = 0; t < 64 / STEP; ++t) {                       // (a loop of loads alone: they are in flight together)
+        const int k = key + t * STEP;
+        const bool o = at_not_finite(p[k * 8]);
+        odd |= o && (shown >> k & 1);
     }
-    // 16 bytes of a tile's values (swizzled rows of 128 bytes; `chunk` counts 16 bytes from the tile's first row; columns from
-    // `col0`): zeros if no row sees the key, else without what is not finite
-    __device__ __forceinline__ void clean(unsigned char* tile, int chunk, int col0, bool hidden, int turn) {
-        uint4* p = reinterpret_cast<uint4*>(tile) + chunk;
-        if (hidden) {
-            *p = make_uint4(0u, 0u, 0u, 0u);
-            return;
-        }
-        if (!at_not_finite(*p)) return;
-        const int key = chunk >> 3, c0 = col0 + ((chunk & 7) ^ (key & 7)) * 8;
+    if (~shown)
+        for (int t = 0; t < 64 / STEP; ++t)
+            if (!(shown >> (key + t * STEP) & 1)) p[(key + t * STEP) * 8] = make_uint4(0u, 0u, 0u, 0u);
+    return odd;
+}
+// Takes what is not finite out of a lane's 16 bytes of a key; every lane of the warp calls it (`on`: this lane has such a part).  Returns
+// those columns of the key's 64, the same in its eight lanes.
+__device__ __forceinline__ unsigned long long at_take_odd(unsigned char* tile, int key, bool on) {
+    const int chunk = threadIdx.x & 7;
+    uint4* p = reinterpret_cast<uint4*>(tile + key * 128) + chunk;
+    unsigned long long odd = 0;
+    if (on && at_not_finite(*p)) {
         unsigned short* v = reinterpret_cast<unsigned short*>(p);
         for (int e = 0; e < 8; ++e)
             if ((v[e] & 0x7f80) == 0x7f80) {
                 v[e] = 0;
-                atomicOr(&keys[turn][c0 + e], 1ull << key);
+                odd |= 1ull << ((chunk ^ (key & 7)) * 8 + e);
             }
-        any[turn] = 1;
+    }
+    for (int o = 1; o < 8; o <<= 1) odd |= __shfl_xor_sync(0xffffffffu, odd, o);
+    return odd;
+}
+// the lowest n of 64 bits
+__device__ __forceinline__ unsigned long long at_below(int n) { return n <= 0 ? 0ull : n >= 64 ? ~0ull : (1ull << n) - 1; }
+template <int PARTS, int MOST>                                  // columns in 64s; keys that find room
+struct AtNotes {
+    unsigned long long cols[MOST][PARTS];
+    int key[MOST];                                              // positions in the request
+    int count, low, high;                                       // keys noted; those that found no room lie from low to high
+    __device__ __forceinline__ void clear() { count = 0; low = 0x7fffffff; high = -1; }
+    // by one lane, for a key's part of the columns; returns the place for other parts, or -1
+    __device__ __forceinline__ int add(int k) {
+        const int i = atomicAdd(&count, 1);
+        if (i < MOST) {
+            key[i] = k;
+            for (int p = 0; p < PARTS; ++p) cols[i][p] = 0;
+            return i;
+        }
+        atomicMin(&low, k);
+        atomicMax(&high, k);
+        return -1;
+    }
+    // the columns 32 w .. that a row with keys [from, pos] and [0, kept) has met such values in (all, if it may see a key without room)
+    __device__ __noinline__ uint32_t met(int w, int pos, int from, int kept) const {
+        uint32_t m = low <= pos && (high >= from || low < kept) ? 0xffffffffu : 0u;
+        for (int i = 0; i < min(count, MOST); ++i)
+            if (key[i] <= pos && (key[i] >= from || key[i] < kept)) m |= (uint32_t)(cols[i][w >> 1] >> ((w & 1) * 32));
+        return m;
     }
 };
-
 __device__ __forceinline__ void at_put_nans(uint32_t (&r)[32], uint32_t which) {
 #pragma unroll
     for (int j = 0; j < 32; ++j)

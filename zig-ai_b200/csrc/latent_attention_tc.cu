@@ -12,9 +12,9 @@
 //
 // Queries and cached rows come by TMA (no multicast) in boxes of 64 columns, the cached rows page by page into LT_STAGES stages; the
 // last box reaches beyond the row and is filled with zeros.  TMEM holds two score and two P buffers, so the scores of tile i + 2
-// are issued behind the product of tile i.  Roles: warp 0 one lane issues the loads, warp 1 one lane the products, warps 2-5 are
-// the softmax.  Blocks are handed out from the last pairs backwards (they have the most keys).  Every wait on an mbarrier is
-// bounded; a block whose wait runs out raises the status word, its roles leave their loops, TMEM is freed and the block returns.
+// are issued behind the product of tile i.  Roles: warp 0 one lane issues the loads (and the warp cleans the values of tiles that
+// not every pair sees whole), warp 1 one lane the products, warps 2-5 are the softmax.  Blocks are handed out from the last pairs
+// backwards (they have the most keys).  Every wait on an mbarrier is bounded; a block whose wait runs out raises the status word, its roles leave their loops, TMEM is freed and the block returns.
 //
 // What bounds it: the chain of a tile (scores, softmax, P, product), 1.8 us of 64 keys, with one block an SM (200 KB of shared memory);
 // the products' tensor time is about 0.8 us of it.  16 heads, R = 256, Dr = 32: 2048 rows 282 us (mma.sync, four warps sharing tiles of
@@ -32,6 +32,8 @@
 #define LT_TMEM_COLS 512                              // two score buffers in columns 0..127, O in 128..383, two P buffers in 384..447
 #define LT_COL_O (2 * LT_BN)
 #define LT_COL_P (LT_COL_O + LT_MAX_R)
+#define LT_LAG 1                                      // tiles that the cleaning is behind the loads (below the number of stages)
+typedef AtNotes<LT_MAX_R / 64, 64> LtNotes;
 
 struct LtArgs {
     bf16* out;                  // [N, H, R]
@@ -70,22 +72,22 @@ __global__ void __launch_bounds__(LT_THREADS) latent_attention_tc_kernel(const _
     uint64_t* s_ready = bars + 1 + 2 * LT_STAGES;               // [2] scores of tile i in buffer i & 1
     uint64_t* p_ready = bars + 3 + 2 * LT_STAGES;               // [2] P of tile i in buffer i & 1
     uint64_t* o_ready = bars + 5 + 2 * LT_STAGES;               // [2] the product of tile i has read P buffer i & 1 and added to O
-    uint32_t& tmem_base_holder = *reinterpret_cast<uint32_t*>(bars + 7 + 2 * LT_STAGES);
-    int* words = reinterpret_cast<int*>(bars + 8 + 2 * LT_STAGES);
+    uint64_t* v_ready = bars + 7 + 2 * LT_STAGES;               // [LT_STAGES] the values of a stage are there and clean
+    uint32_t& tmem_base_holder = *reinterpret_cast<uint32_t*>(bars + 7 + 3 * LT_STAGES);
+    int* words = reinterpret_cast<int*>(bars + 8 + 3 * LT_STAGES);
     int& failed_flag = words[0];
     int& s_seq = words[1];
     int& s_i0 = words[2];
-    AtHidden<LT_MAX_R>& hid = *reinterpret_cast<AtHidden<LT_MAX_R>*>(words + 4);
-    uint32_t* nans = reinterpret_cast<uint32_t*>(&hid + 1);     // [8][LT_BM] the columns of a pair that have met a value that is not finite
+    LtNotes& notes = *reinterpret_cast<LtNotes*>(words + 4);
     volatile int* failed = &failed_flag;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-    for (int t = 0; t < 3; ++t) hid.clear(t, tid, LT_THREADS);
-    for (int i = tid; i < LT_MAX_R / 32 * LT_BM; i += LT_THREADS) nans[i] = 0;
     if (tid == 0) {
         failed_flag = (at_smem(smem_raw) & 1023u) ? 1 : 0;      // the swizzled tiles need 1024-byte alignment
+        notes.clear();
         at_mbar_init(&q_full, 1);
         for (int s = 0; s < LT_STAGES; ++s) {
+            at_mbar_init(&v_ready[s], 1);
             at_mbar_init(&kv_full[s], 1);
             at_mbar_init(&kv_empty[s], 1);
         }
@@ -124,38 +126,63 @@ __global__ void __launch_bounds__(LT_THREADS) latent_attention_tc_kernel(const _
         const int pairs = min(LT_BM, (a.cu_q[s + 1] - row0) * a.H - i0);      // valid pairs of this block
         const int kend = ctx + (i0 + pairs - 1) / a.H + 1;                    // one past the last visible key of the block
         const int n_tiles = (kend + LT_BN - 1) / LT_BN;
+        // the tiles that end behind the first pair's row (the last one counts as such: when its values are ready, so are all)
+        const int p0 = min((ctx + i0 / a.H + 1) / LT_BN, n_tiles - 1);
 
         if (warp == 0) {
+            // ---- loads: the block's queries, then a stage of cached rows per tile, page by page
+            const int* table = a.block_table + (size_t)s * a.table_width;
+            const int ps = a.page_size, box_rows = ps < LT_BN ? ps : LT_BN, per_tile = LT_BN / box_rows;
             if (lane == 0) {
-                // ---- loads: the block's queries, then a stage of cached rows per tile, page by page
-                const int* table = a.block_table + (size_t)s * a.table_width;
-                const int ps = a.page_size, box_rows = ps < LT_BN ? ps : LT_BN, per_tile = LT_BN / box_rows;
                 at_mbar_expect_tx(&q_full, q_bytes);
                 for (int b = 0; b < n_blocks; ++b)
                     at_tma_load_2d(sQ + (size_t)b * LT_Q_BLOCK, b < n_lat ? &map_lat : &map_rot, b < n_lat ? b * 64 : 0, row0 * a.H + i0, &q_full);
-                int issued = 0;
-                for (int i = 0; i < n_tiles; ++i) {
-                    const int st = i % LT_STAGES;
-                    if (!at_mbar_wait(&kv_empty[st], ((i / LT_STAGES) & 1) ^ 1, failed)) break;
-                    at_mbar_expect_tx(&kv_full[st], kv_bytes);
-                    unsigned char* dst = sKV + (size_t)st * kv_bytes;
-                    for (int p = 0; p < per_tile; ++p) {
-                        const int key0 = i * LT_BN + p * box_rows;
-                        const int idx = key0 >> a.page_shift, off = key0 & (ps - 1);
-                        int page = idx < a.table_width ? table[idx] : 0;              // beyond the table: the null page
-                        if ((unsigned)page >= (unsigned)a.num_pages) {                // outside the pool: page 0, and the step is void
-                            zai_raise(a.status, ZAI_ST_PAGE);
-                            page = 0;
+            }
+            int issued = 0;
+            for (int i = p0; i < n_tiles; ++i) {
+                bool ok = true;
+                if (lane == 0)                                  // one lane issues all loads up to LT_LAG tiles behind this one
+                    for (const int end = min(i + LT_LAG + 1, n_tiles); issued < end && ok; ++issued) {
+                        const int st = issued % LT_STAGES;
+                        ok = at_mbar_wait(&kv_empty[st], ((issued / LT_STAGES) & 1) ^ 1, failed);
+                        if (!ok) break;
+                        at_mbar_expect_tx(&kv_full[st], kv_bytes);
+                        unsigned char* dst = sKV + (size_t)st * kv_bytes;
+                        for (int p = 0; p < per_tile; ++p) {
+                            const int key0 = issued * LT_BN + p * box_rows;
+                            const int idx = key0 >> a.page_shift, off = key0 & (ps - 1);
+                            int page = idx < a.table_width ? table[idx] : 0;          // beyond the table: the null page
+                            if ((unsigned)page >= (unsigned)a.num_pages) {            // outside the pool: page 0, and the step is void
+                                zai_raise(a.status, ZAI_ST_PAGE);
+                                page = 0;
+                            }
+                            for (int b = 0; b < n_blocks; ++b)
+                                at_tma_load_2d(dst + (size_t)b * LT_K_BLOCK + (size_t)p * box_rows * 128, &map_kv, b * 64, page * ps + off, &kv_full[st]);
                         }
-                        for (int b = 0; b < n_blocks; ++b)
-                            at_tma_load_2d(dst + (size_t)b * LT_K_BLOCK + (size_t)p * box_rows * 128, &map_kv, b * 64, page * ps + off, &kv_full[st]);
+                        if (issued < p0) at_mbar_arrive(&v_ready[st]);
                     }
-                    issued = i + 1;
-                }
-                if (*failed) {                                  // loads already issued still land here: wait for them
-                    for (int i = max(issued - LT_STAGES, 0); i < issued; ++i) lt_drain(&kv_full[i % LT_STAGES], (i / LT_STAGES) & 1);
-                    lt_drain(&q_full, 0);
-                }
+                // as keys the rows have to stay what they are until the scores are there
+                const int st = i % LT_STAGES;
+                if (!__shfl_sync(0xffffffffu, ok, 0) || !at_mbar_wait_warp(&kv_full[st], (i / LT_STAGES) & 1, failed)
+                    || !at_mbar_wait_warp(&s_ready[i & 1], (i >> 1) & 1, failed)) break;
+                unsigned char* rows = sKV + (size_t)st * kv_bytes + (size_t)(lane >> 3) * LT_K_BLOCK;
+                const bool mine = (lane >> 3) < n_lat;          // (a row a turn, eight lanes a block of 64 columns)
+                const bool odd = mine && at_clean<1>(rows, 0, at_below(kend - i * LT_BN));
+                if (__any_sync(0xffffffffu, odd))
+                    for (int k = 0; k < LT_BN; ++k) {
+                        const unsigned long long cols = at_take_odd(rows, k, mine);
+                        if (!__any_sync(0xffffffffu, cols != 0)) continue;
+                        int e = lane == 0 ? notes.add(i * LT_BN + k) : 0;
+                        e = __shfl_sync(0xffffffffu, e, 0);
+                        if (e >= 0 && (lane & 7) == 0) notes.cols[e][lane >> 3] = cols;
+                    }
+                at_proxy_fence();                               // (generic writes, which the product reads)
+                __syncwarp();
+                if (lane == 0) at_mbar_arrive(&v_ready[st]);
+            }
+            if (lane == 0 && *failed) {                         // loads already issued still land here: wait for them
+                for (int i = max(issued - LT_STAGES, 0); i < issued; ++i) lt_drain(&kv_full[i % LT_STAGES], (i / LT_STAGES) & 1);
+                lt_drain(&q_full, 0);
             }
         } else if (warp == 1) {
             if (lane == 0) {
@@ -183,7 +210,7 @@ __global__ void __launch_bounds__(LT_THREADS) latent_attention_tc_kernel(const _
                 if (ok && n_tiles > 1) ok = scores(1);
                 for (int i = 0; i < n_tiles && ok; ++i) {
                     const int st = i % LT_STAGES;
-                    ok = at_mbar_wait(&p_ready[i & 1], (i >> 1) & 1, failed);
+                    ok = at_mbar_wait(&p_ready[i & 1], (i >> 1) & 1, failed) && (i < p0 || at_mbar_wait(&v_ready[st], (i / LT_STAGES) & 1, failed));
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t aV = at_smem(sKV + (size_t)st * kv_bytes);
@@ -208,34 +235,11 @@ __global__ void __launch_bounds__(LT_THREADS) latent_attention_tc_kernel(const _
             const uint32_t tS = tmem_base + ((uint32_t)(qd * 32) << 16), tO = tS + LT_COL_O, tP = tS + LT_COL_P;
             const float c = a.scale_log2;
             float m = -INFINITY, l = 0.f;                       // m: the pair's reference, in units of the scores
-            int turn3 = 0;
-            bool alive = true, bad = false;
-            for (int i = 0; i < n_tiles; ++i) {
-                if (alive && !at_mbar_wait_warp(&s_ready[i & 1], (i >> 1) & 1, failed)) alive = false;      // (the warp together)
+            bool alive = true;
+            for (int i = 0; i < n_tiles && alive; ++i) {
+                if (!at_mbar_wait_warp(&s_ready[i & 1], (i >> 1) & 1, failed)) { alive = false; break; }    // (the warp leaves together)
                 const uint32_t tSi = tS + (i & 1) * LT_BN, tPi = tP + (i & 1) * (LT_BN / 2);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (i * LT_BN + LT_BN - 1 > ctx + i0 / a.H) {   // some pair sees a part of this tile (a warp that has given up takes part)
-                    const int st = i % LT_STAGES;
-                    hid.clear(turn3 == 2 ? 0 : turn3 + 1, tid - 64, LT_BM);           // (all have left the tile that used it)
-                    if (alive && !at_mbar_wait_warp(&kv_full[st], (i / LT_STAGES) & 1, failed)) alive = false;    // (long since there)
-                    if (alive) {
-                        unsigned char* rows = sKV + (size_t)st * kv_bytes;           // (as keys they have been used: the scores are there)
-                        for (int e = tid - 64; e < n_lat * LT_BN * 8; e += LT_BM) {
-                            const int b = e / (LT_BN * 8), chunk = e % (LT_BN * 8);
-                            hid.clean(rows + (size_t)b * LT_K_BLOCK, chunk, b * 64, i * LT_BN + (chunk >> 3) >= kend, turn3);
-                        }
-                        at_proxy_fence();
-                    }
-                    asm volatile("bar.sync 1, 128;" ::: "memory");
-                    if (hid.any[turn3]) {
-                        bad = true;
-                        const unsigned long long sees = at_below(qpos + 1 - i * LT_BN);
-                        for (int c = 0; c < a.R; ++c)
-                            if (hid.keys[turn3][c] & sees) nans[(c >> 5) * LT_BM + row] |= 1u << (c & 31);
-                    }
-                    turn3 = turn3 == 2 ? 0 : turn3 + 1;
-                }
-                if (!alive) continue;                           // (the other warps' barriers still count on this one)
                 const int hi = valid ? min(qpos + 1 - i * LT_BN, LT_BN) : 0;      // keys of this tile that the pair sees: below hi
                 const bool full = hi >= LT_BN;
                 // the pair's 64 scores: their maximum, their weights against the reference into P, the weights' sum
@@ -263,7 +267,7 @@ __global__ void __launch_bounds__(LT_THREADS) latent_attention_tc_kernel(const _
                     m = mx;
                 }
                 if (i > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
-                    if (!at_mbar_wait_warp(&o_ready[(i - 1) & 1], ((i - 1) >> 1) & 1, failed)) { alive = false; continue; }   // the product before has added to O
+                    if (!at_mbar_wait_warp(&o_ready[(i - 1) & 1], ((i - 1) >> 1) & 1, failed)) { alive = false; break; }   // the product before has added to O
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     for (int c0 = 0; c0 < a.R; c0 += 32) {
                         uint32_t o[32];
@@ -297,7 +301,8 @@ __global__ void __launch_bounds__(LT_THREADS) latent_attention_tc_kernel(const _
                 __syncwarp();
                 if (lane == 0) at_mbar_arrive(&p_ready[i & 1]);
             }
-            if (alive && at_mbar_wait_warp(&o_ready[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1, failed)) {
+            if (alive && at_mbar_wait_warp(&o_ready[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1, failed)
+                && at_mbar_wait_warp(&v_ready[(n_tiles - 1) % LT_STAGES], ((n_tiles - 1) / LT_STAGES) & 1, failed)) {     // (the latter: the notes are seen)
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 float inv = l > 0.f ? 1.f / l : 0.f;
                 if (a.sink) {                                   // one more term of the denominator
@@ -309,7 +314,7 @@ __global__ void __launch_bounds__(LT_THREADS) latent_attention_tc_kernel(const _
                 for (int c0 = 0; c0 < a.R; c0 += 32) {
                     uint32_t o[32];
                     at_tmem_ld32(tO + c0, o);
-                    if (bad) at_put_nans(o, nans[(c0 >> 5) * LT_BM + row]);
+                    if (notes.count) at_put_nans(o, notes.met(c0 >> 5, qpos, 0, 0));
                     if (valid) {
 #pragma unroll
                         for (int d = 0; d < 32; d += 8) {
@@ -367,7 +372,7 @@ ZAI_API int zai_latent_attention_tc(void* out, const void* q_lat, const void* q_
     a.page_shift = 0;
     while ((1 << a.page_shift) < page_size) ++a.page_shift;
     const int n_blocks = R / 64 + (Dr > 0 ? 1 : 0);
-    constexpr size_t words = 256 + sizeof(AtHidden<LT_MAX_R>) + LT_MAX_R / 32 * LT_BM * sizeof(uint32_t);
+    constexpr size_t words = 256 + sizeof(LtNotes);
     static_assert(LT_MAX_BLOCKS * (LT_Q_BLOCK + LT_STAGES * LT_K_BLOCK) + words <= 227 * 1024, "one block an SM");
     const size_t smem = (size_t)n_blocks * (LT_Q_BLOCK + LT_STAGES * LT_K_BLOCK) + words;
     static unsigned long long configured = 0;
