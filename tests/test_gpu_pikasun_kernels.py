@@ -417,3 +417,29 @@ def test_latent_attention_leaves_calls_to_the_general_kernel(q_lens, monkeypatch
     o, case = latent_case(16, 256, 32, 64, [5] * len(q_lens), q_lens, 44, shift=1)
     assert torch.equal(o.latent_attention(*case), o.latent_attention(*case, impl="general"))
     assert o.read_status() == 0
+
+
+@pytest.mark.parametrize("impl", ["tcgen05", "mma"])
+def test_latent_attention_of_a_key_that_decides(impl):
+    """A key with nearly all of the weight, in a later tile than the one before it: its weight is exactly 1, so that the result is as near
+    to 64 bits as its own rounding allows (a weight of 2^4.75 or 2^6.25 in bfloat16 would be off by up to 0.14 %, a third more error)."""
+    o = ops()
+    H, R, ps, n = 16, 64, 32, 200
+    step = make_step(o, torch.bfloat16, [0], [n], ps, 16, 22)
+    g = torch.Generator().manual_seed(46)
+    ids = step.block_tables[0][0].cpu().long()
+    q = torch.zeros(n, H, R, dtype=torch.bfloat16)
+    q[:, :, 0] = 1.0
+    for lead in (4.75, 5.25, 6.25, 7.75):                                 # the later key's lead, in factors of two
+        rows = torch.randn(n, R, generator=g).bfloat16()
+        rows[:, 0] = 0.0
+        rows[0, 0], rows[100, 0] = 40.0, 40.0 + lead                      # (the others' weights are 2^-40 of them)
+        pages = torch.zeros(16, ps, R, dtype=torch.bfloat16)
+        pages[ids] = torch.cat([rows, torch.zeros(-n % ps, R, dtype=torch.bfloat16)]).view(-1, ps, R)
+        got = o.latent_attention(q.cuda(), torch.zeros(n, H, 0, dtype=torch.bfloat16).cuda(), step, CacheView(0, pages.cuda(), step.block_tables[0], ps),
+                                 H, R, 0, 0.6931471805599453, impl=impl)[150, 0].cpu()
+        w = torch.tensor([2.0 ** -lead, 1.0], dtype=torch.float64)
+        want = (w[:, None] * rows[[0, 100]].double()).sum(0) / w.sum()
+        off, least = (got.double() - want)[1:], (want.bfloat16().double() - want)[1:]
+        assert off.square().mean().sqrt() < 1.1 * least.square().mean().sqrt(), (lead, off.square().mean().sqrt() / least.square().mean().sqrt())
+    assert o.read_status() == 0

@@ -7,8 +7,7 @@
 //     S = Q K^T      tcgen05.mma, M = 128 pairs, N = 64 keys, K = R + Dr, operands from shared memory, into TMEM
 //     P = exp2(..)   four warps, a pair a thread: its 64 scores from TMEM, P back into TMEM as the next product's first operand
 //     O += P C       tcgen05.mma, the tile's own first R columns as values: the same bytes that were the keys, read as an MN-major
-//                    operand 64 columns at a time; O (R columns) stays in TMEM and is rescaled there only when a pair's reference
-//                    maximum has to move by more than 2^8
+//                    operand 64 columns at a time; O (R columns) stays in TMEM and is rescaled there when some pair's maximum moves
 //
 // Queries and cached rows come by TMA (no multicast) in boxes of 64 columns, the cached rows page by page into LT_STAGES stages; the
 // last box reaches beyond the row and is filled with zeros.  TMEM holds two score and two P buffers, so the scores of tile i + 2
@@ -226,15 +225,15 @@ __global__ void __launch_bounds__(LT_THREADS) latent_attention_tc_kernel(const _
                 }
             }
         } else {
-            // ---- softmax: thread = pair.  The pair's reference maximum is only moved, and O and the sum rescaled, when a tile's
-            // maximum exceeds it by more than 2^8 (P then stays below 256; the result does not depend on the reference).
+            // ---- softmax: thread = pair.  The pair's reference is its running maximum, so that the largest weight is exactly 1
+            // whatever it is rounded to.
             const int qd = warp & 3;                            // this warp's quarter of the TMEM lanes
             const int row = qd * 32 + lane;
             const bool valid = row < pairs;
             const int qpos = ctx + (i0 + row) / a.H;            // the pair's position: keys 0..qpos are visible
             const uint32_t tS = tmem_base + ((uint32_t)(qd * 32) << 16), tO = tS + LT_COL_O, tP = tS + LT_COL_P;
             const float c = a.scale_log2;
-            float m = -INFINITY, l = 0.f;                       // m: the pair's reference, in units of the scores
+            float m = -INFINITY, l = 0.f;                       // m: the pair's maximum, in units of the scores
             bool alive = true;
             for (int i = 0; i < n_tiles && alive; ++i) {
                 if (!at_mbar_wait_warp(&s_ready[i & 1], (i >> 1) & 1, failed)) { alive = false; break; }    // (the warp leaves together)
@@ -262,7 +261,7 @@ __global__ void __launch_bounds__(LT_THREADS) latent_attention_tc_kernel(const _
                 float alpha = 1.f;
                 if (m == -INFINITY) {
                     m = mx;                                     // nothing summed so far
-                } else if (mx * c > m * c + 8.f) {
+                } else if (mx > m) {
                     alpha = at_exp2(m * c - mx * c);
                     m = mx;
                 }
