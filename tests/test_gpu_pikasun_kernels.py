@@ -419,6 +419,26 @@ def test_latent_attention_leaves_calls_to_the_general_kernel(q_lens, monkeypatch
     assert o.read_status() == 0
 
 
+@pytest.mark.parametrize("H,R,Dr", [(16, 256, 32), (40, 128, 0), (3, 64, 16)])
+@pytest.mark.parametrize("captured", [False, True])
+def test_latent_attention_of_a_step_in_both_kernels(H, R, Dr, captured, monkeypatch):
+    """Spans on both sides of the line between the kernels, in any order, with and without ranges of keys, the long ones or the short ones
+    alone, and laid out like a captured step (more tiles than there are, a span without rows)."""
+    for ctx, q_lens in (([0, 63, 64, 300], [70, 1, 130, 3]), ([900, 5, 0, 40], [1, 2, 64, 1]), ([10, 700, 3], [1, 0, 33]), ([20, 0], [200, 7])):
+        o, case = latent_case(H, R, Dr, 32, ctx, q_lens, 45)
+        step, sink = case[2], torch.randn(H, generator=torch.Generator().manual_seed(1)).cuda()
+        if captured:
+            step.attn_tiles = sum(q_lens) // 128 + len(q_lens)
+        want = ref_ops.latent_attention(*case, sink=sink)
+        for cut in (1, 2, 33, 64, 130, 1 << 30):
+            monkeypatch.setattr(o, "_latent_cut", lambda *a: cut)
+            for wanted in (1, 1 << 30):                               # (mma.sync walks keys whole, or in ranges)
+                monkeypatch.setattr(o, "LATENT_WARPS_WANTED", wanted)
+                got = o.latent_attention(*case, sink=sink)
+                assert torch.allclose(got.float(), want.float(), **tol(torch.bfloat16)), (ctx, cut, float((got.float() - want.float()).abs().max()))
+    assert o.read_status() == 0
+
+
 @pytest.mark.parametrize("impl", ["tcgen05", "mma"])
 def test_latent_attention_of_a_key_that_decides(impl):
     """A key with nearly all of the weight, in a later tile than the one before it: its weight is exactly 1, so that the result is as near

@@ -31,3 +31,24 @@ def test_spans_take_their_kernels_by_the_layers_sizes_alone(cut):
         for d in (1, 8, 16, 32, 64):
             for v in (1, 8, 33, 64, 128, 256):
                 assert 64 <= cut(h, d, v) <= max(256, 32 * h)
+
+
+def test_latent_attention_goes_where_the_keys_are():
+    def cut(ctx, q_lens, heads=16, rank=256, captured=False):
+        s = step_of(q_lens, captured)
+        s.kv_lens = [c + n for c, n in zip(ctx, q_lens)]
+        return ops._latent_cut(s, heads, rank, 32)
+    # a span alone: by its rows, whatever its context
+    for ctx in (0, 1000, 16000):
+        assert cut([ctx], [64]) > 64 and cut([ctx], [128]) <= 128
+    assert cut([4000], [32], heads=128) <= 32 and cut([4000], [128], rank=128) > 128
+    # a few decoding requests far behind, beside a prompt's portion: their tiles would walk their keys alone
+    assert cut([16000] * 12 + [0], [1] * 12 + [100]) > 100
+    assert 1 < cut([16000] * 12 + [6000], [1] * 12 + [400]) <= 400
+    assert cut([16000, 0], [20, 200]) > 20
+    # many short spans together
+    assert cut([500] * 16, [20] * 16) == 1
+    # so many rows that mma.sync would not cut keys into ranges
+    assert cut([16000] * 12 + [0], [1] * 12 + [1900]) == 1
+    # contexts not known: each span by itself
+    assert 100 < cut([16000] * 12 + [0], [1] * 12 + [200], captured=True) <= 200

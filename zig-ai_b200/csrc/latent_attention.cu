@@ -228,6 +228,13 @@ __device__ __forceinline__ void lm_tile(float (&o)[LM_COLS / 8][4], float& m0, f
     }
 }
 
+// With cu_q, rows of spans longer than max_rows are another kernel's
+__device__ __forceinline__ bool lm_mine(int t, const int* __restrict__ seq_idx, const int* __restrict__ cu_q, int max_rows) {
+    if (!cu_q) return true;
+    const int s = seq_idx[t];
+    return cu_q[s + 1] - cu_q[s] <= max_rows;
+}
+
 // The factors that turn a row's unnormalised sums into its output when the denominator also holds 2^(sink log2 e): with
 // M the row's maximum (base 2, scaled) and Mn = max(M, sink'), out = O 2^(M - Mn) / (l 2^(M - Mn) + 2^(sink' - Mn)).
 __device__ __forceinline__ void lm_sink(float& inv0, float& inv1, float l0, float l1, float M0, float M1,
@@ -245,7 +252,7 @@ __global__ void __launch_bounds__(128) latent_attention_mma_kernel(
     const bf16* __restrict__ q_rot, const bf16* __restrict__ pages, const int* __restrict__ block_table, int table_width,
     const int* __restrict__ positions, const int* __restrict__ seq_idx, int page_size, int N, int H, int R, int Dr,
     float scale_log2, int split_keys, int n_splits, int warps_per_block, int num_pages, int* __restrict__ status,
-    const float* __restrict__ sink) {
+    const float* __restrict__ sink, const int* __restrict__ cu_q, int max_rows) {
     extern __shared__ __align__(16) unsigned char lm_smem[];
     const int W = R + Dr, ST = W + 8;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -260,6 +267,7 @@ __global__ void __launch_bounds__(128) latent_attention_mma_kernel(
     w /= RCH;
     const int hg = (int)(w % HG);
     const int t = (int)(w / HG);
+    if (!lm_mine(t, seq_idx, cu_q, max_rows)) return;
     bf16* sq = reinterpret_cast<bf16*>(lm_smem) + (size_t)warp * (16 + 2 * LM_KT) * ST;     // [16][ST] queries
     bf16* sk = sq + 16 * ST;                                                                // 2 x [LM_KT][ST] cached rows
     const int h0 = hg * 16, col0 = rc * LM_COLS;
@@ -360,7 +368,8 @@ __global__ void __launch_bounds__(128) latent_attention_rows_kernel(
     bf16* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml, const bf16* __restrict__ q_lat,
     const bf16* __restrict__ q_rot, const bf16* __restrict__ pages, const int* __restrict__ block_table, int table_width,
     const int* __restrict__ positions, const int* __restrict__ seq_idx, int page_size, int N, int H, int R, int Dr,
-    float scale_log2, int split_keys, int n_splits, int num_pages, int* __restrict__ status, const float* __restrict__ sink) {
+    float scale_log2, int split_keys, int n_splits, int num_pages, int* __restrict__ status, const float* __restrict__ sink,
+    const int* __restrict__ cu_q, int max_rows) {
     extern __shared__ __align__(16) unsigned char lm_smem[];
     __shared__ int s_key[4], s_khi[4];
     const int W = R + Dr, ST = W + 8;
@@ -370,13 +379,14 @@ __global__ void __launch_bounds__(128) latent_attention_rows_kernel(
     pdl_wait();
     // groups of heads fastest, then blocks of columns, then ranges of keys, then rows: neighbours share their cached rows
     long long w = (long long)blockIdx.x * 4 + warp;
-    const bool live = w < (long long)N * n_splits * RCH * HG;
+    bool live = w < (long long)N * n_splits * RCH * HG;
     const int hg = live ? (int)(w % HG) : 0;
     w /= HG;
     const int rc = live ? (int)(w % RCH) : 0;
     w /= RCH;
     const int split = live ? (int)(w % n_splits) : 0;
     const int t = live ? (int)(w / n_splits) : 0;
+    live = live && lm_mine(t, seq_idx, cu_q, max_rows);
     bf16* sq = reinterpret_cast<bf16*>(lm_smem) + (size_t)warp * 16 * ST;         // [16][ST] this warp's queries
     bf16* sk = reinterpret_cast<bf16*>(lm_smem) + (size_t)4 * 16 * ST;            // 2 x [LM_KT][ST] the block's cached rows
     const int h0 = hg * 16, col0 = rc * LM_COLS;
@@ -498,10 +508,12 @@ __global__ void __launch_bounds__(128) latent_attention_rows_kernel(
 
 // out[t, h, :] = sum_c O_c 2^(m_c - m) / sum_c l_c 2^(m_c - m), the ranges taken in order
 __global__ void latent_combine_kernel(bf16* __restrict__ out, const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                      int R, int n_splits, int H, const float* __restrict__ sink) {
+                                      int R, int n_splits, int H, const float* __restrict__ sink, const int* __restrict__ seq_idx,
+                                      const int* __restrict__ cu_q, int max_rows) {
     pdl_trigger();
     pdl_wait();
     const size_t th = blockIdx.x;
+    if (!lm_mine((int)(th / H), seq_idx, cu_q, max_rows)) return;
     const float* ml = part_ml + th * n_splits * 2;
     const float sk = sink ? sink[th % H] * 1.4426950408889634f : -INFINITY;
     float m = sk;
@@ -524,11 +536,12 @@ ZAI_API int zai_latent_attention_mma_supports(int R, int Dr) {
     return R >= 32 && R % 32 == 0 && Dr >= 0 && W % 16 == 0 && (size_t)(4 * 16 + 2 * LM_KT) * (W + 8) * 2 <= 200 * 1024;
 }
 
-// bfloat16; part_o [N, H, n_splits, R] and part_ml [N, H, n_splits, 2] 32-bit scratch (unused with n_splits = 1).
+// bfloat16; part_o [N, H, n_splits, R] and part_ml [N, H, n_splits, 2] 32-bit scratch (unused with n_splits = 1).  With cu_q (first
+// rows of the spans) only rows of spans of at most max_rows rows are run.
 ZAI_API int zai_latent_attention_mma(void* out, float* part_o, float* part_ml, const void* q_lat, const void* q_rot, const void* pages,
                                      const int* block_table, int table_width, const int* positions, const int* seq_idx,
                                      int page_size, int N, int H, int R, int Dr, float scale, int split_keys, int n_splits,
-                                     int num_pages, int* status, const float* sink, cudaStream_t stream) {
+                                     int num_pages, int* status, const float* sink, const int* cu_q, int max_rows, cudaStream_t stream) {
     if (N <= 0) return ZAI_OK;
     if (!zai_latent_attention_mma_supports(R, Dr) || H < 1 || n_splits < 1 || split_keys < LM_KT || split_keys % LM_KT) return ZAI_BAD_SIZE;
     const int cols = R <= 128 ? 128 : 256;
@@ -548,10 +561,10 @@ ZAI_API int zai_latent_attention_mma(void* out, float* part_o, float* part_ml, c
         auto rows_kernel = cols == 128 ? latent_attention_rows_kernel<128> : latent_attention_rows_kernel<256>;
         int rc = launch_pdl(rows_kernel, dim3((unsigned)blocks), dim3(128), smem, stream, (bf16*)out, part_o, part_ml,
                             (const bf16*)q_lat, (const bf16*)q_rot, (const bf16*)pages, block_table, table_width, positions, seq_idx,
-                            page_size, N, H, R, Dr, scale * 1.4426950408889634f, split_keys, n_splits, num_pages, status, sink);
+                            page_size, N, H, R, Dr, scale * 1.4426950408889634f, split_keys, n_splits, num_pages, status, sink, cu_q, max_rows);
         if (rc != 0 || n_splits == 1) return rc;
         return launch_pdl(latent_combine_kernel, dim3((unsigned)((size_t)N * H)), dim3(128), 0, stream, (bf16*)out,
-                          (const float*)part_o, (const float*)part_ml, R, n_splits, H, sink);
+                          (const float*)part_o, (const float*)part_ml, R, n_splits, H, sink, seq_idx, cu_q, max_rows);
     }
     const size_t per_warp = (size_t)(16 + 2 * LM_KT) * (R + Dr + 8) * 2;
     int wpb = (int)((200 * 1024) / per_warp);
@@ -567,10 +580,11 @@ ZAI_API int zai_latent_attention_mma(void* out, float* part_o, float* part_ml, c
     auto kernel = cols == 128 ? latent_attention_mma_kernel<128> : latent_attention_mma_kernel<256>;
     int rc = launch_pdl(kernel, dim3((unsigned)blocks), dim3(128), per_warp * wpb, stream, (bf16*)out, part_o,
                         part_ml, (const bf16*)q_lat, (const bf16*)q_rot, (const bf16*)pages, block_table, table_width, positions,
-                        seq_idx, page_size, N, H, R, Dr, scale * 1.4426950408889634f, split_keys, n_splits, wpb, num_pages, status, sink);
+                        seq_idx, page_size, N, H, R, Dr, scale * 1.4426950408889634f, split_keys, n_splits, wpb, num_pages, status, sink, cu_q,
+                        max_rows);
     if (rc != 0 || n_splits == 1) return rc;
     return launch_pdl(latent_combine_kernel, dim3((unsigned)((size_t)N * H)), dim3(128), 0, stream, (bf16*)out, (const float*)part_o,
-                      (const float*)part_ml, R, n_splits, H, sink);
+                      (const float*)part_ml, R, n_splits, H, sink, seq_idx, cu_q, max_rows);
 }
 
 // out [N, H, R], q_lat [N, H, R], q_rot [N, H, Dr], pages [num_pages, page_size, R + Dr], all in `dtype`; sink [H] 32-bit or null.

@@ -41,7 +41,7 @@ struct LtArgs {
     const int* ctx_lens;        // [S] positions cached before the step
     int* status;
     const float* sink;          // [H] or null
-    int num_pages, table_width, S, page_size, page_shift, H, R, Dr;
+    int num_pages, table_width, S, page_size, page_shift, H, R, Dr, min_rows;
     float scale_log2;
 };
 
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(LT_THREADS) latent_attention_tc_kernel(const _
     if (tid == 0) {
         int t = (int)gridDim.x - 1 - (int)blockIdx.x, s = 0;    // tiles of pairs from the last request's last ones backwards
         for (; s < a.S; ++s) {
-            const int nt = ((a.cu_q[s + 1] - a.cu_q[s]) * a.H + LT_BM - 1) / LT_BM;
+            const int n = a.cu_q[s + 1] - a.cu_q[s], nt = n < a.min_rows ? 0 : (n * a.H + LT_BM - 1) / LT_BM;
             if (t < nt) break;
             t -= nt;
         }
@@ -347,11 +347,12 @@ ZAI_API int zai_latent_attention_tc_supports(int H, int R, int Dr, int page_size
 }
 ZAI_API int zai_latent_attention_tc_pairs() { return LT_BM; }
 
-// out [N, H, R] from q_lat [N, H, R], q_rot [N, H, Dr] and pages [num_pages, page_size, R + Dr], bfloat16; n_tiles: the sum over the
-// spans of their rows x H / 128, rounded up (or more); sink [H] 32-bit or null.
+// out [N, H, R] from q_lat [N, H, R], q_rot [N, H, Dr] and pages [num_pages, page_size, R + Dr], bfloat16; spans of at least min_rows rows
+// are run; n_tiles: the sum over them of their rows x H / 128, rounded up (or more); sink [H] 32-bit or null.
 ZAI_API int zai_latent_attention_tc(void* out, const void* q_lat, const void* q_rot, const void* pages, int num_pages, int* status,
                                     const int* block_table, int table_width, const int* cu_q, const int* ctx_lens, int N, int S,
-                                    int n_tiles, int page_size, int H, int R, int Dr, float scale, const float* sink, cudaStream_t stream) {
+                                    int n_tiles, int page_size, int H, int R, int Dr, float scale, const float* sink, int min_rows,
+                                    cudaStream_t stream) {
     if (N <= 0 || S <= 0 || n_tiles <= 0) return ZAI_OK;
     if (!zai_latent_attention_tc_supports(H, R, Dr, page_size) || (long long)N * H > 0x7fffffffLL) return ZAI_BAD_SIZE;
     if ((reinterpret_cast<uintptr_t>(q_lat) | (Dr ? reinterpret_cast<uintptr_t>(q_rot) : 0) | reinterpret_cast<uintptr_t>(pages) | reinterpret_cast<uintptr_t>(out)) & 15)
@@ -366,7 +367,7 @@ ZAI_API int zai_latent_attention_tc(void* out, const void* q_lat, const void* q_
     if (e) return e;
     LtArgs a;
     a.out = (bf16*)out; a.block_table = block_table; a.cu_q = cu_q; a.ctx_lens = ctx_lens; a.status = status; a.sink = sink;
-    a.num_pages = num_pages; a.table_width = table_width; a.S = S; a.page_size = page_size; a.H = H; a.R = R; a.Dr = Dr;
+    a.num_pages = num_pages; a.table_width = table_width; a.S = S; a.page_size = page_size; a.H = H; a.R = R; a.Dr = Dr; a.min_rows = min_rows;
     a.scale_log2 = scale * 1.4426950408889634f;
     a.page_shift = 0;
     while ((1 << a.page_shift) < page_size) ++a.page_shift;

@@ -34,6 +34,7 @@ class StepBatch:
     decode_only: bool = False      # every span is one token
     q_lens: Sequence[int] = ()
     request_ids: Sequence = ()
+    kv_lens: Sequence[int] = ()    # ctx_len + q_len of every span
     single_first: int = 0          # this many leading spans (0, 8, 16, 32, ...) are one token each: in a step that also
     #                                holds longer spans, attention may run them through the kernel for single tokens
     attn_tiles: Optional[int] = None   # blocks of query rows to launch for span attention (default: from q_lens);
@@ -144,7 +145,7 @@ def batch_views(ops, dtype, dev: torch.Tensor, lay: PackedLayout) -> StepBatch:
         max_q_len=max(lay.q_lens) if lay.q_lens else 0,
         max_kv_len=max((c + n for c, n in zip(lay.ctx, lay.q_lens)), default=0),
         decode_only=all(n == 1 for n in lay.q_lens) and S > 0,
-        q_lens=lay.q_lens, request_ids=lay.request_ids)
+        q_lens=lay.q_lens, request_ids=lay.request_ids, kv_lens=[c + n for c, n in zip(lay.ctx, lay.q_lens)])
 
 
 def pack_step(ops, dtype, device, spans, tables: Dict[int, "np.ndarray"], pin: bool = False) -> StepBatch:

@@ -61,12 +61,12 @@ _SIGNATURES = {
     "latent_attention": {
         "zai_latent_attention": [_P, _P, _P, _P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P, _P, _P],
         "zai_latent_attention_mma_supports": [_I, _I],
-        "zai_latent_attention_mma": [_P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P, _P],
+        "zai_latent_attention_mma": [_P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _I, _I, _I, _P, _P, _P, _I, _P],
     },
     "latent_attention_tc": {
         "zai_latent_attention_tc_supports": [_I, _I, _I, _I],
         "zai_latent_attention_tc_pairs": [],
-        "zai_latent_attention_tc": [_P, _P, _P, _P, _I, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _P, _P],
+        "zai_latent_attention_tc": [_P, _P, _P, _P, _I, _P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _P, _I, _P],
     },
     "activation": {"zai_silu_mul": [_P, _P, _I, _I, _I, _P],
                    "zai_clamped_glu": [_P, _P, _I, _I, _I, _F, _F, _P],
@@ -1037,7 +1037,7 @@ def paged_attention(q, step, cache, heads, kv_heads, head_dim, scale, window=Non
     `impl="general"` with one warp a row and head.  `impl="mma"` / `impl="tcgen05"` pick between the two span kernels.
     `window`: a query sees the last `window` positions; `chunk`: it sees back to the start of its chunk of that
     many positions (the kernels take the chunk as a negative window).
-    Shaped scores (the general kernel): `softcap` (s <- cap tanh(s / cap)), `bias` [distances, heads] 32-bit (added after the
+    Shaped scores (the same kernels, each with the scores shaped inside it): `softcap` (s <- cap tanh(s / cap)), `bias` [distances, heads] 32-bit (added after the
     cap by min(distance, last row)), `sink` [heads] 32-bit (a term of the denominator alone), `keep_first` (with a window:
     the request's first positions stay visible)."""
     _cuda(q, bias, sink)
@@ -1627,22 +1627,51 @@ def latent_prepare(q, dkv, norm_w, eps, table, step, cache, heads, dim, rot_dim,
     return q_rot
 
 
-# From this many rows x groups of 16 heads on, steps with portions run latent attention in tiles of 128 (row, head) pairs on tcgen05:
-# a tile walks its keys at 29 us a thousand whatever the step's size, and the mma.sync kernels take 0.3 us a row, group and thousand
-# keys.  16 heads: 32 rows behind 8000 positions 90 (mma.sync) and 234 us, 128 behind 4000 160 and 124, 512 behind 6000 902
-# and 191, 2048 alone 282 and 66; 16 single tokens and 20 rows behind 6000 87 and 178.
-LATENT_TC_ROWS = 112
 LATENT_SPLIT_KEYS = 256          # keys per range where a step's rows are too few to fill the device
 LATENT_WARPS_WANTED = 1024       # from this many warps (rows x groups of 16 heads x blocks of output columns) on, no ranges
 USE_LATENT_MMA = os.environ.get("ZAI_LATENT_MMA", "1") == "1"
 
 
+def _latent_cut(step, heads, rank, rot_dim):
+    """Spans of this many rows or more run latent attention in tiles of 128 (row, head) pairs on tcgen05, the others with mma.sync.  A
+    tile walks its keys alone at `tile` us a thousand, however few of its pairs are used; mma.sync shares a span's keys among the chip
+    at `row` us a row and thousand keys.  So a span alone is quicker in tiles from tile / row rows on, whatever its context (rank 256 + 32,
+    16 heads, behind 8000: 96 rows 230 us by mma.sync and 236 in tiles, 128 rows 279 and 236; rank 128: 128 rows 136 and 162; 128 heads:
+    32 rows 310 and 246), and a step of several spans is what its longest tile and its other rows take: 12 single tokens behind 16 000
+    beside a prompt of 100 106 and 459, 16 spans of 20 behind 500 80 and 25.  Where the contexts are not known (a captured step shape) each
+    span goes by itself; steps of so many rows that mma.sync would not cut keys into ranges go in tiles (1912 rows, 12 of them behind 16 000:
+    4621 and 514)."""
+    groups, width = -(-heads // 16), rank + rot_dim
+    n = step.n_tokens
+    if n * groups * -(-rank // (128 if rank <= 128 else 256)) >= LATENT_WARPS_WANTED:
+        return 1
+    tile, row = 10.0 + 0.066 * width, 0.00095 * width * groups ** 0.7
+    own = max(int(tile / row), 1)
+    kv = getattr(step, "kv_lens", ()) if not getattr(step, "attn_tiles", None) and step.q_lens else ()
+    if len(kv) < 2:
+        return own
+    # thousands of keys: rows x keys of the spans below `own` and of all, and the tiles' longest walk (or the chip's share of all)
+    short = every = own_top = top = own_all = tiles_all = 0.0
+    for rows, end in zip(step.q_lens, kv):
+        keys = (end - 0.5 * rows) * 1e-3
+        work, share = rows * keys, -(-rows * heads // 128) * keys / 110
+        every += work
+        top, tiles_all = max(top, end * 1e-3), tiles_all + share
+        if rows < own:
+            short += work
+        else:
+            own_top, own_all = max(own_top, end * 1e-3), own_all + share
+    times = ((8 + tile * max(top, tiles_all), 1), (12 + row * every, 1 << 30),
+             ((12 + row * short if short else 0.0) + (8 + tile * max(own_top, own_all) if own_all else 0.0), own))
+    return min(times)[1]
+
+
 @_timed("attention")
 def latent_attention(q_lat, q_rot, step, cache, heads, rank, rot_dim, scale, impl=None, sink=None):
     """Causal attention of every head against the cached rows [latent | rotated key part]: scores
-    (q_lat . latent + q_rot . key part) * scale, output sum_j p_j latent_j, [N, H, rank].  bfloat16 steps with
-    many rows run on tcgen05 where the rank is a multiple of 64 up to 256 and rot_dim one of 16 up to 64 (`impl="tcgen05"` whatever
-    their size); else bfloat16 with a rank that is a multiple of 32 and rank + rot_dim a multiple of 16 runs on the tensor cores (steps of many rows: the four
+    (q_lat . latent + q_rot . key part) * scale, output sum_j p_j latent_j, [N, H, rank].  bfloat16 spans of many
+    rows run on tcgen05 where the rank is a multiple of 64 up to 256 and rot_dim one of 16 up to 64 (`_latent_cut`; `impl="tcgen05"`
+    whatever their size); else bfloat16 with a rank that is a multiple of 32 and rank + rot_dim a multiple of 16 runs on the tensor cores (steps of many rows: the four
     warps of a block share the tiles of cached rows; steps of few rows: a warp a row and range of keys, the ranges added
     up by a second kernel); everything else, and `impl="general"`, runs the general kernel.  `sink` [H] 32-bit: one more
     term exp(sink_h) in every row's denominator (no key, no value, not scaled)."""
@@ -1657,32 +1686,42 @@ def latent_attention(q_lat, q_rot, step, cache, heads, rank, rot_dim, scale, imp
     out = torch.empty((N, H, R), dtype=q_lat.dtype, device=q_lat.device)
     # (the tensor-core kernels' copies start on 16 bytes; ZAI_LATENT_MMA=0 leaves every call to the general kernel)
     tensor_cores = q_lat.dtype == torch.bfloat16 and not (q_lat.data_ptr() | (q_rot.data_ptr() if Dr else 0) | pages.data_ptr()) & 15
+    cut = 1 << 30                                              # (spans of that many rows or more run in tiles of pairs)
     if (tensor_cores and (impl == "tcgen05" or (impl is None and USE_LATENT_MMA)) and not step.decode_only
             and _fn("latent_attention_tc", "zai_latent_attention_tc_supports")(H, R, Dr, cache.page_size)):
-        if impl == "tcgen05" or N * -(-H // 16) >= LATENT_TC_ROWS:
-            pairs = _fn("latent_attention_tc", "zai_latent_attention_tc_pairs")()
-            captured = getattr(step, "attn_tiles", None) or not step.q_lens
-            tiles = N * H // pairs + step.n_seqs if captured else sum(-(-n * H // pairs) for n in step.q_lens)
-            _check(_fn("latent_attention_tc", "zai_latent_attention_tc")(
-                _ptr(out), _ptr(q_lat), _ptr(q_rot), _ptr(pages), pages.shape[0], _status_ptr(q_lat.device), _ptr(bt), bt.shape[1],
-                _ptr(step.cu_q), _ptr(step.ctx_lens), N, step.n_seqs, tiles, cache.page_size, H, R, Dr, float(scale), _ptr(sink),
-                _stream()), "latent_attention_tc")
+        cut = 1 if impl == "tcgen05" else _latent_cut(step, H, R, Dr)
+    long, short = _span_kinds(step, cut)
+    if long:
+        pairs = _fn("latent_attention_tc", "zai_latent_attention_tc_pairs")()
+        if getattr(step, "attn_tiles", None) or not step.q_lens:
+            tiles = N * H // pairs + min(step.n_seqs, N // cut)
+        else:
+            tiles = sum(-(-n * H // pairs) for n in step.q_lens if n >= cut)
+        _check(_fn("latent_attention_tc", "zai_latent_attention_tc")(
+            _ptr(out), _ptr(q_lat), _ptr(q_rot), _ptr(pages), pages.shape[0], _status_ptr(q_lat.device), _ptr(bt), bt.shape[1],
+            _ptr(step.cu_q), _ptr(step.ctx_lens), N, step.n_seqs, tiles, cache.page_size, H, R, Dr, float(scale), _ptr(sink),
+            cut, _stream()), "latent_attention_tc")
+        if not short or cut == 1:
             return out
     if (impl != "general" and (USE_LATENT_MMA or impl in ("mma", "mma_rows", "mma_ranges")) and tensor_cores
             and _fn("latent_attention", "zai_latent_attention_mma_supports")(R, Dr)):
-        warps = N * (-(-H // 16)) * (-(-R // (128 if R <= 128 else 256)))
+        rows = N
+        if long and not getattr(step, "attn_tiles", None) and step.q_lens:       # (up to the last row of a shorter span)
+            rows = sum(step.q_lens[:max(i for i, n in enumerate(step.q_lens) if 0 < n < cut) + 1])
+        warps = rows * (-(-H // 16)) * (-(-R // (128 if R <= 128 else 256)))
         n_splits = 1 if warps >= LATENT_WARPS_WANTED else max(-(-int(step.max_kv_len) // LATENT_SPLIT_KEYS), 1)
         if impl in ("mma_rows", "mma_ranges"):               # (tests pick the kernel whatever the step's size)
             n_splits = 1 if impl == "mma_rows" else max(-(-int(step.max_kv_len) // LATENT_SPLIT_KEYS), 1)
         split_keys = LATENT_SPLIT_KEYS if n_splits > 1 else 1 << 30           # one range: all keys
         part_o = part_ml = None
         if n_splits > 1:
-            part_o = torch.empty((N, H, n_splits, R), dtype=torch.float32, device=q_lat.device)
-            part_ml = torch.empty((N, H, n_splits, 2), dtype=torch.float32, device=q_lat.device)
+            part_o = torch.empty((rows, H, n_splits, R), dtype=torch.float32, device=q_lat.device)
+            part_ml = torch.empty((rows, H, n_splits, 2), dtype=torch.float32, device=q_lat.device)
         _check(_fn("latent_attention", "zai_latent_attention_mma")(
             _ptr(out), _ptr(part_o), _ptr(part_ml), _ptr(q_lat), _ptr(q_rot), _ptr(pages), _ptr(bt), bt.shape[1],
-            _ptr(step.positions), _ptr(step.seq_idx), cache.page_size, N, H, R, Dr, float(scale), split_keys, n_splits,
-            pages.shape[0], _status_ptr(q_lat.device), _ptr(sink), _stream()), "latent_attention_mma", 2 if n_splits > 1 else 1)
+            _ptr(step.positions), _ptr(step.seq_idx), cache.page_size, rows, H, R, Dr, float(scale), split_keys, n_splits,
+            pages.shape[0], _status_ptr(q_lat.device), _ptr(sink), _ptr(step.cu_q) if long else None, cut - 1, _stream()),
+            "latent_attention_mma", 2 if n_splits > 1 else 1)
         return out
     _check(_fn("latent_attention", "zai_latent_attention")(
         _ptr(out), _ptr(q_lat), _ptr(q_rot), _ptr(pages), _dt(q_lat), _ptr(bt), bt.shape[1], _ptr(step.positions), _ptr(step.seq_idx),
