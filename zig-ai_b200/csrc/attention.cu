@@ -103,8 +103,8 @@ __global__ void paged_attention_warp_kernel(T* __restrict__ out, const T* __rest
 // ---- spans of rows: a block owns AT_M (row, query head) pairs of one key/value head and one request (neighbouring rows, the heads
 // that share the keys) and walks the keys in tiles of AT_N, 32-bit multiply-adds throughout.  A thread makes 4 pairs x 4 keys of the
 // scores (rows ty 4 .., keys tx + 16 j) and 4 pairs x DM / 16 columns of the output; the 16 threads of a row are neighbouring lanes,
-// so its maximum, sum and weights need no block barrier.  Key tiles start at multiples of AT_N whatever the span, so a row's result
-// does not depend on how the request was cut into steps or on its batch.
+// so its maximum, sum and weights need no block barrier.  Key tiles start at multiples of AT_N whatever the span: a row's result is
+// the same in any portion and batch (steps of single tokens run the kernel above, whose sums have another order).
 //
 // What bounds it: 32-bit multiply-adds; eight 16-byte loads from shared memory feed 64 of them, and four blocks an SM (two at 128)
 // cover each other's loads and barriers.  A warp a row read every key and value from L2 once per row and head, keys by 32 lanes on

@@ -1053,7 +1053,8 @@ __global__ void __launch_bounds__(256) delta_carry_kernel(const DeltaArgs a) {
     DeltaColumns<DN>* su = ss + 2;                                            // [2] u
     pdl_trigger();
     pdl_wait();
-    const int seq = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * DN;
+    // (one dimension, which holds any number of requests: blocks of columns fastest, then heads, then requests)
+    const int per = (a.V + DN - 1) / DN, h = blockIdx.x / per % a.H, seq = blockIdx.x / per / a.H, v0 = blockIdx.x % per * DN;
     const int r0 = a.cu_q[seq], rows = a.cu_q[seq + 1] - r0;
     if (rows < a.min_rows) return;
     int first = 0;
@@ -1192,7 +1193,9 @@ static int delta_carry(const DeltaArgs& a, cudaStream_t stream) {
         const cudaError_t e = cudaFuncSetAttribute(delta_carry_kernel<DN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
     }
-    return launch_pdl(delta_carry_kernel<DN>, dim3(a.n_seqs, a.H, (a.V + DN - 1) / DN), dim3(256), smem, stream, a);
+    const long long blocks = (long long)a.n_seqs * a.H * ((a.V + DN - 1) / DN);
+    if (blocks > 0x7fffffffLL) return ZAI_BAD_SIZE;
+    return launch_pdl(delta_carry_kernel<DN>, dim3((unsigned)blocks), dim3(256), smem, stream, a);
 }
 
 ZAI_API int zai_gated_delta_chunk_rows() { return DC; }

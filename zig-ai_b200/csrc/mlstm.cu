@@ -14,7 +14,7 @@
 //     of one request and walks the request's rows of the step in order, its column of S in registers, the rows' q, k and gates
 //     staged in shared memory a tile of rows at a time by a second warp (the next tile comes in while a tile is walked); it
 //     leaves S^T q per column, n . q and m per row.  `mlstm_output_kernel` divides, norms per head and gates.
-//   * chunks of 64 rows on the tensor cores (bfloat16, spans of 64 rows or more, heads of up to 128), further below.
+//   * chunks of 64 rows on the tensor cores (bfloat16, longer spans, heads of up to 128), further below.
 #include "mma_helpers.cuh"
 
 // Rows staged at a time: as many as make the staged q and k 2 x 1024 values, at most 32 (a lane computes one row's gates).
@@ -375,13 +375,14 @@ __global__ void __launch_bounds__(256) mlstm_chunk_state_kernel(const MlstmArgs 
     }
 }
 
-// pass 2: a thread carries four neighbouring columns of one row of S across every chunk of a request (blockIdx.x); the maximum's
+// pass 2: a thread carries four neighbouring columns of one row of S across every chunk of a request; the maximum's
 // way is the same sum in every thread.
 __global__ void __launch_bounds__(128) mlstm_state_pass_kernel(const MlstmArgs a) {
     constexpr int AHEAD = 8;                                 // chunks whose loads are in flight
     pdl_trigger();
     pdl_wait();
-    const int s = blockIdx.x, h = blockIdx.y;
+    // (one dimension, which holds any number of requests: blocks of a head's state fastest, then heads, then requests)
+    const int blocks = (a.D * (a.VP / 4) + 127) / 128, h = blockIdx.x / blocks % a.H, s = blockIdx.x / blocks / a.H;
     const int rows = a.cu_q[s + 1] - a.cu_q[s];
     if (rows < a.min_rows) return;
     int c0 = 0;
@@ -390,7 +391,7 @@ __global__ void __launch_bounds__(128) mlstm_state_pass_kernel(const MlstmArgs a
         if (n >= a.min_rows) c0 += (n + MLSTM_Q - 1) / MLSTM_Q;
     }
     const int nc = (rows + MLSTM_Q - 1) / MLSTM_Q, per = a.VP / 4;
-    const int idx = blockIdx.z * blockDim.x + threadIdx.x;
+    const int idx = blockIdx.x % blocks * blockDim.x + threadIdx.x;
     if (idx >= a.D * per) return;
     const int d = idx / per, col = (idx % per) * 4, cols = a.Dv + 1;
     const int slot = zai_checked_slot(a.slot_ids[s], a.num_slots, a.status);
@@ -692,7 +693,9 @@ ZAI_API int zai_mlstm_chunked(void* out, const void* y, int y_stride, int q_at, 
     }
     int rc = launch_pdl(mlstm_chunk_state_kernel, dim3(max_chunks, H, (Dv + 63) / 64), dim3(256), mlstm_state_smem(D), stream, a);
     if (rc) return rc;
-    rc = launch_pdl(mlstm_state_pass_kernel, dim3(n_seqs, H, (D * (a.VP / 4) + 127) / 128), dim3(128), 0, stream, a);
+    const long long blocks = (long long)n_seqs * H * ((D * (a.VP / 4) + 127) / 128);
+    if (blocks > 0x7fffffffLL) return ZAI_BAD_SIZE;
+    rc = launch_pdl(mlstm_state_pass_kernel, dim3((unsigned)blocks), dim3(128), 0, stream, a);
     if (rc) return rc;
     return Dv <= 64 ? mlstm_chunk_out<64>(a, (bf16*)out, weight, eps, max_chunks, stream)
                     : mlstm_chunk_out<128>(a, (bf16*)out, weight, eps, max_chunks, stream);
