@@ -168,7 +168,6 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
     }
     // the softmax threads' state, kept past the roles for a shared tile's combination
     float m = -INFINITY, l = 0.f;                               // m: the row's reference, in units of the scores
-    uint32_t nans = 0;                                          // which of the thread's 32 columns have met a value that is not finite
     bool have_o = false;                                        // the row's O in TMEM is complete
     int row0 = 0, rows = 0;
     if (s < a.S && !failed_flag) {
@@ -188,13 +187,14 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
             n_tiles = min(per, n_tiles - from);
         }
         auto key_of = [&](int i) { return (SHAPED && from + i < n_kept ? from + i : tile0 + from + i - n_kept) * AT_BN; };   // the first key of tile i
-        // the tiles that some row does not see whole: those that end behind the first row (from tile p0 on; the last one counts as such:
-        // when its values are ready, so are all), and those before the last row's first key that are not kept (p1 to p2)
-        const int keep = SHAPED && a.window > 0 ? a.opt.keep_first : 0;
-        auto index_of = [&](int t) { return min(max((t < n_kept ? t : max(t, tile0) - tile0 + n_kept) - from, 0), n_tiles); };
-        const int p0 = min(index_of((ctx + i0 + 1) / AT_BN), n_tiles - 1), p1 = index_of(keep / AT_BN);
-        const int whole = index_of((zai_first_visible(kend - 1, a.window) + AT_BN - 1) / AT_BN), p2 = p1 < whole ? whole : 0;
-        auto part = [&](int i) { return i >= p0 || (i >= p1 && i < p2); };
+        // the tiles that some row does not see whole: those that end behind the first row (from tile p0 on, three at most; the last one
+        // counts as such: when its values are ready, so are all), and those before the last row's first key that are not kept (p1 to p2)
+        auto parts = [&](int& p0, int& p1, int& p2, int keep) {
+            auto index_of = [&](int t) { return min(max((t < n_kept ? t : max(t, tile0) - tile0 + n_kept) - from, 0), n_tiles); };
+            p0 = min(index_of((ctx + i0 + 1) / AT_BN), n_tiles - 1);
+            p1 = index_of(keep / AT_BN);
+            p2 = min(index_of((zai_first_visible(kend - 1, a.window) + AT_BN - 1) / AT_BN), p0);
+        };
 
         if (warp == 0) {
             if (n_tiles > 0) {
@@ -205,34 +205,34 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
                     at_mbar_expect_tx(&q_full, AT_Q_BYTES);
                     at_tma_load_2d(sQ, &map_q, h * AT_D, row0 + i0, &q_full);
                 }
-                int issued = 0;
-                for (int i = 0; i < n_tiles; ++i) {             // (i: the next tile whose values may need cleaning)
-                    i = min(i < p2 ? max(i, p1) : n_tiles, max(i, p0));
-                    bool ok = true;
-                    if (lane == 0)                              // one lane issues all loads up to AT_LAG tiles behind it
-                        for (const int end = min(i + AT_LAG + 1, n_tiles); issued < end && ok; ++issued) {
-                            const int st = issued % STAGES;
-                            ok = at_mbar_wait(&kv_empty[st], ((issued / STAGES) & 1) ^ 1, failed);
-                            if (!ok) break;
-                            at_mbar_expect_tx(&kv_full[st], AT_KV_BYTES);
-                            unsigned char* dst = sKV + (size_t)st * AT_KV_BYTES;
-                            for (int p = 0; p < per_tile; ++p) {
-                                const int key0 = key_of(issued) + p * box_rows;
-                                const int idx = key0 >> a.page_shift, off = key0 & (ps - 1);
-                                int page = idx < a.table_width ? table[idx] : 0;      // beyond the table: the null page
-                                if ((unsigned)page >= (unsigned)a.num_pages) {        // outside the pool: page 0, and the step is void
-                                    zai_raise(a.status, ZAI_ST_PAGE);
-                                    page = 0;
-                                }
-                                const int krow = ((page * 2 + 0) * a.Hkv + hk) * ps + off;
-                                const int vrow = ((page * 2 + 1) * a.Hkv + hk) * ps + off;
-                                at_tma_load_2d(dst + (size_t)p * box_rows * 128, &map_kv, 0, krow, &kv_full[st]);
-                                at_tma_load_2d(dst + AT_BN * 128 + (size_t)p * box_rows * 128, &map_kv, 0, vrow, &kv_full[st]);
+                const int keep = SHAPED && a.window > 0 ? a.opt.keep_first : 0;
+                int p0, p1, p2, issued = 0;
+                parts(p0, p1, p2, keep);
+                auto load = [&](int end) {                      // by one lane: the tiles up to `end`
+                    for (; issued < end; ++issued) {
+                        const int st = issued % STAGES;
+                        if (!at_mbar_wait(&kv_empty[st], ((issued / STAGES) & 1) ^ 1, failed)) break;
+                        at_mbar_expect_tx(&kv_full[st], AT_KV_BYTES);
+                        unsigned char* dst = sKV + (size_t)st * AT_KV_BYTES;
+                        for (int p = 0; p < per_tile; ++p) {
+                            const int key0 = key_of(issued) + p * box_rows;
+                            const int idx = key0 >> a.page_shift, off = key0 & (ps - 1);
+                            int page = idx < a.table_width ? table[idx] : 0;          // beyond the table: the null page
+                            if ((unsigned)page >= (unsigned)a.num_pages) {            // outside the pool: page 0, and the step is void
+                                zai_raise(a.status, ZAI_ST_PAGE);
+                                page = 0;
                             }
-                            if (!part(issued)) at_mbar_arrive(&v_ready[st]);
+                            const int krow = ((page * 2 + 0) * a.Hkv + hk) * ps + off;
+                            const int vrow = ((page * 2 + 1) * a.Hkv + hk) * ps + off;
+                            at_tma_load_2d(dst + (size_t)p * box_rows * 128, &map_kv, 0, krow, &kv_full[st]);
+                            at_tma_load_2d(dst + AT_BN * 128 + (size_t)p * box_rows * 128, &map_kv, 0, vrow, &kv_full[st]);
                         }
+                        if (issued < p0 && (issued < p1 || issued >= p2)) at_mbar_arrive(&v_ready[st]);
+                    }
+                };
+                auto clean = [&](int i) {                       // by the warp: the values of tile i
                     const int st = i % STAGES, tile_key = key_of(i);
-                    if (!__shfl_sync(0xffffffffu, ok, 0) || !at_mbar_wait_warp(&kv_full[st], (i / STAGES) & 1, failed)) break;
+                    if (!at_mbar_wait_warp(&kv_full[st], (i / STAGES) & 1, failed)) return false;
                     unsigned char* values = sKV + (size_t)st * AT_KV_BYTES + AT_KV_BYTES / 2;
                     const unsigned long long shown = at_below(kend - tile_key) & (~at_below(kbeg - tile_key) | at_below(keep - tile_key));
                     if (__any_sync(0xffffffffu, at_clean<4>(values, lane >> 3, shown)))
@@ -246,7 +246,19 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
                     at_proxy_fence();                           // (generic writes, which the product reads)
                     __syncwarp();
                     if (lane == 0) at_mbar_arrive(&v_ready[st]);
+                    return true;
+                };
+                // A window's first tiles with the loads AT_LAG tiles ahead of them, then all other loads by the one lane alone (with the warp
+                // in step beside it a tile's load came a third later), then the last tiles, whose loads need none of their products
+                bool ok = true;
+                for (int i = p1; i < p2 && ok; ++i) {
+                    if (lane == 0) load(min(i + AT_LAG + 1, n_tiles));
+                    __syncwarp();
+                    ok = clean(i);
                 }
+                if (lane == 0) load(n_tiles);
+                __syncwarp();
+                for (int i = p0; i < n_tiles && ok; ++i) ok = clean(i);
                 if (lane == 0 && *failed) {                     // loads already issued still land here: wait for them
                     for (int i = max(issued - STAGES, 0); i < issued; ++i) {
                         const uint32_t addr = at_smem(&kv_full[i % STAGES]);
@@ -293,10 +305,10 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
                 // tile i ends
                 if (ok) ok = scores(0);
                 if (ok && n_tiles > 1) ok = scores(1);
-                for (int i = 0; i < n_tiles && ok; ++i) {
+                auto product = [&](int i, bool wait) {          // O += P V of tile i, and the scores of tile i + 2; `wait`: its values are cleaned
                     const int st = i % STAGES;
-                    ok = at_mbar_wait(&p_ready[i & 1], (i >> 1) & 1, failed) && (!part(i) || at_mbar_wait(&v_ready[st], (i / STAGES) & 1, failed));
-                    if (!ok) break;
+                    ok = at_mbar_wait(&p_ready[i & 1], (i >> 1) & 1, failed) && (!wait || at_mbar_wait(&v_ready[st], (i / STAGES) & 1, failed));
+                    if (!ok) return;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t aV = at_smem(sKV + (size_t)st * AT_KV_BYTES + AT_BN * 128);
 #pragma unroll
@@ -305,7 +317,12 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
                     at_commit(&o_ready[i & 1]);
                     at_commit(&kv_empty[st]);
                     if (i + 2 < n_tiles) ok = scores(i + 2);
-                }
+                };
+                int p0, p1, p2, i = 0;
+                parts(p0, p1, p2, SHAPED && a.window > 0 ? a.opt.keep_first : 0);
+                for (; i < p2 && ok; ++i) product(i, i >= p1);
+                for (; i < p0 && ok; ++i) product(i, false);
+                for (; i < n_tiles && ok; ++i) product(i, true);
             }
         } else if (n_tiles > 0) {
             // ---- softmax: thread = half of a query row (32 of a tile's 64 columns).  O stays in TMEM (the products add to
@@ -433,7 +450,6 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
             if (alive && at_mbar_wait_warp(&o_ready[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1, failed)) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 have_o = at_mbar_wait_warp(&v_ready[(n_tiles - 1) % STAGES], ((n_tiles - 1) / STAGES) & 1, failed);    // (long since; the notes are seen)
-                if (notes.count) nans = notes.met(half, qpos, klo, kept);
                 float inv = l > 0.f ? 1.f / l : 0.f;
                 if (SHAPED && a.opt.sink) {                     // one more term of the denominator
                     const float M = m * c, sk = a.opt.sink[h] * 1.4426950408889634f, top = fmaxf(M, sk);
@@ -444,7 +460,6 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
                 if (!SHARED) {
                     uint32_t r[32];
                     at_tmem_ld32(tO, r);
-                    if (nans) at_put_nans(r, nans);
                     if (valid) {
 #pragma unroll
                         for (int d = 0; d < 32; d += 8) {
@@ -456,6 +471,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
                             }
                             *reinterpret_cast<uint4*>(dst + d) = make_uint4(v[0], v[1], v[2], v[3]);
                         }
+                        if (notes.count) notes.put_nans(dst, 1, half, 1, qpos, klo, kept);
                     }
                 }
             }
@@ -477,9 +493,12 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
         if (ok) {
             uint32_t r[32];
             at_tmem_ld32(tO, r);
-            if (nans) at_put_nans(r, nans);
 #pragma unroll
             for (int j = 0; j < 32; ++j) po[j * AT_BM + row] = __uint_as_float(r[j]);
+            if (notes.count) {
+                const int qpos = a.ctx_lens[s] + i0 + row, klo = zai_first_visible(qpos, a.window);
+                notes.put_nans(po + row, AT_BM, half, 1, qpos, klo, SHAPED && a.window > 0 ? min(a.opt.keep_first, klo) : 0);
+            }
         }
         asm volatile("bar.sync 5, 256;" ::: "memory");          // the eight softmax warps
         if (tid == 64) {

@@ -176,20 +176,20 @@ struct AtNotes {
         atomicMax(&high, k);
         return -1;
     }
-    // the columns 32 w .. that a row with keys [from, pos] and [0, kept) has met such values in (all, if it may see a key without room)
-    __device__ __noinline__ uint32_t met(int w, int pos, int from, int kept) const {
-        uint32_t m = low <= pos && (high >= from || low < kept) ? 0xffffffffu : 0u;
-        for (int i = 0; i < min(count, MOST); ++i)
-            if (key[i] <= pos && (key[i] >= from || key[i] < kept)) m |= (uint32_t)(cols[i][w >> 1] >> ((w & 1) * 32));
-        return m;
+    // NaN into the values of a row's columns [32 w, 32 w + 32 n), `step` values apart, that have met a value that is not finite at a key of
+    // [from, pos] or [0, kept) (all of them, if it may see a key without room).  A call behind the row's stores: rare, and not
+    // to be carried by what comes before it
+    template <typename T>
+    __device__ __noinline__ void put_nans(T* row, size_t step, int w, int n, int pos, int from, int kept) const {
+        for (int k = w; k < w + n; ++k) {
+            uint32_t m = low <= pos && (high >= from || low < kept) ? 0xffffffffu : 0u;
+            for (int i = 0; i < min(count, MOST); ++i)
+                if (key[i] <= pos && (key[i] >= from || key[i] < kept)) m |= (uint32_t)(cols[i][k >> 1] >> ((k & 1) * 32));
+            for (int j = 0; j < 32; ++j)
+                if (m >> j & 1) row[((k - w) * 32 + j) * step] = from_float<T>(__int_as_float(0x7fc00000));
+        }
     }
 };
-__device__ __forceinline__ void at_put_nans(uint32_t (&r)[32], uint32_t which) {
-#pragma unroll
-    for (int j = 0; j < 32; ++j)
-        if (which >> j & 1) r[j] = 0x7fc00000u;
-}
-
 // ------------------------------------------------------------------------------------------ host side
 typedef CUresult (*AtEncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                     const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,

@@ -15,9 +15,9 @@
 // not every pair sees whole), warp 1 one lane the products, warps 2-5 are the softmax.  Blocks are handed out from the last pairs
 // backwards (they have the most keys).  Every wait on an mbarrier is bounded; a block whose wait runs out raises the status word, its roles leave their loops, TMEM is freed and the block returns.
 //
-// What bounds it: the chain of a tile (scores, softmax, P, product), 1.8 us of 64 keys, with one block an SM (200 KB of shared memory);
-// the products' tensor time is about 0.8 us of it.  16 heads, R = 256, Dr = 32: 2048 rows 282 us (mma.sync, four warps sharing tiles of
-// 32) -> 66 us (550 TFLOP/s causal), behind 6144 positions 1505 -> 411 (620 TFLOP/s); 512 rows behind 6000 902 -> 191.
+// What bounds it: the chain of a tile (scores, softmax, P, product), 2.1 us of 64 keys, with one block an SM (200 KB of shared memory);
+// the products' tensor time is about 0.8 us of it.  16 heads, R = 256, Dr = 32, mma.sync (four warps sharing tiles of 32) and here: 2048
+// rows 275 and 77 us, 128 behind 4000 160 and 136 (the reference as the running maximum takes 5 % of it, the cleaning 2 %).
 #include "attention_tc_helpers.cuh"
 
 #define LT_BM 128
@@ -31,7 +31,6 @@
 #define LT_TMEM_COLS 512                              // two score buffers in columns 0..127, O in 128..383, two P buffers in 384..447
 #define LT_COL_O (2 * LT_BN)
 #define LT_COL_P (LT_COL_O + LT_MAX_R)
-#define LT_LAG 1                                      // tiles that the cleaning is behind the loads (below the number of stages)
 typedef AtNotes<LT_MAX_R / 64, 64> LtNotes;
 
 struct LtArgs {
@@ -125,8 +124,8 @@ __global__ void __launch_bounds__(LT_THREADS) latent_attention_tc_kernel(const _
         const int pairs = min(LT_BM, (a.cu_q[s + 1] - row0) * a.H - i0);      // valid pairs of this block
         const int kend = ctx + (i0 + pairs - 1) / a.H + 1;                    // one past the last visible key of the block
         const int n_tiles = (kend + LT_BN - 1) / LT_BN;
-        // the tiles that end behind the first pair's row (the last one counts as such: when its values are ready, so are all)
-        const int p0 = min((ctx + i0 / a.H + 1) / LT_BN, n_tiles - 1);
+        // the tiles that end behind the first pair's row, three at most (the last one counts as such: when its values are ready, so are all)
+        auto first_part = [&]() { return min((ctx + i0 / a.H + 1) / LT_BN, n_tiles - 1); };
 
         if (warp == 0) {
             // ---- loads: the block's queries, then a stage of cached rows per tile, page by page
@@ -137,33 +136,34 @@ __global__ void __launch_bounds__(LT_THREADS) latent_attention_tc_kernel(const _
                 for (int b = 0; b < n_blocks; ++b)
                     at_tma_load_2d(sQ + (size_t)b * LT_Q_BLOCK, b < n_lat ? &map_lat : &map_rot, b < n_lat ? b * 64 : 0, row0 * a.H + i0, &q_full);
             }
+            const int p0 = first_part();
             int issued = 0;
-            for (int i = p0; i < n_tiles; ++i) {
-                bool ok = true;
-                if (lane == 0)                                  // one lane issues all loads up to LT_LAG tiles behind this one
-                    for (const int end = min(i + LT_LAG + 1, n_tiles); issued < end && ok; ++issued) {
-                        const int st = issued % LT_STAGES;
-                        ok = at_mbar_wait(&kv_empty[st], ((issued / LT_STAGES) & 1) ^ 1, failed);
-                        if (!ok) break;
-                        at_mbar_expect_tx(&kv_full[st], kv_bytes);
-                        unsigned char* dst = sKV + (size_t)st * kv_bytes;
-                        for (int p = 0; p < per_tile; ++p) {
-                            const int key0 = issued * LT_BN + p * box_rows;
-                            const int idx = key0 >> a.page_shift, off = key0 & (ps - 1);
-                            int page = idx < a.table_width ? table[idx] : 0;          // beyond the table: the null page
-                            if ((unsigned)page >= (unsigned)a.num_pages) {            // outside the pool: page 0, and the step is void
-                                zai_raise(a.status, ZAI_ST_PAGE);
-                                page = 0;
-                            }
-                            for (int b = 0; b < n_blocks; ++b)
-                                at_tma_load_2d(dst + (size_t)b * LT_K_BLOCK + (size_t)p * box_rows * 128, &map_kv, b * 64, page * ps + off, &kv_full[st]);
+            if (lane == 0)
+                for (; issued < n_tiles; ++issued) {
+                    const int st = issued % LT_STAGES;
+                    if (!at_mbar_wait(&kv_empty[st], ((issued / LT_STAGES) & 1) ^ 1, failed)) break;
+                    at_mbar_expect_tx(&kv_full[st], kv_bytes);
+                    unsigned char* dst = sKV + (size_t)st * kv_bytes;
+                    for (int p = 0; p < per_tile; ++p) {
+                        const int key0 = issued * LT_BN + p * box_rows;
+                        const int idx = key0 >> a.page_shift, off = key0 & (ps - 1);
+                        int page = idx < a.table_width ? table[idx] : 0;              // beyond the table: the null page
+                        if ((unsigned)page >= (unsigned)a.num_pages) {                // outside the pool: page 0, and the step is void
+                            zai_raise(a.status, ZAI_ST_PAGE);
+                            page = 0;
                         }
-                        if (issued < p0) at_mbar_arrive(&v_ready[st]);
+                        for (int b = 0; b < n_blocks; ++b)
+                            at_tma_load_2d(dst + (size_t)b * LT_K_BLOCK + (size_t)p * box_rows * 128, &map_kv, b * 64, page * ps + off, &kv_full[st]);
                     }
+                    if (issued < p0) at_mbar_arrive(&v_ready[st]);
+                }
+            __syncwarp();
+            // the last tiles' values, behind all loads (which need none of their products): with the warp in step beside the one lane a
+            // tile's load came a sixth later
+            for (int i = p0; i < n_tiles; ++i) {
                 // as keys the rows have to stay what they are until the scores are there
                 const int st = i % LT_STAGES;
-                if (!__shfl_sync(0xffffffffu, ok, 0) || !at_mbar_wait_warp(&kv_full[st], (i / LT_STAGES) & 1, failed)
-                    || !at_mbar_wait_warp(&s_ready[i & 1], (i >> 1) & 1, failed)) break;
+                if (!at_mbar_wait_warp(&kv_full[st], (i / LT_STAGES) & 1, failed) || !at_mbar_wait_warp(&s_ready[i & 1], (i >> 1) & 1, failed)) break;
                 unsigned char* rows = sKV + (size_t)st * kv_bytes + (size_t)(lane >> 3) * LT_K_BLOCK;
                 const bool mine = (lane >> 3) < n_lat;          // (a row a turn, eight lanes a block of 64 columns)
                 const bool odd = mine && at_clean<1>(rows, 0, at_below(kend - i * LT_BN));
@@ -207,10 +207,10 @@ __global__ void __launch_bounds__(LT_THREADS) latent_attention_tc_kernel(const _
                 };
                 if (ok) ok = scores(0);
                 if (ok && n_tiles > 1) ok = scores(1);
-                for (int i = 0; i < n_tiles && ok; ++i) {
+                auto product = [&](int i, bool wait) {          // O += P C of tile i, and the scores of tile i + 2; `wait`: its values are cleaned
                     const int st = i % LT_STAGES;
-                    ok = at_mbar_wait(&p_ready[i & 1], (i >> 1) & 1, failed) && (i < p0 || at_mbar_wait(&v_ready[st], (i / LT_STAGES) & 1, failed));
-                    if (!ok) break;
+                    ok = at_mbar_wait(&p_ready[i & 1], (i >> 1) & 1, failed) && (!wait || at_mbar_wait(&v_ready[st], (i / LT_STAGES) & 1, failed));
+                    if (!ok) return;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t aV = at_smem(sKV + (size_t)st * kv_bytes);
                     for (int b = 0; b < n_lat; ++b) {
@@ -222,7 +222,11 @@ __global__ void __launch_bounds__(LT_THREADS) latent_attention_tc_kernel(const _
                     at_commit(&o_ready[i & 1]);
                     at_commit(&kv_empty[st]);
                     if (i + 2 < n_tiles) ok = scores(i + 2);
-                }
+                };
+                const int p0 = first_part();
+                int i = 0;
+                for (; i < p0 && ok; ++i) product(i, false);
+                for (; i < n_tiles && ok; ++i) product(i, true);
             }
         } else {
             // ---- softmax: thread = pair.  The pair's reference is its running maximum, so that the largest weight is exactly 1
@@ -313,7 +317,6 @@ __global__ void __launch_bounds__(LT_THREADS) latent_attention_tc_kernel(const _
                 for (int c0 = 0; c0 < a.R; c0 += 32) {
                     uint32_t o[32];
                     at_tmem_ld32(tO + c0, o);
-                    if (notes.count) at_put_nans(o, notes.met(c0 >> 5, qpos, 0, 0));
                     if (valid) {
 #pragma unroll
                         for (int d = 0; d < 32; d += 8) {
@@ -327,6 +330,7 @@ __global__ void __launch_bounds__(LT_THREADS) latent_attention_tc_kernel(const _
                         }
                     }
                 }
+                if (valid && notes.count) notes.put_nans(dst, 1, 0, a.R / 32, qpos, 0, 0);
             }
         }
     }
