@@ -506,19 +506,21 @@ ZAI_API int zai_gated_rmsnorm(void* out, const float* o, const float* w, const v
 //
 // The first line is a triangular system with the same matrix for every column: its solution for the right sides beta_t v_t (U0)
 // and beta_t e^(c_t) k_t (W) needs no state, and u = U0 - W S_0.  Two kernels:
-//   * `delta_chunk_kernel`, every chunk and head at once: unit norms, decays, A, P, and the system solved by substitution in
-//     32-bit, a thread a right side with its 64 unknowns in registers.  A and P are products of bfloat16 rows, or, with a decay per
-//     channel, of rows in three parts scaled by e^(c_t - c_first) and e^(c_first - c_s) around the first of 16 rows; inside 16 rows
-//     that decay by more than 2^-100 the pairs of rows are taken one by one instead.  Running sums are made in 64-bit and kept in
-//     two parts, so that a difference of two is good to the last bits.
+//   * `delta_chunk_kernel`, every chunk and head at once: unit norms, decays, A, P, and the system solved in four steps of 16 rows,
+//     16 right sides a warp: 32-bit substitution among the 16, their part in later rows on the tensor cores.  A and P are products
+//     of bfloat16 rows, or, with a decay per channel, of rows in three parts scaled by e^(c_t - c_first) and e^(c_first - c_s) around the
+//     first of 16 rows; inside 16 rows that decay by more than 2^-100 the pairs of rows are taken one by one instead.  Running
+//     sums are made in 64-bit and kept in two parts, so that a difference of two is good to the last bits.
 //   * `delta_carry_kernel`, a block a head and DN columns of S: carries S across a request's chunks on the tensor cores (four
 //     warps: u, then the new S) and makes the chunks' read-outs beside that (four more warps).  S, u, W, P and the scaled k and q
 //     are 32-bit and go into bfloat16 products as sums of three parts (24 bits; the six products that reach 2^-24 of the
 //     result), with 32-bit sums by size.  What comes from the first kernel is laid out as a lane's operands of one m16n8k16
 //     product lie, three parts beforehand: 16 bytes a load, nothing to convert.
 // 2048 rows of 16 heads of 64 x 128 (norms, recurrence and output norm): 136 us where the walk takes 480, with a decay per channel
-// 172 (601); of 32 heads 233 (581) and 292 (660).  The first kernel (53 and 88 us of 16 heads) is bound by its phases' latencies
-// with two blocks an SM, the second (58) by a chunk's two dependent products, 1.8 us a chunk at 43 % of the tensor pipe.
+// 172 (601); of 32 heads 233 (581) and 292 (660), before the first kernel's system went to the tensor cores.  The first kernel (16 heads
+// of 2048 rows, a decay per channel: 91 us with a right side a thread, 65 now; 32 heads of 1300 rows, one per head: 77 and 62) is bound by
+// the instructions that a block issues (some 60 000, at half of what two blocks an SM could), the second (58) by a chunk's two
+// dependent products, 1.8 us a chunk at 43 % of the tensor pipe.
 #define DC 64                       // rows of a chunk
 #define DCD 64                      // key size the chunk kernels are made for (smaller heads are filled up with zeros)
 #define DC_LD 68                    // 32-bit row stride in shared memory
@@ -574,6 +576,12 @@ __device__ __forceinline__ float delta_exp2(float x, float y) {
     return fmaf(e, 0.69314718f * y, e);
 }
 
+// an 8 x 8 matrix of 16-bit values, a row four lanes: its rows become its columns
+__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t v) {
+    uint32_t r;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+    return r;
+}
 // 16 sums over 16 neighbouring lanes at once: lane i of the 16 ends with the sum of v[i] in v[0]
 __device__ __forceinline__ void sum16(float (&v)[16], int lane) {
 #pragma unroll
@@ -590,6 +598,7 @@ __device__ __forceinline__ void sum16(float (&v)[16], int lane) {
 // Writes an operand: get(row, column) gives two neighbouring columns (the first even); all 256 threads
 template <typename F>
 __device__ __forceinline__ void delta_put(DeltaOperand* out, F get) {
+#pragma unroll 1
     for (int i = threadIdx.x; i < 4 * 4 * 32; i += 256) {
         const int lane = i & 31, kt = (i >> 5) & 3, mt = i >> 7, g = lane >> 2, tq = lane & 3;
         uint32_t part[4][3];
@@ -616,16 +625,14 @@ struct DeltaShared {
             bf16 left[2][3][16][DR_LD];                      // 16 rows of q and k times e^(c_t - c at their first), in three parts
             bf16 right[3][DC][DR_LD];                        // the rows of k up to them times e^(c at their first - c_s), likewise
         };
+        bf16 a[DC][DR_LD];                                   // before that: what the decays per channel are made of
         bf16 v[DC * (DELTA_V_MAX + 8)];                      // then: the rows of v, V + 8 values apart
     };
-    float m[DC][DC_LD];                                      // beta_t A_ts below the diagonal, P_ts at [s][t] on and above it
-    union {
-        struct {
-            float hi[DC][DCD];                               // running log decays inside the 16 rows (one column: the chunk's), in
-            bf16 lo[DC][DCD];                                // two parts (32 bits of their sums)
-        } c;
-        float w[DC][DC_LD];                                  // W, when the decays are no longer needed
-    };
+    float m[DC][DC_LD];                                      // beta_t A_ts below the diagonal
+    struct {
+        float hi[DC][DCD];                                   // running log decays inside the 16 rows (one column: the chunk's), in
+        bf16 lo[DC][DCD];                                    // two parts (32 bits of their sums)
+    } c;
     float sum[4][DCD], sum_lo[4][DCD];                       // log decay of every 16 rows, in two parts
     float before[5][DCD], after[4][DCD];                     // ... of all 16s before (4: of the chunk), and after
     float beta[DC];
@@ -638,10 +645,13 @@ struct DeltaShared {
         return make_float2(x.x * i, x.y * i);
     }
     __device__ __forceinline__ float2 at(int t, int d) const { return make_float2(c.hi[t][d], to_float(c.lo[t][d])); }
-    // two neighbouring sums: their leading parts and what is left
-    __device__ __forceinline__ void at_two(int t, int d, float2& x, float2& y) const {
-        x = *reinterpret_cast<const float2*>(&c.hi[t][d]);
-        y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&c.lo[t][d]));
+    // four neighbouring sums: their leading parts and what is left
+    __device__ __forceinline__ void at_four(int t, int d, float (&x)[4], float (&y)[4]) const {
+        const float4 hi = *reinterpret_cast<const float4*>(&c.hi[t][d]);
+        const uint2 lo = *reinterpret_cast<const uint2*>(&c.lo[t][d]);
+        x[0] = hi.x, x[1] = hi.y, x[2] = hi.z, x[3] = hi.w;
+        y[0] = __uint_as_float(lo.x << 16), y[1] = __uint_as_float(lo.x & 0xffff0000u);
+        y[2] = __uint_as_float(lo.y << 16), y[3] = __uint_as_float(lo.y & 0xffff0000u);
     }
     __device__ __forceinline__ void keep(int t, int d, double v) {
         c.hi[t][d] = (float)v;
@@ -675,24 +685,34 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_kernel(const DeltaArgs a) 
             sm.qk[which][t][d] = (t < n && d < D) ? a.qkv[(size_t)(t0 + t) * a.qkv_stride + (size_t)(which * a.G + kvh) * D + d] : __float2bfloat16_rn(0.f);
         }
     }
+    if constexpr (CH) {
+        const bf16* from = a.a + (size_t)t0 * a.a_stride + h * D;
+        if (((D | a.a_stride) & 7) == 0 && (reinterpret_cast<uintptr_t>(a.a) & 15) == 0) {
+            for (int i = tid; i < DC * 8; i += 256) {
+                const int t = i >> 3, d = (i & 7) * 8;
+                const bool ok = t < n && d < D;
+                cp_async16(&sm.a[t][d], from + (ok ? (size_t)t * a.a_stride + d : 0), ok);
+            }
+        } else {
+            for (int i = tid; i < DC * DCD; i += 256) {
+                const int t = i >> 6, d = i & 63;
+                sm.a[t][d] = (t < n && d < D) ? from[(size_t)t * a.a_stride + d] : __float2bfloat16_rn(0.f);
+            }
+        }
+    }
     cp_async_commit();
     // decays and beta
     if (tid < DC) sm.beta[tid] = tid < n ? 1.f / (1.f + expf(-to_float(a.b[(size_t)(t0 + tid) * a.b_stride + h]))) : 0.f;
     const float rate = expf(a.a_log[h]);
     if constexpr (CH) {
         const int d = tid & 63, seg = tid >> 6;              // 16 rows of a channel a thread
-        double acc = 0.0;
-        float x[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const int t = seg * 16 + i;
-            x[i] = (t < n && d < D) ? to_float(a.a[(size_t)(t0 + t) * a.a_stride + h * D + d]) : 0.f;
-        }
         const float bias = d < D ? a.dt_bias[h * D + d] : 0.f;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const int t = seg * 16 + i;
-            if (t < n && d < D) acc += delta_log_decay(rate, x[i] + bias);
+        cp_async_wait<0>();
+        __syncthreads();
+        double acc = 0.0;
+#pragma unroll 2
+        for (int t = seg * 16; t < seg * 16 + 16; ++t) {
+            if (t < n && d < D) acc += delta_log_decay(rate, to_float(sm.a[t][d]) + bias);
             sm.keep(t, d, acc);
         }
         sm.sum[seg][d] = (float)acc;
@@ -747,44 +767,58 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_kernel(const DeltaArgs a) 
 
     // A and P on the tensor cores, 16 rows (I) at a time; a warp takes eight columns of one of the two
     const int mi = lane >> 3, r8 = lane & 7, g = lane >> 2, tq = lane & 3;
+    DeltaChunk* out = a.chunks + (size_t)blockIdx.x * a.H + h;
     for (int I = 0; I < 4; ++I) {
         bool fast = true;
         if constexpr (CH) {
             // the largest decay of these 16 rows says whether e^(-c) inside them can be a factor by itself
             fast = !__syncthreads_or(tid < DCD && !(sm.sum[I][tid & 63] > -DELTA_FAST));
             const int rows = 16 * I + (fast ? 16 : 0);
-            for (int i = tid; i < (rows + 32) * (DCD / 2); i += 256) {
-                const int row = i / (DCD / 2), d = (i % (DCD / 2)) * 2;
-                float2 e, x, hi, lo;
+            // (four channels a thread and turn)
+#pragma unroll 1
+            for (int i = tid; i < (rows + 32) * (DCD / 4); i += 256) {
+                const int row = i / (DCD / 4), d = (i % (DCD / 4)) * 4;
+                float e[4], hi[4], lo[4];
+                bf16* dst;
+                int part = DC * DR_LD, which = 1, t = row;
                 if (row < rows) {                            // right: k_s e^(c at the first of the 16 - c_s)
-                    const int s = row, J = s >> 4;
-                    sm.at_two(s, d, hi, lo);
+                    const int J = row >> 4;
+                    sm.at_four(row, d, hi, lo);
+                    dst = &sm.right[0][row][d];
                     if (J == I) {
-                        e = make_float2(delta_exp2(-hi.x, -lo.x), delta_exp2(-hi.y, -lo.y));
-                    } else {
-                        const float2 a0 = *reinterpret_cast<const float2*>(&sm.sum[J][d]), a1 = *reinterpret_cast<const float2*>(&sm.sum_lo[J][d]);
-                        float2 f = make_float2((a0.x - hi.x) + (a1.x - lo.x), (a0.y - hi.y) + (a1.y - lo.y));
-                        for (int K = J + 1; K < I; ++K) {
-                            const float2 more = *reinterpret_cast<const float2*>(&sm.sum[K][d]);
-                            f.x += more.x;
-                            f.y += more.y;
-                        }
-                        e = make_float2(fast_exp2(f.x), fast_exp2(f.y));
-                    }
-                    x = sm.unit_two(1, s, d);
-                } else {                                     // left: q_t, k_t times e^(c_t - c at the first)
-                    const int which = (row - rows) >> 4, t = 16 * I + ((row - rows) & 15);
-                    sm.at_two(t, d, hi, lo);
-                    e = make_float2(delta_exp2(hi.x, lo.x), delta_exp2(hi.y, lo.y));
-                    x = sm.unit_two(which, t, d);
-                }
-                uint32_t p[3];
-                split3_pair(x.x * e.x, x.y * e.y, p);
 #pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    bf16* dst = row < rows ? &sm.right[k][row][d] : &sm.left[(row - rows) >> 4][k][(row - rows) & 15][d];
-                    *reinterpret_cast<uint32_t*>(dst) = p[k];
+                        for (int j = 0; j < 4; ++j) e[j] = delta_exp2(-hi[j], -lo[j]);
+                    } else {
+                        const float4 a0 = *reinterpret_cast<const float4*>(&sm.sum[J][d]), a1 = *reinterpret_cast<const float4*>(&sm.sum_lo[J][d]);
+                        float f[4] = {(a0.x - hi[0]) + (a1.x - lo[0]), (a0.y - hi[1]) + (a1.y - lo[1]), (a0.z - hi[2]) + (a1.z - lo[2]),
+                                      (a0.w - hi[3]) + (a1.w - lo[3])};
+                        for (int K = J + 1; K < I; ++K) {
+                            const float4 more = *reinterpret_cast<const float4*>(&sm.sum[K][d]);
+                            f[0] += more.x;
+                            f[1] += more.y;
+                            f[2] += more.z;
+                            f[3] += more.w;
+                        }
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) e[j] = fast_exp2(f[j]);
+                    }
+                } else {                                     // left: q_t, k_t times e^(c_t - c at the first)
+                    which = (row - rows) >> 4;
+                    t = 16 * I + ((row - rows) & 15);
+                    sm.at_four(t, d, hi, lo);
+                    dst = &sm.left[which][0][t & 15][d];
+                    part = 16 * DR_LD;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) e[j] = delta_exp2(hi[j], lo[j]);
                 }
+                const uint2 raw = *reinterpret_cast<const uint2*>(&sm.qk[which][t][d]);
+                const float inv = sm.inv[which][t];
+                const float2 x0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x)), x1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+                uint32_t p0[3], p1[3];
+                split3_pair(x0.x * inv * e[0], x0.y * inv * e[1], p0);
+                split3_pair(x1.x * inv * e[2], x1.y * inv * e[3], p1);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) *reinterpret_cast<uint2*>(dst + k * part) = make_uint2(p0[k], p1[k]);
             }
             __syncthreads();
         }
@@ -812,14 +846,21 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_kernel(const DeltaArgs a) 
                              *reinterpret_cast<const uint32_t*>(&sm.qk[1][nt * 8 + g][kt * 16 + 2 * tq + 8]));
                 }
             }
+            float w[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int t = 16 * I + g + 8 * (e >> 1), s = nt * 8 + 2 * tq + (e & 1);
-                if (s > t) continue;                         // (what lies there is no part of the sums)
-                float v = acc[0][e] + (acc[1][e] + acc[2][e]);
-                if constexpr (!CH) v = acc[0][e] * sm.inv[which][t] * sm.inv[1][s] * fast_exp2(delta_minus(sm.at(t, 0), sm.at(s, 0)));
-                if (which == 0) sm.m[s][t] = v;
-                else if (s < t) sm.m[t][s] = sm.beta[t] * v;
+                w[e] = acc[0][e] + (acc[1][e] + acc[2][e]);
+                if constexpr (!CH) w[e] = acc[0][e] * sm.inv[which][t] * sm.inv[1][s] * fast_exp2(delta_minus(sm.at(t, 0), sm.at(s, 0)));
+                if (s > t) w[e] = 0.f;                       // (what lies there is no part of the sums)
+                if (which == 1 && s < t) sm.m[t][s] = sm.beta[t] * w[e];
+            }
+            if (which == 0) {                                // P goes out as it lies: half of a tile of 16 columns
+                uint32_t lo[3], hi[3];
+                split3_pair(w[0], w[1], lo);
+                split3_pair(w[2], w[3], hi);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) reinterpret_cast<uint2*>(&out->p.v[k][I][nt >> 1][lane])[nt & 1] = make_uint2(lo[k], hi[k]);
             }
         }
         if (CH && !fast) {
@@ -849,13 +890,16 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_kernel(const DeltaArgs a) 
             sum16(va, lane);
             sum16(vp, lane);
             if (dq < r) sm.m[t][16 * I + dq] = sm.beta[t] * va[0];
-            if (dq <= r) sm.m[16 * I + dq][t] = vp[0];
+            float part[3];
+            split3(dq <= r ? vp[0] : 0.f, part[0], part[1], part[2]);
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                reinterpret_cast<bf16*>(&out->p.v[k][I][I][(r & 7) * 4 + ((dq & 7) >> 1)])[((r >> 3) + 2 * (dq >> 3)) * 2 + (dq & 1)] = __float2bfloat16_rn(part[k]);
         }
         if (CH) __syncthreads();                             // (the next 16 rows' operands take the place of these)
     }
     __syncthreads();
 
-    DeltaChunk* out = a.chunks + (size_t)blockIdx.x * a.H + h;
     // the rows of v come while the operands are put down
     const bool v_here = V <= DELTA_V_MAX;
     const bf16* v = a.qkv + (size_t)t0 * a.qkv_stride + (size_t)2 * a.G * D + (size_t)h * V;
@@ -873,7 +917,6 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_kernel(const DeltaArgs a) 
         }
     }
     cp_async_commit();
-    auto from_start = [&](int t, int d) { return CH ? sm.before[t >> 4][d] + sm.c.hi[t][d] : sm.c.hi[t][0]; };
     delta_put(&out->q, [&](int t, int d) {
         const float2 x = sm.unit_two(0, t, d);
         if (!CH) {
@@ -883,7 +926,6 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_kernel(const DeltaArgs a) 
         const float2 hi = *reinterpret_cast<const float2*>(&sm.c.hi[t][d]), b = *reinterpret_cast<const float2*>(&sm.before[t >> 4][d]);
         return make_float2(x.x * fast_exp2(b.x + hi.x), x.y * fast_exp2(b.y + hi.y));
     });
-    delta_put(&out->p, [&](int t, int s) { return make_float2(s <= t ? sm.m[s][t] : 0.f, s < t ? sm.m[s + 1][t] : 0.f); });
     delta_put(&out->k, [&](int d, int s) {
         float e[2];
 #pragma unroll
@@ -897,51 +939,93 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_kernel(const DeltaArgs a) 
 
     cp_async_wait<0>();
     __syncthreads();
-    // the triangular system, a right side a thread: the columns of e^(c_t) k_t, then those of v
+    // The triangular system, 16 right sides a warp at a time: the columns of e^(c_t) k_t, then those of v.  A lane has its share of
+    // their rows (columns g, g + 8; rows 2 tq, + 1, + 8, + 9 of every 16).  Rows go in four steps of 16: the 16 among themselves are
+    // substituted in 32-bit, and what they take off the later ones is a product on the tensor cores (columns are its rows, so the
+    // solved 16 are its operand as they lie).  The steps are one loop's turns on purpose: every instruction runs once a turn, so
+    // what the loop costs first is fetching its code (unrolled, 64 rows a thread: 106 KB of code, 28 of a block's 55 us).
     float* u0 = a.u0 + ((size_t)blockIdx.x * a.H + h) * DC * a.VP;
-    const int total = V + DCD;
-    for (int c0 = 0; c0 < total; c0 += 256) {
-        const int d = c0 + tid, col = d - DCD;
-        float u[DC];
-        if (col >= 0) {
-            if (v_here) {
+#pragma unroll 1
+    for (int tile = warp; tile < DCD / 16 + (V + 15) / 16; tile += 8) {
+        const int c0 = tile * 16 - DCD;                      // its first column of v
+        float x[4][2][4] = {};                               // [16 rows from this turn's on][tile of 8 rows][...]
+#pragma unroll 1
+        for (int I = 0; I < 4; ++I) {
 #pragma unroll
-                for (int t = 0; t < DC; ++t) u[t] = col < V ? to_float(sm.v[t * (V + 8) + col]) : 0.f;
+            for (int i = 0; i < 8; ++i) {
+                const int t = 16 * I + (i >> 2) * 8 + 2 * tq + (i & 1), col = c0 + g + 8 * (i >> 1 & 1);
+                float r = 0.f;
+                if (c0 < 0) r = sm.unit(1, t, DCD + col) * fast_exp2(CH ? sm.before[I][DCD + col] + sm.c.hi[t][DCD + col] : sm.c.hi[t][0]);
+                else if (col < V && v_here) r = to_float(sm.v[t * (V + 8) + col]);
+                else if (col < V && t < n) r = to_float(v[(size_t)t * a.qkv_stride + col]);
+                x[0][i >> 2][i & 3] = fmaf(sm.beta[t], r, x[0][i >> 2][i & 3]);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {                    // rows 4 q .. of the 16 leave what they weigh in the later ones
+                float4 m4[2][2];
+#pragma unroll
+                for (int i = q >> 1; i < 2; ++i)
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) m4[i][b] = *reinterpret_cast<const float4*>(&sm.m[16 * I + i * 8 + 2 * tq + b][16 * I + 4 * q]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int s = 4 * q + j, from = (lane & ~3) | ((s & 7) >> 1);
+                    const float u_lo = __shfl_sync(0xffffffffu, x[0][s >> 3][s & 1], from), u_hi = __shfl_sync(0xffffffffu, x[0][s >> 3][2 + (s & 1)], from);
+#pragma unroll
+                    for (int i = q >> 1; i < 2; ++i)
+#pragma unroll
+                        for (int b = 0; b < 2; ++b) {
+                            const float m = j == 0 ? m4[i][b].x : j == 1 ? m4[i][b].y : j == 2 ? m4[i][b].z : m4[i][b].w;
+                            const int behind = s - 8 * i - b;        // row 8 i + 2 tq + b lies behind s: 2 tq > this
+                            if (behind < 0 || (behind < 6 && tq > behind / 2)) {
+                                x[0][i][b] = fmaf(-m, u_lo, x[0][i][b]);
+                                x[0][i][2 + b] = fmaf(-m, u_hi, x[0][i][2 + b]);
+                            }
+                        }
+                }
+            }
+            uint32_t up[4][3];                               // the solved rows in three parts: a product's first operand
+#pragma unroll
+            for (int i = 0; i < 4; ++i) split3_pair(x[0][i >> 1][2 * (i & 1)], x[0][i >> 1][2 * (i & 1) + 1], up[i]);
+            if (c0 < 0) {                                    // W, its rows and columns changed over
+#pragma unroll
+                for (int k = 0; k < 3; ++k)
+                    out->w.v[k][I][tile][lane] = make_uint4(movmatrix_trans(up[0][k]), movmatrix_trans(up[2][k]), movmatrix_trans(up[1][k]), movmatrix_trans(up[3][k]));
             } else {
 #pragma unroll
-                for (int t = 0; t < DC; ++t) u[t] = (t < n && col < V) ? to_float(v[(size_t)t * a.qkv_stride + col]) : 0.f;
-            }
-        } else {
-#pragma unroll
-            for (int t = 0; t < DC; ++t) u[t] = sm.unit(1, t, d) * fast_exp2(from_start(t, d));
-        }
-        __syncthreads();                                     // (W takes the decays' place)
-        if (c0 + warp * 32 >= total) continue;
-#pragma unroll
-        for (int t = 0; t < DC; ++t) {
-            float p0 = sm.beta[t] * u[t], p1 = 0.f, p2 = 0.f, p3 = 0.f;
-#pragma unroll
-            for (int s = 0; s + 4 <= t; s += 4) {
-                const float4 m4 = *reinterpret_cast<const float4*>(&sm.m[t][s]);
-                p0 = fmaf(-m4.x, u[s], p0);
-                p1 = fmaf(-m4.y, u[s + 1], p1);
-                p2 = fmaf(-m4.z, u[s + 2], p2);
-                p3 = fmaf(-m4.w, u[s + 3], p3);
+                for (int i = 0; i < 8; ++i) {
+                    const int t = 16 * I + (i >> 2) * 8 + 2 * tq + (i & 1), col = c0 + g + 8 * (i >> 1 & 1);
+                    if (col < V) u0[(size_t)t * a.VP + col] = x[0][i >> 2][i & 3];
+                }
             }
 #pragma unroll
-            for (int s = t & ~3; s < t; ++s) p1 = fmaf(-sm.m[t][s], u[s], p1);
-            u[t] = (p0 + p1) + (p2 + p3);
-        }
-        if (col < 0) {
+            for (int j = 1; j < 4; ++j) {
+                if (I + j > 3) break;
 #pragma unroll
-            for (int t = 0; t < DC; ++t) sm.w[t][d] = u[t];
-        } else if (col < V) {
+                for (int nt = 0; nt < 2; ++nt) {
+                    uint32_t fb[2][3];
+                    float acc[3][4] = {};
 #pragma unroll
-            for (int t = 0; t < DC; ++t) u0[(size_t)t * a.VP + col] = u[t];
+                    for (int k = 0; k < 2; ++k) {
+                        const float2 m2 = *reinterpret_cast<const float2*>(&sm.m[16 * (I + j) + nt * 8 + g][16 * I + 2 * tq + 8 * k]);
+                        split3_pair(-m2.x, -m2.y, fb[k]);
+                    }
+#pragma unroll
+                    for (int pa = 0; pa < 3; ++pa) {
+                        const uint32_t f[4] = {up[0][pa], up[1][pa], up[2][pa], up[3][pa]};
+#pragma unroll
+                        for (int pb = 0; pa + pb < 3; ++pb) mma_bf16(acc[pa + pb], f, fb[0][pb], fb[1][pb]);
+                    }
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) x[j][nt][e] += acc[0][e] + (acc[1][e] + acc[2][e]);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+#pragma unroll
+                for (int e = 0; e < 8; ++e) x[j][e >> 2][e & 3] = x[j + 1][e >> 2][e & 3];
         }
     }
-    __syncthreads();
-    delta_put(&out->w, [&](int t, int d) { return *reinterpret_cast<const float2*>(&sm.w[t][d]); });
 }
 
 __device__ __forceinline__ void stmatrix_x4_trans(void* p, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {

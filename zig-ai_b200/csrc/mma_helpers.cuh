@@ -42,14 +42,13 @@ __device__ __forceinline__ void split3(float v, float& hi, float& mid, float& lo
     mid = __bfloat162float(__float2bfloat16_rn(r));
     lo = r - mid;
 }
-// two neighbouring values, each split: p[k] holds the k-th parts
+// two neighbouring values, each split: p[k] holds the k-th parts (rounded two at a time: eleven instructions)
 __device__ __forceinline__ void split3_pair(float v0, float v1, uint32_t (&p)[3]) {
-    float a0, a1, a2, b0, b1, b2;
-    split3(v0, a0, a1, a2);
-    split3(v1, b0, b1, b2);
-    p[0] = pack_bf16(a0, b0);
-    p[1] = pack_bf16(a1, b1);
-    p[2] = pack_bf16(a2, b2);
+    p[0] = pack_bf16(v0, v1);
+    v0 -= __uint_as_float(p[0] << 16);
+    v1 -= __uint_as_float(p[0] & 0xffff0000u);
+    p[1] = pack_bf16(v0, v1);
+    p[2] = pack_bf16(v0 - __uint_as_float(p[1] << 16), v1 - __uint_as_float(p[1] & 0xffff0000u));
 }
 
 // 2^x by the special-function unit (2 ulp; x = -inf gives 0, which the masked scores rely on).  The
