@@ -7,32 +7,27 @@
 // run: a block owns 128 query rows of one head; per tile of 64 keys
 //
 //     S = Q K^T      tcgen05.mma, M = 128 (query rows = TMEM lanes), N = 64 keys, K = 64, into TMEM
-//     P = exp2(..)   eight warps, half of a query row's 64 scores per thread, from TMEM with tcgen05.ld; P goes
-//                    back into TMEM (tcgen05.st, two bfloat16 a column) as the next product's A operand
-//     O_t = P V      tcgen05.mma with A in TMEM, N = 64, K = 64 keys, V read straight from its page
-//                    layout [key][64] as an MN-major operand, accumulated into O in TMEM; the threads
-//                    rescale O there only when a row's reference maximum has to move
+//     P = exp2(..)   four warps, a query row a thread, from TMEM with tcgen05.ld; P goes back into TMEM (tcgen05.st, two
+//                    bfloat16 a column) as the next product's A operand
+//     O += P V       tcgen05.mma with A in TMEM, N = 64, K = 64 keys, V read straight from its page
+//                    layout [key][64] as an MN-major operand; the threads rescale O there only when a row's reference moves
 //
-// TMEM holds two score buffers and two P buffers (tile i uses buffer i & 1), so the products run a
-// tile ahead of the softmax: the scores of tile i + 2 are issued when the softmax has read those of
-// tile i, and the softmax of tile i + 1 finds its scores ready when it has written P of tile i.
+// Eight softmax warps take the tiles by turns, four the even ones and four the odd ones, each turn with a score buffer and a
+// P buffer: tile i + 1 is in the softmax of the other turn while tile i's P is multiplied and tile i + 2's scores are made.
+// A product is issued as soon as what it needs is there, in whatever order that comes.
 //
-// After a row's first tile the threads do not look for a tile's maximum first: they compute P against
-// the reference as it is and find the maximum on the way; only if it lies more than 2^8 above the
-// reference in some row of the warp does the reference move and the tile get walked again.  The two warps
-// that share rows exchange their maxima through shared memory once a tile (a barrier of 64 threads), so both
-// decide alike; a warp that has given up a wait still takes part in that barrier.
-//
-// TMEM allows two blocks an SM and a tile is a chain (scores, softmax, P, product), of which the softmax is the
-// longest link: with four warps, a row a thread, 2330 of a tile's 3700 cycles.  With eight (us, 32 heads of 64 over 8): 2048 rows 54 -> 46,
-// behind 6144 positions 258 -> 251, 8192 rows 543 -> 510; 16 heads, 32 rows behind 16 384 positions 76 -> 49.
+// What bounds it: of a turn's 2900 cycles a tile, 1100 are exponentials and packing (512 of them the special-function unit's for
+// one warp), 700 the scores' load and maximum, the rest waits and what goes with them; two blocks an SM (TMEM allows no more)
+// run beside each other.  us, 32 heads of 64 over 8, 2048 rows behind 6144 positions: 271 with half a row a thread and the two
+// halves' maxima exchanged every tile, 243 with a row a thread and products issued by one lane behind `lane == 0`, 212 now.
 //
 // Shaped scores (`ZaiScoreOptions` in common.cuh) are an instantiation of their own: the cap by a tanh without a branch, the bias by distance
 // from shared memory (a head's column of the table; neighbouring rows read neighbouring distances), the sink in the
 // normalisation, kept first positions as tiles of their own ahead of the window's.  What bounds them is the shaping (a tile's
-// 64 x 128 scores cost twice what its exponentials do).  Against the walk by mma.sync they take the place of (us, cap, bias and
-// sink): 16 heads of 64 over 8, 2048 rows 164 -> 119, behind 6144 positions 630 -> 477, 8192 rows 1391 -> 870, 32 rows behind 16 384
-// positions 684 -> 100; 32 heads, 2048 rows 299 -> 134; a window of 1024 with 4 kept positions, 2048 rows 97 -> 58.
+// scores cost four times what its exponentials do); it takes two numbers an instruction (fma.rn.f32x2).  16 heads of 64 over 4,
+// 2048 rows, cap, bias and sink: 103 -> 90 us.  Before that, against the walk by mma.sync (us, cap, bias and sink): 16 heads of 64 over
+// 8, 2048 rows 164 -> 119, behind 6144 positions 630 -> 477, 8192 rows 1391 -> 870, 32 rows behind 16 384 positions 684 -> 100;
+// 32 heads, 2048 rows 299 -> 134; a window of 1024 with 4 kept positions, 2048 rows 97 -> 58.
 // Their error against 64 bits is 0.93 to 1.00 of that walk's (relative 1.71e-3 to 2.10e-3, what bfloat16 P and results make it).
 //
 // Q, K and V reach shared memory by TMA (cp.async.bulk.tensor, no multicast), K and V page by page
@@ -54,7 +49,8 @@
 #define AT_SHAPED_STAGES 4                            // (shaped scores: the bias by distance has the fifth's place, and more)
 #define AT_Q_BYTES (AT_BM * AT_D * 2)                 // 16 KB
 #define AT_KV_BYTES (2 * AT_BN * AT_D * 2)            // keys then values: 16 KB
-#define AT_TMEM_COLS 256                              // two score buffers in columns 0..127, O in 128..191, two P buffers in 192..255
+#define AT_TMEM_COLS 256                              // two score buffers in columns 0..127, O in 128..191, two P buffers in 192..255; shaped
+                                                      // scores: P in the first half of its scores' columns, a second O in 192..255
 #define AT_COL_O (2 * AT_BN)
 #define AT_COL_P (2 * AT_BN + AT_D)
 #define AT_LAG 2                                      // tiles that the cleaning is behind the loads (below the number of stages)
@@ -79,14 +75,53 @@ struct AtArgs {
     ZaiScoreOptions opt;        // (shaped scores)
 };
 
-// tanh without a branch, so that a warp of mixed scores takes one way: the Taylor series up to x^9 below 0.3 (the next term is under
-// 6e-8 of it there), the identity 1 - 2 / (1 + e^2x) beyond (a relative error of 4e-7 at most).
-__device__ __forceinline__ float at_tanh(float x) {
-    const float q = x * x;
-    const float small = fmaf(x * q, fmaf(q, fmaf(q, fmaf(q, 62.f / 2835.f, -17.f / 315.f), 2.f / 15.f), -1.f / 3.f), x);
-    const float large = 1.f - __fdividef(2.f, 1.f + at_exp2(x * 2.8853900817779268f));
-    return fabsf(x) < 0.3f ? small : large;
+// two 32-bit numbers in one instruction
+__device__ __forceinline__ float2 at_fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(reinterpret_cast<unsigned long long&>(d))
+        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)), "l"(reinterpret_cast<unsigned long long&>(c)));
+    return d;
 }
+__device__ __forceinline__ float2 at_mul2(float2 a, float2 b) {
+    float2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<unsigned long long&>(d))
+        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+    return d;
+}
+__device__ __forceinline__ float2 at_add2(float2 a, float2 b) {
+    float2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<unsigned long long&>(d))
+        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+    return d;
+}
+__device__ __forceinline__ uint32_t at_pack(float2 v) {
+    __nv_bfloat162 p = __floats2bfloat162_rn(v.x, v.y);
+    return *reinterpret_cast<uint32_t*>(&p);
+}
+__device__ __forceinline__ float2 at_two(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float at_max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+// tanh of two numbers without a branch, so that a warp of mixed scores takes one way: the Taylor series up to x^9 below 0.3 (the next
+// term is under 6e-8 of it there), the identity 1 - 2 / (1 + e^2x) beyond (a relative error of 4e-7 at most).
+__device__ __forceinline__ float2 at_tanh2(float2 x) {
+    const float2 q = at_mul2(x, x);
+    float2 small = at_fma2(q, at_two(62.f / 2835.f), at_two(-17.f / 315.f));
+    small = at_fma2(q, small, at_two(2.f / 15.f));
+    small = at_fma2(q, small, at_two(-1.f / 3.f));
+    small = at_fma2(at_mul2(x, q), small, x);
+    const float2 z = at_mul2(x, at_two(2.8853900817779268f));
+    const float2 d = at_add2(make_float2(at_exp2(z.x), at_exp2(z.y)), at_two(1.f));
+    const float2 large = at_fma2(make_float2(__fdividef(1.f, d.x), __fdividef(1.f, d.y)), at_two(-2.f), at_two(1.f));
+    return make_float2(fabsf(x.x) < 0.3f ? small.x : large.x, fabsf(x.y) < 0.3f ? small.y : large.y);
+}
+
+// A row's reference on its way from the warp that has tile i to the one with its rows in tile i + 1: a barrier of 64 threads, of which
+// the one side arrives and goes on
+__device__ __forceinline__ void at_pass_on(int qd, int i) { asm volatile("bar.arrive %0, 64;" ::"r"(2 + qd * 2 + (i & 1)) : "memory"); }
+__device__ __forceinline__ void at_pass_wait(int qd, int i) { asm volatile("bar.sync %0, 64;" ::"r"(2 + qd * 2 + (i & 1)) : "memory"); }
 
 // SHARED: several blocks (grid z) share a tile of query rows' keys; SHAPED: the scores pass `opt`
 template <bool SHARED, bool SHAPED>
@@ -104,14 +139,14 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
     uint64_t* kv_empty = bars + 1 + STAGES;                  // [STAGES]
     uint64_t* s_ready = bars + 1 + 2 * STAGES;               // [2] scores of tile i in buffer i & 1
     uint64_t* p_ready = bars + 3 + 2 * STAGES;               // [2] P of tile i in buffer i & 1
-    uint64_t* o_ready = bars + 5 + 2 * STAGES;               // [2] the product of tile i has read P buffer i & 1 and added to O
+    uint64_t* s_empty = bars + 5 + 2 * STAGES;               // [2] the scores of buffer i & 1 have been read
     uint64_t* v_ready = bars + 7 + 2 * STAGES;               // [STAGES] the values of a stage are there and clean
     uint32_t& tmem_base_holder = *reinterpret_cast<uint32_t*>(bars + 7 + 3 * STAGES);
     int* words = reinterpret_cast<int*>(bars + 8 + 3 * STAGES);
     int& failed_flag = words[0];
     int& s_seq = words[1];
     int& s_i0 = words[2];
-    float* exch = reinterpret_cast<float*>(words + 4);          // [2][2][128]: a tile's maxima by half, by turns; then the sums
+    float* exch = reinterpret_cast<float*>(words + 4);          // [2][2][128]: the references by turn (even, odd tiles), then the sums
     AtTileNotes& notes = *reinterpret_cast<AtTileNotes*>(exch + 4 * AT_BM);
     float* bias = reinterpret_cast<float*>(&notes + 1);         // [bias_rows] the head's bias by distance
     volatile int* failed = &failed_flag;
@@ -128,8 +163,8 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
         }
         for (int b = 0; b < 2; ++b) {
             at_mbar_init(&s_ready[b], 1);
-            at_mbar_init(&p_ready[b], 8);                       // one arrival per softmax warp
-            at_mbar_init(&o_ready[b], 1);
+            at_mbar_init(&p_ready[b], 4);                       // one arrival per softmax warp of the tile
+            at_mbar_init(&s_empty[b], 4);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -167,8 +202,9 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
         __syncthreads();
     }
     // the softmax threads' state, kept past the roles for a shared tile's combination
-    float m = -INFINITY, l = 0.f;                               // m: the row's reference, in units of the scores
-    bool have_o = false;                                        // the row's O in TMEM is complete
+    float m = -INFINITY, l = 0.f;                               // m: the row's reference, in the exponent's units
+    bool have_o = false;                                        // the row's O is complete
+    float out[32];                                              // ... a half of it
     int row0 = 0, rows = 0;
     if (s < a.S && !failed_flag) {
         const int hk = h / (a.Hq / a.Hkv);
@@ -211,7 +247,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
                 auto load = [&](int end) {                      // by one lane: the tiles up to `end`
                     for (; issued < end; ++issued) {
                         const int st = issued % STAGES;
-                        if (!at_mbar_wait(&kv_empty[st], ((issued / STAGES) & 1) ^ 1, failed)) break;
+                        if (!at_mbar_wait<AT_NAP_NS>(&kv_empty[st], ((issued / STAGES) & 1) ^ 1, failed)) break;
                         at_mbar_expect_tx(&kv_full[st], AT_KV_BYTES);
                         unsigned char* dst = sKV + (size_t)st * AT_KV_BYTES;
                         for (int p = 0; p < per_tile; ++p) {
@@ -280,199 +316,243 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
                 }
             }
         } else if (warp == 1) {
-            if (lane == 0 && n_tiles > 0) {
-                // ---- products.  Instruction descriptors: D 32-bit, A and B bfloat16, M = 128, N = 64; the
-                // scores have both operands K-major; O_t has A (P) in TMEM and B (the values) MN-major.
+            if (n_tiles > 0 && at_elect()) {
+                // ---- products.  (By the lane that elect.sync picks: the compiler then knows that one lane is left and issues a product in
+                // half the time that it takes behind `lane == 0`, where a tile's eight products and three commits took 2000 cycles,
+                // more than its softmax.)
+                // Instruction descriptors: D 32-bit, A and B bfloat16, M = 128, N = 64; the scores have both operands K-major; O has
+                // A (P) in TMEM and B (the values) MN-major.
                 constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(AT_BN >> 3) << 17) | ((uint32_t)(AT_BM >> 4) << 24);
                 constexpr uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(AT_D >> 3) << 17) |
                                              ((uint32_t)(AT_BM >> 4) << 24);
                 const uint32_t tS = tmem_base, tO = tmem_base + AT_COL_O, tP = tmem_base + AT_COL_P;
                 const uint32_t aQ = at_smem(sQ);
+                int p0, p1, p2;
+                parts(p0, p1, p2, SHAPED && a.window > 0 ? a.opt.keep_first : 0);
                 bool ok = at_mbar_wait(&q_full, 0, failed);
-                auto scores = [&](int i) {                      // S = Q K^T of tile i into score buffer i & 1
-                    const int st = i % STAGES;
-                    if (!at_mbar_wait(&kv_full[st], (i / STAGES) & 1, failed)) return false;
+                // A stage's release is also what says that its product, and all before it, are in O.
+                auto scores = [&](int i) {
+                    const uint32_t aK = at_smem(sKV + (size_t)(i % STAGES) * AT_KV_BYTES);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t aK = at_smem(sKV + (size_t)st * AT_KV_BYTES);
 #pragma unroll
                     for (int k = 0; k < AT_D / 16; ++k)
                         at_umma(tS + (i & 1) * AT_BN, at_desc(aQ + k * 32), at_desc(aK + k * 32), idesc_s, k > 0 ? 1u : 0u);
                     at_commit(&s_ready[i & 1]);
-                    return true;
                 };
-                // the scores run a tile ahead of the softmax: those of tile i + 2 are issued when the softmax
-                // has read those of tile i (same buffer), so tile i + 1's are ready when the softmax of
-                // tile i ends
-                if (ok) ok = scores(0);
-                if (ok && n_tiles > 1) ok = scores(1);
-                auto product = [&](int i, bool wait) {          // O += P V of tile i, and the scores of tile i + 2; `wait`: its values are cleaned
-                    const int st = i % STAGES;
-                    ok = at_mbar_wait(&p_ready[i & 1], (i >> 1) & 1, failed) && (!wait || at_mbar_wait(&v_ready[st], (i / STAGES) & 1, failed));
-                    if (!ok) return;
+                auto product = [&](int i) {
+                    const uint32_t aV = at_smem(sKV + (size_t)(i % STAGES) * AT_KV_BYTES + AT_BN * 128);
+                    const uint32_t d = SHAPED ? tO + (i & 1) * AT_D : tO, p = SHAPED ? tS + (i & 1) * AT_BN : tP + (i & 1) * (AT_BN / 2);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t aV = at_smem(sKV + (size_t)st * AT_KV_BYTES + AT_BN * 128);
 #pragma unroll
                     for (int kk = 0; kk < AT_BN / 16; ++kk)     // 16 keys a step: eight columns of P, two groups of 8 keys of V
-                        at_umma_ts(tO, tP + (i & 1) * (AT_BN / 2) + kk * 8, at_desc(aV + kk * 2048), idesc_o, (i > 0 || kk > 0) ? 1u : 0u);
-                    at_commit(&o_ready[i & 1]);
-                    at_commit(&kv_empty[st]);
-                    if (i + 2 < n_tiles) ok = scores(i + 2);
+                        at_umma_ts(d, p + kk * 8, at_desc(aV + kk * 2048), idesc_o, (i > (SHAPED ? 1 : 0) || kk > 0) ? 1u : 0u);
                 };
-                int p0, p1, p2, i = 0;
-                parts(p0, p1, p2, SHAPED && a.window > 0 ? a.opt.keep_first : 0);
-                for (; i < p2 && ok; ++i) product(i, i >= p1);
-                for (; i < p0 && ok; ++i) product(i, false);
-                for (; i < n_tiles && ok; ++i) product(i, true);
+                auto cleaned = [&](int i) { return i >= p0 || (i >= p1 && i < p2); };
+                if (SHAPED) {
+                    // P lies over its scores, so the scores of tile i + 2 are issued behind the product of tile i (products of one
+                    // thread run in order); the other turn's tile i + 1 is in the softmax meanwhile
+#pragma unroll 1
+                    for (int i = -2; i < n_tiles && ok; ++i) {
+                        if (i >= 0) {
+                            ok = (!cleaned(i) || at_mbar_wait(&v_ready[i % STAGES], (i / STAGES) & 1, failed)) && at_mbar_wait(&p_ready[i & 1], (i >> 1) & 1, failed);
+                            if (ok) product(i);
+                        }
+                        if (ok && i + 2 < n_tiles) {
+                            ok = at_mbar_wait(&kv_full[(i + 2) % STAGES], ((i + 2) / STAGES) & 1, failed);
+                            if (ok) scores(i + 2);
+                        }
+                        if (ok && i >= 0) at_commit(&kv_empty[i % STAGES]);
+                    }
+                } else {
+                    // Scores as soon as their buffer has been read, products as soon as their P is there, whichever comes first (in a
+                    // fixed order each waited for the other turn's warps: a turn took 3000 cycles)
+                    int s_at = 0, p_at = 0;
+                    for (int spin = 0; p_at < n_tiles && ok; ++spin) {
+                        if (s_at < n_tiles && at_mbar_test(&kv_full[s_at % STAGES], (s_at / STAGES) & 1)
+                            && (s_at < 2 || at_mbar_test(&s_empty[s_at & 1], ((s_at - 2) >> 1) & 1))) {
+                            scores(s_at++);
+                            spin = 0;
+                        }
+                        if (at_mbar_test(&p_ready[p_at & 1], (p_at >> 1) & 1)
+                            && (!cleaned(p_at) || at_mbar_test(&v_ready[p_at % STAGES], (p_at / STAGES) & 1))) {
+                            product(p_at);
+                            at_commit(&kv_empty[p_at++ % STAGES]);
+                            spin = 0;
+                        }
+                        if (spin >= AT_SPIN_LIMIT) *failed = 1;
+                        if (spin > 0 && *failed) ok = false;
+                    }
+                }
             }
         } else if (n_tiles > 0) {
-            // ---- softmax: thread = half of a query row (32 of a tile's 64 columns).  O stays in TMEM (the products add to
-            // it); the row's reference maximum is only moved, and O and the sum rescaled, when a tile's maximum exceeds
-            // it by more than 2^8 (P then stays below 256, exact enough in bfloat16 and 32-bit sums; the
-            // result O / l does not depend on the reference).
-            const int qd = warp & 3, half = (warp - 2) >> 2;    // this warp's quarter of the TMEM lanes, its half of the columns
+            // ---- softmax: thread = a query row; four warps have the even tiles, four the odd ones.  O stays in TMEM (the products add
+            // to it); a row's reference is only moved, and O and the sums rescaled, when a tile's maximum exceeds it by more than
+            // 2^8 (P then stays below 256, exact enough in bfloat16 and 32-bit sums; the result O / l does not depend on the
+            // reference).  The reference goes from tile to tile through shared memory, so from one turn's warp to the other's,
+            // early in a tile.  Shaped scores have the running maximum as their reference, which moves in most tiles: there each
+            // turn has a reference, a sum and an O of its own.
+            const int qd = warp & 3, turn = (warp - 2) >> 2;    // this warp's quarter of the TMEM lanes, the tiles it has
             const int row = qd * 32 + lane;
             const bool valid = row < rows;
             const int qpos = ctx + i0 + row;                    // the row's position: keys 0..qpos are visible
             const int klo = zai_first_visible(qpos, a.window);
             const int kept = SHAPED && a.window > 0 ? min(a.opt.keep_first, klo) : 0;
-            const uint32_t tS = tmem_base + ((uint32_t)(qd * 32) << 16) + half * 32, tO = tS + AT_COL_O, tP = tmem_base + ((uint32_t)(qd * 32) << 16) + AT_COL_P + half * 16;
+            const uint32_t lanes = tmem_base + ((uint32_t)(qd * 32) << 16), tS = lanes + turn * AT_BN, tO = lanes + AT_COL_O + (SHAPED ? turn * AT_D : 0),
+                           tP = SHAPED ? tS : lanes + AT_COL_P + turn * (AT_BN / 2);
             const float c = SHAPED ? 1.f : a.scale_log2;        // (shaped scores are made in the exponent's units)
             const float unit = SHAPED && a.opt.softcap > 0.f ? a.opt.scale / a.opt.softcap : 0.f, cap = a.opt.softcap * 1.4426950408889634f;
             bool alive = true;
-            for (int i = 0; i < n_tiles; ++i) {
-                const int key0 = key_of(i) + half * 32;
-                if (alive && !at_mbar_wait_warp(&s_ready[i & 1], (i >> 1) & 1, failed)) alive = false;      // (the warp together)
-                const uint32_t tSi = tS + (i & 1) * AT_BN, tPi = tP + (i & 1) * (AT_BN / 2);
+            for (int i = turn; i < n_tiles; i += 2) {
+                const int key0 = key_of(i);
+                if (alive) alive = at_mbar_wait_warp(&s_ready[turn], (i >> 1) & 1, failed);                   // (the warp together)
+                if (!alive) {                                   // (the other turn's warps still wait for this one's word)
+                    if (SHAPED) break;
+                    if (i > 0) at_pass_wait(qd, i - 1);
+                    if (i + 1 < n_tiles) at_pass_on(qd, i);
+                    continue;
+                }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                // keys of this half that the row sees: [lo, hi), and those below `first`
-                const int lo = valid ? max(klo - key0, 0) : 32, hi = valid ? min(qpos + 1 - key0, 32) : 0;
+                uint32_t x[2][32];
+                at_tmem_ld32_nowait(tS, x[0]);
+                at_tmem_ld32_nowait(tS + 32, x[1]);
+                at_tmem_wait_ld(x[0]);
+                at_tmem_wait_ld(x[1]);
+                if (!SHAPED) {
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    if (lane == 0) at_mbar_arrive(&s_empty[turn]);
+                }
+                if (SHAPED) {
+                    const int far = qpos - key0, last = a.opt.bias_rows - 1;
+                    // a distance below zero is a hidden key's (what it reads lies in this block's shared memory); beyond the
+                    // table its last entry counts.  Most tiles lie on one side of that for the whole warp.
+                    const bool near = __all_sync(0xffffffffu, far <= last);
+                    const float* from = bias + far;
+                    auto shape = [&](auto entry) {
+#pragma unroll
+                        for (int j = 0; j < 64; j += 2) {
+                            float2 v = make_float2(__uint_as_float(x[j >> 5][j & 31]), __uint_as_float(x[j >> 5][(j & 31) + 1]));
+                            const float2 add = make_float2(entry(j), entry(j + 1));
+                            v = a.opt.softcap > 0.f ? at_fma2(at_tanh2(at_mul2(v, at_two(unit))), at_two(cap), add) : at_fma2(v, at_two(a.scale_log2), add);
+                            x[j >> 5][j & 31] = __float_as_uint(v.x);
+                            x[j >> 5][(j & 31) + 1] = __float_as_uint(v.y);
+                        }
+                    };
+                    if (!a.opt.bias) shape([](int) { return 0.f; });
+                    else if (near) shape([&](int j) { return from[-j]; });
+                    else shape([&](int j) { return bias[min(max(far - j, 0), last)]; });
+                }
+                // keys that the row sees: [lo, hi), and those below `first`
+                const int lo = valid ? max(klo - key0, 0) : 64, hi = valid ? min(qpos + 1 - key0, 64) : 0;
                 const int first = valid ? kept - key0 : 0;
-                const bool full = lo <= 0 && hi >= 32;          // the row sees them all: no masking needed
-                // the 32 scores, shaped and with the hidden ones at minus infinity
-                auto load = [&](uint32_t (&x)[32]) {
-                    at_tmem_ld32_nowait(tSi, x);
-                    at_tmem_wait_ld(x);
-                    if (SHAPED) {
+                if (__any_sync(0xffffffffu, lo > 0 || hi < 64)) {                       // (the warp's branch: no tile without it pays for its instructions)
+                    // (a hidden score may be anything, also NaN: it is replaced before the exponential)
+                    const unsigned long long seen = (at_below(hi) & ~at_below(lo)) | (SHAPED ? at_below(first) : 0ull);
+                    const uint32_t some[2] = {(uint32_t)seen, (uint32_t)(seen >> 32)};
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            float v = __uint_as_float(x[j]);
-                            v = a.opt.softcap > 0.f ? cap * at_tanh(v * unit) : v * a.scale_log2;
-                            if (a.opt.bias) v += bias[min(max(qpos - key0 - j, 0), a.opt.bias_rows - 1)];
-                            x[j] = __float_as_uint(v);
-                        }
-                    }
-                    if (!full) {
-                        // (a hidden score may be anything, also NaN: it is replaced before the exponential)
-#pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (!((j >= lo && j < hi) || (SHAPED && j < first))) x[j] = __float_as_uint(-INFINITY);
-                    }
-                };
-                // one walk over them: their maximum (`mx`), and with `emit` the probabilities against `ref` into P and their sum (`lt`)
-                auto walk = [&](const uint32_t (&x)[32], bool emit, float ref, float& mx, float& lt) {
-                    float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}, lt4[4] = {0.f, 0.f, 0.f, 0.f};   // four chains each, not one of 32 links
-                    if (!emit) {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) mx4[j & 3] = fmaxf(mx4[j & 3], __uint_as_float(x[j]));
-                    } else {
-                        uint32_t pk[16];
-#pragma unroll
-                        for (int j = 0; j < 32; j += 2) {
-                            const float s0 = __uint_as_float(x[j]), s1 = __uint_as_float(x[j + 1]);
-                            mx4[(j >> 1) & 3] = fmaxf(mx4[(j >> 1) & 3], fmaxf(s0, s1));
-                            const float p0 = at_exp2(s0 * c - ref), p1 = at_exp2(s1 * c - ref);
-                            lt4[(j >> 1) & 3] += p0 + p1;
-                            __nv_bfloat162 v = __floats2bfloat162_rn(p0, p1);
-                            pk[j >> 1] = *reinterpret_cast<uint32_t*>(&v);
-                        }
-                        // (This P buffer was read by the product of the tile two before.  That product was issued
-                        // before this tile's scores, and the commit behind the scores covers every product issued
-                        // before it: the scores being ready says the buffer is free.)
-                        at_tmem_st16(tPi, pk);                  // 32 keys = 16 columns of P
-                    }
-                    mx = fmaxf(mx, fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])));
-                    lt += (lt4[0] + lt4[1]) + (lt4[2] + lt4[3]);
-                };
-                // With a reference in every row of the warp, the tile is walked once against it; else the
-                // maximum is found first, as a walk of its own.  Shaped scores are dear: they stay in registers, their maximum is
-                // always found first, and the reference is the row's running maximum itself.
-                uint32_t x[32];
-                const bool speculate = !SHAPED && i > 0 && __all_sync(0xffffffffu, m != -INFINITY || !valid);
-                float mx = -INFINITY, lt = 0.f;
-                if (alive) {
-                    load(x);
-                    walk(x, speculate, m == -INFINITY ? 0.f : m * c, mx, lt);
+                    for (int j = 0; j < 64; ++j)
+                        if (!(some[j >> 5] >> (j & 31) & 1)) x[j >> 5][j & 31] = __float_as_uint(-INFINITY);
                 }
-                // the row's maximum over both halves, which the two warps then decide by alike
-                float* turn = exch + (i & 1) * (2 * AT_BM);
-                turn[half * AT_BM + row] = mx;
-                asm volatile("bar.sync %0, 64;" ::"r"(1 + qd) : "memory");
-                mx = fmaxf(mx, turn[(half ^ 1) * AT_BM + row]);
-                if (!alive) continue;                           // (this warp has given up; the other one must not wait for it)
+                float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};            // four chains, not one of 32 links
+#pragma unroll
+                for (int j = 0; j < 64; j += 2)
+                    mx4[(j >> 1) & 3] = at_max3(mx4[(j >> 1) & 3], __uint_as_float(x[j >> 5][j & 31]), __uint_as_float(x[j >> 5][(j & 31) + 1]));
+                const float mx = fmaxf(at_max3(mx4[0], mx4[1], mx4[2]), mx4[3]) * c;
                 // move the reference?  (warp-wide decision: the TMEM accesses below are the whole warp's)
-                float alpha = 1.f;
-                if (m == -INFINITY) {
-                    m = mx;                                     // nothing summed so far (O and l are 0, or this is the first tile)
-                } else if (mx * c > m * c + (SHAPED ? 0.f : 8.f)) {
-                    alpha = at_exp2(m * c - mx * c);
-                    m = mx;
+                float alpha = 1.f, ref = m;
+                if (!SHAPED && i > 0) {
+                    at_pass_wait(qd, i - 1);
+                    ref = exch[((i - 1) & 1) * AT_BM + row];
                 }
-                const bool moved = __any_sync(0xffffffffu, alpha != 1.f);
-                float again = -INFINITY;
-                if (SHAPED) walk(x, true, m == -INFINITY ? 0.f : m * c, again, lt);       // (before the rescaling: x is in registers no longer then)
-                if (i > 0 && moved) {
-                    if (!at_mbar_wait_warp(&o_ready[(i - 1) & 1], ((i - 1) >> 1) & 1, failed)) { alive = false; continue; }   // the product before (and with it all before) has added to O
+                if (ref == -INFINITY) {
+                    ref = mx;                                   // nothing summed so far (O and l are 0, or this is the first tile)
+                } else if (mx > ref + (SHAPED ? 0.f : 8.f)) {
+                    alpha = at_exp2(ref - mx);
+                    ref = mx;
+                }
+                if (!SHAPED && i + 1 < n_tiles) {
+                    exch[(i & 1) * AT_BM + row] = ref;
+                    at_pass_on(qd, i);
+                }
+                if (m != ref && m != -INFINITY) l *= at_exp2(m - ref);
+                m = ref;
+                if (__any_sync(0xffffffffu, alpha != 1.f)) {
+                    // (shaped: this tile's scores came behind the turn's products so far, so those are in O)
+                    if (!SHAPED) alive = at_mbar_wait_warp(&kv_empty[(i - 1) % STAGES], ((i - 1) / STAGES) & 1, failed);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    uint32_t r[32];
-                    at_tmem_ld32(tO, r);
+#pragma unroll 1
+                    for (int d = 0; d < AT_D; d += 16) {
+                        uint32_t r[16];
+                        at_tmem_ld16(tO + d, r);
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * alpha);
-                    at_tmem_st32(tO, r);
-                    l *= alpha;
+                        for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * alpha);
+                        at_tmem_st16(tO + d, r);
+                    }
                 }
-                if (!SHAPED && (!speculate || moved)) {
-                    lt = 0.f;
-                    load(x);
-                    walk(x, true, m == -INFINITY ? 0.f : m * c, again, lt);   // no key seen so far: every p is 0
+                // P, two keys a column; its sum on the way
+                const float2 c2 = at_two(c), minus = at_two(m == -INFINITY ? 0.f : -m);  // (no key seen so far: every p is 0)
+                float2 lt[4] = {};
+                // (plain scores: the product of tile i - 2 reads this P buffer)
+                if (!SHAPED && i > 1 && alive) alive = at_mbar_wait_warp(&kv_empty[(i - 2) % STAGES], ((i - 2) / STAGES) & 1, failed);
+#pragma unroll
+                for (int j0 = 0; j0 < 64; j0 += 16) {           // (16 keys a store: with 64 the registers for them cost moves and spills)
+                    uint32_t pk[8];
+#pragma unroll
+                    for (int j = j0; j < j0 + 16; j += 2) {
+                        const float2 z = at_fma2(make_float2(__uint_as_float(x[j >> 5][j & 31]), __uint_as_float(x[j >> 5][(j & 31) + 1])), c2, minus);
+                        const float2 p = make_float2(at_exp2(z.x), at_exp2(z.y));
+                        lt[(j >> 1) & 3] = at_add2(lt[(j >> 1) & 3], p);
+                        pk[(j - j0) >> 1] = at_pack(p);
+                    }
+                    at_tmem_st8(tP + j0 / 2, pk);
                 }
-                l += lt;
+                const float2 sum = at_add2(at_add2(lt[0], lt[1]), at_add2(lt[2], lt[3]));
+                l += sum.x + sum.y;
                 // P (and a rescaled O) are in TMEM before the product-issuing thread hears of it
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) at_mbar_arrive(&p_ready[i & 1]);
+                if (lane == 0) at_mbar_arrive(&p_ready[turn]);
             }
-            // the row's sum over both halves
-            float* turn = exch + (n_tiles & 1) * (2 * AT_BM);
-            turn[half * AT_BM + row] = l;
-            asm volatile("bar.sync %0, 64;" ::"r"(1 + qd) : "memory");
-            l += turn[(half ^ 1) * AT_BM + row];
-            if (alive && at_mbar_wait_warp(&o_ready[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1, failed)) {
+            // the row's two parts: what weighs them, and the sum over both
+            if (!SHAPED) asm volatile("bar.sync 1, 256;" ::: "memory");     // (the last reference has been read)
+            exch[turn * AT_BM + row] = m;
+            exch[(2 + turn) * AT_BM + row] = l;
+            asm volatile("bar.sync 1, 256;" ::: "memory");      // the eight softmax warps
+            const float m0 = exch[row], m1 = exch[AT_BM + row], l0 = exch[2 * AT_BM + row], l1 = exch[3 * AT_BM + row];
+            m = fmaxf(m0, m1);
+            const float f0 = m0 == -INFINITY ? 0.f : at_exp2(m0 - m), f1 = m1 == -INFINITY ? 0.f : at_exp2(m1 - m);
+            l = l0 * f0 + l1 * f1;
+            if (alive && at_mbar_wait_warp(&kv_empty[(n_tiles - 1) % STAGES], ((n_tiles - 1) / STAGES) & 1, failed)) {      // the last product is in O
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 have_o = at_mbar_wait_warp(&v_ready[(n_tiles - 1) % STAGES], ((n_tiles - 1) / STAGES) & 1, failed);    // (long since; the notes are seen)
                 float inv = l > 0.f ? 1.f / l : 0.f;
                 if (SHAPED && a.opt.sink) {                     // one more term of the denominator
-                    const float M = m * c, sk = a.opt.sink[h] * 1.4426950408889634f, top = fmaxf(M, sk);
-                    const float e = at_exp2(M - top);
+                    const float sk = a.opt.sink[h] * 1.4426950408889634f, top = fmaxf(m, sk);
+                    const float e = at_exp2(m - top);
                     inv = e / (l * e + at_exp2(sk - top));
                 }
-                bf16* dst = a.out + ((size_t)(row0 + i0 + row) * a.Hq + h) * AT_D + half * 32;
-                if (!SHARED) {
-                    uint32_t r[32];
-                    at_tmem_ld32(tO, r);
-                    if (valid) {
+                // this thread's half of the columns of O, the two parts together
+                uint32_t o0[32], o1[32];
+                at_tmem_ld32(lanes + AT_COL_O + turn * 32, o0);
+                if (SHAPED && n_tiles > 1) at_tmem_ld32(lanes + AT_COL_O + AT_D + turn * 32, o1);
 #pragma unroll
-                        for (int d = 0; d < 32; d += 8) {
-                            uint32_t v[4];
+                for (int j = 0; j < 32; ++j) {
+                    out[j] = __uint_as_float(o0[j]) * (SHAPED ? f0 : 1.f);
+                    if (SHAPED && n_tiles > 1) out[j] = fmaf(__uint_as_float(o1[j]), f1, out[j]);
+                }
+                bf16* dst = a.out + ((size_t)(row0 + i0 + row) * a.Hq + h) * AT_D + turn * 32;
+                if (!SHARED && valid) {
 #pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                __nv_bfloat162 p = __floats2bfloat162_rn(__uint_as_float(r[d + 2 * e]) * inv, __uint_as_float(r[d + 2 * e + 1]) * inv);
-                                v[e] = *reinterpret_cast<uint32_t*>(&p);
-                            }
-                            *reinterpret_cast<uint4*>(dst + d) = make_uint4(v[0], v[1], v[2], v[3]);
+                    for (int d = 0; d < 32; d += 8) {
+                        uint32_t v[4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            __nv_bfloat162 p = __floats2bfloat162_rn(out[d + 2 * e] * inv, out[d + 2 * e + 1] * inv);
+                            v[e] = *reinterpret_cast<uint32_t*>(&p);
                         }
-                        if (notes.count) notes.put_nans(dst, 1, half, 1, qpos, klo, kept);
+                        *reinterpret_cast<uint4*>(dst + d) = make_uint4(v[0], v[1], v[2], v[3]);
                     }
+                    if (notes.count) notes.put_nans(dst, 1, turn, 1, qpos, klo, kept);
                 }
             }
         }
@@ -480,21 +560,18 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
     if (SHARED && s < a.S && warp >= 2) {
         // ---- a shared tile of query rows: this block's part into memory, a ticket, and the last one combines
         const int qd = warp & 3, half = (warp - 2) >> 2, row = qd * 32 + lane;
-        const uint32_t tO = tmem_base + ((uint32_t)(qd * 32) << 16) + AT_COL_O + half * 32;
         const int slot = ((int)gridDim.y - 1 - (int)blockIdx.y) * a.Hq + h;
         const size_t mine = (size_t)slot * a.splits + blockIdx.z;
         float* po = a.part_o + mine * (AT_D * AT_BM) + half * 32 * AT_BM;
         float* pml = a.part_ml + mine * (2 * AT_BM);
         const bool ok = have_o && !failed_flag;                 // (a block without key tiles, or one that gave up, has no part)
         if (half == 0) {
-            pml[row] = (ok && m != -INFINITY) ? m * (SHAPED ? 1.f : a.scale_log2) : -INFINITY;
+            pml[row] = ok ? m : -INFINITY;
             pml[AT_BM + row] = ok ? l : 0.f;
         }
         if (ok) {
-            uint32_t r[32];
-            at_tmem_ld32(tO, r);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) po[j * AT_BM + row] = __uint_as_float(r[j]);
+            for (int j = 0; j < 32; ++j) po[j * AT_BM + row] = out[j];
             if (notes.count) {
                 const int qpos = a.ctx_lens[s] + i0 + row, klo = zai_first_visible(qpos, a.window);
                 notes.put_nans(po + row, AT_BM, half, 1, qpos, klo, SHAPED && a.window > 0 ? min(a.opt.keep_first, klo) : 0);

@@ -5,7 +5,14 @@
 #include "common.cuh"
 
 #define AT_SPIN_LIMIT 4000000
+#define AT_NAP_NS 100
 
+// true in one lane of a warp in step
+__device__ __forceinline__ bool at_elect() {
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one != 0;
+}
 __device__ __forceinline__ uint32_t at_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void at_mbar_init(uint64_t* bar, int count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(at_smem(bar)), "r"(count));
@@ -16,23 +23,32 @@ __device__ __forceinline__ void at_mbar_expect_tx(uint64_t* bar, uint32_t bytes)
 __device__ __forceinline__ void at_mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(at_smem(bar)) : "memory");
 }
+// NAP: how long a try that finds the phase open sleeps before the next (a waiting lane without that issues instructions all the time)
+template <int NAP = 0>
 __device__ __forceinline__ bool at_mbar_wait(uint64_t* bar, uint32_t parity, volatile int* failed) {
     const uint32_t a = at_smem(bar);
+#pragma unroll 1
     for (int it = 0; it < AT_SPIN_LIMIT; ++it) {
         uint32_t ok;
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                      : "=r"(ok) : "r"(a), "r"(parity) : "memory");
         if (ok) return true;
         if (*failed) return false;
+        if (NAP > 0) __nanosleep(NAP);
     }
     *failed = 1;
     return false;
 }
-// A warp's wait: lane 0 watches the barrier, the others hear the outcome.
+// Is the phase over?  (Does not wait.)
+__device__ __forceinline__ bool at_mbar_test(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(at_smem(bar)), "r"(parity) : "memory");
+    return ok != 0;
+}
+// A warp's wait, all lanes in step
 __device__ __forceinline__ bool at_mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* failed) {
-    int ok = 1;
-    if ((threadIdx.x & 31) == 0) ok = at_mbar_wait(bar, parity, failed) ? 1 : 0;
-    return __shfl_sync(0xffffffffu, ok, 0) != 0;
+    return __all_sync(0xffffffffu, at_mbar_wait(bar, parity, failed));
 }
 __device__ __forceinline__ void at_tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -88,11 +104,22 @@ __device__ __forceinline__ void at_tmem_st32(uint32_t taddr, const uint32_t (&r)
                  : "memory");
 }
 
+__device__ __forceinline__ void at_tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void at_tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
                  ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
                    "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
                  : "memory");
+}
+__device__ __forceinline__ void at_tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 // A product whose A operand lies in TMEM (row = lane, two bfloat16 of k per 32-bit column)
 __device__ __forceinline__ void at_umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
