@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(LT_THREADS) latent_attention_tc_kernel(const _
                 lt_drain(&q_full, 0);
             }
         } else if (warp == 1) {
-            if (lane == 0) {
+            if (at_elect()) {                                   // (issued behind `lane == 0` a product takes twice as long)
                 // ---- products.  Instruction descriptors: D 32-bit, A and B bfloat16, M = 128, N = 64; the scores have both
                 // operands K-major; O has A (P) in TMEM and B (the cached rows' first R columns) MN-major.
                 constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(LT_BN >> 3) << 17) | ((uint32_t)(LT_BM >> 4) << 24);
@@ -220,13 +220,12 @@ __global__ void __launch_bounds__(LT_THREADS) latent_attention_tc_kernel(const _
                                        (i > 0 || kk > 0) ? 1u : 0u);
                     }
                     at_commit(&o_ready[i & 1]);
-                    at_commit(&kv_empty[st]);
                     if (i + 2 < n_tiles) ok = scores(i + 2);
+                    at_commit(&kv_empty[st]);
                 };
                 const int p0 = first_part();
-                int i = 0;
-                for (; i < p0 && ok; ++i) product(i, false);
-                for (; i < n_tiles && ok; ++i) product(i, true);
+#pragma unroll 1
+                for (int i = 0; i < n_tiles && ok; ++i) product(i, i >= p0);
             }
         } else {
             // ---- softmax: thread = pair.  The pair's reference is its running maximum, so that the largest weight is exactly 1
