@@ -123,6 +123,91 @@ __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1
 
 __device__ __forceinline__ float sg_gelu_tanh(float z) { return 0.5f * z * (1.f + tanhf(0.79788456080286536f * (z + 0.044715f * z * z * z))); }
 
+#define SG_SUM_BYTES 512             // [8 warps][16 rows] of 32-bit sums at most
+
+__device__ __forceinline__ float4 skinny_sum4(float4 v, uint2 d) {
+    const float2 d0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&d.x)), d1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&d.y));
+    return make_float4(v.x + d0.x, v.y + d0.y, v.z + d1.x, v.w + d1.y);
+}
+__device__ __forceinline__ uint2 skinny_round4(float4 v, float4 gm) {
+    __nv_bfloat162 lo = __floats2bfloat162_rn(v.x * gm.x, v.y * gm.y), hi = __floats2bfloat162_rn(v.z * gm.z, v.w * gm.w);
+    return make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+}
+// A warp's columns of up to R rows from m0 on: everything of a chunk of 1024 columns is asked for before the first of it is used
+// (lane m's `source` is the source of row m).  sums [rows]: the rows' sums of squares over these columns.
+template <int R>
+__device__ __forceinline__ void skinny_stage(const SkinnyArgs& a, bf16* xs, int XS, float* sums, int m0, int source, int lane, int warp) {
+    const int K = a.K;
+    size_t src[R];
+    float ss[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        src[r] = (size_t)__shfl_sync(0xffffffffu, source, min(m0 + r, a.M - 1)) * K;
+        ss[r] = 0.f;
+    }
+#pragma unroll 1
+    for (int k = warp * 128 + lane * 4; k < K; k += SG_WARPS * 128) {
+        float4 v[R];
+        uint2 d[R];
+        const float4 gm = *reinterpret_cast<const float4*>(a.gamma + k);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            v[r] = *reinterpret_cast<const float4*>(a.h + src[r] + k);
+            d[r] = a.delta ? *reinterpret_cast<const uint2*>(a.delta + src[r] + k) : make_uint2(0u, 0u);
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if (m0 + r >= a.M) break;
+            const float4 w = a.delta ? skinny_sum4(v[r], d[r]) : v[r];
+            if (a.h_out && blockIdx.x == 0) *reinterpret_cast<float4*>(a.h_out + (size_t)(m0 + r) * K + k) = w;
+            ss[r] += w.x * w.x + w.y * w.y + w.z * w.z + w.w * w.w;
+            *reinterpret_cast<uint2*>(xs + (size_t)(m0 + r) * XS + k) = skinny_round4(w, gm);
+        }
+    }
+    // R sums over the warp at once: after the halving steps lane i has row i % R's
+#pragma unroll
+    for (int o = R / 2; o > 0; o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+            const float send = up ? ss[i] : ss[i + o], keep = up ? ss[i + o] : ss[i];
+            ss[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+#pragma unroll
+    for (int o = R; o < 32; o <<= 1) ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], o);
+    if (lane < R && m0 + lane < a.M) sums[m0 + lane] = ss[0];
+}
+// The same for a layer norm, whose mean is taken off before the squares: a warp a row, and a first walk over it for the mean (the second
+// one hits the cache).  sums [warps][stride]
+__device__ __forceinline__ void skinny_stage_centered(const SkinnyArgs& a, bf16* xs, int XS, float* sums, int stride, int source, int lane, int warp) {
+    const int K = a.K;
+    for (int m = warp; m < a.M; m += SG_WARPS) {
+        const size_t src = (size_t)__shfl_sync(0xffffffffu, source, m) * K;
+        auto at = [&](int k) {
+            const float4 v = *reinterpret_cast<const float4*>(a.h + src + k);
+            return a.delta ? skinny_sum4(v, *reinterpret_cast<const uint2*>(a.delta + src + k)) : v;
+        };
+        float mean = 0.f, ss = 0.f;
+#pragma unroll 2
+        for (int k = lane * 4; k < K; k += 128) {
+            const float4 w = at(k);
+            mean += (w.x + w.y) + (w.z + w.w);
+        }
+        mean = warp_sum(mean) / (float)K;
+#pragma unroll 2
+        for (int k = lane * 4; k < K; k += 128) {
+            float4 w = at(k);
+            if (a.h_out && blockIdx.x == 0) *reinterpret_cast<float4*>(a.h_out + (size_t)m * K + k) = w;
+            w.x -= mean; w.y -= mean; w.z -= mean; w.w -= mean;
+            ss += w.x * w.x + w.y * w.y + w.z * w.z + w.w * w.w;
+            *reinterpret_cast<uint2*>(xs + (size_t)m * XS + k) = skinny_round4(w, *reinterpret_cast<const float4*>(a.gamma + k));
+        }
+        ss = warp_sum(ss);
+        if (lane < SG_WARPS) sums[lane * stride + m] = lane == 0 ? ss : 0.f;
+    }
+}
+
 // Blocks are persistent: block b takes the work units b, b + gridDim.x, ...; a unit is `tpc` tiles of
 // 16 weight rows, each tile's K cut into `sk` slices, one slice per warp (8 warps).  A block uses
 // at most half of an SM's shared memory and registers, so the blocks of the next kernel on the stream
@@ -131,9 +216,8 @@ template <int MT, int EPI, bool NORM>
 __global__ void __launch_bounds__(SG_WARPS * 32, 2) skinny_gemm_kernel(const SkinnyArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int K = a.K, XS = K + 8;
-    float* inv_s = reinterpret_cast<float*>(smem_raw);        // [8*MT] 1/rms of each row (64 floats reserved)
-    bf16* xs = reinterpret_cast<bf16*>(smem_raw + 256);      // [8*MT][K + 8]
-    float* gs = reinterpret_cast<float*>(smem_raw + 256 + (size_t)8 * MT * XS * sizeof(bf16));   // [K] the norm's weight
+    float* sums = reinterpret_cast<float*>(smem_raw);         // [warps][8*MT] each row's sum of squares over the columns that a warp staged
+    bf16* xs = reinterpret_cast<bf16*>(smem_raw + SG_SUM_BYTES);   // [M][K + 8]
     float* red = reinterpret_cast<float*>(smem_raw + a.red_offset);   // [warps][MT*4][32]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
@@ -180,7 +264,8 @@ __global__ void __launch_bounds__(SG_WARPS * 32, 2) skinny_gemm_kernel(const Ski
     // the same ring, right behind the weights of their block (they depend on the kernel before this
     // one, so they are issued after the wait; every warp loads only its own K slice of x).
     constexpr int NT = EPI == EPI_CONV ? 2 : 1;             // 16-row operands per tile
-    constexpr int SLOT = (2 * NT + (NORM ? 0 : MT)) * 512;  // bytes of one 32-k block in a warp's ring
+    constexpr int WB = EPI == EPI_CONV ? 1536 : 1024;       // bytes of one 32-k block's weights (of the convolution's second operand one half)
+    constexpr int SLOT = WB + (NORM ? 0 : MT) * 512;        // ... with the token rows: a block in a warp's ring
     const int ring_rounds = a.ring_rounds;
     unsigned char* ring = smem_raw + a.ring_offset + (size_t)warp * ring_rounds * 4 * SLOT;
     auto issue_w = [&](int r) {
@@ -198,7 +283,7 @@ __global__ void __launch_bounds__(SG_WARPS * 32, 2) skinny_gemm_kernel(const Ski
                     const bool ok = (kb + u) < kb1 && k0 + 8 * t < K;   // past the slice or past K: zeros
                     unsigned char* slot = ring + (size_t)((r % ring_rounds) * 4 + u) * SLOT + j * 1024 + lane * 16;
                     cp_async16_zfill(slot, w_lo + k0, ok && row_lo >= 0);
-                    cp_async16_zfill(slot + 512, w_hi + k0, ok && row_hi >= 0);
+                    if (j == 0) cp_async16_zfill(slot + 512, w_hi + k0, ok && row_hi >= 0);
                 }
             }
         }
@@ -210,7 +295,7 @@ __global__ void __launch_bounds__(SG_WARPS * 32, 2) skinny_gemm_kernel(const Ski
             for (int u = 0; u < 4; ++u) {
                 const int k0 = (kb + u) << 5;
                 const bool ok = (kb + u) < kb1 && k0 + 8 * t < K;
-                unsigned char* slot = ring + (size_t)((r % ring_rounds) * 4 + u) * SLOT + NT * 1024 + lane * 16;
+                unsigned char* slot = ring + (size_t)((r % ring_rounds) * 4 + u) * SLOT + WB + lane * 16;
 #pragma unroll
                 for (int nt = 0; nt < MT; ++nt) {
                     const int m = nt * 8 + g;
@@ -247,20 +332,25 @@ __global__ void __launch_bounds__(SG_WARPS * 32, 2) skinny_gemm_kernel(const Ski
             }
         }
     }
-    // ---- the convolution's inputs of a unit (state, taps, bias of the lane's channel and tokens) are
-    // asked for at the start of the unit and used in its epilogue, so their way from memory is hidden
-    // behind the product (after the wait: the kernel before this one may have written the state)
+    // ---- the convolution's inputs of a unit.  Taps, bias and slots are no kernel's output: the first unit's are asked for before the
+    // wait.  The state is asked for at the start of the unit (the kernel before this one may have written it) and used in its
+    // epilogue, so its way from memory is hidden behind the product.
     float cv_prev[EPI == EPI_CONV ? MT : 1][2][SG_CONV_TAPS - 1], cv_w[SG_CONV_TAPS], cv_b = 0.f;
     int cv_slot[EPI == EPI_CONV ? MT : 1][2];
-    auto conv_inputs = [&](int unit) {
-        if (EPI != EPI_CONV || kslice != 0) return;
+    bool bad_slot = false;                                    // (raised once, at the end: no atomic in the unrolled loops)
+    auto conv_channel = [&](int unit, int& ch) {
         const int tile = (blockIdx.x + unit * gridDim.x) * a.tpc + tile_in_unit;
-        const int ch = tile * 8 + g;
-        const bool vc = tile < a.n_tiles && ch < a.F;
+        ch = tile * 8 + g;
+        return tile < a.n_tiles && ch < a.F;
+    };
+    auto conv_fixed = [&](int unit) {
+        if (EPI != EPI_CONV || kslice != 0) return;
+        int ch;
+        const bool vc = conv_channel(unit, ch);
         cv_b = (vc && a.conv_b) ? a.conv_b[ch] : 0.f;
 #pragma unroll
         for (int j = 0; j < SG_CONV_TAPS; ++j) cv_w[j] = (vc && j < a.taps) ? a.conv_w[(size_t)ch * a.taps + j] : 0.f;
-        bool bad_slot = false;                                // (raised once, below: no atomic in the unrolled loops)
+        if (unit > 0) return;                                 // (the slots are the same for every unit)
 #pragma unroll
         for (int nt = 0; nt < (EPI == EPI_CONV ? MT : 1); ++nt)
 #pragma unroll
@@ -270,112 +360,72 @@ __global__ void __launch_bounds__(SG_WARPS * 32, 2) skinny_gemm_kernel(const Ski
                 const bool bad = (unsigned)slot >= (unsigned)a.num_slots;     // outside the slots: slot 0, and the step is void
                 bad_slot |= bad;
                 cv_slot[nt][e] = bad ? 0 : slot;
+            }
+    };
+    auto conv_states = [&](int unit) {
+        if (EPI != EPI_CONV || kslice != 0) return;
+        int ch;
+        const bool vc = conv_channel(unit, ch);
+#pragma unroll
+        for (int nt = 0; nt < (EPI == EPI_CONV ? MT : 1); ++nt)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
 #pragma unroll
                 for (int j = 0; j < SG_CONV_TAPS - 1; ++j)
-                    cv_prev[nt][e][j] = (vc && tok < a.M && j < a.taps - 1)
+                    cv_prev[nt][e][j] = (vc && nt * 8 + 2 * t + e < a.M && j < a.taps - 1)
                         ? a.conv_state[((size_t)cv_slot[nt][e] * a.state_rows + j) * a.F + ch] : 0.f;
-            }
-        if (bad_slot) zai_raise(a.status, ZAI_ST_SLOT);
     };
-    // the norm's weight and the rows' source indices are written by no kernel of the step: they are
-    // fetched before the wait, the weight into shared memory
-    int src_row0 = warp, src_row1 = warp + SG_WARPS;
-    if (NORM) {
-        for (int k = tid * 4; k < K; k += SG_WARPS * 32 * 4) *reinterpret_cast<float4*>(gs + k) = *reinterpret_cast<const float4*>(a.gamma + k);
-        if (a.row_idx) {
-            if (src_row0 < a.M) src_row0 = a.row_idx[src_row0];
-            if (src_row1 < a.M) src_row1 = a.row_idx[src_row1];
-        }
-    }
+    if (n_units > 0) conv_fixed(0);
+    int source = lane;                                       // lane m: the source of row m (no kernel's output either)
+    if (NORM && a.row_idx && lane < a.M) source = a.row_idx[lane];
     if (a.next.when == 1 && warp == SG_WARPS - 1) ask_next_weights(a.next, lane);
-    pdl_trigger();
     pdl_wait_at(__LINE__, 1 + EPI * 2 + (NORM ? 1 : 0));
+    pdl_trigger();                                           // (before the wait the next kernel's loads run beside this one's: 323 us instead of 318)
     if (a.next.when == 2 && warp == SG_WARPS - 1) ask_next_weights(a.next, lane);
-    if (n_units > 0) conv_inputs(0);                         // asked for now, used in the epilogue
-    if (NORM) __syncthreads();                               // gs is complete
+    if (n_units > 0) conv_states(0);                         // asked for now, used in the epilogue
     if (!NORM) {
         for (int r = 0; r < ring_rounds; ++r) issue_x(r);
         cp_async_commit_group();
     }
 
-    // ---- x into shared memory, once per block.  With the norm, x = (h + delta) * gamma rounded to
-    // bfloat16; the row's factor rsqrt(mean((h + delta)^2) + eps) is applied to the sums afterwards.
-    // A warp takes a row; a lane asks for up to eight 16-byte pieces of h and of delta before it uses
-    // the first, so a row of up to 1024 values costs one trip to memory.
+    // ---- x into shared memory, once per block.  With the norm, x = (h + delta) * gamma rounded to bfloat16; the row's factor
+    // rsqrt(mean((h + delta)^2) + eps) is applied to the sums afterwards.  A warp takes 128 of every 1024 columns of all rows, four a
+    // lane, so rows of up to 1024 values are one trip to memory and eight warps share the work of even a single row.  (A warp a row:
+    // 1.7 us from the wait to the products for one row, 2.2 for eight; so 1.4 and 1.9.  A decode step of the 350M shape, with the
+    // convolution's slots and taps asked for before the wait: one request 350 -> 318 us, eight 377 -> 365.)
     if (NORM) {
-        for (int m = warp; m < 8 * MT; m += SG_WARPS) {
-            bf16* dst = xs + (size_t)m * XS;
-            if (m >= a.M) {
-                for (int k = lane * 8; k < K; k += 256) *reinterpret_cast<uint4*>(dst + k) = zero4;
-                if (lane == 0) inv_s[m] = 0.f;
-                continue;
+        if (a.center) skinny_stage_centered(a, xs, XS, sums, 8 * MT, source, lane, warp);
+        else {
+#pragma unroll 1
+            for (int m0 = 0; m0 < a.M; m0 += 8) {
+                const int rows = a.M - m0;
+                if (rows == 1) skinny_stage<1>(a, xs, XS, sums + warp * 8 * MT, m0, source, lane, warp);
+                else if (rows <= 4) skinny_stage<4>(a, xs, XS, sums + warp * 8 * MT, m0, source, lane, warp);
+                else skinny_stage<8>(a, xs, XS, sums + warp * 8 * MT, m0, source, lane, warp);
             }
-            const size_t src = (size_t)(m < SG_WARPS ? src_row0 : src_row1) * K;
-            float mean = 0.f;
-            if (a.center) {                                  // a first walk over the row for its mean (the second one hits the cache)
-                float s4 = 0.f;
-                for (int k = lane * 4; k < K; k += 128) {
-                    const float4 v = *reinterpret_cast<const float4*>(a.h + src + k);
-                    s4 += (v.x + v.y) + (v.z + v.w);
-                    if (a.delta) {
-                        const uint2 d = *reinterpret_cast<const uint2*>(a.delta + src + k);
-                        const __nv_bfloat162 d0 = *reinterpret_cast<const __nv_bfloat162*>(&d.x);
-                        const __nv_bfloat162 d1 = *reinterpret_cast<const __nv_bfloat162*>(&d.y);
-                        s4 += (__low2float(d0) + __high2float(d0)) + (__low2float(d1) + __high2float(d1));
-                    }
-                }
-                mean = warp_sum(s4) / (float)K;
-            }
-            float ss = 0.f;
-            for (int kq = lane * 4; kq < K; kq += 1024) {
-                float4 v[8];
-                uint2 d[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const int k = kq + u * 128;
-                    if (k < K) {
-                        v[u] = *reinterpret_cast<const float4*>(a.h + src + k);
-                        if (a.delta) d[u] = *reinterpret_cast<const uint2*>(a.delta + src + k);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const int k = kq + u * 128;
-                    if (k < K) {
-                        float4 w = v[u];
-                        const float4 gm = *reinterpret_cast<const float4*>(gs + k);
-                        if (a.delta) {
-                            const __nv_bfloat162 d0 = *reinterpret_cast<const __nv_bfloat162*>(&d[u].x);
-                            const __nv_bfloat162 d1 = *reinterpret_cast<const __nv_bfloat162*>(&d[u].y);
-                            w.x += __low2float(d0); w.y += __high2float(d0); w.z += __low2float(d1); w.w += __high2float(d1);
-                        }
-                        if (a.h_out && blockIdx.x == 0) *reinterpret_cast<float4*>(a.h_out + (size_t)m * K + k) = w;
-                        w.x -= mean; w.y -= mean; w.z -= mean; w.w -= mean;
-                        ss += w.x * w.x + w.y * w.y + w.z * w.z + w.w * w.w;
-                        __nv_bfloat162 o0 = __floats2bfloat162_rn(w.x * gm.x, w.y * gm.y);
-                        __nv_bfloat162 o1 = __floats2bfloat162_rn(w.z * gm.z, w.w * gm.w);
-                        uint2 o;
-                        o.x = *reinterpret_cast<uint32_t*>(&o0);
-                        o.y = *reinterpret_cast<uint32_t*>(&o1);
-                        *reinterpret_cast<uint2*>(dst + k) = o;
-                    }
-                }
-            }
-            ss = warp_sum(ss);
-            if (lane == 0) inv_s[m] = rsqrtf(ss / (float)K + a.eps);
         }
+        __syncthreads();
     }
-    if (NORM) __syncthreads();
     float inv_tok[MT][2];
 #pragma unroll
-    for (int nt = 0; nt < MT; ++nt) {
-        inv_tok[nt][0] = NORM ? inv_s[nt * 8 + 2 * t] : 1.f;
-        inv_tok[nt][1] = NORM ? inv_s[nt * 8 + 2 * t + 1] : 1.f;
-    }
+    for (int nt = 0; nt < MT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            inv_tok[nt][e] = 1.f;
+            if (NORM && kslice == 0 && nt * 8 + 2 * t + e < a.M) {
+                float ss = 0.f;
+#pragma unroll
+                for (int w2 = 0; w2 < SG_WARPS; ++w2) ss += sums[w2 * 8 * MT + nt * 8 + 2 * t + e];
+                inv_tok[nt][e] = rsqrtf(ss / (float)K + a.eps);
+            }
+        }
 
     const bf16* xrow = xs + (size_t)g * XS + 8 * t;
     for (int unit = 0; unit < n_units; ++unit) {
-        if (unit > 0) conv_inputs(unit);
+        if (unit > 0) {
+            conv_fixed(unit);
+            conv_states(unit);
+        }
         // ---- the products of this unit's slice: a round's slots are refilled as soon as it is read
         float c[NT][MT][4];
 #pragma unroll
@@ -410,7 +460,7 @@ __global__ void __launch_bounds__(SG_WARPS * 32, 2) skinny_gemm_kernel(const Ski
 #pragma unroll
                     for (int nt = 0; nt < MT; ++nt) {
                         uint4 b4;
-                        if (NORM) b4 = kin ? *reinterpret_cast<const uint4*>(xrow + (size_t)nt * 8 * XS + k0) : zero4;
+                        if (NORM) b4 = kin && nt * 8 + g < a.M ? *reinterpret_cast<const uint4*>(xrow + (size_t)nt * 8 * XS + k0) : zero4;
                         else b4 = bx[u][nt];
                         mma16816(c[0][nt], wl[u].x, wh[u].x, wl[u].y, wh[u].y, b4.x, b4.y);
                         mma16816(c[0][nt], wl[u].z, wh[u].z, wl[u].w, wh[u].w, b4.z, b4.w);
@@ -426,13 +476,13 @@ __global__ void __launch_bounds__(SG_WARPS * 32, 2) skinny_gemm_kernel(const Ski
                     uint4 b4[MT];
 #pragma unroll
                     for (int nt = 0; nt < MT; ++nt) {
-                        if (NORM) b4[nt] = kin ? *reinterpret_cast<const uint4*>(xrow + (size_t)nt * 8 * XS + k0) : zero4;
-                        else b4[nt] = *reinterpret_cast<const uint4*>(slot + NT * 1024 + nt * 512);
+                        if (NORM) b4[nt] = kin && nt * 8 + g < a.M ? *reinterpret_cast<const uint4*>(xrow + (size_t)nt * 8 * XS + k0) : zero4;
+                        else b4[nt] = *reinterpret_cast<const uint4*>(slot + WB + nt * 512);
                     }
 #pragma unroll
                     for (int j = 0; j < NT; ++j) {
                         const uint4 wl = *reinterpret_cast<const uint4*>(slot + j * 1024);
-                        const uint4 wh = *reinterpret_cast<const uint4*>(slot + j * 1024 + 512);
+                        const uint4 wh = j == 0 ? *reinterpret_cast<const uint4*>(slot + 512) : zero4;
 #pragma unroll
                         for (int nt = 0; nt < MT; ++nt) {
                             mma16816(c[j][nt], wl.x, wh.x, wl.y, wh.y, b4[nt].x, b4[nt].y);
@@ -560,6 +610,7 @@ __global__ void __launch_bounds__(SG_WARPS * 32, 2) skinny_gemm_kernel(const Ski
             }
         }
     }
+    if (EPI == EPI_CONV && bad_slot) zai_raise(a.status, ZAI_ST_SLOT);
     cp_async_wait_rounds(0);
 }
 
@@ -820,6 +871,12 @@ static int sg_slots() {
     }
     return v;
 }
+// What a block takes: x (with the norm the rows that there are, and their sums), the sums of the K slices, the rings
+static size_t skinny_block_x_bytes(int M, int K, bool norm) {
+    return norm ? (SG_SUM_BYTES + (size_t)M * (K + 8) * sizeof(bf16) + 1023) / 1024 * 1024 : 0;
+}
+static size_t skinny_block_round_bytes(int mt, bool norm, int nt) { return (size_t)SG_WARPS * 4 * ((nt == 2 ? 3 : 2) + (norm ? 0 : mt)) * 512; }
+// (the bounds on the sizes that the kernel takes, and the depth of its rings, are counted for the largest block of its variant)
 static size_t skinny_x_bytes(int mt, int K, bool norm) {
     if (!norm) return 1024;                                 // x travels through the rings
     return (256 + (size_t)8 * mt * (K + 8) * sizeof(bf16) + (size_t)K * sizeof(float) + 1023) / 1024 * 1024;
@@ -867,7 +924,7 @@ static void skinny_plan(int rows, bool may_halve, int K, int* n_tiles, int* half
 
 template <int MT, int EPI, bool NORM>
 static int skinny_launch(const SkinnyArgs& a, cudaStream_t stream) {
-    const size_t smem = (size_t)a.ring_offset + skinny_round_bytes(MT, NORM, EPI == EPI_CONV ? 2 : 1) * a.ring_rounds;
+    const size_t smem = (size_t)a.ring_offset + skinny_block_round_bytes(MT, NORM, EPI == EPI_CONV ? 2 : 1) * a.ring_rounds;
     static size_t configured = 0;
     if (smem > configured) {
         cudaError_t e = cudaFuncSetAttribute(skinny_gemm_kernel<MT, EPI, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -910,7 +967,7 @@ static int skinny_run(SkinnyArgs& a, int epilogue, cudaStream_t stream) {
         const int rounds = rpu * ((a.units + grid - 1) / grid);
         if (a.ring_rounds > rounds) a.ring_rounds = rounds;
     }
-    a.red_offset = (int)skinny_x_bytes(mt, a.K, norm);
+    a.red_offset = (int)skinny_block_x_bytes(a.M, a.K, norm);
     a.ring_offset = a.red_offset + (int)skinny_red_bytes(mt, nt);
     a.l2_prefetch_bytes = skinny_l2_prefetch_bytes();
     if (epilogue == EPI_BF16) return norm ? skinny_dispatch_mt<EPI_BF16, true>(a, stream) : skinny_dispatch_mt<EPI_BF16, false>(a, stream);
