@@ -163,10 +163,7 @@ class CacheManager:
     def _fits_already(self, rc: RequestCache, total_tokens: int) -> bool:
         """True if the pages the request holds already cover `total_tokens` positions and no window
         has anything to give back (the common case of a decoded token inside its last page)."""
-        if self._has_window:
-            return False
-        n_logical = -(-total_tokens // self.page_size)
-        return all(len(t) >= n_logical for t in rc.tables.values())
+        return not self._has_window and total_tokens <= rc.capacity
 
     def _set_row(self, gi: int, slot: int, j: int, page: int) -> None:
         rows = self._rows[gi]

@@ -75,6 +75,7 @@ class ModelRunner:
         `trusted`: the caller (the scheduler) has checked the tokens and reserved the pages."""
         if not entries:
             raise StepError("a step needs at least one entry")
+        arrays = {}                                       # longer spans' tokens, made into arrays once
         if not trusted:
             seen = set()
             V, max_pos = self.model.vocab_size, self.model.spec.max_positions
@@ -84,14 +85,19 @@ class ModelRunner:
                 seen.add(rid)
                 if rid not in self.processed:
                     raise StepError(f"request {rid!r} was not added")
-                if len(tokens) < 1:
+                n = len(tokens)
+                if n < 1:
                     raise StepError(f"request {rid!r} brings no tokens")
-                arr = np.asarray(tokens)
-                if arr.dtype.kind not in "iu" or arr.min() < 0 or arr.max() >= V:
-                    bad = [int(t) for t in tokens if not 0 <= int(t) < V]
-                    raise StepError(f"request {rid!r}: token ids {bad[:8]} are outside the vocabulary of {V}")
-                if self.processed[rid] + len(tokens) > max_pos:
-                    raise StepError(f"request {rid!r} would reach {self.processed[rid] + len(tokens)} positions; "
+                # (one token, the case of every decoded request, without an array: 4 us a request)
+                if n > 1 or type(tokens[0]) is not int or not 0 <= tokens[0] < V:
+                    arr = np.asarray(tokens)
+                    if arr.dtype.kind not in "iu" or arr.min() < 0 or arr.max() >= V:
+                        bad = [int(t) for t in tokens if not 0 <= int(t) < V]
+                        raise StepError(f"request {rid!r}: token ids {bad[:8]} are outside the vocabulary of {V}")
+                    if arr.ndim == 1:
+                        arrays[rid] = arr
+                if self.processed[rid] + n > max_pos:
+                    raise StepError(f"request {rid!r} would reach {self.processed[rid] + n} positions; "
                                     f"the model allows {max_pos}")
             # all-or-nothing reservation over the whole step
             demand: Dict[int, int] = {}
@@ -107,7 +113,7 @@ class ModelRunner:
             for rid, tokens, _want in entries:
                 self.cache.reserve(rid, self.processed[rid] + len(tokens))
         requests = self.cache.requests
-        spans = [(rid, self.processed[rid], tokens, want, requests[rid].slot) for rid, tokens, want in entries]
+        spans = [(rid, self.processed[rid], arrays.get(rid, tokens), want, requests[rid].slot) for rid, tokens, want in entries]
         rids = [e[0] for e in entries]
         ps = self.cache.page_size
         longest = max(self.processed[rid] + len(tokens) for rid, tokens, _ in entries)
