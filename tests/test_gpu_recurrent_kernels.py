@@ -141,6 +141,29 @@ def test_gated_delta(dtype, H, G, D, V):
     assert torch.equal(state_a[0], state_b[0])
 
 
+@pytest.mark.parametrize("channel", [False, True])
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("singles,spans", [(8, [2]), (9, [70, 5]), (17, [64, 0, 63]), (32, [66]), (7, [130])])
+def test_gated_delta_of_decoded_tokens_ahead_of_spans(singles, spans, dtype, channel):
+    """Leading spans of one token take the one kernel, eight or sixteen of them, the others of the step what their length says."""
+    o = ops()
+    g = torch.Generator().manual_seed(27)
+    H, G, D, V = 4, 2, 64, 128
+    q_lens = [1] * singles + spans
+    N = sum(q_lens)
+    step = make_step(o, dtype, [3] * len(q_lens), q_lens, 8, 256, 5)
+    assert step.single_first == (singles if singles == 8 else 0 if singles < 8 else 1 << (singles.bit_length() - 1))
+    qkv, b, a, gate, a_log, dt_bias, norm_w = (t.to(dtype) if t.dtype == torch.bfloat16 else t for t in delta_inputs(H, G, D, V, N, channel, g))
+    state_a = (torch.randn(len(q_lens) + 3, H, D, V, generator=g) * 0.3).cuda()
+    state_b = state_a.clone()
+    ya = o.gated_delta(qkv, b, a, gate, a_log, dt_bias, norm_w, 1e-5, state_a, step, H, G, D, V, True, channel_decay=channel)
+    yb = ref_ops.gated_delta(qkv, b, a, gate, a_log, dt_bias, norm_w, 1e-5, state_b, step, H, G, D, V, True, channel_decay=channel)
+    # the limits of test_gated_delta
+    assert torch.allclose(ya.float(), yb.float(), **tol(dtype))
+    assert torch.allclose(state_a, state_b, atol=1e-4, rtol=1e-4)
+    assert o.read_status() == 0
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_empty_spans_change_nothing(dtype):
     """A step may hold spans without tokens (a captured step shape is filled up with them)."""

@@ -1327,12 +1327,12 @@ def _scan_chunks(step, n_rows, channel_blocks=16):
     return chunk, n_rows // chunk + step.n_seqs
 
 
-def _span_kinds(step, cut):
-    """Whether a step has spans of `cut` rows or more, and whether it has shorter ones.  A captured step shape is replayed with
+def _span_kinds(step, cut, skip=0):
+    """Whether a step has spans of `cut` rows or more, and whether it has shorter ones behind the first `skip`.  A captured step shape is replayed with
     other spans than it was captured with (it launches a bound of its attention tiles, `attn_tiles`): it may have both."""
     if getattr(step, "attn_tiles", None) or not step.q_lens:
         return step.n_tokens >= cut, True
-    return max(step.q_lens) >= cut, any(0 < n < cut for n in step.q_lens)
+    return max(step.q_lens) >= cut, any(0 < n < cut for n in step.q_lens[skip:])
 
 
 def _chunked_spans(step, cut):
@@ -1483,16 +1483,31 @@ def gated_delta(qkv, b, a, gate, a_log, dt_bias, norm_w, eps, state, step, heads
         return out
     o = torch.empty((N, H * V), dtype=torch.float32, device=dev)
     out = torch.empty((N, H * V), dtype=qkv.dtype, device=dev)
+    # 8 to 16 leading spans of one token beside longer ones (`StepBatch.single_first`): the one kernel too.  The walk's two kernels go over
+    # all of the step's rows for them: 8 beside 1272 rows of 32 heads of 64 x 128, 49 us where this takes 6
+    ns = 0
+    if impl is None and not step.decode_only and _fn(lib, "zai_gated_delta_single_supports")(D, V):
+        ns = int(getattr(step, "single_first", 0))
+        if ns > DELTA_SINGLE_MAX_ROWS:
+            ns = 0
+    es = qkv.element_size()
+    cu, slots, n_seqs = step.cu_q.data_ptr(), step.slot_ids.data_ptr(), step.n_seqs - ns
+    if ns:
+        _check(_fn(lib, "zai_gated_delta_single")(
+            _ptr(out), qp, qs, bp, bs, ap, as_, gp, gs, _dt(qkv), _ptr(a_log), _ptr(dt_bias), _ptr(norm_w), float(eps),
+            float(unit_eps), _ptr(state), slots, ns, H, G, D, V, int(bool(write_state)), state.shape[0], _status_ptr(dev), ch, act,
+            _stream()), "gated_delta_single")
+        cu, slots = cu + 4 * ns, slots + 4 * ns
     cut = 1 << 30                                              # (spans of that many rows or more run in chunks, the others are walked)
     if impl != "walk" and not step.decode_only and qkv.dtype == torch.bfloat16 and _fn(lib, "zai_gated_delta_chunked_supports")(D, V):
         cut = 1 if impl == "chunks" else _delta_cut(H, D, V)
-    long, short = _span_kinds(step, cut)
+    long, short = _span_kinds(step, cut, ns)
     if long:
         max_chunks = _chunk_bound(step, cut, _fn(lib, "zai_gated_delta_chunk_rows")())
         scratch = torch.empty(max_chunks * H * _fn(lib, "zai_gated_delta_chunk_bytes")(V), dtype=torch.uint8, device=dev)
         _check(_fn(lib, "zai_gated_delta_chunked")(
-            _ptr(o), qp, qs, bp, bs, ap, as_, _ptr(a_log), _ptr(dt_bias), float(unit_eps), _ptr(state), _ptr(step.cu_q), _ptr(step.slot_ids),
-            state.shape[0], _status_ptr(dev), step.n_seqs, H, G, D, V, ch, int(bool(write_state)), cut, _chunked_spans(step, cut),
+            _ptr(o), qp, qs, bp, bs, ap, as_, _ptr(a_log), _ptr(dt_bias), float(unit_eps), _ptr(state), cu, slots,
+            state.shape[0], _status_ptr(dev), n_seqs, H, G, D, V, ch, int(bool(write_state)), cut, _chunked_spans(step, cut),
             _ptr(scratch), max_chunks, _stream()), "gated_delta_chunked", 2)
     if short and cut > 1:
         qk = torch.empty((N, 2, G, D), dtype=torch.float32, device=dev)
@@ -1501,12 +1516,11 @@ def gated_delta(qkv, b, a, gate, a_log, dt_bias, norm_w, eps, state, step, heads
         _check(_fn(lib, "zai_delta_prepare")(_ptr(qk), _ptr(bg), _ptr(gch), qp, qs, bp, bs, ap, as_, _dt(qkv), _ptr(a_log), _ptr(dt_bias),
                                              N, H, G, D, float(unit_eps), _ptr(step.cu_q), _ptr(step.seq_idx) if long else None, cut - 1,
                                              _stream()), "delta_prepare")
-        vp = qp + 2 * G * D * qkv.element_size()
-        _check(_fn(lib, "zai_gated_delta")(_ptr(o), _ptr(qk), _ptr(bg), _ptr(gch), vp, qs, _dt(qkv), _ptr(state), _ptr(step.cu_q),
-                                           _ptr(step.slot_ids), N, step.n_seqs, H, G, D, V, int(bool(write_state)), state.shape[0],
-                                           _status_ptr(dev), cut - 1, _stream()), "gated_delta")
-    _check(_fn(lib, "zai_gated_rmsnorm")(_ptr(out), _ptr(o), _ptr(norm_w), gp, gs, _dt(qkv), float(eps), N, H, V, act, _stream()),
-           "gated_rmsnorm")
+        vp = qp + 2 * G * D * es
+        _check(_fn(lib, "zai_gated_delta")(_ptr(o), _ptr(qk), _ptr(bg), _ptr(gch), vp, qs, _dt(qkv), _ptr(state), cu, slots, N, n_seqs, H, G,
+                                           D, V, int(bool(write_state)), state.shape[0], _status_ptr(dev), cut - 1, _stream()), "gated_delta")
+    _check(_fn(lib, "zai_gated_rmsnorm")(out.data_ptr() + ns * H * V * es, o.data_ptr() + ns * H * V * 4, _ptr(norm_w), gp + ns * gs * es, gs,
+                                         _dt(qkv), float(eps), N - ns, H, V, act, _stream()), "gated_rmsnorm")
     return out
 
 
