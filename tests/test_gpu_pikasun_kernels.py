@@ -60,7 +60,9 @@ def test_rotation_table_plain_and_stretched(scaling):
 
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("H,G,D,Dv,rot,scope", [(4, 2, 16, 16, 8, 2), (3, 1, 32, 8, 32, 2), (6, 3, 24, 40, 0, 2), (2, 2, 128, 128, 64, 2),
-                                                (5, 5, 10, 6, 4, 1), (8, 2, 64, 64, 64, 0), (8, 1, 128, 64, 32, 2)])
+                                                (5, 5, 10, 6, 4, 1), (8, 2, 64, 64, 64, 0), (8, 1, 128, 64, 32, 2),
+                                                # rows normed whole in registers: one load a thread, some, and four (with a rotation: halves of a pair)
+                                                (8, 8, 16, 16, 0, 2), (8, 8, 16, 16, 16, 2), (16, 4, 64, 64, 32, 2), (64, 32, 64, 64, 64, 2)])
 def test_qkv_prepare(dtype, H, G, D, Dv, rot, scope):
     """q, k and v from a wider stacked projection (a gate's columns behind them): the norm in its three scopes, the
     rotation, heads padded to the cache's size, and the rows written at the right page and offset."""
