@@ -289,3 +289,22 @@ def test_span_attention_and_values_that_are_not_finite(ps, form, bad):
             assert not torch.isfinite(got[hit]).any(), (ctx, p)
             assert torch.equal(got[~hit], want[~hit]), (ctx, p)
     assert o.read_status() == 0
+
+
+@pytest.mark.parametrize("dim,window", [(64, None), (64, 50), (24, None)])
+def test_32_bit_spans_in_few_and_in_many_tiles(dim, window):
+    """Up to two blocks an SM bring the next tile of keys ahead, larger grids do not: the same results, to the bit, for the same request."""
+    o = ops()
+    g = torch.Generator().manual_seed(71)
+    ctx, q_lens, ps, heads = [70, 3], [37, 900], 16, 16            # 16 heads of their own keys: 2 x 16 blocks, and 29 x 16 more
+    num_pages = 80
+    both = make_step(o, torch.float32, ctx, q_lens, ps, num_pages, 72)
+    pages = fill_pages(both, ctx, q_lens, ps, heads, dim, torch.float32, num_pages, g)
+    q = torch.randn(sum(q_lens), heads * dim, generator=g).cuda()
+    run = lambda step, rows, table: o.paged_attention(rows, step, CacheView(0, pages, table, ps), heads, heads, dim, dim ** -0.5, window)
+    many = run(both, q, both.block_tables[0])
+    want = ref_ops.paged_attention(q, both, CacheView(0, pages, both.block_tables[0], ps), heads, heads, dim, dim ** -0.5, window)
+    assert torch.allclose(many, want, atol=2e-5, rtol=2e-5)        # sums of a thousand weights of 32 bits
+    first = make_step(o, torch.float32, ctx[:1], q_lens[:1], ps, num_pages, 72)
+    assert torch.equal(run(first, q[:37], both.block_tables[0][:1].contiguous()), many[:37])
+    assert o.read_status() == 0

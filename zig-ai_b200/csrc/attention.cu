@@ -137,7 +137,8 @@ __device__ __forceinline__ float4 at_four(const bf16* p, int d, int D, bool vec)
                        d + 3 < D ? to_float(p[d + 3]) : 0.f);
 }
 
-template <typename T, int DM, bool EXT>
+// AHEAD: a tile's keys and values are asked for while the tile before is used, and wait in registers
+template <typename T, int DM, bool EXT, bool AHEAD>
 __global__ void __launch_bounds__(128) paged_attention_tile_kernel(
     T* __restrict__ out, const T* __restrict__ q, const T* __restrict__ pages, const int* __restrict__ block_table, int table_width,
     const int* __restrict__ positions, const int* __restrict__ cu_q, int n_seqs, int page_size, int Hq, int Hkv, int D, float scale,
@@ -201,25 +202,49 @@ __global__ void __launch_bounds__(128) paged_attention_tile_kernel(
 #pragma unroll
         for (int c = 0; c < NC; ++c) o[i][c] = 0.f;
     }
+    constexpr int PER = AT_N * (DM / 4) / 128;               // fours of keys (and of values) a thread brings of a tile
+    float4 next_k[AHEAD ? PER : 1], next_v[AHEAD ? PER : 1];
+    auto fetch = [&](int n, int r, float4& kv, float4& vv) { // the r-th of them
+        const int i = tid + r * 128, j = i / (DM / 4), d = (i % (DM / 4)) * 4;
+        const long long at = sm.row[n & 1][j];
+        kv = vv = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (at >= 0) {
+            kv = at_four(pages + at, d, D, vec);
+            vv = at_four(pages + at + v_off, d, D, vec);
+        }
+    };
     find_rows(0);
+    if (AHEAD) {
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < PER; ++r) fetch(0, r, next_k[r], next_v[r]);
+    }
     for (int n = 0; n < n_tiles; ++n) {
         bool odd = false;                                    // one of the thread's values is infinite or NaN
         __syncthreads();                                     // the tile before has been used; this one's rows are known
-#pragma unroll 4
-        for (int i = tid; i < AT_N * (DM / 4); i += 128) {
-            const int j = i / (DM / 4), d = (i % (DM / 4)) * 4;
-            const long long at = sm.row[n & 1][j];
-            float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), vv = kv;
-            if (at >= 0) {
-                kv = at_four(pages + at, d, D, vec);
-                vv = at_four(pages + at + v_off, d, D, vec);
-            }
+        auto put = [&](int r, const float4& kv, const float4& vv) {
+            const int i = tid + r * 128, j = i / (DM / 4), d = (i % (DM / 4)) * 4;
             *reinterpret_cast<float4*>(&sm.k[j][d]) = kv;
             *reinterpret_cast<float4*>(&sm.v[j][d]) = vv;
             odd |= !(fmaf(vv.x, 0.f, fmaf(vv.y, 0.f, fmaf(vv.z, 0.f, vv.w * 0.f))) == 0.f);       // (NaN for either)
+        };
+        if (AHEAD) {
+#pragma unroll
+            for (int r = 0; r < PER; ++r) put(r, next_k[r], next_v[r]);
+        } else {
+#pragma unroll 4
+            for (int r = 0; r < PER; ++r) {
+                float4 kv, vv;
+                fetch(n, r, kv, vv);
+                put(r, kv, vv);
+            }
         }
         find_rows(n + 1);
         odd = __syncthreads_or(odd);
+        if (AHEAD && n + 1 < n_tiles) {
+#pragma unroll
+            for (int r = 0; r < PER; ++r) fetch(n + 1, r, next_k[r], next_v[r]);
+        }
         float s[4][4] = {};
 #pragma unroll 4
         for (int d = 0; d < DM; d += 4) {
@@ -334,18 +359,36 @@ ZAI_API int zai_paged_attention_tiles_supports(int D, int Hq, int Hkv) { return 
 // rows of a tile: n_tiles of the launcher is the sum over the spans of their rows divided by this, rounded up (or more)
 ZAI_API int zai_paged_attention_tile_rows(int Hq, int Hkv) { return AT_M / (Hq / Hkv); }
 
-template <typename T, int DM, bool EXT>
-static int launch_tiles(void* out, const void* q, const void* pages, const int* block_table, int table_width, const int* positions,
+template <typename T, int DM, bool EXT, bool AHEAD>
+static int launch_tiles_of(void* out, const void* q, const void* pages, const int* block_table, int table_width, const int* positions,
                         const int* cu_q, int n_seqs, int n_tiles, int page_size, int Hq, int Hkv, int D, float scale, int window,
                         int num_pages, int* status, const ZaiScoreOptions& opt, cudaStream_t stream) {
     static unsigned long long done = 0;
     if (zai_first_on_device(&done)) {
-        const cudaError_t e = cudaFuncSetAttribute(paged_attention_tile_kernel<T, DM, EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AtTile<DM>));
+        const cudaError_t e = cudaFuncSetAttribute(paged_attention_tile_kernel<T, DM, EXT, AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AtTile<DM>));
         if (e != cudaSuccess) return (int)e;
     }
-    return launch_pdl(paged_attention_tile_kernel<T, DM, EXT>, dim3(n_tiles, Hkv), dim3(128), sizeof(AtTile<DM>), stream, (T*)out,
+    return launch_pdl(paged_attention_tile_kernel<T, DM, EXT, AHEAD>, dim3(n_tiles, Hkv), dim3(128), sizeof(AtTile<DM>), stream, (T*)out,
                       (const T*)q, (const T*)pages, block_table, table_width, positions, cu_q, n_seqs, page_size, Hq, Hkv, D, scale,
                       window, num_pages, status, opt);
+}
+// Grids of at most two blocks an SM bring the next tile while one is used (a tile's trip to memory is not hidden by other blocks
+// there): a layer of 384 rows behind 128 positions, 16 heads of 64 over 8, 176 -> 157 us.  Larger ones do without its 64 registers a thread.
+template <typename T, int DM, bool EXT>
+static int launch_tiles(void* out, const void* q, const void* pages, const int* block_table, int table_width, const int* positions,
+                        const int* cu_q, int n_seqs, int n_tiles, int page_size, int Hq, int Hkv, int D, float scale, int window,
+                        int num_pages, int* status, const ZaiScoreOptions& opt, cudaStream_t stream) {
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 148;
+    }
+    if constexpr (DM <= 64)
+        if ((long long)n_tiles * Hkv <= 2LL * sms)
+            return launch_tiles_of<T, DM, EXT, true>(out, q, pages, block_table, table_width, positions, cu_q, n_seqs, n_tiles, page_size, Hq, Hkv, D,
+                                                     scale, window, num_pages, status, opt, stream);
+    return launch_tiles_of<T, DM, EXT, false>(out, q, pages, block_table, table_width, positions, cu_q, n_seqs, n_tiles, page_size, Hq, Hkv, D,
+                                              scale, window, num_pages, status, opt, stream);
 }
 
 // A step's spans in tiles of rows (positions of a span's rows follow one another); the score options as below, all off by zeros
