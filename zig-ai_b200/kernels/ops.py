@@ -1484,7 +1484,7 @@ def gated_delta(qkv, b, a, gate, a_log, dt_bias, norm_w, eps, state, step, heads
     o = torch.empty((N, H * V), dtype=torch.float32, device=dev)
     out = torch.empty((N, H * V), dtype=qkv.dtype, device=dev)
     # 8 to 16 leading spans of one token beside longer ones (`StepBatch.single_first`): the one kernel too.  The walk's two kernels go over
-    # all of the step's rows for them: 8 beside 1272 rows of 32 heads of 64 x 128, 49 us where this takes 6
+    # all of the step's rows for them: 8 beside 1272 rows of 32 heads of 64 x 128, 49 us where this takes 11
     ns = 0
     if impl is None and not step.decode_only and _fn(lib, "zai_gated_delta_single_supports")(D, V):
         ns = int(getattr(step, "single_first", 0))
