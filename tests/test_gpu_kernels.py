@@ -490,6 +490,24 @@ def test_skinny_gemm_with_norm_residual_and_gathered_rows(M, O, K, eps):
     assert torch.equal(lazy.residual.data, h)
 
 
+@pytest.mark.parametrize("layer_norm", [False, True])
+@pytest.mark.parametrize("O,K", [(96, 264), (64, 512), (128, 1000), (1536, 1024), (512, 2048)])
+def test_rows_normed_before_a_product_do_not_depend_on_their_number(O, K, layer_norm):
+    """A row among others is the row alone, to the bit: its sum of squares is added in one order whatever the step's rows."""
+    from zig_ai_b200.parts.base import LazyNorm, Residual
+    o = ops()
+    g = torch.Generator().manual_seed(3)
+    h = (torch.randn(16, K, generator=g) * 2 + 0.5).cuda()
+    delta = torch.randn(16, K, generator=g).to(torch.bfloat16).cuda()
+    gamma = (1 + 0.2 * torch.randn(K, generator=g)).cuda()
+    beta = dict(beta=(0.5 * torch.randn(K, generator=g)).cuda()) if layer_norm else {}
+    w = (torch.randn(O, K, generator=g) * K ** -0.5).to(torch.bfloat16).cuda()
+    run = lambda a, b: o.linear(LazyNorm(Residual(h[a:b].clone()), delta[a:b].clone(), gamma, 1e-5, torch.bfloat16, **beta), w, out_dtype=torch.float32)
+    alone = torch.cat([run(i, i + 1) for i in range(16)])
+    for M in (3, 4, 5, 8, 9, 12, 13, 16):
+        assert torch.equal(run(0, M), alone[:M]), M
+
+
 @pytest.mark.parametrize("M", [1, 5, 8, 13, 16])
 @pytest.mark.parametrize("C,K,taps,bias,norm", [(1024, 1024, 3, False, True), (96, 96, 3, True, True), (100, 64, 4, True, False),
                                                 (517, 1000, 2, False, True), (72, 40, 1, True, False)])

@@ -160,23 +160,27 @@ __device__ __forceinline__ void skinny_stage(const SkinnyArgs& a, bf16* xs, int 
             if (m0 + r >= a.M) break;
             const float4 w = a.delta ? skinny_sum4(v[r], d[r]) : v[r];
             if (a.h_out && blockIdx.x == 0) *reinterpret_cast<float4*>(a.h_out + (size_t)(m0 + r) * K + k) = w;
-            ss[r] += w.x * w.x + w.y * w.y + w.z * w.z + w.w * w.w;
+            ss[r] += fmaf(w.w, w.w, fmaf(w.z, w.z, fmaf(w.y, w.y, w.x * w.x)));
             *reinterpret_cast<uint2*>(xs + (size_t)(m0 + r) * XS + k) = skinny_round4(w, gm);
         }
     }
-    // R sums over the warp at once: after the halving steps lane i has row i % R's
+    // R sums over the warp at once, by exchanges over lane distances 1, 2, 4, 8, 16 whatever R is (a row's sum does not depend on how
+    // many rows the step has): the first of them halve the rows that a lane has, the others add up what is left of one
+    int mine = 0;                                            // the row that the lane is left with
 #pragma unroll
-    for (int o = R / 2; o > 0; o >>= 1) {
+    for (int o = 1; o < R; o <<= 1) {
         const bool up = lane & o;
+        const int left = R / 2 / o;                          // rows that a lane has behind this exchange
+        mine += up ? left : 0;
 #pragma unroll
-        for (int i = 0; i < o; ++i) {
-            const float send = up ? ss[i] : ss[i + o], keep = up ? ss[i + o] : ss[i];
+        for (int i = 0; i < left; ++i) {
+            const float send = up ? ss[i] : ss[i + left], keep = up ? ss[i + left] : ss[i];
             ss[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
         }
     }
 #pragma unroll
     for (int o = R; o < 32; o <<= 1) ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], o);
-    if (lane < R && m0 + lane < a.M) sums[m0 + lane] = ss[0];
+    if (lane < R && m0 + mine < a.M) sums[m0 + mine] = ss[0];
 }
 // The same for a layer norm, whose mean is taken off before the squares: a warp a row, and a first walk over it for the mean (the second
 // one hits the cache).  sums [warps][stride]
