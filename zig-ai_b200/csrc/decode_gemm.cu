@@ -183,29 +183,46 @@ __device__ __forceinline__ void skinny_stage(const SkinnyArgs& a, bf16* xs, int 
     if (lane < R && m0 + mine < a.M) sums[m0 + mine] = ss[0];
 }
 // The same for a layer norm, whose mean is taken off before the squares: a warp a row, and a first walk over it for the mean (the second
-// one hits the cache).  sums [warps][stride]
-__device__ __forceinline__ void skinny_stage_centered(const SkinnyArgs& a, bf16* xs, int XS, float* sums, int stride, int source, int lane, int warp) {
+// one hits the cache).  Eight 16-byte loads of a lane are in flight, and the norm's weight (`gs`) is in shared memory since before the
+// wait: read behind it, in a second walk of two loads at a time, it was four trips to memory more (us a layer of norm, gated product
+// and down product, 1024 columns: one row 10.9 and 9.7, eight 11.2 and 10.9, sixteen 17.2 and 14.5; 2048: sixteen 55.9 and 44.9).
+// sums [warps][stride]
+__device__ __forceinline__ void skinny_stage_centered(const SkinnyArgs& a, bf16* xs, int XS, float* sums, int stride, const float* gs, int source,
+                                                      int lane, int warp) {
     const int K = a.K;
     for (int m = warp; m < a.M; m += SG_WARPS) {
         const size_t src = (size_t)__shfl_sync(0xffffffffu, source, m) * K;
-        auto at = [&](int k) {
-            const float4 v = *reinterpret_cast<const float4*>(a.h + src + k);
-            return a.delta ? skinny_sum4(v, *reinterpret_cast<const uint2*>(a.delta + src + k)) : v;
-        };
-        float mean = 0.f, ss = 0.f;
-#pragma unroll 2
+        float mean = 0.f;
         for (int k = lane * 4; k < K; k += 128) {
-            const float4 w = at(k);
+            float4 w = *reinterpret_cast<const float4*>(a.h + src + k);
+            if (a.delta) w = skinny_sum4(w, *reinterpret_cast<const uint2*>(a.delta + src + k));
             mean += (w.x + w.y) + (w.z + w.w);
         }
         mean = warp_sum(mean) / (float)K;
-#pragma unroll 2
-        for (int k = lane * 4; k < K; k += 128) {
-            float4 w = at(k);
-            if (a.h_out && blockIdx.x == 0) *reinterpret_cast<float4*>(a.h_out + (size_t)m * K + k) = w;
-            w.x -= mean; w.y -= mean; w.z -= mean; w.w -= mean;
-            ss += w.x * w.x + w.y * w.y + w.z * w.z + w.w * w.w;
-            *reinterpret_cast<uint2*>(xs + (size_t)m * XS + k) = skinny_round4(w, *reinterpret_cast<const float4*>(a.gamma + k));
+        float ss = 0.f;
+#pragma unroll 1
+        for (int kq = lane * 4; kq < K; kq += 1024) {
+            float4 v[8];
+            uint2 d[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int k = kq + u * 128;
+                if (k < K) {
+                    v[u] = *reinterpret_cast<const float4*>(a.h + src + k);
+                    if (a.delta) d[u] = *reinterpret_cast<const uint2*>(a.delta + src + k);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int k = kq + u * 128;
+                if (k < K) {
+                    float4 w = a.delta ? skinny_sum4(v[u], d[u]) : v[u];
+                    if (a.h_out && blockIdx.x == 0) *reinterpret_cast<float4*>(a.h_out + (size_t)m * K + k) = w;
+                    w.x -= mean; w.y -= mean; w.z -= mean; w.w -= mean;
+                    ss += w.x * w.x + w.y * w.y + w.z * w.z + w.w * w.w;
+                    *reinterpret_cast<uint2*>(xs + (size_t)m * XS + k) = skinny_round4(w, *reinterpret_cast<const float4*>(gs + k));
+                }
+            }
         }
         ss = warp_sum(ss);
         if (lane < SG_WARPS) sums[lane * stride + m] = lane == 0 ? ss : 0.f;
@@ -222,6 +239,7 @@ __global__ void __launch_bounds__(SG_WARPS * 32, 2) skinny_gemm_kernel(const Ski
     const int K = a.K, XS = K + 8;
     float* sums = reinterpret_cast<float*>(smem_raw);         // [warps][8*MT] each row's sum of squares over the columns that a warp staged
     bf16* xs = reinterpret_cast<bf16*>(smem_raw + SG_SUM_BYTES);   // [M][K + 8]
+    float* gs = reinterpret_cast<float*>(xs + (NORM ? (size_t)a.M * XS : 0));   // [K] a layer norm's weight
     float* red = reinterpret_cast<float*>(smem_raw + a.red_offset);   // [warps][MT*4][32]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
@@ -382,6 +400,8 @@ __global__ void __launch_bounds__(SG_WARPS * 32, 2) skinny_gemm_kernel(const Ski
     if (n_units > 0) conv_fixed(0);
     int source = lane;                                       // lane m: the source of row m (no kernel's output either)
     if (NORM && a.row_idx && lane < a.M) source = a.row_idx[lane];
+    if (NORM && EPI != EPI_CONV && a.center)                // ... nor is a layer norm's weight
+        for (int k = tid * 4; k < K; k += SG_WARPS * 32 * 4) *reinterpret_cast<float4*>(gs + k) = *reinterpret_cast<const float4*>(a.gamma + k);
     if (a.next.when == 1 && warp == SG_WARPS - 1) ask_next_weights(a.next, lane);
     pdl_wait_at(__LINE__, 1 + EPI * 2 + (NORM ? 1 : 0));
     pdl_trigger();                                           // (before the wait the next kernel's loads run beside this one's: 323 us instead of 318)
@@ -398,8 +418,10 @@ __global__ void __launch_bounds__(SG_WARPS * 32, 2) skinny_gemm_kernel(const Ski
     // 1.7 us from the wait to the products for one row, 2.2 for eight; so 1.4 and 1.9.  A decode step of the 350M shape, with the
     // convolution's slots and taps asked for before the wait: one request 350 -> 318 us, eight 377 -> 365.)
     if (NORM) {
-        if (a.center) skinny_stage_centered(a, xs, XS, sums, 8 * MT, source, lane, warp);
-        else {
+        if (EPI != EPI_CONV && a.center) {                   // (no convolution behind a layer norm)
+            __syncthreads();                                 // gs is complete
+            skinny_stage_centered(a, xs, XS, sums, 8 * MT, gs, source, lane, warp);
+        } else {
 #pragma unroll 1
             for (int m0 = 0; m0 < a.M; m0 += 8) {
                 const int rows = a.M - m0;
@@ -875,9 +897,9 @@ static int sg_slots() {
     }
     return v;
 }
-// What a block takes: x (with the norm the rows that there are, and their sums), the sums of the K slices, the rings
-static size_t skinny_block_x_bytes(int M, int K, bool norm) {
-    return norm ? (SG_SUM_BYTES + (size_t)M * (K + 8) * sizeof(bf16) + 1023) / 1024 * 1024 : 0;
+// What a block takes: x (with the norm the rows that there are, their sums and a layer norm's weight), the sums of the K slices, the rings
+static size_t skinny_block_x_bytes(int M, int K, bool norm, bool center) {
+    return norm ? (SG_SUM_BYTES + (size_t)M * (K + 8) * sizeof(bf16) + (center ? (size_t)K * sizeof(float) : 0) + 1023) / 1024 * 1024 : 0;
 }
 static size_t skinny_block_round_bytes(int mt, bool norm, int nt) { return (size_t)SG_WARPS * 4 * ((nt == 2 ? 3 : 2) + (norm ? 0 : mt)) * 512; }
 // (the bounds on the sizes that the kernel takes, and the depth of its rings, are counted for the largest block of its variant)
@@ -971,7 +993,7 @@ static int skinny_run(SkinnyArgs& a, int epilogue, cudaStream_t stream) {
         const int rounds = rpu * ((a.units + grid - 1) / grid);
         if (a.ring_rounds > rounds) a.ring_rounds = rounds;
     }
-    a.red_offset = (int)skinny_block_x_bytes(a.M, a.K, norm);
+    a.red_offset = (int)skinny_block_x_bytes(a.M, a.K, norm, a.center != 0);
     a.ring_offset = a.red_offset + (int)skinny_red_bytes(mt, nt);
     a.l2_prefetch_bytes = skinny_l2_prefetch_bytes();
     if (epilogue == EPI_BF16) return norm ? skinny_dispatch_mt<EPI_BF16, true>(a, stream) : skinny_dispatch_mt<EPI_BF16, false>(a, stream);
