@@ -491,7 +491,7 @@ def test_skinny_gemm_with_norm_residual_and_gathered_rows(M, O, K, eps):
 
 
 @pytest.mark.parametrize("layer_norm", [False, True])
-@pytest.mark.parametrize("O,K", [(96, 264), (64, 512), (128, 1000), (1536, 1024), (512, 2048)])
+@pytest.mark.parametrize("O,K", [(96, 64), (96, 136), (96, 264), (64, 512), (128, 1000), (1536, 1024), (512, 2048)])
 def test_rows_normed_before_a_product_do_not_depend_on_their_number(O, K, layer_norm):
     """A row among others is the row alone, to the bit: its sum of squares is added in one order whatever the step's rows."""
     from zig_ai_b200.parts.base import LazyNorm, Residual

@@ -133,6 +133,27 @@ __device__ __forceinline__ uint2 skinny_round4(float4 v, float4 gm) {
     __nv_bfloat162 lo = __floats2bfloat162_rn(v.x * gm.x, v.y * gm.y), hi = __floats2bfloat162_rn(v.z * gm.z, v.w * gm.w);
     return make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
 }
+// R sums over the warp at once; returns which of them the lane has, in ss[0] (lanes below R).  The exchanges go over lane distances 1, 2,
+// 4, 8, 16 whatever R is, so that a row's sum does not depend on how many rows the step has: the first of them halve the sums that a
+// lane has, the others add up what is left of one.
+template <int R>
+__device__ __forceinline__ int skinny_warp_sums(float (&ss)[R], int lane) {
+    int mine = 0;
+#pragma unroll
+    for (int o = 1; o < R; o <<= 1) {
+        const bool up = lane & o;
+        const int left = R / 2 / o;                          // sums that a lane has behind this exchange
+        mine += up ? left : 0;
+#pragma unroll
+        for (int i = 0; i < left; ++i) {
+            const float send = up ? ss[i] : ss[i + left], keep = up ? ss[i + left] : ss[i];
+            ss[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+#pragma unroll
+    for (int o = R; o < 32; o <<= 1) ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], o);
+    return mine;
+}
 // A warp's columns of up to R rows from m0 on: everything of a chunk of 1024 columns is asked for before the first of it is used
 // (lane m's `source` is the source of row m).  sums [rows]: the rows' sums of squares over these columns.
 template <int R>
@@ -164,30 +185,51 @@ __device__ __forceinline__ void skinny_stage(const SkinnyArgs& a, bf16* xs, int 
             *reinterpret_cast<uint2*>(xs + (size_t)(m0 + r) * XS + k) = skinny_round4(w, gm);
         }
     }
-    // R sums over the warp at once, by exchanges over lane distances 1, 2, 4, 8, 16 whatever R is (a row's sum does not depend on how
-    // many rows the step has): the first of them halve the rows that a lane has, the others add up what is left of one
-    int mine = 0;                                            // the row that the lane is left with
-#pragma unroll
-    for (int o = 1; o < R; o <<= 1) {
-        const bool up = lane & o;
-        const int left = R / 2 / o;                          // rows that a lane has behind this exchange
-        mine += up ? left : 0;
-#pragma unroll
-        for (int i = 0; i < left; ++i) {
-            const float send = up ? ss[i] : ss[i + left], keep = up ? ss[i + left] : ss[i];
-            ss[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
-    }
-#pragma unroll
-    for (int o = R; o < 32; o <<= 1) ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], o);
+    const int mine = skinny_warp_sums<R>(ss, lane);
     if (lane < R && m0 + mine < a.M) sums[m0 + mine] = ss[0];
+}
+// The same for rows of fewer parts of 128 columns than there are warps, a warp a row: the parts' sums are those that the warps of
+// `skinny_stage` make, to the bit.  `gs`: the norm's weight in shared memory.  sums [parts][stride]
+__device__ __forceinline__ void skinny_stage_short(const SkinnyArgs& a, bf16* xs, int XS, float* sums, int stride, int parts, const float* gs,
+                                                   int source, int lane, int warp) {
+    const int K = a.K;
+#pragma unroll 1
+    for (int m = warp; m < a.M; m += SG_WARPS) {
+        const size_t src = (size_t)__shfl_sync(0xffffffffu, source, m) * K;
+        float4 v[8];
+        uint2 d[8];
+        float ss[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int k = lane * 4 + u * 128;
+            v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            d[u] = make_uint2(0u, 0u);
+            if (k < K) {
+                v[u] = *reinterpret_cast<const float4*>(a.h + src + k);
+                if (a.delta) d[u] = *reinterpret_cast<const uint2*>(a.delta + src + k);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int k = lane * 4 + u * 128;
+            ss[u] = 0.f;
+            if (k < K) {
+                const float4 w = a.delta ? skinny_sum4(v[u], d[u]) : v[u];
+                if (a.h_out && blockIdx.x == 0) *reinterpret_cast<float4*>(a.h_out + (size_t)m * K + k) = w;
+                ss[u] += fmaf(w.w, w.w, fmaf(w.z, w.z, fmaf(w.y, w.y, w.x * w.x)));
+                *reinterpret_cast<uint2*>(xs + (size_t)m * XS + k) = skinny_round4(w, *reinterpret_cast<const float4*>(gs + k));
+            }
+        }
+        const int mine = skinny_warp_sums<8>(ss, lane);
+        if (lane < 8 && mine < parts) sums[mine * stride + m] = ss[0];
+    }
 }
 // The same for a layer norm, whose mean is taken off before the squares: a warp a row, and a first walk over it for the mean (the second
 // one hits the cache).  Eight 16-byte loads of a lane are in flight, and the norm's weight (`gs`) is in shared memory since before the
 // wait: read behind it, in a second walk of two loads at a time, it was four trips to memory more (us a layer of norm, gated product
 // and down product, 1024 columns: one row 10.9 and 9.7, eight 11.2 and 10.9, sixteen 17.2 and 14.5; 2048: sixteen 55.9 and 44.9).
 // sums [warps][stride]
-__device__ __forceinline__ void skinny_stage_centered(const SkinnyArgs& a, bf16* xs, int XS, float* sums, int stride, const float* gs, int source,
+__device__ __forceinline__ void skinny_stage_centered(const SkinnyArgs& a, bf16* xs, int XS, float* sums, int stride, int parts, const float* gs, int source,
                                                       int lane, int warp) {
     const int K = a.K;
     for (int m = warp; m < a.M; m += SG_WARPS) {
@@ -225,7 +267,7 @@ __device__ __forceinline__ void skinny_stage_centered(const SkinnyArgs& a, bf16*
             }
         }
         ss = warp_sum(ss);
-        if (lane < SG_WARPS) sums[lane * stride + m] = lane == 0 ? ss : 0.f;
+        if (lane < parts) sums[lane * stride + m] = lane == 0 ? ss : 0.f;
     }
 }
 
@@ -233,13 +275,15 @@ __device__ __forceinline__ void skinny_stage_centered(const SkinnyArgs& a, bf16*
 // 16 weight rows, each tile's K cut into `sk` slices, one slice per warp (8 warps).  A block uses
 // at most half of an SM's shared memory and registers, so the blocks of the next kernel on the stream
 // become resident beside it and start their own weight stream while this kernel still runs.
-template <int MT, int EPI, bool NORM>
+// ROWS: a norm's rows are staged by a warp each (layer norms, five and more short rows) and not by columns.  (Variants of their own: with
+// both in one, everything else paid 1 to 2 % for the code.)
+template <int MT, int EPI, bool NORM, bool ROWS>
 __global__ void __launch_bounds__(SG_WARPS * 32, 2) skinny_gemm_kernel(const SkinnyArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int K = a.K, XS = K + 8;
     float* sums = reinterpret_cast<float*>(smem_raw);         // [warps][8*MT] each row's sum of squares over the columns that a warp staged
     bf16* xs = reinterpret_cast<bf16*>(smem_raw + SG_SUM_BYTES);   // [M][K + 8]
-    float* gs = reinterpret_cast<float*>(xs + (NORM ? (size_t)a.M * XS : 0));   // [K] a layer norm's weight
+    float* gs = reinterpret_cast<float*>(xs + (ROWS ? (size_t)a.M * XS : 0));   // [K] the norm's weight, where rows are staged by a warp each
     float* red = reinterpret_cast<float*>(smem_raw + a.red_offset);   // [warps][MT*4][32]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
@@ -400,7 +444,8 @@ __global__ void __launch_bounds__(SG_WARPS * 32, 2) skinny_gemm_kernel(const Ski
     if (n_units > 0) conv_fixed(0);
     int source = lane;                                       // lane m: the source of row m (no kernel's output either)
     if (NORM && a.row_idx && lane < a.M) source = a.row_idx[lane];
-    if (NORM && EPI != EPI_CONV && a.center)                // ... nor is a layer norm's weight
+    const int parts = min((K + 127) / 128, SG_WARPS);        // sums of squares that a row has
+    if (ROWS)                                                // (... nor is the norm's weight)
         for (int k = tid * 4; k < K; k += SG_WARPS * 32 * 4) *reinterpret_cast<float4*>(gs + k) = *reinterpret_cast<const float4*>(a.gamma + k);
     if (a.next.when == 1 && warp == SG_WARPS - 1) ask_next_weights(a.next, lane);
     pdl_wait_at(__LINE__, 1 + EPI * 2 + (NORM ? 1 : 0));
@@ -416,11 +461,14 @@ __global__ void __launch_bounds__(SG_WARPS * 32, 2) skinny_gemm_kernel(const Ski
     // rsqrt(mean((h + delta)^2) + eps) is applied to the sums afterwards.  A warp takes 128 of every 1024 columns of all rows, four a
     // lane, so rows of up to 1024 values are one trip to memory and eight warps share the work of even a single row.  (A warp a row:
     // 1.7 us from the wait to the products for one row, 2.2 for eight; so 1.4 and 1.9.  A decode step of the 350M shape, with the
-    // convolution's slots and taps asked for before the wait: one request 350 -> 318 us, eight 377 -> 365.)
+    // convolution's slots and taps asked for before the wait: one request 350 -> 318 us, eight 377 -> 365.)  Shorter rows leave warps
+    // without columns that way: from five of them on a warp takes a row.  (us a layer of norm, SwiGLU product and
+    // down product, by columns and by rows: 512 columns, one row 5.3 and 5.7, eight 6.5 and 6.0, sixteen 8.8 and 8.3; 768: eight 7.8 and 7.3.)
     if (NORM) {
-        if (EPI != EPI_CONV && a.center) {                   // (no convolution behind a layer norm)
+        if (ROWS) {
             __syncthreads();                                 // gs is complete
-            skinny_stage_centered(a, xs, XS, sums, 8 * MT, gs, source, lane, warp);
+            if (a.center) skinny_stage_centered(a, xs, XS, sums, 8 * MT, parts, gs, source, lane, warp);
+            else skinny_stage_short(a, xs, XS, sums, 8 * MT, parts, gs, source, lane, warp);
         } else {
 #pragma unroll 1
             for (int m0 = 0; m0 < a.M; m0 += 8) {
@@ -441,7 +489,7 @@ __global__ void __launch_bounds__(SG_WARPS * 32, 2) skinny_gemm_kernel(const Ski
             if (NORM && kslice == 0 && nt * 8 + 2 * t + e < a.M) {
                 float ss = 0.f;
 #pragma unroll
-                for (int w2 = 0; w2 < SG_WARPS; ++w2) ss += sums[w2 * 8 * MT + nt * 8 + 2 * t + e];
+                for (int w2 = 0; w2 < SG_WARPS; ++w2) ss += w2 < parts ? sums[w2 * 8 * MT + nt * 8 + 2 * t + e] : 0.f;
                 inv_tok[nt][e] = rsqrtf(ss / (float)K + a.eps);
             }
         }
@@ -897,9 +945,10 @@ static int sg_slots() {
     }
     return v;
 }
-// What a block takes: x (with the norm the rows that there are, their sums and a layer norm's weight), the sums of the K slices, the rings
-static size_t skinny_block_x_bytes(int M, int K, bool norm, bool center) {
-    return norm ? (SG_SUM_BYTES + (size_t)M * (K + 8) * sizeof(bf16) + (center ? (size_t)K * sizeof(float) : 0) + 1023) / 1024 * 1024 : 0;
+// What a block takes: x (with the norm the rows that there are, their sums and, where a warp stages a row, the norm's weight), the sums of the
+// K slices, the rings
+static size_t skinny_block_x_bytes(int M, int K, bool norm, bool by_rows) {
+    return norm ? (SG_SUM_BYTES + (size_t)M * (K + 8) * sizeof(bf16) + (by_rows ? (size_t)K * sizeof(float) : 0) + 1023) / 1024 * 1024 : 0;
 }
 static size_t skinny_block_round_bytes(int mt, bool norm, int nt) { return (size_t)SG_WARPS * 4 * ((nt == 2 ? 3 : 2) + (norm ? 0 : mt)) * 512; }
 // (the bounds on the sizes that the kernel takes, and the depth of its rings, are counted for the largest block of its variant)
@@ -948,12 +997,12 @@ static void skinny_plan(int rows, bool may_halve, int K, int* n_tiles, int* half
     *units = (*n_tiles + *tpc - 1) / *tpc;
 }
 
-template <int MT, int EPI, bool NORM>
+template <int MT, int EPI, bool NORM, bool ROWS>
 static int skinny_launch(const SkinnyArgs& a, cudaStream_t stream) {
     const size_t smem = (size_t)a.ring_offset + skinny_block_round_bytes(MT, NORM, EPI == EPI_CONV ? 2 : 1) * a.ring_rounds;
     static size_t configured = 0;
     if (smem > configured) {
-        cudaError_t e = cudaFuncSetAttribute(skinny_gemm_kernel<MT, EPI, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(skinny_gemm_kernel<MT, EPI, NORM, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
         if (e != cudaSuccess) return (int)e;
         configured = smem;
@@ -961,13 +1010,14 @@ static int skinny_launch(const SkinnyArgs& a, cudaStream_t stream) {
     const int grid = a.units < sg_slots() ? a.units : sg_slots();
     SkinnyArgs b = a;
     b.next = take_hint(grid);
-    return launch_pdl(skinny_gemm_kernel<MT, EPI, NORM>, dim3(grid), dim3(SG_WARPS * 32), smem, stream, b);
+    return launch_pdl(skinny_gemm_kernel<MT, EPI, NORM, ROWS>, dim3(grid), dim3(SG_WARPS * 32), smem, stream, b);
 }
 
-template <int EPI, bool NORM>
-static int skinny_dispatch_mt(const SkinnyArgs& a, cudaStream_t stream) {
-    if (a.M <= 8) return skinny_launch<1, EPI, NORM>(a, stream);
-    return skinny_launch<2, EPI, NORM>(a, stream);
+template <int EPI>
+static int skinny_dispatch(const SkinnyArgs& a, bool by_rows, cudaStream_t stream) {
+    if (!a.h) return a.M <= 8 ? skinny_launch<1, EPI, false, false>(a, stream) : skinny_launch<2, EPI, false, false>(a, stream);
+    if (!by_rows) return a.M <= 8 ? skinny_launch<1, EPI, true, false>(a, stream) : skinny_launch<2, EPI, true, false>(a, stream);
+    return a.M <= 8 ? skinny_launch<1, EPI, true, true>(a, stream) : skinny_launch<2, EPI, true, true>(a, stream);
 }
 
 // 1 if the kernel takes these sizes (else the caller uses the library product and separate kernels)
@@ -993,13 +1043,14 @@ static int skinny_run(SkinnyArgs& a, int epilogue, cudaStream_t stream) {
         const int rounds = rpu * ((a.units + grid - 1) / grid);
         if (a.ring_rounds > rounds) a.ring_rounds = rounds;
     }
-    a.red_offset = (int)skinny_block_x_bytes(a.M, a.K, norm, a.center != 0);
+    const bool by_rows = norm && (a.center || (a.K <= (SG_WARPS - 1) * 128 && a.M > 4));      // (see skinny_stage and what follows it)
+    a.red_offset = (int)skinny_block_x_bytes(a.M, a.K, norm, by_rows);
     a.ring_offset = a.red_offset + (int)skinny_red_bytes(mt, nt);
     a.l2_prefetch_bytes = skinny_l2_prefetch_bytes();
-    if (epilogue == EPI_BF16) return norm ? skinny_dispatch_mt<EPI_BF16, true>(a, stream) : skinny_dispatch_mt<EPI_BF16, false>(a, stream);
-    if (epilogue == EPI_F32) return norm ? skinny_dispatch_mt<EPI_F32, true>(a, stream) : skinny_dispatch_mt<EPI_F32, false>(a, stream);
-    if (epilogue == EPI_SWIGLU) return norm ? skinny_dispatch_mt<EPI_SWIGLU, true>(a, stream) : skinny_dispatch_mt<EPI_SWIGLU, false>(a, stream);
-    if (epilogue == EPI_CONV) return norm ? skinny_dispatch_mt<EPI_CONV, true>(a, stream) : skinny_dispatch_mt<EPI_CONV, false>(a, stream);
+    if (epilogue == EPI_BF16) return skinny_dispatch<EPI_BF16>(a, by_rows, stream);
+    if (epilogue == EPI_F32) return skinny_dispatch<EPI_F32>(a, by_rows, stream);
+    if (epilogue == EPI_SWIGLU) return skinny_dispatch<EPI_SWIGLU>(a, by_rows, stream);
+    if (epilogue == EPI_CONV) return skinny_dispatch<EPI_CONV>(a, by_rows, stream);
     return ZAI_BAD_SIZE;
 }
 
