@@ -949,6 +949,27 @@ def test_qk_norm_rope_many_rows(Hq, Hkv, D, ps, qk_norm):
     assert pages_a[0].abs().sum() == 0 and o.read_status() == 0
 
 
+@pytest.mark.parametrize("Hq,Hkv,D", [(8, 2, 32), (16, 4, 24), (32, 8, 16)])
+def test_qk_norm_rope_32_bit_rows_among_few_and_many(Hq, Hkv, D):
+    """Blocks of 4, 8 and 16 warps (chosen by rows and heads): the same rows to the bit, pages included."""
+    o = ops()
+    g = torch.Generator().manual_seed(18)
+    N, ps = 2400, 64
+    qkv = torch.randn(N, (Hq + 2 * Hkv) * D, generator=g).cuda()
+    w = (1 + 0.1 * torch.randn(D, generator=g)).cuda()
+    want = None
+    for n in (N, 1184, 800, 444, 5):
+        step = make_step(o, torch.float32, [0], [n], ps, 40, 19)
+        pages = torch.zeros(40, 2, Hkv, ps, D, device="cuda")
+        q, k = o.qk_norm_rope(qkv[:n].contiguous(), w, w, 1e-5, D, 10000.0, step, CacheView(0, pages, step.block_tables[0], ps), Hq, Hkv, D, True, True, True)
+        rows = pages[step.block_tables[0][0].long()].transpose(1, 3).reshape(-1, Hkv, 2, D)[:n]
+        if want is None:
+            want = q, k, rows
+        for got, ref in zip((q, k, rows), want):
+            assert torch.equal(got, ref[:n]), n
+    assert o.read_status() == 0
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("Hq,Hkv,D", [(4, 2, 64), (3, 3, 24), (6, 2, 100), (32, 1, 12), (33, 1, 20), (5, 1, 128), (2, 1, 1)])
 def test_attention_in_tiles_of_rows(dtype, Hq, Hkv, D):

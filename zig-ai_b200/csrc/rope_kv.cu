@@ -374,6 +374,15 @@ ZAI_API int zai_rope_table_scaled(float2* table, const int* positions, const dou
                       magnitude);
 }
 
+static int sm_count() {
+    static int n = 0;
+    if (!n) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 148;
+    }
+    return n;
+}
+
 // q_map > 0: the rows hold Hq / 2 query heads, each two maps of q_map and D - q_map values; q_out has a query head per map with
 // zeros in the other map's place (no norm, no rotation).
 ZAI_API int zai_qk_norm_rope(const void* qkv, int qkv_cols, int dtype, const float* q_gamma, const float* k_gamma,
@@ -399,12 +408,19 @@ ZAI_API int zai_qk_norm_rope(const void* qkv, int qkv_cols, int dtype, const flo
         ZAI_QK_VEC(2) ZAI_QK_VEC(4) ZAI_QK_VEC(8) ZAI_QK_VEC(16) ZAI_QK_VEC(32)
 #undef ZAI_QK_VEC
     }
-    // a warp a head, as far as 16 warps and the shared memory for their rows go (four warps took a row's heads by turns, a trip to
-    // memory each: 384 rows of 32 heads of 64 in 32 bits 11.8 us, so 6.9)
-    int threads = 128;
+    // A warp a head, up to 16 warps, as far as the shared memory for their rows goes and the grid stays one wave (an SM holds 1536 of these
+    // threads): four warps take a row's heads by turns, a trip to memory each.  More blocks than a wave holds cover those trips
+    // themselves and wide ones only leave warps idle; from 24 heads on eight warps still pay with up to 16 rows an SM, from 48 on 16
+    // with up to 8.  32 bits, us with 4, 8 and 16 warps: 32 heads of 64, 384 rows 10.4, 8.5, 6.1; 768 rows 13.8, 9.4, 11.0; 2048 rows
+    // 23.0, 20.5, 23.9; 8192 rows 79 and, with 16, 110; 12 heads of 128, 384 rows 6.5, 6.3, 4.5; 768 rows 9.1, 7.1, 8.1; 2048 rows
+    // 13.9, 14.9, 17.0; 80 heads of 64, 1024 rows 41.8, 30.5, 27.8; 2048 rows 62.6, 52.8, 53.7.
+    const int heads = Hq + (has_kv ? 2 * Hkv : 0);
+    const long long wave = (long long)sm_count() * 1536;
     const auto bytes = [&](int n) { return (size_t)(rot + (n / 32) * D) * sizeof(float); };
+    int threads = 128;
     if (bytes(threads) > 48 * 1024) return ZAI_BAD_SIZE;
-    while (threads < 512 && threads / 32 < Hq + (has_kv ? 2 * Hkv : 0) && bytes(2 * threads) <= 48 * 1024) threads *= 2;
+    if (heads > 8 && bytes(512) <= 48 * 1024 && (N * 512LL <= wave || (heads >= 48 && N <= 8LL * sm_count()))) threads = 512;
+    else if (heads > 4 && bytes(256) <= 48 * 1024 && (N * 256LL <= wave || (heads >= 24 && N <= 16LL * sm_count()))) threads = 256;
     const size_t smem = bytes(threads);
     ZAI_DISPATCH(dtype, return launch_pdl(qk_norm_rope_kernel<T>, dim3(N), dim3(threads), smem, stream,
         (const T*)qkv, qkv_cols, q_gamma, k_gamma, eps, cs_table, rot, positions, seq_idx, block_table,
