@@ -291,9 +291,9 @@ def test_span_attention_and_values_that_are_not_finite(ps, form, bad):
     assert o.read_status() == 0
 
 
-@pytest.mark.parametrize("dim,window", [(64, None), (64, 50), (24, None)])
+@pytest.mark.parametrize("dim,window", [(64, None), (64, 50), (32, None), (24, None)])
 def test_32_bit_spans_in_few_and_in_many_tiles(dim, window):
-    """Up to two blocks an SM bring the next tile of keys ahead, larger grids do not: the same results, to the bit, for the same request."""
+    """Up to 7/4 blocks an SM bring the next tile of keys ahead (heads of 32 and 64), larger grids do not: the same results, to the bit, for the same request."""
     o = ops()
     g = torch.Generator().manual_seed(71)
     ctx, q_lens, ps, heads = [70, 3], [37, 900], 16, 16            # 16 heads of their own keys: 2 x 16 blocks, and 29 x 16 more

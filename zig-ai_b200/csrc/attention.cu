@@ -16,6 +16,8 @@
 // `zai_paged_attention_scored` is the same kernel with the options of designs that shape their scores (`ZaiScoreOptions`
 // in common.cuh: a cap, a bias by distance, a sink, kept first positions under a window; here with the exact `tanhf`).
 // The kept positions are a second range of keys, walked before the window's, again in steps of 32 from position 0.
+#include <type_traits>
+
 #include "common.cuh"
 
 
@@ -372,21 +374,28 @@ static int launch_tiles_of(void* out, const void* q, const void* pages, const in
                       (const T*)q, (const T*)pages, block_table, table_width, positions, cu_q, n_seqs, page_size, Hq, Hkv, D, scale,
                       window, num_pages, status, opt);
 }
-// Grids of at most two blocks an SM bring the next tile while one is used (a tile's trip to memory is not hidden by other blocks
-// there): a layer of 384 rows behind 128 positions, 16 heads of 64 over 8, 176 -> 157 us.  Larger ones do without its 64 registers a thread.
+// Whether a tile of keys is brought while the one before is used.  A tile's trip to memory is not hidden by other blocks in grids of up
+// to about 7/4 blocks an SM; fuller ones do without the 40 registers a thread.  For 32-bit heads of 32 and 64 values whose rows are all
+// 16-byte loads, and requests of more than two tiles of keys (known by the width of the table).  us without and with, 8 heads of 64: 20
+// rows alone 8.8, 9.5, behind 60 positions 13.5, 13.7, behind 200 23.2, 21.9; 400 behind 400 (104 blocks) 66.9, 59.4; 800 rows (200)
+// 83.3, 72.5; 1000 (256) 110, 107; 1184 behind 1000 (296) 239, 245; 3000 (752) 455, 477.  Of 32: 20 alone 7.0, 7.5, 400 behind 400
+// 42.3, 39.0, 880 rows (224 blocks) 60, 57, 2048 rows of 4 heads (256) 129, 132.  Of 40 (bounds in every load) 590 rows 56.7, 59.0; heads
+// of 128 would wait in 128 registers more.  bfloat16 of 40, whose values would wait as 32-bit numbers: 400 behind 400 72, 107.
 template <typename T, int DM, bool EXT>
 static int launch_tiles(void* out, const void* q, const void* pages, const int* block_table, int table_width, const int* positions,
                         const int* cu_q, int n_seqs, int n_tiles, int page_size, int Hq, int Hkv, int D, float scale, int window,
                         int num_pages, int* status, const ZaiScoreOptions& opt, cudaStream_t stream) {
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 148;
-    }
-    if constexpr (DM <= 64)
-        if ((long long)n_tiles * Hkv <= 2LL * sms)
+    if constexpr (std::is_same<T, float>::value && DM <= 64) {
+        static int sms = 0;
+        if (!sms) {
+            int dev = 0;
+            if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 148;
+        }
+        if (D == DM && ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(pages)) & 15) == 0
+            && (long long)table_width * page_size > 2 * AT_N && (long long)n_tiles * Hkv * 8 <= (DM == 64 ? 14LL : 13LL) * sms)
             return launch_tiles_of<T, DM, EXT, true>(out, q, pages, block_table, table_width, positions, cu_q, n_seqs, n_tiles, page_size, Hq, Hkv, D,
                                                      scale, window, num_pages, status, opt, stream);
+    }
     return launch_tiles_of<T, DM, EXT, false>(out, q, pages, block_table, table_width, positions, cu_q, n_seqs, n_tiles, page_size, Hq, Hkv, D,
                                               scale, window, num_pages, status, opt, stream);
 }
