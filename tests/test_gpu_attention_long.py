@@ -291,6 +291,43 @@ def test_span_attention_and_values_that_are_not_finite(ps, form, bad):
     assert o.read_status() == 0
 
 
+@pytest.mark.parametrize("ps", [16, 64])
+@pytest.mark.parametrize("opts", [dict(softcap=20.0, bias=40, sink=True), dict(sink=True), dict(window=20, keep_first=3, sink=True),
+                                  dict(softcap=2.0), dict(bias=300)])
+def test_shaped_span_attention_of_one_tile_of_keys(ps, opts):
+    """Spans whose rows see one tile of 64 keys, whose halves are made apart: rows that see keys of one half, of both, of the last key
+    of the first; a value that is not finite reaches the rows that see it.  A result is a weighted mean of values below 5.2: weights
+    and both results rounded to bfloat16, 3 * 2^-9 * 5.2."""
+    o = ops()
+    g = torch.Generator().manual_seed(81)
+    opts = dict(opts)
+    if "bias" in opts:
+        opts["bias"] = (torch.randn(opts["bias"], Hq, generator=g) * 1.5).cuda()
+    if "sink" in opts:
+        opts["sink"] = (torch.randn(Hq, generator=g) * 2).cuda()
+    ctx, q_lens = [0, 0, 31, 32, 63, 5, 0, 0], [64, 33, 2, 32, 1, 30, 1, 65]
+    num_pages = sum(-(-(c + n) // ps) for c, n in zip(ctx, q_lens)) + 8
+    step = make_step(o, BF16, ctx, q_lens, ps, num_pages, 82)
+    fill = lambda junk: fill_pages(step, ctx, q_lens, ps, Hkv, D, BF16, num_pages, torch.Generator().manual_seed(83), junk=junk).clamp(-5.2, 5.2)
+    q = torch.randn(sum(q_lens), Hq * D, generator=g).to(BF16).cuda()
+    run = lambda at, pages: at(q, step, CacheView(0, pages, step.block_tables[0], ps), Hq, Hkv, D, D ** -0.5, **opts)
+    got, want = run(o.paged_attention, fill(0.0)), run(ref_ops.paged_attention, fill(0.0))
+    assert torch.allclose(got.float(), want.float(), atol=3e-2, rtol=0), (got.float() - want.float()).abs().max()
+    assert torch.equal(run(o.paged_attention, fill(float("nan"))), got)
+    kv, col = 3, 17
+    for p in (0, 31, 32, 63):
+        pages = fill(float("nan"))
+        pages[int(step.block_tables[0][0, p // ps]), 1, kv, p % ps, col] = float("inf")
+        pos = torch.arange(64)
+        sees = (p <= pos) & ((p > pos - opts.get("window", 1000)) | (p < opts.get("keep_first", 0)))
+        hit = torch.zeros(sum(q_lens), Hq, D, dtype=torch.bool)
+        hit[:64, kv * G:(kv + 1) * G, col] = sees[:, None]
+        hit = hit.view(-1, Hq * D).cuda()
+        now = run(o.paged_attention, pages)
+        assert not torch.isfinite(now[hit]).any() and torch.equal(now[~hit], got[~hit]), p
+    assert o.read_status() == 0
+
+
 @pytest.mark.parametrize("dim,window", [(64, None), (64, 50), (32, None), (24, None)])
 def test_32_bit_spans_in_few_and_in_many_tiles(dim, window):
     """Up to 7/4 blocks an SM bring the next tile of keys ahead (heads of 32 and 64), larger grids do not: the same results, to the bit, for the same request."""

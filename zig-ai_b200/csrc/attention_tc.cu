@@ -39,6 +39,8 @@
 // (scores, softmax, P, product), and the longest blocks of every head should start first.
 // Every wait on an mbarrier is bounded; a block whose wait runs out raises the status word, its roles
 // leave their loops, TMEM is freed and the block returns.
+#include <type_traits>
+
 #include "attention_tc_helpers.cuh"
 
 #define AT_D 64
@@ -348,7 +350,20 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
                         at_umma_ts(d, p + kk * 8, at_desc(aV + kk * 2048), idesc_o, (i > (SHAPED ? 1 : 0) || kk > 0) ? 1u : 0u);
                 };
                 auto cleaned = [&](int i) { return i >= p0 || (i >= p1 && i < p2); };
-                if (SHAPED) {
+                if (SHAPED && n_tiles == 1) {
+                    // a tile alone: the turns have half of its keys each, for an O each
+                    if (ok) ok = at_mbar_wait(&kv_full[0], 0, failed);
+                    if (ok) scores(0);
+                    if (ok) ok = at_mbar_wait(&v_ready[0], 0, failed) && at_mbar_wait(&p_ready[0], 0, failed) && at_mbar_wait(&p_ready[1], 0, failed);
+                    if (ok) {
+                        const uint32_t aV = at_smem(sKV + AT_BN * 128);
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                        for (int kk = 0; kk < AT_BN / 16; ++kk)
+                            at_umma_ts(tO + (kk >> 1) * AT_D, tS + (kk >> 1) * 32 + (kk & 1) * 8, at_desc(aV + kk * 2048), idesc_o, kk & 1);
+                        at_commit(&kv_empty[0]);
+                    }
+                } else if (SHAPED) {
                     // P lies over its scores, so the scores of tile i + 2 are issued behind the product of tile i (products of one
                     // thread run in order); the other turn's tile i + 1 is in the softmax meanwhile
 #pragma unroll 1
@@ -398,25 +413,27 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
             const int klo = zai_first_visible(qpos, a.window);
             const int kept = SHAPED && a.window > 0 ? min(a.opt.keep_first, klo) : 0;
             const uint32_t lanes = tmem_base + ((uint32_t)(qd * 32) << 16), tS = lanes + turn * AT_BN, tO = lanes + AT_COL_O + (SHAPED ? turn * AT_D : 0),
-                           tP = SHAPED ? tS : lanes + AT_COL_P + turn * (AT_BN / 2);
+                           tPlain = lanes + AT_COL_P + turn * (AT_BN / 2);
             const float c = SHAPED ? 1.f : a.scale_log2;        // (shaped scores are made in the exponent's units)
             const float unit = SHAPED && a.opt.softcap > 0.f ? a.opt.scale / a.opt.softcap : 0.f, cap = a.opt.softcap * 1.4426950408889634f;
             bool alive = true;
-            for (int i = turn; i < n_tiles; i += 2) {
-                const int key0 = key_of(i);
-                if (alive) alive = at_mbar_wait_warp(&s_ready[turn], (i >> 1) & 1, failed);                   // (the warp together)
+            // tile i's keys from key0 on (64 of them, or 32), whose scores come into column tSc
+            auto tile = [&](int i, int key0, uint32_t tSc, uint64_t* scores_ready, auto keys_of) {
+                constexpr int KEYS = decltype(keys_of)::value;
+                const uint32_t tP = SHAPED ? tSc : tPlain;
+                if (alive) alive = at_mbar_wait_warp(scores_ready, (i >> 1) & 1, failed);   // (the warp together)
                 if (!alive) {                                   // (the other turn's warps still wait for this one's word)
-                    if (SHAPED) break;
+                    if (SHAPED) return;
                     if (i > 0) at_pass_wait(qd, i - 1);
                     if (i + 1 < n_tiles) at_pass_on(qd, i);
-                    continue;
+                    return;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                uint32_t x[2][32];
-                at_tmem_ld32_nowait(tS, x[0]);
-                at_tmem_ld32_nowait(tS + 32, x[1]);
-                at_tmem_wait_ld(x[0]);
-                at_tmem_wait_ld(x[1]);
+                uint32_t x[KEYS / 32][32];
+#pragma unroll
+                for (int j = 0; j < KEYS / 32; ++j) at_tmem_ld32_nowait(tSc + j * 32, x[j]);
+#pragma unroll
+                for (int j = 0; j < KEYS / 32; ++j) at_tmem_wait_ld(x[j]);
                 if (!SHAPED) {
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     if (lane == 0) at_mbar_arrive(&s_empty[turn]);
@@ -429,7 +446,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
                     const float* from = bias + far;
                     auto shape = [&](auto entry) {
 #pragma unroll
-                        for (int j = 0; j < 64; j += 2) {
+                        for (int j = 0; j < KEYS; j += 2) {
                             float2 v = make_float2(__uint_as_float(x[j >> 5][j & 31]), __uint_as_float(x[j >> 5][(j & 31) + 1]));
                             const float2 add = make_float2(entry(j), entry(j + 1));
                             v = a.opt.softcap > 0.f ? at_fma2(at_tanh2(at_mul2(v, at_two(unit))), at_two(cap), add) : at_fma2(v, at_two(a.scale_log2), add);
@@ -442,19 +459,19 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
                     else shape([&](int j) { return bias[min(max(far - j, 0), last)]; });
                 }
                 // keys that the row sees: [lo, hi), and those below `first`
-                const int lo = valid ? max(klo - key0, 0) : 64, hi = valid ? min(qpos + 1 - key0, 64) : 0;
+                const int lo = valid ? max(klo - key0, 0) : KEYS, hi = valid ? min(qpos + 1 - key0, KEYS) : 0;
                 const int first = valid ? kept - key0 : 0;
-                if (__any_sync(0xffffffffu, lo > 0 || hi < 64)) {                       // (the warp's branch: no tile without it pays for its instructions)
+                if (__any_sync(0xffffffffu, lo > 0 || hi < KEYS)) {                     // (the warp's branch: no tile without it pays for its instructions)
                     // (a hidden score may be anything, also NaN: it is replaced before the exponential)
                     const unsigned long long seen = (at_below(hi) & ~at_below(lo)) | (SHAPED ? at_below(first) : 0ull);
                     const uint32_t some[2] = {(uint32_t)seen, (uint32_t)(seen >> 32)};
 #pragma unroll
-                    for (int j = 0; j < 64; ++j)
+                    for (int j = 0; j < KEYS; ++j)
                         if (!(some[j >> 5] >> (j & 31) & 1)) x[j >> 5][j & 31] = __float_as_uint(-INFINITY);
                 }
                 float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};            // four chains, not one of 32 links
 #pragma unroll
-                for (int j = 0; j < 64; j += 2)
+                for (int j = 0; j < KEYS; j += 2)
                     mx4[(j >> 1) & 3] = at_max3(mx4[(j >> 1) & 3], __uint_as_float(x[j >> 5][j & 31]), __uint_as_float(x[j >> 5][(j & 31) + 1]));
                 const float mx = fmaxf(at_max3(mx4[0], mx4[1], mx4[2]), mx4[3]) * c;
                 // move the reference?  (warp-wide decision: the TMEM accesses below are the whole warp's)
@@ -494,7 +511,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
                 // (plain scores: the product of tile i - 2 reads this P buffer)
                 if (!SHAPED && i > 1 && alive) alive = at_mbar_wait_warp(&kv_empty[(i - 2) % STAGES], ((i - 2) / STAGES) & 1, failed);
 #pragma unroll
-                for (int j0 = 0; j0 < 64; j0 += 16) {           // (16 keys a store: with 64 the registers for them cost moves and spills)
+                for (int j0 = 0; j0 < KEYS; j0 += 16) {         // (16 keys a store: with 64 the registers for them cost moves and spills)
                     uint32_t pk[8];
 #pragma unroll
                     for (int j = j0; j < j0 + 16; j += 2) {
@@ -512,6 +529,13 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) at_mbar_arrive(&p_ready[turn]);
+            };
+            if (SHAPED && n_tiles == 1) {
+                // a tile alone: each turn has 32 of its keys, or half of the warps would have nothing to do.  (64 rows, cap, bias and sink, 16
+                // heads: 9.0 us with all keys in one turn, 7.2 so; 64 spans of 40 rows 45 and 39.)
+                if constexpr (SHAPED) tile(0, key_of(0) + turn * 32, lanes + turn * 32, &s_ready[0], std::integral_constant<int, 32>{});
+            } else {
+                for (int i = turn; i < n_tiles; i += 2) tile(i, key_of(i), tS, &s_ready[turn], std::integral_constant<int, AT_BN>{});
             }
             // the row's two parts: what weighs them, and the sum over both
             if (!SHAPED) asm volatile("bar.sync 1, 256;" ::: "memory");     // (the last reference has been read)
@@ -534,11 +558,11 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
                 // this thread's half of the columns of O, the two parts together
                 uint32_t o0[32], o1[32];
                 at_tmem_ld32(lanes + AT_COL_O + turn * 32, o0);
-                if (SHAPED && n_tiles > 1) at_tmem_ld32(lanes + AT_COL_O + AT_D + turn * 32, o1);
+                if (SHAPED) at_tmem_ld32(lanes + AT_COL_O + AT_D + turn * 32, o1);
 #pragma unroll
                 for (int j = 0; j < 32; ++j) {
                     out[j] = __uint_as_float(o0[j]) * (SHAPED ? f0 : 1.f);
-                    if (SHAPED && n_tiles > 1) out[j] = fmaf(__uint_as_float(o1[j]), f1, out[j]);
+                    if (SHAPED) out[j] = fmaf(__uint_as_float(o1[j]), f1, out[j]);
                 }
                 bf16* dst = a.out + ((size_t)(row0 + i0 + row) * a.Hq + h) * AT_D + turn * 32;
                 if (!SHARED && valid) {
