@@ -143,24 +143,45 @@ def test_gated_delta(dtype, H, G, D, V):
 
 @pytest.mark.parametrize("channel", [False, True])
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("singles,spans", [(8, [2]), (9, [70, 5]), (17, [64, 0, 63]), (32, [66]), (7, [130])])
-def test_gated_delta_of_decoded_tokens_ahead_of_spans(singles, spans, dtype, channel):
-    """Leading spans of one token take the one kernel, eight or sixteen of them, the others of the step what their length says."""
+@pytest.mark.parametrize("singles,spans", [(8, [2]), (9, [70, 5]), (17, [64, 0, 63]), (32, [66]), (7, [130]), (8, [70]), (12, [64, 0, 130]),
+                                           (16, [66]), (8, [0, 0]), (17, [64, 0])])
+@pytest.mark.parametrize("captured", [False, True])
+def test_gated_delta_of_decoded_tokens_ahead_of_spans(singles, spans, captured, dtype, channel):
+    """Eight and more leading spans of one token take the one kernel where every other span goes in chunks (rows and states are then those of
+    a step of the same requests alone, to the bit, and the walk's kernels do not run); everything else is walked, and so is a step in
+    the layout of a captured shape (empty spans, counts of chunks and spans rounded up)."""
     o = ops()
     g = torch.Generator().manual_seed(27)
     H, G, D, V = 4, 2, 64, 128
-    q_lens = [1] * singles + spans
+    q_lens = [1] * singles + spans + ([0, 0] if captured else [])
     N = sum(q_lens)
     step = make_step(o, dtype, [3] * len(q_lens), q_lens, 8, 256, 5)
+    if captured:
+        step.attn_tiles = N // 128 + len(q_lens)
     assert step.single_first == (singles if singles == 8 else 0 if singles < 8 else 1 << (singles.bit_length() - 1))
     qkv, b, a, gate, a_log, dt_bias, norm_w = (t.to(dtype) if t.dtype == torch.bfloat16 else t for t in delta_inputs(H, G, D, V, N, channel, g))
     state_a = (torch.randn(len(q_lens) + 3, H, D, V, generator=g) * 0.3).cuda()
-    state_b = state_a.clone()
+    state_b, state_c = state_a.clone(), state_a.clone()
+    before = o.launches
     ya = o.gated_delta(qkv, b, a, gate, a_log, dt_bias, norm_w, 1e-5, state_a, step, H, G, D, V, True, channel_decay=channel)
+    launches = o.launches - before
     yb = ref_ops.gated_delta(qkv, b, a, gate, a_log, dt_bias, norm_w, 1e-5, state_b, step, H, G, D, V, True, channel_decay=channel)
     # the limits of test_gated_delta
     assert torch.allclose(ya.float(), yb.float(), **tol(dtype))
     assert torch.allclose(state_a, state_b, atol=1e-4, rtol=1e-4)
+    chunked = dtype == torch.bfloat16
+    if not captured and singles >= 8 and all(n == 0 or (n >= 64 and chunked) for n in spans):
+        for i in range(0, singles, 16):                          # (steps of up to 16 single tokens are that kernel's)
+            k = min(i + 16, singles)
+            alone = make_step(o, dtype, [3] * (k - i), [1] * (k - i), 8, 256, 5, slots=list(range(i + 1, k + 1)))
+            yc = o.gated_delta(*(t[i:k].contiguous() for t in (qkv, b, a, gate)), a_log, dt_bias, norm_w, 1e-5, state_c, alone, H, G, D, V, True,
+                               channel_decay=channel)
+            assert torch.equal(ya[i:k], yc)
+        assert torch.equal(state_a[1:singles + 1], state_c[1:singles + 1])
+        assert launches == 2 + (2 if any(spans) else 0)          # the one kernel, the chunks' two, the norm of their rows
+    else:
+        long = N >= 64 if captured else any(n >= 64 for n in spans)
+        assert launches == 3 + (2 if long and chunked else 0)    # the walk's two, the chunks' two, the norm
     assert o.read_status() == 0
 
 

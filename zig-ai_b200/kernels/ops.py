@@ -1436,8 +1436,9 @@ def min_gru(zxg, b_z, b_x, state, step, write_state=True):
 
 
 def _delta_cut(heads, dim, vdim):
-    """Spans of this many rows or more run the delta rule in chunks (bfloat16).  It depends on the layer's sizes alone, so that a
-    request's results depend neither on its neighbours nor on capture.  us walked and in chunks, spans x rows: a span alone gains from
+    """Spans of this many rows or more run the delta rule in chunks (bfloat16).  It depends on the layer's sizes alone, so that the
+    results of a span of two rows or more depend neither on its neighbours nor on capture (a span of one row may take the kernel for
+    single tokens, whose sums have an order of their own: few requests' decode steps, and `_delta_singles`).  us walked and in chunks, spans x rows: a span alone gains from
     about 64 rows on (16 heads of 64 x 128: 1x128 39 and 27, 1x2048 474 and 132; 32 heads of 32 x 64: 1x256 60 and 35), and beside longer
     spans a shorter one had better not be a chain of its own (32 heads of 64 x 128, 777 and 301 rows with 130 and 64: 307 with the 64
     walked, 266 with all in chunks).  Where spans fill the chip the walk costs by D x V and the chunks by the head: 16 heads of 64 x
@@ -1448,6 +1449,19 @@ def _delta_cut(heads, dim, vdim):
     if dim * vdim >= 64 * 64:
         return 128
     return max(256, heads * (8 if dim * vdim >= 1024 else 32))
+
+
+def _delta_singles(step, cut):
+    """How many leading spans of one token take the kernel for single tokens in a step that also has longer spans: eight and more of
+    them where that spares the walk, so where every other span is of `cut` rows or more.  The walk's two kernels go over all of the
+    step's rows for them (us walked and so, 32 heads of 64 x 128: 8 beside 1272 rows 172 and 161, 24 195 and 180, 100 293 and 254; 16
+    heads, 64 beside 64 rows 85 and 55; fewer than eight gain up to 14 % or lose as much).  Beside a span that is walked anyway a kernel
+    of their own is one launch more (16 beside 40 rows of 32 heads 35 and 38, 24 in two parts 41 and 46; 8 beside 70, 5 and 200 of 16
+    heads 53 and 60).  Captured step shapes walk: what lies behind the leading spans differs from replay to replay."""
+    if step.decode_only or getattr(step, "attn_tiles", None) or not step.q_lens:
+        return 0
+    n = next((i for i, x in enumerate(step.q_lens) if x != 1), len(step.q_lens))
+    return n if n >= 8 and not any(0 < x < cut for x in step.q_lens[n:]) else 0
 
 
 @_timed("recurrence")
@@ -1483,13 +1497,10 @@ def gated_delta(qkv, b, a, gate, a_log, dt_bias, norm_w, eps, state, step, heads
         return out
     o = torch.empty((N, H * V), dtype=torch.float32, device=dev)
     out = torch.empty((N, H * V), dtype=qkv.dtype, device=dev)
-    # 8 to 16 leading spans of one token beside longer ones (`StepBatch.single_first`): the one kernel too.  The walk's two kernels go over
-    # all of the step's rows for them: 8 beside 1272 rows of 32 heads of 64 x 128, 49 us where this takes 11
-    ns = 0
-    if impl is None and not step.decode_only and _fn(lib, "zai_gated_delta_single_supports")(D, V):
-        ns = int(getattr(step, "single_first", 0))
-        if ns > DELTA_SINGLE_MAX_ROWS:
-            ns = 0
+    cut = 1 << 30                                              # (spans of that many rows or more run in chunks, the others are walked)
+    if impl != "walk" and not step.decode_only and qkv.dtype == torch.bfloat16 and _fn(lib, "zai_gated_delta_chunked_supports")(D, V):
+        cut = 1 if impl == "chunks" else _delta_cut(H, D, V)
+    ns = _delta_singles(step, cut) if impl is None and _fn(lib, "zai_gated_delta_single_supports")(D, V) else 0
     es = qkv.element_size()
     cu, slots, n_seqs = step.cu_q.data_ptr(), step.slot_ids.data_ptr(), step.n_seqs - ns
     if ns:
@@ -1498,9 +1509,6 @@ def gated_delta(qkv, b, a, gate, a_log, dt_bias, norm_w, eps, state, step, heads
             float(unit_eps), _ptr(state), slots, ns, H, G, D, V, int(bool(write_state)), state.shape[0], _status_ptr(dev), ch, act,
             _stream()), "gated_delta_single")
         cu, slots = cu + 4 * ns, slots + 4 * ns
-    cut = 1 << 30                                              # (spans of that many rows or more run in chunks, the others are walked)
-    if impl != "walk" and not step.decode_only and qkv.dtype == torch.bfloat16 and _fn(lib, "zai_gated_delta_chunked_supports")(D, V):
-        cut = 1 if impl == "chunks" else _delta_cut(H, D, V)
     long, short = _span_kinds(step, cut, ns)
     if long:
         max_chunks = _chunk_bound(step, cut, _fn(lib, "zai_gated_delta_chunk_rows")())
