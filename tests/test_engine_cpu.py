@@ -187,6 +187,20 @@ def test_a_raised_status_word_voids_the_step(tiny_models):
     assert ref_ops.read_status() == 0
 
 
+@pytest.mark.parametrize("one", [b"a", {0: 5}, {5}, "5", [True], [5.0], [-1], [1 << 40], ["5"], [None]])
+def test_a_token_that_is_none_is_refused(tiny_models, one):
+    """One token as well as several: what is no list of ids inside the vocabulary ends in `StepError` before anything is reserved."""
+    from zig_ai_b200.engine.runner import StepError
+    r = make_runner(tiny_models["A"], "A")
+    r.add_request("a")
+    with pytest.raises((StepError, TypeError) if one == [None] else StepError):
+        r.step([("a", one, [0])])
+    assert r.processed["a"] == 0 and r.cache.requests["a"].num_tokens == 0
+    for fine in ([5], (5,), __import__("numpy").array([5], dtype="uint16"), torch.tensor([5]), range(5, 6)):
+        r.step([("a", fine, [0])])
+    assert r.processed["a"] == 5
+
+
 def test_the_engine_reads_the_status_word_with_the_token_ids(tiny_models):
     from zig_ai_b200.engine.engine import Engine
     from zig_ai_b200.engine.runner import StepError

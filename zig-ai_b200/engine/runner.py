@@ -88,8 +88,8 @@ class ModelRunner:
                 n = len(tokens)
                 if n < 1:
                     raise StepError(f"request {rid!r} brings no tokens")
-                # (one token, the case of every decoded request, without an array: 4 us a request)
-                if n > 1 or type(tokens[0]) is not int or not 0 <= tokens[0] < V:
+                # (one token in a list or tuple, the case of every decoded request, without an array: 4 us a request)
+                if n > 1 or type(tokens) not in (list, tuple) or type(tokens[0]) is not int or not 0 <= tokens[0] < V:
                     arr = np.asarray(tokens)
                     if arr.dtype.kind not in "iu" or arr.min() < 0 or arr.max() >= V:
                         bad = [int(t) for t in tokens if not 0 <= int(t) < V]
