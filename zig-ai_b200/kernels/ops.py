@@ -1311,6 +1311,7 @@ def weighted_sum(a, b, wa, wb):
 
 
 DELTA_SINGLE_MAX_ROWS = 16      # single-token steps of at most this many requests run the delta rule as one kernel
+DELTA_SINGLES_BESIDE = 128      # ... and at most this many decoded tokens ahead of spans in chunks (`_delta_singles`; gains measured up to it)
 CHUNKED_SCAN_MIN_ROWS = 256     # steps with prompt portions of this many rows or more run the linear recurrences in chunks
 
 
@@ -1452,16 +1453,17 @@ def _delta_cut(heads, dim, vdim):
 
 
 def _delta_singles(step, cut):
-    """How many leading spans of one token take the kernel for single tokens in a step that also has longer spans: eight and more of
-    them where that spares the walk, so where every other span is of `cut` rows or more.  The walk's two kernels go over all of the
-    step's rows for them (us walked and so, 32 heads of 64 x 128: 8 beside 1272 rows 172 and 161, 24 195 and 180, 100 293 and 254; 16
-    heads, 64 beside 64 rows 85 and 55; fewer than eight gain up to 14 % or lose as much).  Beside a span that is walked anyway a kernel
-    of their own is one launch more (16 beside 40 rows of 32 heads 35 and 38, 24 in two parts 41 and 46; 8 beside 70, 5 and 200 of 16
-    heads 53 and 60).  Captured step shapes walk: what lies behind the leading spans differs from replay to replay."""
+    """How many leading spans of one token take the kernel for single tokens in a step that also has longer spans: 8 to
+    `DELTA_SINGLES_BESIDE` of them where that spares the walk, so where every other span is of `cut` rows or more.  The walk's two
+    kernels go over all of the step's rows for them (us walked and so, 32 heads of 64 x 128: 8 beside 1272 rows 172 and 161, 24 195 and
+    180, 128 328 and 282; 16 heads, 64 beside 64 rows 85 and 55; fewer than eight gain up to 14 % or lose as much).  Beside a span that
+    is walked anyway a kernel of their own is one launch more (16 beside 40 rows of 32 heads 35 and 38, 24 in two parts 41 and 46; 8
+    beside 70, 5 and 200 of 16 heads 53 and 60).  Captured step shapes walk: what lies behind the leading spans differs from replay to
+    replay."""
     if step.decode_only or getattr(step, "attn_tiles", None) or not step.q_lens:
         return 0
     n = next((i for i, x in enumerate(step.q_lens) if x != 1), len(step.q_lens))
-    return n if n >= 8 and not any(0 < x < cut for x in step.q_lens[n:]) else 0
+    return n if 8 <= n <= DELTA_SINGLES_BESIDE and not any(0 < x < cut for x in step.q_lens[n:]) else 0
 
 
 @_timed("recurrence")
