@@ -147,7 +147,7 @@ def test_gated_delta(dtype, H, G, D, V):
                                            (16, [66]), (8, [0, 0]), (17, [64, 0])])
 @pytest.mark.parametrize("captured", [False, True])
 def test_gated_delta_of_decoded_tokens_ahead_of_spans(singles, spans, captured, dtype, channel):
-    """Eight and more leading spans of one token take the one kernel where every other span goes in chunks (rows and states are then those of
+    """Leading spans of one token (8 to 128) take the one kernel where every other span goes in chunks (rows and states are then those of
     a step of the same requests alone, to the bit, and the walk's kernels do not run); everything else is walked, and so is a step in
     the layout of a captured shape (empty spans, counts of chunks and spans rounded up)."""
     o = ops()
@@ -315,6 +315,28 @@ def delta_inputs(H, G, D, V, N, channel, g):
     qkv, a = torch.randn(N, 2 * G * D + H * V, generator=g).bfloat16().cuda(), torch.randn(N, cols_a, generator=g).bfloat16().cuda()
     gate, b = torch.randn(N, H * V, generator=g).bfloat16().cuda(), torch.randn(N, H, generator=g).bfloat16().cuda()
     return qkv, b, a, gate, a_log, dt_bias, torch.ones(V).cuda()
+
+
+@pytest.mark.parametrize("H,G,D,V", [(16, 8, 64, 128), (16, 4, 40, 72), (16, 16, 64, 256), (16, 8, 64, 64)])
+def test_gated_delta_in_few_chunks_and_in_many(H, G, D, V):
+    """Few chunks are made by two blocks each (heads of more than 64 values), many by one: a request's rows and state are the same, to the
+    bit, and one of 130 rows is the reference's within the limits of test_gated_delta."""
+    o = ops()
+    g = torch.Generator().manual_seed(29)
+    q_lens = [130, 900, 700]
+    qkv, b, a, gate, a_log, dt_bias, norm_w = delta_inputs(H, G, D, V, sum(q_lens), False, g)
+    state = (torch.randn(6, H, D, V, generator=g) * 0.3).cuda()
+
+    def run(at, lens, n, **kw):
+        st = state.clone()
+        step = make_step(o, torch.bfloat16, [3] * len(lens), lens, 64, 64, 5)
+        y = at.gated_delta(qkv[:n].contiguous(), b[:n].contiguous(), a[:n].contiguous(), gate[:n].contiguous(), a_log, dt_bias, norm_w, 1e-5, st,
+                           step, H, G, D, V, True, **kw)
+        return y[:130].float(), st[1]
+    alone, many, want = run(o, [130], 130, impl="chunks"), run(o, q_lens, sum(q_lens), impl="chunks"), run(ref_ops, [130], 130)
+    assert torch.equal(alone[0], many[0]) and torch.equal(alone[1], many[1])
+    assert torch.allclose(alone[0], want[0], **tol(torch.bfloat16)) and torch.allclose(alone[1], want[1], atol=1e-4, rtol=1e-4)
+    assert o.read_status() == 0
 
 
 @pytest.mark.parametrize("H,G,D,V", [(4, 2, 64, 128), (2, 2, 24, 40)])

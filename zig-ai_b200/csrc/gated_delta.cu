@@ -671,6 +671,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_kernel(const DeltaArgs a) 
     const int h = blockIdx.y, kvh = h / (a.H / a.G), n = t1 - t0;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int D = a.D, V = a.V;
+    const int part = CH ? 0 : blockIdx.z, parts = CH ? 1 : gridDim.z;      // (few chunks: two blocks make A each and share what comes of it)
 
     // the rows of q and k (zeros beyond the chunk and beyond D)
     if (((D | a.qkv_stride) & 7) == 0 && (reinterpret_cast<uintptr_t>(a.qkv) & 15) == 0) {
@@ -855,7 +856,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_kernel(const DeltaArgs a) 
                 if (s > t) w[e] = 0.f;                       // (what lies there is no part of the sums)
                 if (which == 1 && s < t) sm.m[t][s] = sm.beta[t] * w[e];
             }
-            if (which == 0) {                                // P goes out as it lies: half of a tile of 16 columns
+            if (which == 0 && part == 0) {                   // P goes out as it lies: half of a tile of 16 columns
                 uint32_t lo[3], hi[3];
                 split3_pair(w[0], w[1], lo);
                 split3_pair(w[2], w[3], hi);
@@ -890,11 +891,11 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_kernel(const DeltaArgs a) 
             sum16(va, lane);
             sum16(vp, lane);
             if (dq < r) sm.m[t][16 * I + dq] = sm.beta[t] * va[0];
-            float part[3];
-            split3(dq <= r ? vp[0] : 0.f, part[0], part[1], part[2]);
+            float third[3];
+            split3(dq <= r ? vp[0] : 0.f, third[0], third[1], third[2]);
 #pragma unroll
             for (int k = 0; k < 3; ++k)
-                reinterpret_cast<bf16*>(&out->p.v[k][I][I][(r & 7) * 4 + ((dq & 7) >> 1)])[((r >> 3) + 2 * (dq >> 3)) * 2 + (dq & 1)] = __float2bfloat16_rn(part[k]);
+                reinterpret_cast<bf16*>(&out->p.v[k][I][I][(r & 7) * 4 + ((dq & 7) >> 1)])[((r >> 3) + 2 * (dq >> 3)) * 2 + (dq & 1)] = __float2bfloat16_rn(third[k]);
         }
         if (CH) __syncthreads();                             // (the next 16 rows' operands take the place of these)
     }
@@ -917,7 +918,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_kernel(const DeltaArgs a) 
         }
     }
     cp_async_commit();
-    delta_put(&out->q, [&](int t, int d) {
+    if (part == 0) delta_put(&out->q, [&](int t, int d) {
         const float2 x = sm.unit_two(0, t, d);
         if (!CH) {
             const float e = fast_exp2(sm.c.hi[t][0]);
@@ -926,7 +927,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_kernel(const DeltaArgs a) 
         const float2 hi = *reinterpret_cast<const float2*>(&sm.c.hi[t][d]), b = *reinterpret_cast<const float2*>(&sm.before[t >> 4][d]);
         return make_float2(x.x * fast_exp2(b.x + hi.x), x.y * fast_exp2(b.y + hi.y));
     });
-    delta_put(&out->k, [&](int d, int s) {
+    if (part == parts - 1) delta_put(&out->k, [&](int d, int s) {
         float e[2];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
@@ -935,7 +936,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_kernel(const DeltaArgs a) 
         }
         return make_float2(sm.unit(1, s, d) * fast_exp2(e[0]), sm.unit(1, s + 1, d) * fast_exp2(e[1]));
     });
-    if (tid < DCD) out->keep[tid] = fast_exp2(CH ? sm.before[4][tid] : sm.c.hi[DC - 1][0]);
+    if (part == 0 && tid < DCD) out->keep[tid] = fast_exp2(CH ? sm.before[4][tid] : sm.c.hi[DC - 1][0]);
 
     cp_async_wait<0>();
     __syncthreads();
@@ -946,7 +947,7 @@ __global__ void __launch_bounds__(256, 2) delta_chunk_kernel(const DeltaArgs a) 
     // what the loop costs first is fetching its code (unrolled, 64 rows a thread: 106 KB of code, 28 of a block's 55 us).
     float* u0 = a.u0 + ((size_t)blockIdx.x * a.H + h) * DC * a.VP;
 #pragma unroll 1
-    for (int tile = warp; tile < DCD / 16 + (V + 15) / 16; tile += 8) {
+    for (int tile = warp * parts + part; tile < DCD / 16 + (V + 15) / 16; tile += 8 * parts) {
         const int c0 = tile * 16 - DCD;                      // its first column of v
         float x[4][2][4] = {};                               // [16 rows from this turn's on][tile of 8 rows][...]
 #pragma unroll 1
@@ -1306,15 +1307,21 @@ ZAI_API int zai_gated_delta_chunked(float* o_out, const void* qkv, int qkv_strid
         if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DeltaShared));
         if (e != cudaSuccess) return (int)e;
     }
-    const int rc = channel ? launch_pdl(delta_chunk_kernel<true>, dim3(max_chunks, H), dim3(256), sizeof(DeltaShared), stream, a)
-                           : launch_pdl(delta_chunk_kernel<false>, dim3(max_chunks, H), dim3(256), sizeof(DeltaShared), stream, a);
-    if (rc) return rc;
-    // 16 columns a block while that leaves no SM with two, else 32 (half the operand loads a column; the same sums a column)
     static int sms = 0;
     if (!sms) {
         int dev = 0;
         if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 148;
     }
+    // Few chunks and more tiles of right sides than a block has warps: two blocks a chunk, or the last round of tiles is a few warps'
+    // work while most SMs have none.  One decay a head, us with one and two: 4 heads of 64 x 128, 64 rows 23.8 and 18.5, 256 rows 28.7
+    // and 23.4; 16 heads, 64 rows 24.5 and 23.3, 512 rows (144 blocks) 44.8 and 39.3, 1024 (256; two an SM) 71.7 and 81.6.  With a decay
+    // per channel, where A and P are more of a block's time, it goes up as often as down (16 heads, 64 rows 35.7 and 37.9, 100 rows 46.7
+    // and 39.6).
+    const int parts = !channel && V > 64 && (long long)max_chunks * H <= sms ? 2 : 1;
+    const int rc = channel ? launch_pdl(delta_chunk_kernel<true>, dim3(max_chunks, H), dim3(256), sizeof(DeltaShared), stream, a)
+                           : launch_pdl(delta_chunk_kernel<false>, dim3(max_chunks, H, parts), dim3(256), sizeof(DeltaShared), stream, a);
+    if (rc) return rc;
+    // 16 columns a block while that leaves no SM with two, else 32 (half the operand loads a column; the same sums a column)
     if ((long long)((V + 15) / 16) * H * n_spans <= sms) return delta_carry<16>(a, stream);
     return delta_carry<32>(a, stream);
 }
