@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) prefill_tc_kernel(const __grid_
                 }
             }
         } else if (warp == 1) {
-            if (n_tiles > 0 && at_elect()) {
+            if (n_tiles > 0 && zai_elect()) {
                 // ---- products.  (By the lane that elect.sync picks: the compiler then knows that one lane is left and issues a product in
                 // half the time that it takes behind `lane == 0`, where a tile's eight products and three commits took 2000 cycles,
                 // more than its softmax.)

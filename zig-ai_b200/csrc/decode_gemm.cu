@@ -951,7 +951,9 @@ static size_t skinny_block_x_bytes(int M, int K, bool norm, bool by_rows) {
     return norm ? (SG_SUM_BYTES + (size_t)M * (K + 8) * sizeof(bf16) + (by_rows ? (size_t)K * sizeof(float) : 0) + 1023) / 1024 * 1024 : 0;
 }
 static size_t skinny_block_round_bytes(int mt, bool norm, int nt) { return (size_t)SG_WARPS * 4 * ((nt == 2 ? 3 : 2) + (norm ? 0 : mt)) * 512; }
-// (the bounds on the sizes that the kernel takes, and the depth of its rings, are counted for the largest block of its variant)
+// Which K the kernel takes (zai_skinny_gemm_supports) and how deep its rings are go by these two instead, which count 8 mt rows, the
+// norm's weight and four parts of a convolution's weights whatever a block holds of them: more than any block takes (but for a
+// round-up of 1 KB), kept as the line because other lengths and depths than these were not measured.
 static size_t skinny_x_bytes(int mt, int K, bool norm) {
     if (!norm) return 1024;                                 // x travels through the rings
     return (256 + (size_t)8 * mt * (K + 8) * sizeof(bf16) + (size_t)K * sizeof(float) + 1023) / 1024 * 1024;

@@ -63,13 +63,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     *failed = 1;
     return false;
 }
-// true in one lane of a warp in step.  (The compiler then knows that one lane is left: behind `lane == 0` a product takes 110 to 125 cycles
-// to issue, behind this 75.  Grouped products of 2048 rows, 8 experts of 2048 x 3072: 174 -> 164 us both.)
-__device__ __forceinline__ bool elect_one() {
-    uint32_t one;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
-    return one != 0;
-}
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                  ::"r"(smem_addr(dst)), "l"(map), "r"(smem_addr(bar)), "r"(c0), "r"(c1) : "memory");
@@ -158,7 +151,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
     pdl_wait();
 
     if (warp == 0) {
-        if (elect_one()) {
+        if (zai_elect()) {
             int issued = 0, it = 0;                            // `it` counts k-blocks over all of this block's tiles
             bool ok = true;
             for (int t = blockIdx.x; t < a.tiles && ok; t += gridDim.x) {
@@ -193,7 +186,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
             }
         }
     } else if (warp == 1) {
-        if (elect_one()) {
+        if (zai_elect()) {
             // instruction descriptor: D fp32, A and B bfloat16, both K-major, N = BN, M = 128
             constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
             bool ok = true;

@@ -82,12 +82,6 @@ __device__ __forceinline__ bool tp_mbar_wait(uint64_t* bar, uint32_t parity, vol
 }
 // One block's tile into its own shared memory; the bytes count on the barrier at `bar_cluster_addr`,
 // which may lie in the other block of the pair.
-// true in one lane of a warp in step
-__device__ __forceinline__ bool tp_elect() {
-    uint32_t one;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
-    return one != 0;
-}
 __device__ __forceinline__ void tp_tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint32_t bar_cluster_addr) {
     asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                  ::"r"(tp_smem(dst)), "l"(map), "r"(bar_cluster_addr), "r"(c0), "r"(c1) : "memory");
@@ -216,7 +210,7 @@ __global__ void __launch_bounds__(TP_THREADS) gemm_pair_kernel(const __grid_cons
     pdl_wait();
 
     if (warp == 0) {
-        if (tp_elect()) {
+        if (zai_elect()) {
             int it = 0, issued = 0;                            // `it` counts k-blocks over all of this pair's tiles
             bool ok = true;
             for (int t = pair; t < a.tiles && ok; t += n_pairs) {
@@ -252,7 +246,7 @@ __global__ void __launch_bounds__(TP_THREADS) gemm_pair_kernel(const __grid_cons
             }
         }
     } else if (warp == 1) {
-        if (rank == 0 && tp_elect()) {
+        if (rank == 0 && zai_elect()) {
             // instruction descriptor: D fp32, A and B bfloat16, both K-major, N = BN, M = 256 over the pair
             constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((2 * TP_BM) >> 4) << 24);
             bool ok = true;

@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(LT_THREADS) latent_attention_tc_kernel(const _
                 lt_drain(&q_full, 0);
             }
         } else if (warp == 1) {
-            if (at_elect()) {                                   // (issued behind `lane == 0` a product takes twice as long)
+            if (zai_elect()) {                                   // (issued behind `lane == 0` a product takes twice as long)
                 // ---- products.  Instruction descriptors: D 32-bit, A and B bfloat16, M = 128, N = 64; the scores have both
                 // operands K-major; O has A (P) in TMEM and B (the cached rows' first R columns) MN-major.
                 constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(LT_BN >> 3) << 17) | ((uint32_t)(LT_BM >> 4) << 24);
