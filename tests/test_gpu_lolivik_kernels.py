@@ -46,7 +46,9 @@ def test_add_cast(dtype, N, H):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("H,G,D,Dv,scope,rot,ps", [(4, 2, 16, 8, 2, 0, 8), (3, 1, 24, 40, 1, 8, 16), (8, 1, 64, 32, 2, 0, 64), (6, 3, 12, 12, 1, 12, 4)])
+@pytest.mark.parametrize("H,G,D,Dv,scope,rot,ps", [(4, 2, 16, 8, 2, 0, 8), (3, 1, 24, 40, 1, 8, 16), (8, 1, 64, 32, 2, 0, 64), (6, 3, 12, 12, 1, 12, 4),
+                                                      # rows normed whole in registers: one load a thread, several, four
+                                                      (8, 8, 16, 16, 2, 0, 8), (16, 4, 64, 64, 2, 32, 16), (64, 32, 64, 64, 2, 0, 64)])
 def test_qkv_prepare_temperature_and_mixed_values(dtype, H, G, D, Dv, scope, rot, ps):
     o = ops()
     g = torch.Generator().manual_seed(3)
