@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(SG_WARPS * 32, 2) skinny_gemm_kernel(const Ski
             if (NORM && kslice == 0 && nt * 8 + 2 * t + e < a.M) {
                 float ss = 0.f;
 #pragma unroll
-                for (int w2 = 0; w2 < SG_WARPS; ++w2) ss += w2 < parts ? sums[w2 * 8 * MT + nt * 8 + 2 * t + e] : 0.f;
+                for (int w2 = 0; w2 < SG_WARPS; ++w2) ss += !ROWS || w2 < parts ? sums[w2 * 8 * MT + nt * 8 + 2 * t + e] : 0.f;
                 inv_tok[nt][e] = rsqrtf(ss / (float)K + a.eps);
             }
         }
@@ -1018,8 +1018,8 @@ static int skinny_launch(const SkinnyArgs& a, cudaStream_t stream) {
 template <int EPI>
 static int skinny_dispatch(const SkinnyArgs& a, bool by_rows, cudaStream_t stream) {
     if (!a.h) return a.M <= 8 ? skinny_launch<1, EPI, false, false>(a, stream) : skinny_launch<2, EPI, false, false>(a, stream);
-    if (!by_rows) return a.M <= 8 ? skinny_launch<1, EPI, true, false>(a, stream) : skinny_launch<2, EPI, true, false>(a, stream);
-    return a.M <= 8 ? skinny_launch<1, EPI, true, true>(a, stream) : skinny_launch<2, EPI, true, true>(a, stream);
+    if (by_rows) return a.M <= 8 ? skinny_launch<1, EPI, true, true>(a, stream) : skinny_launch<2, EPI, true, true>(a, stream);
+    return a.M <= 8 ? skinny_launch<1, EPI, true, false>(a, stream) : skinny_launch<2, EPI, true, false>(a, stream);
 }
 
 // 1 if the kernel takes these sizes (else the caller uses the library product and separate kernels)
@@ -1045,7 +1045,10 @@ static int skinny_run(SkinnyArgs& a, int epilogue, cudaStream_t stream) {
         const int rounds = rpu * ((a.units + grid - 1) / grid);
         if (a.ring_rounds > rounds) a.ring_rounds = rounds;
     }
-    const bool by_rows = norm && (a.center || (a.K <= (SG_WARPS - 1) * 128 && a.M > 4));      // (see skinny_stage and what follows it)
+    // (see skinny_stage and what follows it.  With the convolution and more than eight rows registers are short, and columns stay the
+    // quicker way beyond 384 of them: projection with convolution and out-projection, us by columns and by rows, 512 columns, eight
+    // rows 6.5 and 6.1, nine 8.6 and 9.0; 768, nine 10.0 and 10.7; 384, sixteen 10.3 and 10.0)
+    const bool by_rows = norm && (a.center || (a.K <= (SG_WARPS - 1) * 128 && a.M > 4 && (epilogue != EPI_CONV || a.M <= 8 || a.K <= 384)));
     a.red_offset = (int)skinny_block_x_bytes(a.M, a.K, norm, by_rows);
     a.ring_offset = a.red_offset + (int)skinny_red_bytes(mt, nt);
     a.l2_prefetch_bytes = skinny_l2_prefetch_bytes();
